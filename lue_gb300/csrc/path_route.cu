@@ -1,6 +1,6 @@
 // path_route.cu — the path engine (see path_route.cuh): heavy-path layout of the flow forest, built once
-// per raster, and accu_threshold / accu_fraction / accu_capacity (float32) as one prefix scan per path
-// level.
+// per raster, and accu_threshold / accu_fraction / accu_capacity / accu_trigger (float32) as one prefix scan
+// per path level.
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -437,22 +437,39 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
 // Per call
 // ---------------------------------------------------------------------------------------------------
 
-// A map x -> op(x + a, b) with op = max (threshold) or min (capacity), or x -> a * x + b (fraction); a and
-// b float-float.  flags bit 0: the map of a path's top cell, which ignores its input (its value is b);
-// bit 1: no-data (NaN) from the cell itself or from upstream.
+// Kinds of maps, from a cell's inflow along its path to its outflow: x -> max(x + a, b) (threshold),
+// x -> min(x + a, b) (capacity), x -> a * x + b (fraction), and x -> x + b where x >= a, else c (trigger).
+//
+// The trigger's maps compose into maps of the same form because every one of them is monotone on x >= 0 and c
+// is its value at 0: m2 after m1, with c1 >= a2, passes everything on (x >= a1 gives x + b1 >= c1 >= a2):
+// (a1, b1 + b2, c1 + b2); with c1 < a2 what m1 holds back stays held back: (max(a1, a2 - b1), b1 + b2, c2).
+//
+// On the stage engine accu_trigger was bound by its chain of rounds (1500^2: 1595 us a call); as a scan it
+// takes 319 us.
+constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2, kTrigger = 3;
+
+// a, b and c float-float.  flags bit 0: the map of a path's top cell, which ignores its input (its value is
+// value()); bit 1: no-data (NaN) from the cell itself or from upstream.
+template <int K>
 struct PMap {
     float ah, al, bh, bl;
     int flags;
+    __device__ FF value() const { return FF{bh, bl}; }
+};
+template <>
+struct PMap<kTrigger> {
+    float ah, al, bh, bl;
+    int flags;
+    float ch, cl;
+    __device__ FF value() const { return FF{ch, cl}; }
 };
 
-// Kinds of maps: x -> max(x + a, b) (threshold), x -> min(x + a, b) (capacity), x -> a * x + b (fraction).
-constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2;
-
 template <int K>
-__device__ __forceinline__ PMap pm_identity()
+__device__ __forceinline__ PMap<K> pm_identity()
 {
-    if (K == kAffine) return PMap{1.0f, 0.0f, 0.0f, 0.0f, 0};
-    return PMap{0.0f, 0.0f, K == kMinPlus ? INFINITY : -INFINITY, 0.0f, 0};
+    if constexpr (K == kAffine) return PMap<K>{1.0f, 0.0f, 0.0f, 0.0f, 0};
+    else if constexpr (K == kTrigger) return PMap<K>{-INFINITY, 0.0f, 0.0f, 0.0f, 0, 0.0f, 0.0f};
+    else return PMap<K>{0.0f, 0.0f, K == kMinPlus ? INFINITY : -INFINITY, 0.0f, 0};
 }
 
 // x + y for float-float values; a sum that is not finite is kept with lo = 0 (two_sum's error terms would
@@ -495,87 +512,129 @@ __device__ __forceinline__ void ff_mul(float xh, float xl, float yh, float yl, f
 
 // m1 first, then m2.
 template <int K>
-__device__ __forceinline__ PMap compose(const PMap& m1, const PMap& m2)
+__device__ __forceinline__ PMap<K> compose(const PMap<K>& m1, const PMap<K>& m2)
 {
     if (m2.flags & 1) return m2;
-    PMap r;
+    PMap<K> r;
     r.flags = (m1.flags & 1) | ((m1.flags | m2.flags) & 2);
-    if (K == kAffine) {  // a2 * (a1 * x + b1) + b2
+    if constexpr (K == kAffine) {  // a2 * (a1 * x + b1) + b2
         ff_mul(m1.ah, m1.al, m2.ah, m2.al, r.ah, r.al);
         float th, tl;
         ff_mul(m2.ah, m2.al, m1.bh, m1.bl, th, tl);
         ff_sum(th, tl, m2.bh, m2.bl, r.bh, r.bl);
-        return r;
+    } else if constexpr (K == kTrigger) {
+        float th, tl, uh, ul;
+        ff_sum(m1.bh, m1.bl, m2.bh, m2.bl, r.bh, r.bl);
+        ff_sum(m2.ah, m2.al, -m1.bh, -m1.bl, th, tl);
+        ff_sum(m1.ch, m1.cl, m2.bh, m2.bl, uh, ul);
+        const bool holds = ff_less(m1.ch, m1.cl, m2.ah, m2.al);
+        const bool later = holds && ff_less(m1.ah, m1.al, th, tl);
+        r.ah = later ? th : m1.ah;
+        r.al = later ? tl : m1.al;
+        r.ch = holds ? m2.ch : uh;
+        r.cl = holds ? m2.cl : ul;
+    } else {
+        ff_sum(m1.ah, m1.al, m2.ah, m2.al, r.ah, r.al);
+        float th, tl;
+        ff_sum(m1.bh, m1.bl, m2.ah, m2.al, th, tl);
+        const bool take = K == kMinPlus ? ff_less(th, tl, m2.bh, m2.bl) : ff_less(m2.bh, m2.bl, th, tl);
+        r.bh = take ? th : m2.bh;
+        r.bl = take ? tl : m2.bl;
     }
-    ff_sum(m1.ah, m1.al, m2.ah, m2.al, r.ah, r.al);
-    float th, tl;
-    ff_sum(m1.bh, m1.bl, m2.ah, m2.al, th, tl);
-    const bool take = K == kMinPlus ? ff_less(th, tl, m2.bh, m2.bl) : ff_less(m2.bh, m2.bl, th, tl);
-    r.bh = take ? th : m2.bh;
-    r.bl = take ? tl : m2.bl;
     return r;
 }
 
 // The map of one cell: s = its material plus the outflow of its light upstream neighbours, b its
-// threshold or capacity.
-template <Rule R>
-__device__ __forceinline__ PMap cell_map(bool top, float sh, float sl, float b, bool nan)
+// threshold, fraction, capacity or trigger.
+template <Rule R, int K>
+__device__ __forceinline__ PMap<K> cell_map(bool top, float sh, float sl, float b, bool nan)
 {
-    if (nan) return PMap{0.0f, 0.0f, 0.0f, 0.0f, 2 | (top ? 1 : 0)};
+    PMap<K> m{0.0f, 0.0f, 0.0f, 0.0f, nan ? 2 | (top ? 1 : 0) : 0};
+    if (nan) return m;
     if (top) {
         float oh = 0.0f, ol = 0.0f, rem = 0.0f;
         rule_f32<R>(FF{sh, sl}, false, 0.0f, b, oh, ol, rem);
-        return PMap{0.0f, 0.0f, oh, ol, 1};
+        m.flags = 1;
+        if constexpr (K == kTrigger) {
+            m.ah = INFINITY;
+            m.ch = oh;
+            m.cl = ol;
+        } else {
+            m.bh = oh;
+            m.bl = ol;
+        }
+    } else if constexpr (K == kMaxPlus) {  // max(x + (s - threshold), 0)
+        ff_sum(sh, sl, -b, 0.0f, m.ah, m.al);
+    } else if constexpr (K == kAffine) {  // fraction * x + fraction * s
+        m.ah = b;
+        ff_mul(b, 0.0f, sh, sl, m.bh, m.bl);
+    } else if constexpr (K == kTrigger) {  // x + s where that reaches the trigger, else 0
+        ff_sum(b, 0.0f, -sh, -sl, m.ah, m.al);
+        m.bh = sh;
+        m.bl = sl;
+        const bool passes = !ff_less(sh, sl, b, 0.0f);
+        m.ch = passes ? sh : 0.0f;
+        m.cl = passes ? sl : 0.0f;
+    } else {  // capacity: min(x + s, capacity)
+        m.ah = sh;
+        m.al = sl;
+        m.bh = b;
     }
-    if (R == Rule::threshold) {  // max(x + (s - threshold), 0)
-        float dh, dl;
-        ff_sum(sh, sl, -b, 0.0f, dh, dl);
-        return PMap{dh, dl, 0.0f, 0.0f, 0};
-    }
-    if (R == Rule::fraction) {  // fraction * x + fraction * s
-        float qh, ql;
-        ff_mul(b, 0.0f, sh, sl, qh, ql);
-        return PMap{b, 0.0f, qh, ql, 0};
-    }
-    return PMap{sh, sl, b, 0.0f, 0};  // capacity: min(x + s, capacity)
+    return m;
 }
 
-__device__ __forceinline__ PMap shfl_up(const PMap& m, int d)
+// Every word of a map, moved by f (shuffles and loads).
+template <int K, class F>
+__device__ __forceinline__ PMap<K> pm_each(const PMap<K>& m, F f)
 {
-    PMap r;
-    r.ah = __shfl_up_sync(0xffffffffu, m.ah, d);
-    r.al = __shfl_up_sync(0xffffffffu, m.al, d);
-    r.bh = __shfl_up_sync(0xffffffffu, m.bh, d);
-    r.bl = __shfl_up_sync(0xffffffffu, m.bl, d);
-    r.flags = __shfl_up_sync(0xffffffffu, m.flags, d);
+    PMap<K> r;
+    r.ah = f(m.ah);
+    r.al = f(m.al);
+    r.bh = f(m.bh);
+    r.bl = f(m.bl);
+    r.flags = f(m.flags);
+    if constexpr (K == kTrigger) {
+        r.ch = f(m.ch);
+        r.cl = f(m.cl);
+    }
     return r;
+}
+template <int K>
+__device__ __forceinline__ PMap<K> shfl_up(const PMap<K>& m, int d)
+{
+    return pm_each(m, [d](auto v) { return __shfl_up_sync(0xffffffffu, v, d); });
+}
+template <int K>
+__device__ __forceinline__ PMap<K> shfl_down(const PMap<K>& m, int d)
+{
+    return pm_each(m, [d](auto v) { return __shfl_down_sync(0xffffffffu, v, d); });
 }
 
 // Exclusive scan of the threads' maps in thread order; `total` is the composition of all of them.
 template <int K, int NT>
-__device__ __forceinline__ PMap block_excl_scan(const PMap& v, PMap* s_warp, PMap& total)
+__device__ __forceinline__ PMap<K> block_excl_scan(const PMap<K>& v, PMap<K>* s_warp, PMap<K>& total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    PMap x = v;
+    PMap<K> x = v;
     for (int d = 1; d < 32; d <<= 1) {
-        const PMap y = shfl_up(x, d);
+        const PMap<K> y = shfl_up(x, d);
         if (lane >= d) x = compose<K>(y, x);
     }
-    PMap ex = shfl_up(x, 1);
+    PMap<K> ex = shfl_up(x, 1);
     if (lane == 0) ex = pm_identity<K>();
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
     if (warp == 0) {
-        PMap w = lane < NT / 32 ? s_warp[lane] : pm_identity<K>();
+        PMap<K> w = lane < NT / 32 ? s_warp[lane] : pm_identity<K>();
         for (int d = 1; d < 32; d <<= 1) {
-            const PMap y = shfl_up(w, d);
+            const PMap<K> y = shfl_up(w, d);
             if (lane >= d) w = compose<K>(y, w);
         }
         if (lane < NT / 32) s_warp[lane] = w;
     }
     __syncthreads();
     total = s_warp[NT / 32 - 1];
-    const PMap r = warp ? compose<K>(s_warp[warp - 1], ex) : ex;
+    const PMap<K> r = warp ? compose<K>(s_warp[warp - 1], ex) : ex;
     __syncthreads();
     return r;
 }
@@ -634,29 +693,14 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v)
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ PMap ld_map(const PMap* m)
-{
-    return PMap{__ldcg(&m->ah), __ldcg(&m->al), __ldcg(&m->bh), __ldcg(&m->bl), __ldcg(&m->flags)};
-}
-
-__device__ __forceinline__ PMap shfl_down(const PMap& m, int d)
-{
-    PMap r;
-    r.ah = __shfl_down_sync(0xffffffffu, m.ah, d);
-    r.al = __shfl_down_sync(0xffffffffu, m.al, d);
-    r.bh = __shfl_down_sync(0xffffffffu, m.bh, d);
-    r.bl = __shfl_down_sync(0xffffffffu, m.bl, d);
-    r.flags = __shfl_down_sync(0xffffffffu, m.flags, d);
-    return r;
-}
-
 // Decoupled look-back of one level's launch: CTAs take tiles in ticket order; each publishes the
 // composition of its tile's maps (state 1), then the composition of everything before and including its
 // tile (state 2).  Status words carry the launch's epoch, so the arrays need no clearing between launches.
+template <int K>
 struct PathScan {
     int* status;  // [tiles] epoch << 2 | state
-    PMap* aggm;   // [tiles] the tile's own composition
-    PMap* inclm;  // [tiles] the composition up to and including the tile
+    PMap<K>* aggm;   // [tiles] the tile's own composition
+    PMap<K>* inclm;  // [tiles] the composition up to and including the tile
     int* ticket;  // zeroed before the launch
     int epoch;
     int polls;    // poll limit of one wait
@@ -668,14 +712,14 @@ constexpr int kPathPolls = 1 << 20;
 // a time, until a tile with a published prefix is among them.  Every wait is bounded: a wait that gives
 // up (or finds that another one did) sets flag[1], after which the walk engine redoes the call.
 template <int K>
-__device__ PMap look_back(const PathScan& q, int64_t tile, unsigned long long* flag)
+__device__ PMap<K> look_back(const PathScan<K>& q, int64_t tile, unsigned long long* flag)
 {
     const int lane = threadIdx.x & 31;
-    PMap running = pm_identity<K>();
+    PMap<K> running = pm_identity<K>();
     for (int64_t j = tile - 1;; j -= 32) {
         const int64_t idx = j - lane;
         int st = 2;
-        PMap m = pm_identity<K>();
+        PMap<K> m = pm_identity<K>();
         if (idx >= 0) {
             int v = 0, k = 0;
             for (; k < q.polls; ++k) {
@@ -688,7 +732,7 @@ __device__ PMap look_back(const PathScan& q, int64_t tile, unsigned long long* f
                 st = -1;
             } else {
                 st = v & 3;
-                m = ld_map(st == 2 ? q.inclm + idx : q.aggm + idx);
+                m = pm_each(*(st == 2 ? q.inclm + idx : q.aggm + idx), [](const auto& v) { return __ldcg(&v); });
             }
         }
         if (__ballot_sync(0xffffffffu, st < 0)) {
@@ -699,12 +743,10 @@ __device__ PMap look_back(const PathScan& q, int64_t tile, unsigned long long* f
         if (incl && lane > __ffs(incl) - 1) m = pm_identity<K>();
         // lanes 31 .. 0 in this order (farther tiles come first)
         for (int d = 1; d < 32; d <<= 1) {
-            const PMap o = shfl_down(m, d);
+            const PMap<K> o = shfl_down(m, d);
             if (lane + d < 32) m = compose<K>(o, m);
         }
-        const PMap window = PMap{__shfl_sync(0xffffffffu, m.ah, 0), __shfl_sync(0xffffffffu, m.al, 0),
-                                 __shfl_sync(0xffffffffu, m.bh, 0), __shfl_sync(0xffffffffu, m.bl, 0),
-                                 __shfl_sync(0xffffffffu, m.flags, 0)};
+        const PMap<K> window = pm_each(m, [](auto v) { return __shfl_sync(0xffffffffu, v, 0); });
         running = compose<K>(window, running);
         if (incl) return running;
     }
@@ -722,7 +764,7 @@ struct Chunk {
     FF sum[PER];
     bool nan[PER];
 
-    __device__ __forceinline__ PMap load(const PathCall& p, int64_t first, int64_t lo, int64_t hi)
+    __device__ __forceinline__ PMap<K> load(const PathCall& p, int64_t first, int64_t lo, int64_t hi)
     {
 #pragma unroll
         for (int j = 0; j < PER; ++j) on[j] = first + j >= lo && first + j < hi;
@@ -755,7 +797,7 @@ struct Chunk {
                 }
             }
         }
-        PMap acc = pm_identity<K>();
+        PMap<K> acc = pm_identity<K>();
         bool odd = false;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
@@ -765,13 +807,13 @@ struct Chunk {
             sum[j].add(e[j]);
             sum[j].normalise();
             odd |= !nan[j] && (isinf(e[j]) || isinf(b[j]) || isinf(sum[j].hi));
-            acc = compose<K>(acc, cell_map<R>(w[j] < 0, sum[j].hi, sum[j].lo, b[j], nan[j]));
+            acc = compose<K>(acc, cell_map<R, K>(w[j] < 0, sum[j].hi, sum[j].lo, b[j], nan[j]));
         }
         if (odd) p.flag[1] = 1;  // +-inf: the walk engine redoes the call
         return acc;
     }
 
-    __device__ __forceinline__ void store(const PathCall& p, int64_t first, int64_t p1, PMap E)
+    __device__ __forceinline__ void store(const PathCall& p, int64_t first, int64_t p1, PMap<K> E)
     {
         // the position after this thread's last one: is it the top of a path (then the last one is a bottom)?
         const int32_t after = first + PER < p1 ? __ldg(p.order + first + PER) : -1;
@@ -784,7 +826,7 @@ struct Chunk {
             bool nn = nan[j];
             if (!top) {
                 nn |= (E.flags & 2) != 0;
-                t = FF{E.bh, E.bl};
+                t = E.value();
             }
             t.add(sum[j].hi, sum[j].lo);
             float oh = 0.0f, ol = 0.0f, rem = 0.0f;
@@ -797,7 +839,7 @@ struct Chunk {
             p.rem[c] = rem;
             const int32_t next = j + 1 < PER ? w[(j + 1) % PER] : after;
             if (first + j + 1 >= p1 || next < 0) p.lo[c] = ol;  // a path bottom
-            E = compose<K>(E, cell_map<R>(top, sum[j].hi, sum[j].lo, b[j], nan[j]));
+            E = compose<K>(E, cell_map<R, K>(top, sum[j].hi, sum[j].lo, b[j], nan[j]));
         }
     }
 };
@@ -807,19 +849,19 @@ struct Chunk {
 // One level in one pass, for levels with long paths: tiles in ticket order, the composition of the
 // tiles before each one by decoupled look-back.
 template <Rule R, int K, int PER, bool LIGHT>
-__global__ void PATH_BOUNDS(PER) k_path_level(PathCall p, int64_t p0, int64_t p1, PathScan q)
+__global__ void PATH_BOUNDS(PER) k_path_level(PathCall p, int64_t p0, int64_t p1, PathScan<K> q)
 {
-    __shared__ PMap s_warp[kPathThreads / 32];
-    __shared__ PMap s_prefix;
+    __shared__ PMap<K> s_warp[kPathThreads / 32];
+    __shared__ PMap<K> s_prefix;
     __shared__ int64_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(q.ticket, 1);
     __syncthreads();
     const int64_t tile = s_tile;
     const int64_t first = chunk_base<PER>(p0) + tile * (kPathThreads * PER) + (int64_t)threadIdx.x * PER;
     Chunk<R, K, PER, LIGHT, true> ch;
-    const PMap acc = ch.load(p, first, p0, p1);
-    PMap total;
-    PMap E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
+    const PMap<K> acc = ch.load(p, first, p0, p1);
+    PMap<K> total;
+    PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
     if (threadIdx.x < 32) {
         if (tile == 0) {
             if (threadIdx.x == 0) {
@@ -834,7 +876,7 @@ __global__ void PATH_BOUNDS(PER) k_path_level(PathCall p, int64_t p0, int64_t p1
                 __threadfence();
                 st_release_gpu(q.status + tile, (q.epoch << 2) | 1);
             }
-            const PMap before = look_back<K>(q, tile, p.flag);
+            const PMap<K> before = look_back<K>(q, tile, p.flag);
             if (threadIdx.x == 0) {
                 q.inclm[tile] = compose<K>(before, total);
                 __threadfence();
@@ -867,8 +909,8 @@ constexpr int kPathFreeLongest = 2048;
 template <Rule R, int K, int PER, bool LIGHT>
 __global__ void PATH_BOUNDS(PER) k_path_free(PathCall p, int64_t p0, int64_t p1)
 {
-    __shared__ PMap s_warp[kPathThreads / 32];
-    __shared__ PMap s_carry;
+    __shared__ PMap<K> s_warp[kPathThreads / 32];
+    __shared__ PMap<K> s_carry;
     __shared__ int64_t s_range[2];
     const int64_t T = (int64_t)kPathThreads * PER;
     const int64_t s0 = p0 + (int64_t)blockIdx.x * T;
@@ -886,11 +928,11 @@ __global__ void PATH_BOUNDS(PER) k_path_free(PathCall p, int64_t p0, int64_t p1)
     for (int64_t c0 = lo; c0 < hi; c0 += T) {
         const int64_t first = c0 + (int64_t)threadIdx.x * PER;
         Chunk<R, K, PER, LIGHT, false> ch;
-        const PMap acc = ch.load(p, first, c0, min(hi, c0 + T));
-        PMap total;
+        const PMap<K> acc = ch.load(p, first, c0, min(hi, c0 + T));
+        PMap<K> total;
         // the scan's barriers come after thread 0's update of s_carry for the previous chunk
-        const PMap ex = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
-        const PMap E = compose<K>(s_carry, ex);
+        const PMap<K> ex = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
+        const PMap<K> E = compose<K>(s_carry, ex);
         __syncthreads();  // every thread has read s_carry
         if (threadIdx.x == 0) s_carry = compose<K>(s_carry, total);
         ch.store(p, first, p1, E);
@@ -951,7 +993,7 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
     const char* what = "path engine buffers";
     const int64_t nt = std::max<int64_t>(pc->tiles, 1);
     int rc = LUE_GPU_OK;
-    if ((rc = cuda_status(cudaMalloc(&t->path_maps, 2 * nt * sizeof(PMap)), what)) ||
+    if ((rc = cuda_status(cudaMalloc(&t->path_maps, 2 * nt * sizeof(PMap<kTrigger>)), what)) ||
         (rc = cuda_status(cudaMalloc(&t->path_status, (nt + kPathMaxLevels) * sizeof(int)), what)) ||
         (rc = cuda_status(cudaMalloc(&t->path_flag, 2 * sizeof(unsigned long long)), what)) ||
         (rc = cuda_status(cudaMemsetAsync(t->path_status, 0, (nt + kPathMaxLevels) * sizeof(int), stream), what))) {
@@ -959,7 +1001,7 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
         return rc;
     }
     t->path_epoch = 0;
-    t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap) + (nt + kPathMaxLevels) * 4 + 16;
+    t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (nt + kPathMaxLevels) * 4 + 16;
     return LUE_GPU_OK;
 }
 
@@ -991,7 +1033,7 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const float* a, flo
     int free_longest = kPathFreeLongest, polls = kPathPolls;
     if (const char* e = getenv("LUE_GB300_PATH_FREE_LONGEST")) free_longest = std::max(0, atoi(e));
     if (const char* e = getenv("LUE_GB300_PATH_POLLS")) polls = std::max(0, atoi(e));
-    PMap* aggm = static_cast<PMap*>(t->path_maps);
+    PMap<K>* aggm = static_cast<PMap<K>*>(t->path_maps);
     int launches = 1;
     for (int l = 0; l < levels; ++l) {
         const int64_t p0 = pc->level_offsets[l], p1 = pc->level_offsets[l + 1];
@@ -1019,7 +1061,7 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const float* a, flo
             ++launches;
             continue;
         }
-        PathScan q{t->path_status, aggm, aggm + nt_max, tickets + l, t->path_epoch, polls};
+        PathScan<K> q{t->path_status, aggm, aggm + nt_max, tickets + l, t->path_epoch, polls};
         switch (per * 2 + (l > 0)) {
             case 16: k_path_level<R, K, 8, false><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
             case 17: k_path_level<R, K, 8, true><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
@@ -1048,7 +1090,8 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
 {
     *done = false;
     if (path_engine_off()) return LUE_GPU_OK;
-    if (rule != (int)Rule::threshold && rule != (int)Rule::capacity && rule != (int)Rule::fraction)
+    if (rule != (int)Rule::threshold && rule != (int)Rule::capacity && rule != (int)Rule::fraction &&
+        rule != (int)Rule::trigger)
         return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     if (int rc = path_core_get(t, stream, &pc)) return rc;
@@ -1058,6 +1101,8 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
         return path_run<Rule::threshold, kMaxPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_threshold_f32 (paths)");
     if (rule == (int)Rule::fraction)
         return path_run<Rule::fraction, kAffine>(t, pc, a, as, b, bs, out, rem, stream, "accu_fraction_f32 (paths)");
+    if (rule == (int)Rule::trigger)
+        return path_run<Rule::trigger, kTrigger>(t, pc, a, as, b, bs, out, rem, stream, "accu_trigger_f32 (paths)");
     return path_run<Rule::capacity, kMinPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_capacity_f32 (paths)");
 }
 

@@ -188,8 +188,8 @@ extern "C" int lue_gpu_accu_fraction_f64(lue_gpu_topology* t, const double* infl
                                      "accu_fraction_f64");
 }
 
-// The path engine (path_route.cuh) takes float32 accu_threshold, accu_fraction and accu_capacity on acyclic
-// rasters.
+// The path engine (path_route.cuh) takes float32 accu_threshold, accu_fraction, accu_capacity and accu_trigger
+// on acyclic rasters.
 static int path_first(lue_gpu_topology* t, int rule, const float* a, float as, const float* b, float bs, float* out,
                       float* rem, cudaStream_t stream, bool* done)
 {
