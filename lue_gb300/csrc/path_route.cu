@@ -108,34 +108,52 @@ __global__ void k_path_jump(int32_t* next, int64_t n)
     }
 }
 
+constexpr int kPathMaxLevels = 254;
+constexpr int kPathTile = 64;                            // paths are grouped by the 64 x 64 tile of their bottom
+constexpr int kPathTileCells = kPathTile * kPathTile;
+
 // key[c] = path level of c if c is the bottom of its path, else 255; stats: [0] largest level,
-// [1] longest path, [2] cells whose next is not a bottom (must be 0).
-__global__ void k_path_keys(const int32_t* next, const int32_t* plev, const int32_t* dtop, int64_t n, uint8_t* key,
-                            int* stats)
+// [1] longest path, [2] cells whose next is not a bottom (must be 0), [3 + l] longest path of level l;
+// cells[l]: cells of the paths of level l.
+__global__ void __launch_bounds__(256) k_path_keys(const int32_t* next, const int32_t* plev, const int32_t* dtop,
+                                                   int64_t n, uint8_t* key, int* stats, unsigned long long* cells)
 {
-    int lmax = -1, longest = 0, bad = 0;
+    __shared__ unsigned s_cells[256];
+    __shared__ int s_longest[256];
+    s_cells[threadIdx.x] = 0;
+    s_longest[threadIdx.x] = 0;
+    __syncthreads();
+    int lmax = -1, bad = 0;
     for (int64_t c = grid_stride_begin(); c < n; c += grid_stride()) {
         const int32_t v = next[c];
         uint8_t k = 255;
         if (v >= 0) {
             if (next[v] != v) ++bad;
             if (v == c) {
-                const int l = plev[c];
-                k = (uint8_t)min(l, 254);
+                const int l = min(plev[c], kPathMaxLevels), len = dtop[c] + 1;
+                k = (uint8_t)l;
                 lmax = max(lmax, l);
-                longest = max(longest, dtop[c] + 1);
+                atomicMax(&s_longest[l], len);
+                atomicAdd(&s_cells[l], (unsigned)len);
             }
         }
         key[c] = k;
     }
-    if (lmax >= 0) atomicMax(stats, lmax);
-    if (longest) atomicMax(stats + 1, longest);
-    if (bad) atomicAdd(stats + 2, bad);
+    lmax = __reduce_max_sync(0xffffffffu, lmax);
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (lmax >= 0) atomicMax(stats, lmax);
+        if (bad) atomicAdd(stats + 2, bad);
+    }
+    __syncthreads();
+    if (s_cells[threadIdx.x]) {
+        atomicAdd(cells + threadIdx.x, (unsigned long long)s_cells[threadIdx.x]);
+        atomicMax(stats + 3 + threadIdx.x, s_longest[threadIdx.x]);
+        atomicMax(stats + 1, s_longest[threadIdx.x]);
+    }
 }
 
-constexpr int kCompactPer = 32;                          // cells per thread
-constexpr int kCompactCells = 256 * kCompactPer;         // cells per CTA
-
+// Exclusive sum over a CTA of NT threads; ends with a block barrier.
 template <int NT>
 __device__ __forceinline__ long long block_excl_sum(long long v, long long* s_warp, long long& total)
 {
@@ -162,80 +180,119 @@ __device__ __forceinline__ long long block_excl_sum(long long v, long long* s_wa
     return before + x - v;
 }
 
-// Per CTA of cells: the positions taken by the paths of level `lvl` whose bottom lies in it; longest[lvl]:
-// the longest path of the level.
-__global__ void __launch_bounds__(256) k_level_sums(const uint8_t* key, const int32_t* dtop, int lvl, int64_t n,
-                                                    long long* bsum, int* longest)
-{
-    __shared__ long long s_warp[8];
-    const int64_t c0 = (int64_t)blockIdx.x * kCompactCells + (int64_t)threadIdx.x * kCompactPer;
-    long long s = 0;
-    int lmax = 0;
-    for (int j = 0; j < kCompactPer; ++j) {
-        const int64_t c = c0 + j;
-        if (c < n && key[c] == lvl) {
-            s += dtop[c] + 1;
-            lmax = max(lmax, dtop[c] + 1);
-        }
+struct PathGeom {
+    int64_t rows, cols, tcols, ntiles;
+    __device__ __forceinline__ bool cell(int64_t tile, int loc, int64_t& c) const
+    {
+        const int64_t r = tile / tcols * kPathTile + loc / kPathTile, col = tile % tcols * kPathTile + loc % kPathTile;
+        c = r * cols + col;
+        return r < rows && col < cols;
     }
-    long long total = 0;
-    block_excl_sum<256>(s, s_warp, total);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-    for (int d = 16; d; d >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, d));
-    if ((threadIdx.x & 31) == 0 && lmax) atomicMax(longest + lvl, lmax);
-}
+};
 
-// Exclusive scan of the per-CTA sums of one level, after the positions of the lower levels
-// (running[0]); offsets[lvl + 1] = running[0] afterwards.
-__global__ void __launch_bounds__(1024) k_level_scan(long long* bsum, int64_t nblk, long long* running,
-                                                     long long* offsets, int lvl)
+// Per tile and level: the cells of the paths whose bottom lies in the tile, counts[level * ntiles + tile].
+__global__ void __launch_bounds__(256) k_paths_count(const uint8_t* key, const int32_t* dtop, PathGeom g, int levels,
+                                                     int32_t* counts)
 {
-    __shared__ long long s_warp[32];
-    const int64_t per = (nblk + 1023) / 1024;
-    const int64_t b0 = (int64_t)threadIdx.x * per, b1 = min(nblk, b0 + per);
-    long long s = 0;
-    for (int64_t b = b0; b < b1; ++b) s += bsum[b];
-    long long total = 0;
-    long long x = block_excl_sum<1024>(s, s_warp, total) + running[0];
-    for (int64_t b = b0; b < b1; ++b) {
-        const long long v = bsum[b];
-        bsum[b] = x;
-        x += v;
+    __shared__ int s_cells[kPathMaxLevels + 1];
+    for (int i = threadIdx.x; i < levels; i += 256) s_cells[i] = 0;
+    __syncthreads();
+    const int64_t tile = blockIdx.x;
+    for (int i = threadIdx.x; i < kPathTileCells; i += 256) {
+        int64_t c;
+        if (g.cell(tile, i, c) && key[c] != 255) atomicAdd(&s_cells[key[c]], dtop[c] + 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        offsets[lvl] = running[0];
-        running[0] += total;
-        offsets[lvl + 1] = running[0];
+    for (int i = threadIdx.x; i < levels; i += 256) counts[i * g.ntiles + tile] = s_cells[i];
+}
+
+// counts -> the first position of each level's paths of each tile (a CTA per level; starts[level]: the level's
+// first position).
+__global__ void __launch_bounds__(1024) k_paths_scan(int32_t* counts, int64_t ntiles, const int32_t* starts)
+{
+    __shared__ long long s_warp[32];
+    int32_t* x = counts + blockIdx.x * ntiles;
+    const int64_t per = (ntiles + 1023) / 1024;
+    const int64_t t0 = min(ntiles, (int64_t)threadIdx.x * per), t1 = min(ntiles, t0 + per);
+    long long s = 0, total = 0;
+    for (int64_t t = t0; t < t1; ++t) s += x[t];
+    long long v = starts[blockIdx.x] + block_excl_sum<1024>(s, s_warp, total);
+    for (int64_t t = t0; t < t1; ++t) {
+        const int32_t y = x[t];
+        x[t] = (int32_t)v;
+        v += y;
     }
 }
 
-// base[b]: first position of the path whose bottom is b (paths of one level in cell order of bottoms).
-__global__ void __launch_bounds__(256) k_level_assign(const uint8_t* key, const int32_t* dtop, int lvl, int64_t n,
-                                                      const long long* bsum, int32_t* base)
+// Per tile: its paths sorted by level and cell, and with that their positions.  base[b]: first position of the
+// path whose bottom is b.
+__global__ void __launch_bounds__(256)
+    k_paths_assign(const uint8_t* key, const int32_t* dtop, PathGeom g, const int32_t* counts, int32_t* base)
 {
+    __shared__ uint32_t s_key[kPathTileCells];
+    __shared__ int s_pos[kPathMaxLevels + 1];
     __shared__ long long s_warp[8];
-    const int64_t c0 = (int64_t)blockIdx.x * kCompactCells + (int64_t)threadIdx.x * kCompactPer;
-    long long s = 0;
-    for (int j = 0; j < kCompactPer; ++j) {
-        const int64_t c = c0 + j;
-        if (c < n && key[c] == lvl) s += dtop[c] + 1;
+    __shared__ int s_n;
+    const int64_t tile = blockIdx.x;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kPathTileCells; i += 256) {
+        int64_t c;
+        if (g.cell(tile, i, c) && key[c] != 255) s_key[atomicAdd(&s_n, 1)] = ((unsigned)key[c] << 12) | (unsigned)i;
     }
-    long long total = 0;
-    long long x = block_excl_sum<256>(s, s_warp, total) + bsum[blockIdx.x];
-    for (int j = 0; j < kCompactPer; ++j) {
-        const int64_t c = c0 + j;
-        if (c < n && key[c] == lvl) {
-            base[c] = (int32_t)x;
-            x += dtop[c] + 1;
+    __syncthreads();
+    const int n = s_n;
+    int size = 256;
+    while (size < n) size <<= 1;
+    for (int i = n + threadIdx.x; i < size; i += 256) s_key[i] = 0xFFFFFFFFu;
+    __syncthreads();
+    for (int k = 2; k <= size; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < size; i += 256) {
+                const int o = i ^ j;
+                if (o > i) {
+                    const uint32_t a = s_key[i], b = s_key[o];
+                    if ((a > b) == ((i & k) == 0)) {
+                        s_key[i] = b;
+                        s_key[o] = a;
+                    }
+                }
+            }
+            __syncthreads();
         }
     }
+    const int per = size / 256, i0 = threadIdx.x * per;
+    long long sum = 0, total = 0;
+    for (int i = i0; i < min(n, i0 + per); ++i) {
+        int64_t c;
+        g.cell(tile, (int)(s_key[i] & 0xFFFu), c);
+        sum += dtop[c] + 1;
+    }
+    const int before = (int)block_excl_sum<256>(sum, s_warp, total);
+    int at = before;
+    for (int i = i0; i < min(n, i0 + per); ++i) {
+        int64_t c;
+        g.cell(tile, (int)(s_key[i] & 0xFFFu), c);
+        if (i == 0 || (s_key[i - 1] >> 12) != (s_key[i] >> 12)) s_pos[s_key[i] >> 12] = at;
+        at += dtop[c] + 1;
+    }
+    __syncthreads();
+    at = before;
+    for (int i = i0; i < min(n, i0 + per); ++i) {
+        int64_t c;
+        g.cell(tile, (int)(s_key[i] & 0xFFFu), c);
+        const unsigned l = s_key[i] >> 12;
+        base[c] = counts[l * g.ntiles + tile] + at - s_pos[l];
+        at += dtop[c] + 1;
+    }
 }
 
-// order / light by position (order starts as all ones: no cell).  bad counts positions outside
-// [0, npos) and positions written twice; the build then fails instead of handing on a wrong layout.
+// order and the number of light upstream neighbours by position (order starts as all ones: no cell).  bad counts
+// positions outside [0, npos) and positions written twice; the build then fails instead of handing on a wrong
+// layout.
 __global__ void k_path_place(const int32_t* next, const int32_t* base, const int32_t* dtop, const int32_t* heavy,
-                             const uint8_t* upmask, int64_t n, int64_t npos, int32_t* order, uint8_t* light, int* bad)
+                             const uint8_t* upmask, int64_t n, int64_t npos, int64_t slot_base, int32_t* order,
+                             uint8_t* light, int* bad)
 {
     int nbad = 0;
     for (int64_t c = grid_stride_begin(); c < n; c += grid_stride()) {
@@ -250,7 +307,9 @@ __global__ void k_path_place(const int32_t* next, const int32_t* base, const int
         const int32_t old = atomicExch(order + pos, (int32_t)((uint32_t)c | (dt == 0 ? 0x80000000u : 0u)));
         if (old != -1) ++nbad;
         const int hk = heavy[c];
-        light[pos] = (uint8_t)(__ldg(upmask + c) & ~(hk < 8 ? 1u << hk : 0u));
+        const unsigned m = __ldg(upmask + c) & ~(hk < 8 ? 1u << hk : 0u);
+        if (pos >= slot_base) light[pos - slot_base] = (uint8_t)__popc(m);
+        else if (m) ++nbad;  // a cell of level 0 has no light inflow
     }
     if (nbad) atomicAdd(bad, nbad);
 }
@@ -263,36 +322,119 @@ __global__ void k_path_unwritten(const int32_t* order, int64_t npos, int* bad)
     if (nbad) atomicAdd(bad, nbad);
 }
 
+constexpr int kLightPer = 32;                  // positions per thread
+constexpr int kLightBlock = 256 * kLightPer;   // positions per CTA
+
+// slot_first = exclusive sums of the light neighbour counts: sums of blocks, their scan, the positions.
+__global__ void __launch_bounds__(256) k_light_sums(const uint8_t* light, int64_t n, long long* bsum)
+{
+    __shared__ long long s_warp[8];
+    const int64_t i0 = (int64_t)blockIdx.x * kLightBlock + (int64_t)threadIdx.x * kLightPer;
+    long long s = 0;
+    for (int64_t i = i0; i < min(n, i0 + kLightPer); ++i) s += light[i];
+    long long total = 0;
+    block_excl_sum<256>(s, s_warp, total);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(1024) k_light_scan(long long* bsum, int64_t nblk)
+{
+    __shared__ long long s_warp[32];
+    const int64_t per = (nblk + 1023) / 1024;
+    const int64_t b0 = min(nblk, (int64_t)threadIdx.x * per), b1 = min(nblk, b0 + per);
+    long long s = 0;
+    for (int64_t b = b0; b < b1; ++b) s += bsum[b];
+    long long total = 0;
+    long long x = block_excl_sum<1024>(s, s_warp, total);
+    for (int64_t b = b0; b < b1; ++b) {
+        const long long v = bsum[b];
+        bsum[b] = x;
+        x += v;
+    }
+    if (threadIdx.x == 0) bsum[nblk] = total;
+}
+__global__ void __launch_bounds__(256) k_light_apply(const uint8_t* light, int64_t n, const long long* bsum,
+                                                     int64_t nblk, int32_t* first)
+{
+    __shared__ long long s_warp[8];
+    const int64_t i0 = (int64_t)blockIdx.x * kLightBlock + (int64_t)threadIdx.x * kLightPer;
+    long long s = 0;
+    for (int64_t i = i0; i < min(n, i0 + kLightPer); ++i) s += light[i];
+    long long total = 0;
+    long long x = block_excl_sum<256>(s, s_warp, total) + bsum[blockIdx.x];
+    for (int64_t i = i0; i < min(n, i0 + kLightPer); ++i) {
+        first[i] = (int32_t)x;
+        x += light[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) first[n] = (int32_t)bsum[nblk];
+}
+
+// The slot that takes each path's outflow, at the position of its bottom: that of the bottom among the light
+// neighbours of the cell below.
+__global__ void k_path_slots(const uint8_t* fd, const uint8_t* upmask, const uint8_t* key, const int32_t* next,
+                             const int32_t* base, const int32_t* dtop, const int32_t* heavy,
+                             const int32_t* slot_first, int64_t slot_base, int64_t rows, int64_t cols,
+                             int32_t* path_slot, int* bad)
+{
+    for (int64_t c = grid_stride_begin(); c < rows * cols; c += grid_stride()) {
+        if (key[c] == 255) continue;
+        const uint8_t code = __ldg(fd + c);
+        int32_t slot = -1;
+        int64_t d = 0;
+        if (downstream(code, c / cols, c % cols, rows, cols, d) && __ldg(fd + d) != kNoData) {
+            const int64_t pos = (int64_t)base[next[d]] + dtop[d];
+            const int k = inflow_slot(code), hk = heavy[d];
+            const unsigned m = __ldg(upmask + d) & ~(hk < 8 ? 1u << hk : 0u);
+            if (pos >= slot_base && k >= 0 && ((m >> k) & 1u))
+                slot = slot_first[pos - slot_base] + __popc(m & ((1u << k) - 1u));
+            else
+                atomicAdd(bad, 1);
+        }
+        path_slot[base[c] + dtop[c]] = slot;
+    }
+}
+
+// The first path top at or after position s (p1 if none), for every lane of a warp.
+__device__ __forceinline__ int64_t next_top(const int32_t* order, int64_t s, int64_t p1)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t pos = s; pos < p1; pos += 32) {
+        const unsigned m = __ballot_sync(0xffffffffu, pos + lane < p1 && __ldg(order + pos + lane) < 0);
+        if (m) return pos + __ffs(m) - 1;
+    }
+    return p1;
+}
+
+// One warp per cut of a level's positions: every `step` positions, moved to the next path top.
+__global__ void k_path_cuts(const int32_t* order, int64_t p0, int64_t p1, int64_t step, int64_t ncut, int32_t* cut)
+{
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i > ncut) return;
+    const int64_t at = i == 0 ? p0 : next_top(order, min(p0 + i * step, p1), p1);
+    if ((threadIdx.x & 31) == 0) cut[i] = (int32_t)at;
+}
+
 // Position arrays are padded to whole 8-position chunks plus one chunk, for the vector loads of the
 // per-call kernels.
 static int64_t path_padded(int64_t npos) { return ((npos + 7) / 8 + 1) * 8; }
 
-// Positions per thread of a level: LUE_GB300_PATH_PER (1, 2, 4 or 8; default 4, the fastest at 16384^2:
-// 8.7 ms against 9.8 ms for 8 and 9.3 ms for 2) for large levels, 1 for small ones (of long paths: short
+// Positions per thread of a level's scan: 4 on large levels (2 and 8 were slower there), 1 on small ones (short
 // chains of dependent loads per thread).
 constexpr int64_t kPathSmallLevel = 1 << 20;
-static int path_per_large()
-{
-    static const int per = [] {
-        const char* e = getenv("LUE_GB300_PATH_PER");
-        const int v = e ? atoi(e) : 4;
-        return v == 1 || v == 2 || v == 8 ? v : 4;
-    }();
-    return per;
-}
-static int path_per(int64_t p0, int64_t p1) { return p1 - p0 < kPathSmallLevel ? 1 : path_per_large(); }
-static int64_t path_level_tiles(int64_t p0, int64_t p1, int per)
-{
-    if (p1 <= p0) return 0;
-    const int64_t base = per > 1 ? (p0 & ~int64_t(per - 1)) : p0;
-    return (p1 - base + kPathThreads * per - 1) / (kPathThreads * per);
-}
+
+// A level scans without look-back when its longest path is at most kPathFreeChunks chunks of a CTA; its CTA ranges
+// are then that many chunks, cut at path tops.  One chunk leaves most ranges a second one that is nearly empty
+// and more levels with look-back (accu_threshold at 16384^2: 11.3 ms), four lengthen the serial part of a CTA (6.8
+// ms; accu_fraction at 2311 x 1501: 189 us against 136 us); two: 6.6 ms.
+constexpr int kPathFreeChunks = 2;
+static int64_t path_cut_step(int per) { return (int64_t)kPathThreads * per * kPathFreeChunks; }
 
 void path_core_free(PathCore* pc)
 {
     if (!pc) return;
     cudaFree(pc->order);
-    cudaFree(pc->light);
+    cudaFree(pc->path_slot);
+    cudaFree(pc->slot_first);
+    cudaFree(pc->cut);
     delete pc;
 }
 
@@ -300,134 +442,161 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
 {
     *out = nullptr;
     const int64_t n = core->n, rows = core->rows, cols = core->cols;
-    if (n >= (int64_t(1) << 31)) return fail(LUE_GPU_ERANGE, "path topology: 2^31 cells or more");
+    // positions are 32-bit, and a CTA of the scan may look past the last one
+    if (n >= (int64_t(1) << 31) - 65536) return fail(LUE_GPU_ERANGE, "path topology: about 2^31 cells or more");
     const int64_t npos = core->stats.valid_cells;
     auto* pc = new (std::nothrow) PathCore();
     if (!pc) return fail(LUE_GPU_ENOMEM, "path topology: host allocation");
     pc->npos = npos;
+    const PathGeom g{rows, cols, (cols + kPathTile - 1) / kPathTile,
+                     (cols + kPathTile - 1) / kPathTile * ((rows + kPathTile - 1) / kPathTile)};
     int32_t *size = nullptr, *dtop = nullptr, *plev = nullptr, *heavy = nullptr, *next = nullptr;
-    uint8_t* key = nullptr;
-    long long* scan = nullptr;  // [0] running, [1..] offsets, then per-CTA sums
+    uint8_t *key = nullptr, *light = nullptr;
+    long long* bsum = nullptr;
+    int32_t *counts = nullptr, *starts = nullptr;
+    unsigned long long* cells = nullptr;
     int* stats = nullptr;
-    const int64_t nblk = (n + kCompactCells - 1) / kCompactCells;
-    const int kMaxLevels = 255;
-    int rc = LUE_GPU_OK;
-    int hstats[3] = {0, 0, 0};
+    constexpr int kStats = 3 + 256;
+    int rc = LUE_GPU_OK, levels = 0, hstats[kStats] = {}, launches = 6;
+    unsigned long long hcells[256] = {};
+    std::vector<int32_t> hstart;
+    int64_t ncuts = 0, nlight = 0, nblk = 0;
     const char* what = "path topology";
-    auto cleanup = [&]() {
-        cudaFree(size);
-        cudaFree(dtop);
-        cudaFree(plev);
-        cudaFree(heavy);
-        cudaFree(next);
-        cudaFree(key);
-        cudaFree(scan);
-        cudaFree(stats);
-    };
-    if ((rc = cuda_status(cudaMalloc(&size, n * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&dtop, n * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&plev, n * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&heavy, n * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&next, n * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&key, n), what)) ||
-        (rc = cuda_status(cudaMalloc(&scan, (2 + kMaxLevels + 1 + nblk) * sizeof(long long)), what)) ||
-        (rc = cuda_status(cudaMalloc(&stats, (3 + kMaxLevels) * sizeof(int)), what)) ||
-        (rc = cuda_status(cudaMalloc(&pc->order, path_padded(npos) * sizeof(int32_t)), what)) ||
-        (rc = cuda_status(cudaMalloc(&pc->light, path_padded(npos)), what))) {
-        cleanup();
-        path_core_free(pc);
-        return rc;
-    }
-    pc->bytes = path_padded(npos) * 5;
+#define TRY(call) \
+    if ((rc = cuda_status((call), what))) goto done
+    TRY(cudaMalloc(&size, n * sizeof(int32_t)));
+    TRY(cudaMalloc(&dtop, n * sizeof(int32_t)));
+    TRY(cudaMalloc(&plev, n * sizeof(int32_t)));
+    TRY(cudaMalloc(&heavy, n * sizeof(int32_t)));
+    TRY(cudaMalloc(&next, n * sizeof(int32_t)));
+    TRY(cudaMalloc(&key, n));
+    TRY(cudaMalloc(&stats, kStats * sizeof(int)));
+    TRY(cudaMalloc(&cells, sizeof hcells));
+    TRY(cudaMalloc(&pc->order, path_padded(npos) * sizeof(int32_t)));
     // 1. sizes, heavy neighbours, cells above on the path, path levels
     k_fill<<<grid_for(n, 256), 256, 0, stream>>>(heavy, n, 8);
-    cudaMemcpyAsync(work, core->count, words_for(n) * 4, cudaMemcpyDeviceToDevice, stream);
+    TRY(cudaMemcpyAsync(work, core->count, words_for(n) * 4, cudaMemcpyDeviceToDevice, stream));
     {
-        WalkGrid g{core->fd, core->count, work, rows, cols, n};
+        WalkGrid wg{core->fd, core->count, work, rows, cols, n};
         PathVisitor v{core->upmask, size, dtop, plev, heavy, cols};
-        k_walk<<<grid_all(n, 256), 256, 0, stream>>>(g, v);
+        k_walk<<<grid_all(n, 256), 256, 0, stream>>>(wg, v);
     }
     // 2. bottom of each cell's path: pointer jumping over the path links
     k_path_next<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, heavy, rows, cols, n, next);
-    int rounds = 1;
-    while ((int64_t(1) << rounds) < core->stats.max_level + 2) ++rounds;
-    for (int i = 0; i <= rounds; ++i) k_path_jump<<<grid_for(n, 256), 256, 0, stream>>>(next, n);
-    // 3. keys and level count
-    cudaMemsetAsync(stats, 0, 3 * sizeof(int), stream);
-    k_path_keys<<<grid_for(n, 256), 256, 0, stream>>>(next, plev, dtop, n, key, stats);
-    if ((rc = cuda_status(cudaMemcpyAsync(hstats, stats, sizeof hstats, cudaMemcpyDeviceToHost, stream), what)) ||
-        (rc = cuda_status(cudaStreamSynchronize(stream), what))) {
-        cleanup();
-        path_core_free(pc);
-        return rc;
+    {
+        int rounds = 1;
+        while ((int64_t(1) << rounds) < core->stats.max_level + 2) ++rounds;
+        for (int i = 0; i <= rounds; ++i) k_path_jump<<<grid_for(n, 256), 256, 0, stream>>>(next, n);
+        launches += rounds + 1;
     }
-    if (hstats[2] != 0 || hstats[0] >= 254) {
-        cleanup();
-        path_core_free(pc);
-        return fail(LUE_GPU_ERANGE, "path topology: " + std::to_string(hstats[2]) + " cells without a bottom, " +
-                                        std::to_string(hstats[0] + 1) + " levels");
+    // 3. levels
+    TRY(cudaMemsetAsync(stats, 0, kStats * sizeof(int), stream));
+    TRY(cudaMemsetAsync(cells, 0, sizeof hcells, stream));
+    k_path_keys<<<grid_for(n, 256), 256, 0, stream>>>(next, plev, dtop, n, key, stats, cells);
+    TRY(cudaMemcpyAsync(hstats, stats, sizeof hstats, cudaMemcpyDeviceToHost, stream));
+    TRY(cudaMemcpyAsync(hcells, cells, sizeof hcells, cudaMemcpyDeviceToHost, stream));
+    TRY(cudaStreamSynchronize(stream));
+    if (hstats[2] != 0 || hstats[0] >= kPathMaxLevels) {
+        rc = fail(LUE_GPU_ERANGE, "path topology: " + std::to_string(hstats[2]) + " cells without a bottom, " +
+                                      std::to_string(hstats[0] + 1) + " levels");
+        goto done;
     }
-    const int levels = npos > 0 ? hstats[0] + 1 : 0;
-    pc->longest_path = hstats[1];
-    // 4. positions: levels in order, paths of a level in cell order of their bottoms
-    int32_t* base = size;  // sizes are no longer needed
-    long long* running = scan;
-    long long* offsets = scan + 1;
-    long long* bsum = scan + 2 + kMaxLevels;
-    cudaMemsetAsync(scan, 0, (2 + kMaxLevels) * sizeof(long long), stream);
-    int* longest = stats + 3;
-    cudaMemsetAsync(longest, 0, kMaxLevels * sizeof(int), stream);
+    levels = npos > 0 ? hstats[0] + 1 : 0;
+    // 4. positions: levels in order, and the paths of a level tile by tile
+    pc->levels.resize(levels);
+    hstart.resize(levels + 1);
     for (int l = 0; l < levels; ++l) {
-        k_level_sums<<<(unsigned)nblk, 256, 0, stream>>>(key, dtop, l, n, bsum, longest);
-        k_level_scan<<<1, 1024, 0, stream>>>(bsum, nblk, running, offsets, l);
-        k_level_assign<<<(unsigned)nblk, 256, 0, stream>>>(key, dtop, l, n, bsum, base);
+        PathLevel& v = pc->levels[l];
+        if (hcells[l] > (unsigned long long)(npos - hstart[l])) {
+            rc = fail(LUE_GPU_ERANGE, "path topology: more positions than cells");
+            goto done;
+        }
+        v.p0 = hstart[l];
+        v.p1 = hstart[l + 1] = (int32_t)(hstart[l] + (int64_t)hcells[l]);
+        v.longest = hstats[3 + l];
+        v.per = v.p1 - v.p0 < kPathSmallLevel ? 1 : 4;
+        v.cut0 = (int32_t)ncuts;
+        v.ncut = (int32_t)((v.p1 - v.p0 + path_cut_step(v.per) - 1) / path_cut_step(v.per));
+        ncuts += v.ncut + 1;
+        pc->tiles = std::max<int64_t>(pc->tiles, (v.p1 - v.p0) / (kPathThreads * v.per) + 2);
     }
-    cudaMemsetAsync(pc->order, 0xFF, path_padded(npos) * sizeof(int32_t), stream);
-    cudaMemsetAsync(pc->light, 0, path_padded(npos), stream);
-    cudaMemsetAsync(stats + 2, 0, sizeof(int), stream);
-    k_path_place<<<grid_for(n, 256), 256, 0, stream>>>(next, base, dtop, heavy, core->upmask, n, npos, pc->order,
-                                                       pc->light, stats + 2);
-    k_path_unwritten<<<grid_for(npos, 256), 256, 0, stream>>>(pc->order, npos, stats + 2);
-    std::vector<long long> hoff(levels + 1, 0);
-    std::vector<int> hlong(std::max(levels, 1), 0);
-    if (levels > 0 &&
-        ((rc = cuda_status(cudaMemcpyAsync(hoff.data(), offsets, (levels + 1) * sizeof(long long),
-                                           cudaMemcpyDeviceToHost, stream),
-                           what)) ||
-         (rc = cuda_status(cudaMemcpyAsync(hlong.data(), longest, levels * sizeof(int), cudaMemcpyDeviceToHost,
-                                           stream),
-                           what)))) {
-        cleanup();
-        path_core_free(pc);
-        return rc;
+    if (hstart[levels] != npos) {
+        rc = fail(LUE_GPU_ERANGE, "path topology: " + std::to_string(hstart[levels]) + " positions for " +
+                                      std::to_string(npos) + " cells");
+        goto done;
     }
-    int bad = 0;
-    rc = cuda_status(cudaMemcpyAsync(&bad, stats + 2, sizeof(int), cudaMemcpyDeviceToHost, stream), what);
-    if (!rc) rc = cuda_status(cudaStreamSynchronize(stream), what);
-    if (!rc) rc = cuda_status(cudaGetLastError(), what);
-    cleanup();
-    count_launches(8 + rounds + 3 * levels);
+    pc->slot_base = levels > 0 ? pc->levels[0].p1 : 0;
+    nlight = npos - pc->slot_base;
+    nblk = (nlight + kLightBlock - 1) / kLightBlock;
+    TRY(cudaMalloc(&counts, std::max<int64_t>(1, levels * g.ntiles) * sizeof(int32_t)));
+    TRY(cudaMalloc(&starts, (levels + 1) * sizeof(int32_t)));
+    TRY(cudaMalloc(&pc->path_slot, std::max<int64_t>(1, npos) * sizeof(int32_t)));
+    TRY(cudaMalloc(&pc->slot_first, (nlight + 1) * sizeof(int32_t)));
+    TRY(cudaMalloc(&pc->cut, std::max<int64_t>(1, ncuts) * sizeof(int32_t)));
+    TRY(cudaMalloc(&light, std::max<int64_t>(1, nlight)));
+    TRY(cudaMalloc(&bsum, (nblk + 1) * sizeof(long long)));
+    pc->bytes = path_padded(npos) * 4 + npos * 4 + (nlight + 1) * 4 + ncuts * 4;
+    if (levels > 0) {
+        int32_t* base = size;  // no longer needed
+        TRY(cudaMemcpyAsync(starts, hstart.data(), (levels + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+        k_paths_count<<<(unsigned)g.ntiles, 256, 0, stream>>>(key, dtop, g, levels, counts);
+        k_paths_scan<<<(unsigned)levels, 1024, 0, stream>>>(counts, g.ntiles, starts);
+        k_paths_assign<<<(unsigned)g.ntiles, 256, 0, stream>>>(key, dtop, g, counts, base);
+        TRY(cudaMemsetAsync(pc->order, 0xFF, path_padded(npos) * sizeof(int32_t), stream));
+        TRY(cudaMemsetAsync(stats + 2, 0, sizeof(int), stream));
+        k_path_place<<<grid_for(n, 256), 256, 0, stream>>>(next, base, dtop, heavy, core->upmask, n, npos,
+                                                          pc->slot_base, pc->order, light, stats + 2);
+        k_path_unwritten<<<grid_for(npos, 256), 256, 0, stream>>>(pc->order, npos, stats + 2);
+        // 5. slots
+        if (nlight > 0) k_light_sums<<<(unsigned)nblk, 256, 0, stream>>>(light, nlight, bsum);
+        k_light_scan<<<1, 1024, 0, stream>>>(bsum, nblk);
+        if (nlight > 0) k_light_apply<<<(unsigned)nblk, 256, 0, stream>>>(light, nlight, bsum, nblk, pc->slot_first);
+        k_path_slots<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, core->upmask, key, next, base, dtop, heavy,
+                                                          pc->slot_first, pc->slot_base, rows, cols, pc->path_slot,
+                                                          stats + 2);
+        // 6. CTA ranges of the scans
+        for (const PathLevel& v : pc->levels)
+            if (v.ncut > 0)
+                k_path_cuts<<<(unsigned)(((v.ncut + 1) * 32 + 255) / 256), 256, 0, stream>>>(
+                    pc->order, v.p0, v.p1, path_cut_step(v.per), v.ncut, pc->cut + v.cut0);
+        launches += 8 + levels;
+        long long hslots = 0;
+        int bad = 0;
+        TRY(cudaMemcpyAsync(&hslots, bsum + nblk, sizeof hslots, cudaMemcpyDeviceToHost, stream));
+        TRY(cudaMemcpyAsync(&bad, stats + 2, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        TRY(cudaStreamSynchronize(stream));
+        TRY(cudaGetLastError());
+        pc->nslots = hslots;
+        if (bad) {
+            rc = fail(LUE_GPU_ERANGE, "path topology: inconsistent layout (" + std::to_string(bad) + " misplaced)");
+            goto done;
+        }
+    }
+    count_launches(launches);
+    if (getenv("LUE_GB300_VERBOSE")) {
+        fprintf(stderr, "path topology: %lld cells, %d levels, %lld slots, longest path %d cells; positions (longest path) "
+                        "by level:",
+                (long long)npos, levels, (long long)pc->nslots, hstats[1]);
+        for (const PathLevel& v : pc->levels) fprintf(stderr, " %d (%d)", v.p1 - v.p0, v.longest);
+        fprintf(stderr, "\n");
+    }
+done:
+#undef TRY
+    cudaFree(size);
+    cudaFree(dtop);
+    cudaFree(plev);
+    cudaFree(heavy);
+    cudaFree(next);
+    cudaFree(key);
+    cudaFree(light);
+    cudaFree(bsum);
+    cudaFree(counts);
+    cudaFree(starts);
+    cudaFree(cells);
+    cudaFree(stats);
     if (rc) {
         path_core_free(pc);
         return rc;
-    }
-    if ((levels > 0 && hoff[levels] != npos) || bad) {
-        path_core_free(pc);
-        return fail(LUE_GPU_ERANGE, "path topology: inconsistent layout (" + std::to_string(levels ? hoff[levels] : 0) +
-                                        " positions for " + std::to_string(npos) + " cells, " + std::to_string(bad) +
-                                        " misplaced)");
-    }
-    pc->level_offsets.assign(hoff.begin(), hoff.end());
-    pc->level_longest.assign(hlong.begin(), hlong.begin() + levels);
-    pc->tiles = 0;
-    for (int l = 0; l < levels; ++l)  // as many as one position per thread would need
-        pc->tiles = std::max(pc->tiles, path_level_tiles(hoff[l], hoff[l + 1], 1));
-    if (getenv("LUE_GB300_VERBOSE")) {
-        fprintf(stderr, "path topology: %lld cells, %d levels, %lld tiles, longest path %lld cells; positions "
-                        "(longest path) by level:",
-                (long long)npos, levels, (long long)pc->tiles, (long long)pc->longest_path);
-        for (int l = 0; l < levels; ++l) fprintf(stderr, " %lld (%d)", hoff[l + 1] - hoff[l], hlong[l]);
-        fprintf(stderr, "\n");
     }
     *out = pc;
     return LUE_GPU_OK;
@@ -446,7 +615,7 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
 //
 // On the stage engine accu_trigger was bound by its chain of rounds (1500^2: 1595 us a call); as a scan it
 // takes 319 us.
-constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2, kTrigger = 3;
+constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2, kTrigger = 3, kSum = 4;
 
 // a, b and c float-float.  flags bit 0: the map of a path's top cell, which ignores its input (its value is
 // value()); bit 1: no-data (NaN) from the cell itself or from upstream.
@@ -464,28 +633,34 @@ struct PMap<kTrigger> {
     __device__ FF value() const { return FF{ch, cl}; }
 };
 
+// x -> x + b in float64 (accu); the value of a top cell's map is b.
+template <>
+struct PMap<kSum> {
+    double b;
+    int flags;
+    __device__ double value() const { return b; }
+};
+
 template <int K>
 __device__ __forceinline__ PMap<K> pm_identity()
 {
+    if constexpr (K == kSum) return PMap<K>{0.0, 0};
+    else
     if constexpr (K == kAffine) return PMap<K>{1.0f, 0.0f, 0.0f, 0.0f, 0};
     else if constexpr (K == kTrigger) return PMap<K>{-INFINITY, 0.0f, 0.0f, 0.0f, 0, 0.0f, 0.0f};
     else return PMap<K>{0.0f, 0.0f, K == kMinPlus ? INFINITY : -INFINITY, 0.0f, 0};
 }
 
 // x + y for float-float values; a sum that is not finite is kept with lo = 0 (two_sum's error terms would
-// turn an infinity into NaN).
+// turn an infinity into NaN).  Selects, no branches: a warp composes many maps at once.
 __device__ __forceinline__ void ff_sum(float xh, float xl, float yh, float yl, float& rh, float& rl)
 {
     float s, e;
     two_sum(xh, yh, s, e);
-    if (!isfinite(s)) {
-        rh = s;
-        rl = 0.0f;
-        return;
-    }
     e = __fadd_rn(e, __fadd_rn(xl, yl));
+    e = fabsf(s) < INFINITY ? e : 0.0f;
     rh = __fadd_rn(s, e);
-    rl = __fsub_rn(e, __fsub_rn(rh, s));
+    rl = fabsf(s) < INFINITY ? __fsub_rn(e, __fsub_rn(rh, s)) : 0.0f;
 }
 
 __device__ __forceinline__ bool ff_less(float xh, float xl, float yh, float yl)
@@ -493,31 +668,28 @@ __device__ __forceinline__ bool ff_less(float xh, float xl, float yh, float yl)
     return xh < yh || (xh == yh && xl < yl);
 }
 
-// x * y for float-float values: the exact product of the high parts by FMA (two-product), plus the cross
-// terms, renormalised.
+// x * y for finite float-float values: the exact product of the high parts by FMA (two-product), plus the
+// cross terms, renormalised.
 __device__ __forceinline__ void ff_mul(float xh, float xl, float yh, float yl, float& rh, float& rl)
 {
     const float p = __fmul_rn(xh, yh);
     float e = __fmaf_rn(xh, yh, -p);
     e = __fmaf_rn(xh, yl, e);
     e = __fmaf_rn(xl, yh, e);
-    if (!isfinite(p)) {
-        rh = p;
-        rl = 0.0f;
-        return;
-    }
     rh = __fadd_rn(p, e);
     rl = __fsub_rn(e, __fsub_rn(rh, p));
 }
 
-// m1 first, then m2.
+// m1 first, then m2.  No branches: the constant map of a path's top is one on which the same formulas give
+// a constant (a = -inf, +inf, 0 and +inf for the four float32 kinds), so only its flags are chosen.
 template <int K>
 __device__ __forceinline__ PMap<K> compose(const PMap<K>& m1, const PMap<K>& m2)
 {
-    if (m2.flags & 1) return m2;
     PMap<K> r;
-    r.flags = (m1.flags & 1) | ((m1.flags | m2.flags) & 2);
-    if constexpr (K == kAffine) {  // a2 * (a1 * x + b1) + b2
+    r.flags = m2.flags & 1 ? m2.flags : m1.flags | m2.flags;
+    if constexpr (K == kSum) {
+        r.b = m2.flags & 1 ? m2.b : m1.b + m2.b;
+    } else if constexpr (K == kAffine) {  // a2 * (a1 * x + b1) + b2
         ff_mul(m1.ah, m1.al, m2.ah, m2.al, r.ah, r.al);
         float th, tl;
         ff_mul(m2.ah, m2.al, m1.bh, m1.bl, th, tl);
@@ -544,41 +716,131 @@ __device__ __forceinline__ PMap<K> compose(const PMap<K>& m1, const PMap<K>& m2)
     return r;
 }
 
-// The map of one cell: s = its material plus the outflow of its light upstream neighbours, b its
-// threshold, fraction, capacity or trigger.
-template <Rule R, int K>
-__device__ __forceinline__ PMap<K> cell_map(bool top, float sh, float sl, float b, bool nan)
+// The two kinds of numbers: float32 operations carry float-float values, float64 operations plain doubles.  A
+// cell's sum s is its material plus its light inflow; total() adds what comes along its path.
+struct F32 {
+    using T = float;
+    using V = FF;
+    using Slot = float2;  // hi (NaN: no-data), lo
+    static __device__ __forceinline__ void light(FF& s, bool& nan, float2 v)
+    {
+        nan |= isnan(v.x);
+        float h, e;
+        two_sum(s.hi, v.x, h, e);
+        s.hi = h;
+        s.lo = __fadd_rn(__fadd_rn(s.lo, e), v.y);
+    }
+    static __device__ __forceinline__ FF from(float x) { return FF{x, 0.0f}; }
+    static __device__ __forceinline__ FF cell(FF s, float x) { return total(s, FF{x, 0.0f}); }
+    static __device__ __forceinline__ FF total(FF x, FF s)
+    {
+        float h, e;
+        two_sum(x.hi, s.hi, h, e);
+        e = __fadd_rn(e, __fadd_rn(x.lo, s.lo));
+        const float r = __fadd_rn(h, e);
+        return FF{r, __fsub_rn(e, __fsub_rn(r, h))};
+    }
+    static __device__ __forceinline__ FF zero() { return FF{0.0f, 0.0f}; }
+    static __device__ __forceinline__ float hi(FF v) { return v.hi; }
+    static __device__ __forceinline__ Slot slot(FF v, bool nan)
+    {
+        return nan ? make_float2(__int_as_float(0x7fc00000), 0.0f) : make_float2(v.hi, v.lo);
+    }
+};
+struct F64 {
+    using T = double;
+    using V = double;
+    using Slot = double;
+    static __device__ __forceinline__ void light(double& s, bool& nan, double v)
+    {
+        nan |= isnan(v);
+        s += v;
+    }
+    static __device__ __forceinline__ double from(double x) { return x; }
+    static __device__ __forceinline__ double cell(double s, double x) { return s + x; }
+    static __device__ __forceinline__ double total(double x, double s) { return x + s; }
+    static __device__ __forceinline__ double zero() { return 0.0; }
+    static __device__ __forceinline__ double hi(double v) { return v; }
+    static __device__ __forceinline__ double slot(double v, bool nan) { return nan ? qnan<double>() : v; }
+};
+
+// The rules of rule_f32 / rule_f64 on a finite total t (float-float: normalised), inputs in the domain.
+template <Rule R>
+__device__ __forceinline__ void rule_total(FF t, float b, FF& out, float& rem)
 {
-    PMap<K> m{0.0f, 0.0f, 0.0f, 0.0f, nan ? 2 | (top ? 1 : 0) : 0};
-    if (nan) return m;
-    if (top) {
-        float oh = 0.0f, ol = 0.0f, rem = 0.0f;
-        rule_f32<R>(FF{sh, sl}, false, 0.0f, b, oh, ol, rem);
-        m.flags = 1;
-        if constexpr (K == kTrigger) {
-            m.ah = INFINITY;
-            m.ch = oh;
-            m.cl = ol;
+    if constexpr (R == Rule::fraction) {
+        const float ph = __fmul_rn(b, t.hi);
+        float pl = __fmaf_rn(b, t.hi, -ph);
+        pl = __fmaf_rn(b, t.lo, pl);
+        out.hi = __fadd_rn(ph, pl);
+        out.lo = __fsub_rn(pl, __fsub_rn(out.hi, ph));
+        const float h = __fsub_rn(t.hi, out.hi);  // |t| >= |out|: the rounding error of h is exact
+        const float e = __fsub_rn(__fsub_rn(t.hi, h), out.hi);
+        rem = __fadd_rn(h, __fadd_rn(e, __fsub_rn(t.lo, out.lo)));
+    } else if constexpr (R == Rule::trigger) {
+        const bool stays = t.hi < b || (t.hi == b && t.lo < 0.0f);
+        rem = stays ? t.hi : 0.0f;
+        out.hi = stays ? 0.0f : t.hi;
+        out.lo = stays ? 0.0f : t.lo;
+    } else {  // threshold, capacity: what is above b
+        const bool above = t.hi > b || (t.hi == b && t.lo > 0.0f);
+        const float h = __fsub_rn(t.hi, b);  // t.hi >= b >= 0 where it is used: exact error
+        const float e = __fadd_rn(__fsub_rn(__fsub_rn(t.hi, h), b), t.lo);
+        const float dh = __fadd_rn(h, e), dl = __fsub_rn(e, __fsub_rn(dh, h));
+        if constexpr (R == Rule::threshold) {
+            rem = above ? b : t.hi;
+            out.hi = above ? dh : 0.0f;
+            out.lo = above ? dl : 0.0f;
         } else {
-            m.bh = oh;
-            m.bl = ol;
+            rem = above ? dh : 0.0f;
+            out.hi = above ? b : t.hi;
+            out.lo = above ? 0.0f : t.lo;
         }
-    } else if constexpr (K == kMaxPlus) {  // max(x + (s - threshold), 0)
-        ff_sum(sh, sl, -b, 0.0f, m.ah, m.al);
-    } else if constexpr (K == kAffine) {  // fraction * x + fraction * s
-        m.ah = b;
-        ff_mul(b, 0.0f, sh, sl, m.bh, m.bl);
+    }
+}
+template <Rule R>
+__device__ __forceinline__ void rule_total(double t, double b, double& out, double& rem)
+{
+    static_assert(R == Rule::accu, "float64 paths carry sums only");
+    out = t;
+}
+
+// The map of one cell: s = its material plus the outflow of its light upstream neighbours, b its
+// threshold, fraction, capacity or trigger (both 0 in a no-data cell).  By selects, as compose().
+template <Rule R, int K, class V, class T>
+__device__ __forceinline__ PMap<K> cell_map(bool top, V s, T b, bool nan)
+{
+    PMap<K> m;
+    m.flags = (top ? 1 : 0) | (nan ? 2 : 0);
+    if constexpr (K == kSum) {
+        m.b = s;
+    } else if constexpr (K == kAffine) {  // fraction * x + fraction * s; top: fraction * s
+        m.ah = top ? 0.0f : b;
+        m.al = 0.0f;
+        ff_mul(b, 0.0f, s.hi, s.lo, m.bh, m.bl);
     } else if constexpr (K == kTrigger) {  // x + s where that reaches the trigger, else 0
-        ff_sum(b, 0.0f, -sh, -sl, m.ah, m.al);
-        m.bh = sh;
-        m.bl = sl;
-        const bool passes = !ff_less(sh, sl, b, 0.0f);
-        m.ch = passes ? sh : 0.0f;
-        m.cl = passes ? sl : 0.0f;
-    } else {  // capacity: min(x + s, capacity)
-        m.ah = sh;
-        m.al = sl;
-        m.bh = b;
+        ff_sum(b, 0.0f, -s.hi, -s.lo, m.ah, m.al);
+        const bool passes = m.ah <= 0.0f;
+        m.ah = top ? INFINITY : m.ah;
+        m.al = top ? 0.0f : m.al;
+        m.bh = s.hi;
+        m.bl = s.lo;
+        m.ch = passes ? s.hi : 0.0f;
+        m.cl = passes ? s.lo : 0.0f;
+    } else if constexpr (K == kMaxPlus) {  // max(x + (s - threshold), 0); top: max(s - threshold, 0)
+        float dh, dl;
+        ff_sum(s.hi, s.lo, -b, 0.0f, dh, dl);
+        const bool over = top && dh > 0.0f;
+        m.ah = top ? -INFINITY : dh;
+        m.al = top ? 0.0f : dl;
+        m.bh = over ? dh : 0.0f;
+        m.bl = over ? dl : 0.0f;
+    } else {  // capacity: min(x + s, capacity); top: min(s, capacity)
+        const bool under = top && ff_less(s.hi, s.lo, b, 0.0f);
+        m.ah = top ? INFINITY : s.hi;
+        m.al = top ? 0.0f : s.lo;
+        m.bh = under ? s.hi : b;
+        m.bl = under ? s.lo : 0.0f;
     }
     return m;
 }
@@ -588,6 +850,11 @@ template <int K, class F>
 __device__ __forceinline__ PMap<K> pm_each(const PMap<K>& m, F f)
 {
     PMap<K> r;
+    if constexpr (K == kSum) {
+        r.b = f(m.b);
+        r.flags = f(m.flags);
+        return r;
+    } else {
     r.ah = f(m.ah);
     r.al = f(m.al);
     r.bh = f(m.bh);
@@ -598,6 +865,7 @@ __device__ __forceinline__ PMap<K> pm_each(const PMap<K>& m, F f)
         r.cl = f(m.cl);
     }
     return r;
+    }
 }
 template <int K>
 __device__ __forceinline__ PMap<K> shfl_up(const PMap<K>& m, int d)
@@ -617,6 +885,7 @@ __device__ __forceinline__ PMap<K> block_excl_scan(const PMap<K>& v, PMap<K>* s_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PMap<K> x = v;
     for (int d = 1; d < 32; d <<= 1) {
+        if (__all_sync(0xffffffffu, lane < d || (x.flags & 1))) break;  // every map is a constant by now
         const PMap<K> y = shfl_up(x, d);
         if (lane >= d) x = compose<K>(y, x);
     }
@@ -639,47 +908,43 @@ __device__ __forceinline__ PMap<K> block_excl_scan(const PMap<K>& v, PMap<K>* s_
     return r;
 }
 
+template <class N>
 struct PathCall {
     const int32_t* __restrict__ order;
-    const uint8_t* __restrict__ light;
-    const float* __restrict__ a;  // material
-    float as;
-    const float* __restrict__ b;  // threshold / fraction / capacity
-    float bs;
-    float* out;
-    float* rem;
-    float* lo;                    // float-float residual of the outflow (path bottoms: read as light inflow)
+    const int32_t* __restrict__ path_slot;   // by position, at the bottoms of paths
+    const int32_t* __restrict__ slot_first;  // by position (the engine's array minus its base)
+    const typename N::T* __restrict__ a;     // material
+    typename N::T as;
+    const typename N::T* __restrict__ b;     // threshold / fraction / capacity / trigger
+    typename N::T bs;
+    typename N::T* out;
+    typename N::T* rem;
+    typename N::Slot* slots;                 // what leaves each path; written by a level, read by higher ones
     unsigned long long* flag;
-    int64_t cols;
 };
+
+// The inputs of a cell are in the domain and not NaN.
+template <Rule R, class T>
+__device__ __forceinline__ bool in_domain(T e, T b)
+{
+    if constexpr (R == Rule::accu) return e >= T(0);
+    else if constexpr (R == Rule::fraction) return e >= T(0) && b >= T(0) && b <= T(1);
+    else return e >= T(0) && b >= T(0);
+}
 
 // The order entries of PER consecutive positions from `first` (a multiple of PER), read with vector
 // loads; the position arrays are padded by one 8-position chunk, so a chunk that starts before the end
 // of the array stays inside it.
-template <int PER>
-__device__ __forceinline__ void load_order(const PathCall& p, int64_t first, int32_t (&w)[PER])
+template <int PER, class P>
+__device__ __forceinline__ void load_order(const P& p, int64_t first, int32_t (&w)[PER])
 {
     if (PER == 4) {
         const int4 x = __ldg(reinterpret_cast<const int4*>(p.order + first));
         w[0] = x.x; w[1 % PER] = x.y; w[2 % PER] = x.z; w[3 % PER] = x.w;
-    } else if (PER == 2) {
-        const int2 x = __ldg(reinterpret_cast<const int2*>(p.order + first));
-        w[0] = x.x; w[1 % PER] = x.y;
-    } else if (PER == 8) {
-        const int4 x = __ldg(reinterpret_cast<const int4*>(p.order + first));
-        const int4 y = __ldg(reinterpret_cast<const int4*>(p.order + first) + 1);
-        w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
-        w[4 % PER] = y.x; w[5 % PER] = y.y; w[6 % PER] = y.z; w[7 % PER] = y.w;
     } else {
 #pragma unroll
         for (int j = 0; j < PER; ++j) w[j] = __ldg(p.order + first + j);
     }
-}
-
-template <int PER>
-__device__ __forceinline__ int64_t chunk_base(int64_t p0)
-{
-    return PER > 1 ? (p0 & ~int64_t(PER - 1)) : p0;
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p)
@@ -752,116 +1017,138 @@ __device__ PMap<K> look_back(const PathScan<K>& q, int64_t tile, unsigned long l
     }
 }
 
-// The positions of one thread in one chunk: PER consecutive positions from `first`, those in [lo, hi)
-// active.  load(): inputs, light inflow and the cells' maps, composed in order; store(): from the
-// composition E of everything before the first position, each cell's rule and outputs.  VEC: `first` is
-// a multiple of PER and the order array is read with vector loads.
-template <Rule R, int K, int PER, bool LIGHT, bool VEC>
+// The positions of one thread in one chunk of a scan: PER consecutive positions from `first`, those in
+// [lo, hi) active.  order() and gather() issue the loads, light() adds the light inflow, maps() composes the
+// cells' maps, and store() applies, from the composition E of everything before the first position, each cell's
+// rule.
+template <class N, Rule R, int K, int PER, bool LIGHT>
 struct Chunk {
-    int32_t w[PER];
-    bool on[PER];
-    float b[PER];
-    FF sum[PER];
-    bool nan[PER];
+    using T = typename N::T;
+    int32_t w[PER];          // order entries: cell, top bit
+    unsigned on;             // bit j: position j is active
+    unsigned nan;            // bit j: no-data from the cell itself or its light inflow
+    T e[PER], b[PER];
+    typename N::V sum[PER];
 
-    __device__ __forceinline__ PMap<K> load(const PathCall& p, int64_t first, int64_t lo, int64_t hi)
+    // VEC: `first` is a multiple of PER and the order array is read with vector loads.
+    template <bool VEC>
+    __device__ __forceinline__ void order(const PathCall<N>& p, int32_t first, int32_t lo, int32_t hi)
     {
+        on = 0;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) on[j] = first + j >= lo && first + j < hi;
-        if (VEC && first < hi) {
-            load_order<PER>(p, first, w);
+        for (int j = 0; j < PER; ++j) on |= first + j >= lo && first + j < hi ? 1u << j : 0u;
+        if (VEC) {
+            if (on) load_order<PER>(p, first, w);
         } else {
 #pragma unroll
-            for (int j = 0; j < PER; ++j) w[j] = on[j] ? __ldg(p.order + first + j) : 0;
+            for (int j = 0; j < PER; ++j) w[j] = (on >> j) & 1u ? __ldg(p.order + first + j) : 0;
         }
-        float e[PER];
+    }
+
+    __device__ __forceinline__ void gather(const PathCall<N>& p)
+    {
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const int64_t c = (int64_t)(w[j] & 0x7fffffff);
-            e[j] = on[j] ? value_at(p.a, p.as, c) : 0.0f;
-            b[j] = on[j] ? value_at(p.b, p.bs, c) : 0.0f;
-            sum[j] = FF{0.0f, 0.0f};
-            nan[j] = false;
+            const int32_t c = w[j] & 0x7fffffff;
+            e[j] = p.as;
+            b[j] = p.bs;
+            if ((on >> j) & 1u) {
+                if (p.a) e[j] = __ldg(p.a + c);
+                if (R != Rule::accu && p.b) b[j] = __ldg(p.b + c);
+            }
         }
+    }
+
+    // The cells' sums and the composition of their maps; inactive positions are the identity.
+    __device__ __forceinline__ PMap<K> maps(const PathCall<N>& p, int32_t first)
+    {
+        nan = 0;
         if (LIGHT) {
+            int32_t f[PER + 1];
+#pragma unroll
+            for (int j = 0; j <= PER; ++j)
+                f[j] = ((on >> (j < PER ? j : PER - 1)) & 1u) || (j > 0 && ((on >> (j - 1)) & 1u))
+                           ? __ldg(p.slot_first + first + j)
+                           : 0;
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
-                if (!on[j]) continue;
-                const int64_t c = (int64_t)(w[j] & 0x7fffffff);
-                for (unsigned lm = __ldg(p.light + first + j); lm; lm &= lm - 1) {
-                    const int k = __ffs(lm) - 1;
-                    const int64_t u = c + nb_dr(k) * p.cols + nb_dc(k);
-                    const float vh = p.out[u];
-                    nan[j] |= isnan(vh);
-                    sum[j].add(vh, p.lo[u]);
-                }
+                sum[j] = N::zero();
+                if (!((on >> j) & 1u)) continue;
+                bool bad = false;
+                for (int32_t k = f[j]; k < f[j + 1]; ++k) N::light(sum[j], bad, p.slots[k]);
+                nan |= bad ? 1u << j : 0u;
             }
         }
         PMap<K> acc = pm_identity<K>();
         bool odd = false;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            if (!on[j]) continue;
-            nan[j] |= isnan(e[j]) || isnan(b[j]) || !(e[j] >= 0.0f && b[j] >= 0.0f) ||
-                      (R == Rule::fraction && !(b[j] <= 1.0f));
-            sum[j].add(e[j]);
-            sum[j].normalise();
-            odd |= !nan[j] && (isinf(e[j]) || isinf(b[j]) || isinf(sum[j].hi));
-            acc = compose<K>(acc, cell_map<R, K>(w[j] < 0, sum[j].hi, sum[j].lo, b[j], nan[j]));
+            const bool act = (on >> j) & 1u;
+            bool bad = LIGHT && ((nan >> j) & 1u);
+            bad = bad || !in_domain<R>(e[j], b[j]);
+            if constexpr (LIGHT) sum[j] = N::cell(sum[j], e[j]);
+            else sum[j] = N::from(e[j]);
+            odd |= act && !bad && !(N::hi(sum[j]) < T(INFINITY) && b[j] < T(INFINITY));
+            if (bad) {
+                sum[j] = N::zero();
+                b[j] = T(0);
+                nan |= 1u << j;
+            }
+            const PMap<K> m = cell_map<R, K>(w[j] < 0, sum[j], b[j], bad);
+            if (act) acc = j == 0 ? m : compose<K>(acc, m);
         }
-        if (odd) p.flag[1] = 1;  // +-inf: the walk engine redoes the call
+        if (odd) p.flag[1] = 1;  // +inf: the walk engine redoes the call
         return acc;
     }
 
-    __device__ __forceinline__ void store(const PathCall& p, int64_t first, int64_t p1, PMap<K> E)
+    // hi: the end of the CTA's positions, where a path ends.
+    __device__ __forceinline__ void store(const PathCall<N>& p, int32_t first, int32_t hi, const PMap<K>& E)
     {
         // the position after this thread's last one: is it the top of a path (then the last one is a bottom)?
-        const int32_t after = first + PER < p1 ? __ldg(p.order + first + PER) : -1;
+        const int32_t after = first + PER < hi ? __ldg(p.order + first + PER) : -1;
+        // everything before the first position composes to a constant: a path's top is among it
+        typename N::V x = E.value();
+        bool xnan = (E.flags & 2) != 0, odd = false;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            if (!on[j]) continue;
-            const int64_t c = (int64_t)(w[j] & 0x7fffffff);
+            if (!((on >> j) & 1u)) continue;
+            const int32_t c = w[j] & 0x7fffffff;
             const bool top = w[j] < 0;
-            FF t{0.0f, 0.0f};
-            bool nn = nan[j];
-            if (!top) {
-                nn |= (E.flags & 2) != 0;
-                t = E.value();
+            xnan = ((nan >> j) & 1u) || (!top && xnan);
+            const typename N::V t = top ? sum[j] : N::total(x, sum[j]);
+            T rem = T(0);
+            rule_total<R>(t, b[j], x, rem);
+            odd |= !xnan && !(N::hi(t) < T(INFINITY));
+            p.out[c] = xnan ? qnan<T>() : N::hi(x);
+            if (R != Rule::accu) p.rem[c] = xnan ? qnan<T>() : rem;
+            const int32_t next = j + 1 < PER && first + j + 1 < hi ? w[(j + 1) % PER] : after;
+            if (next < 0) {  // a path bottom
+                const int32_t slot = __ldg(p.path_slot + first + j);
+                if (slot >= 0) p.slots[slot] = N::slot(x, xnan);
             }
-            t.add(sum[j].hi, sum[j].lo);
-            float oh = 0.0f, ol = 0.0f, rem = 0.0f;
-            if (!rule_f32<R>(t, nn, 0.0f, b[j], oh, ol, rem)) {
-                oh = __int_as_float(0x7fc00000);
-                ol = 0.0f;
-                rem = oh;
-            }
-            p.out[c] = oh;
-            p.rem[c] = rem;
-            const int32_t next = j + 1 < PER ? w[(j + 1) % PER] : after;
-            if (first + j + 1 >= p1 || next < 0) p.lo[c] = ol;  // a path bottom
-            E = compose<K>(E, cell_map<R, K>(top, sum[j].hi, sum[j].lo, b[j], nan[j]));
         }
+        if (odd) p.flag[1] = 1;
     }
 };
 
-#define PATH_BOUNDS(PER) __launch_bounds__(kPathThreads, PER >= 8 ? 2 : (PER == 4 ? 4 : (PER == 2 ? 5 : 6)))
-
-// One level in one pass, for levels with long paths: tiles in ticket order, the composition of the
-// tiles before each one by decoupled look-back.
-template <Rule R, int K, int PER, bool LIGHT>
-__global__ void PATH_BOUNDS(PER) k_path_level(PathCall p, int64_t p0, int64_t p1, PathScan<K> q)
+// The scan of one level with very long paths: tiles in ticket order, the composition of the tiles before each
+// one by decoupled look-back.
+template <class N, Rule R, int K, int PER, bool LIGHT>
+__global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, PathLevel v, PathScan<K> q)
 {
     __shared__ PMap<K> s_warp[kPathThreads / 32];
     __shared__ PMap<K> s_prefix;
-    __shared__ int64_t s_tile;
+    __shared__ int s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(q.ticket, 1);
     __syncthreads();
-    const int64_t tile = s_tile;
-    const int64_t first = chunk_base<PER>(p0) + tile * (kPathThreads * PER) + (int64_t)threadIdx.x * PER;
-    Chunk<R, K, PER, LIGHT, true> ch;
-    const PMap<K> acc = ch.load(p, first, p0, p1);
+    const int tile = s_tile;
+    const int32_t first = (v.p0 & ~(PER - 1)) + tile * (kPathThreads * PER) + (int32_t)threadIdx.x * PER;
+    Chunk<N, R, K, PER, LIGHT> ch;
+    ch.template order<true>(p, first, v.p0, v.p1);
+    ch.gather(p);
+    const PMap<K> acc = ch.maps(p, first);
     PMap<K> total;
-    PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
+    const PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
     if (threadIdx.x < 32) {
         if (tile == 0) {
             if (threadIdx.x == 0) {
@@ -886,65 +1173,58 @@ __global__ void PATH_BOUNDS(PER) k_path_level(PathCall p, int64_t p0, int64_t p1
         }
     }
     __syncthreads();
-    ch.store(p, first, p1, compose<K>(s_prefix, E));
+    ch.store(p, first, v.p1, compose<K>(s_prefix, E));
 }
 
-// The first path top at or after position s (p1 if none), for every lane of a warp.
-__device__ __forceinline__ int64_t next_top(const int32_t* order, int64_t s, int64_t p1)
-{
-    const int lane = threadIdx.x & 31;
-    for (int64_t pos = s; pos < p1; pos += 32) {
-        const unsigned m = __ballot_sync(0xffffffffu, pos + lane < p1 && __ldg(order + pos + lane) < 0);
-        if (m) return pos + __ffs(m) - 1;
-    }
-    return p1;
-}
-
-// Levels whose paths are all short (at most kPathFreeLongest cells): each CTA's range of positions is
-// cut at path tops (its nominal range with both ends moved forward to the next top), so no path crosses
-// from one CTA to another and CTAs do not wait for one another; a range is processed in chunks of
-// kPathThreads * PER positions with the composition carried from chunk to chunk.
-constexpr int kPathFreeLongest = 2048;
-
-template <Rule R, int K, int PER, bool LIGHT>
-__global__ void PATH_BOUNDS(PER) k_path_free(PathCall p, int64_t p0, int64_t p1)
+// The scan of one level with shorter paths: each CTA's range of positions begins and ends at path tops (`cut`, laid
+// out once), so no path crosses from one CTA to another and CTAs do not wait for one another; a range is processed
+// in chunks of kPathThreads * PER positions with the composition carried from chunk to chunk.  The next
+// chunk's order is read before this chunk's scan, and its inputs before this chunk's rules, so that the two
+// dependent loads overlap the arithmetic.
+//
+// Bound by instruction issue (50 % of the slots) and by the requests of its scattered stores about equally: 270
+// thread instructions per position on level 0 at 8192^2, 0.71 ms; with branches in the compositions, a second
+// composition per cell in store() and 64-bit positions it was 486 and 1.0 ms.  accu_threshold at 16384^2: 8.4 -> 6.6
+// ms.  Tried and slower: one thread per short path (up to 16, 64 or 256 cells) with the cell rule itself, sorted by
+// length within a tile: 50 instructions per cell, but every lane of a store is a request of its own (8.3-10 ms at
+// 16384^2, with the results of a tile collected in shared memory as well); CTAs of 128 threads (6.9 ms).
+template <class N, Rule R, int K, int PER, bool LIGHT>
+__global__ void __launch_bounds__(kPathThreads, 4)
+    k_path_free(PathCall<N> p, PathLevel v, const int32_t* __restrict__ cut)
 {
     __shared__ PMap<K> s_warp[kPathThreads / 32];
     __shared__ PMap<K> s_carry;
-    __shared__ int64_t s_range[2];
-    const int64_t T = (int64_t)kPathThreads * PER;
-    const int64_t s0 = p0 + (int64_t)blockIdx.x * T;
-    if (threadIdx.x < 32) {
-        const int64_t lo = blockIdx.x == 0 ? p0 : next_top(p.order, s0, p1);
-        const int64_t hi = next_top(p.order, min(s0 + T, p1), p1);
-        if (threadIdx.x == 0) {
-            s_range[0] = lo;
-            s_range[1] = hi;
-            s_carry = pm_identity<K>();
-        }
-    }
-    __syncthreads();
-    const int64_t lo = s_range[0], hi = s_range[1];
-    for (int64_t c0 = lo; c0 < hi; c0 += T) {
-        const int64_t first = c0 + (int64_t)threadIdx.x * PER;
-        Chunk<R, K, PER, LIGHT, false> ch;
-        const PMap<K> acc = ch.load(p, first, c0, min(hi, c0 + T));
+    constexpr int32_t T = kPathThreads * PER;
+    const int32_t lo = __ldg(cut + v.cut0 + blockIdx.x), hi = __ldg(cut + v.cut0 + blockIdx.x + 1);
+    if (threadIdx.x == 0) s_carry = pm_identity<K>();
+    const int32_t at = (int32_t)threadIdx.x * PER;
+    Chunk<N, R, K, PER, LIGHT> ch, nx;
+    ch.template order<false>(p, lo + at, lo, hi);
+    ch.gather(p);
+    for (int32_t c0 = lo; c0 < hi; c0 += T) {  // uniform
+        const int32_t first = c0 + at;
+        const bool more = c0 + T < hi;
+        if (more) nx.template order<false>(p, first + T, lo, hi);
+        const PMap<K> acc = ch.maps(p, first);
         PMap<K> total;
         // the scan's barriers come after thread 0's update of s_carry for the previous chunk
         const PMap<K> ex = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
         const PMap<K> E = compose<K>(s_carry, ex);
         __syncthreads();  // every thread has read s_carry
         if (threadIdx.x == 0) s_carry = compose<K>(s_carry, total);
-        ch.store(p, first, p1, E);
+        if (more) nx.gather(p);
+        ch.store(p, first, hi, E);
+        ch = nx;
     }
 }
 
-__global__ void k_path_no_data(const uint8_t* fd, int64_t n, float* out, float* rem)
+template <class T>
+__global__ void k_path_no_data(const uint8_t* fd, int64_t n, T* out, T* rem)
 {
     for (int64_t i = grid_stride_begin(); i < n; i += grid_stride())
         if (__ldg(fd + i) == kNoData) {
-            out[i] = __int_as_float(0x7fc00000);
-            rem[i] = __int_as_float(0x7fc00000);
+            out[i] = qnan<T>();
+            if (rem) rem[i] = qnan<T>();
         }
 }
 
@@ -978,30 +1258,33 @@ static int path_core_get(lue_gpu_topology* t, cudaStream_t stream, const PathCor
 void path_buffers_free(lue_gpu_topology* t)
 {
     cudaFree(t->path_maps);
-    cudaFree(t->path_status);
-    cudaFree(t->path_flag);
+    cudaFree(t->path_ctl);
+    cudaFree(t->path_slots);
     t->path_maps = nullptr;
-    t->path_status = nullptr;
-    t->path_flag = nullptr;
+    t->path_ctl = nullptr;
+    t->path_slots = nullptr;
 }
 
-constexpr int kPathMaxLevels = 256;
+// path_ctl: the redo flag (two words of 8 bytes) and one ticket per level, zeroed before each call, then the
+// status words of the scan tiles.
+constexpr size_t kPathCtlZeroed = 2 * sizeof(unsigned long long) + (kPathMaxLevels + 2) * sizeof(int);
 
 static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t stream)
 {
     if (t->path_maps) return LUE_GPU_OK;
     const char* what = "path engine buffers";
-    const int64_t nt = std::max<int64_t>(pc->tiles, 1);
+    const int64_t nt = std::max<int64_t>(pc->tiles, 1), ns = std::max<int64_t>(pc->nslots, 1);
+    const size_t ctl = kPathCtlZeroed + nt * sizeof(int);
     int rc = LUE_GPU_OK;
     if ((rc = cuda_status(cudaMalloc(&t->path_maps, 2 * nt * sizeof(PMap<kTrigger>)), what)) ||
-        (rc = cuda_status(cudaMalloc(&t->path_status, (nt + kPathMaxLevels) * sizeof(int)), what)) ||
-        (rc = cuda_status(cudaMalloc(&t->path_flag, 2 * sizeof(unsigned long long)), what)) ||
-        (rc = cuda_status(cudaMemsetAsync(t->path_status, 0, (nt + kPathMaxLevels) * sizeof(int), stream), what))) {
+        (rc = cuda_status(cudaMalloc(&t->path_ctl, ctl), what)) ||
+        (rc = cuda_status(cudaMalloc(&t->path_slots, ns * sizeof(double)), what)) ||
+        (rc = cuda_status(cudaMemsetAsync(t->path_ctl, 0, ctl, stream), what))) {
         path_buffers_free(t);
         return rc;
     }
     t->path_epoch = 0;
-    t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (nt + kPathMaxLevels) * 4 + 16;
+    t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (int64_t)ctl + ns * 8;
     return LUE_GPU_OK;
 }
 
@@ -1011,78 +1294,76 @@ int path_prepare(lue_gpu_topology* t, cudaStream_t stream)
     return path_core_get(t, stream, &pc);
 }
 
-template <Rule R, int K>
-static int path_run(lue_gpu_topology* t, const PathCore* pc, const float* a, float as, const float* b, float bs,
-                    float* out, float* rem, cudaStream_t stream, const char* what)
+template <class N, Rule R, int K, int PER, bool LIGHT>
+static void launch_level(bool free, unsigned blocks, cudaStream_t stream, const PathCall<N>& p, const PathLevel& v,
+                         const PathScan<K>& q, const int32_t* cut)
+{
+    if (free) k_path_free<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, cut);
+    else k_path_level<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, q);
+}
+
+template <class N, Rule R, int K, class Visitor>
+static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T* a, typename N::T as,
+                    const typename N::T* b, typename N::T bs, typename N::T* out, typename N::T* rem,
+                    const Visitor& redo, cudaStream_t stream, const char* what)
 {
     const TopologyCore* core = t->core;
     const int64_t n = core->n;
-    const int levels = (int)pc->level_offsets.size() - 1;
-    if (levels > kPathMaxLevels) return fail(LUE_GPU_ERANGE, std::string(what) + ": too many path levels");
     if (int rc = path_buffers(t, pc, stream)) return rc;
     const int64_t nt_max = std::max<int64_t>(pc->tiles, 1);
-    int* tickets = t->path_status + nt_max;
-    if (int rc = cuda_status(cudaMemsetAsync(t->path_flag, 0, 2 * sizeof(unsigned long long), stream), what))
-        return rc;
-    if (int rc = cuda_status(cudaMemsetAsync(tickets, 0, kPathMaxLevels * sizeof(int), stream), what)) return rc;
-    k_path_no_data<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, n, out, rem);
-    PathCall p{pc->order, pc->light, a, as, b, bs, out, rem, t->lo, t->path_flag, core->cols};
+    unsigned long long* flag = static_cast<unsigned long long*>(t->path_ctl);
+    int* tickets = reinterpret_cast<int*>(flag + 2);
+    int* status = tickets + kPathMaxLevels + 2;
+    if (int rc = cuda_status(cudaMemsetAsync(flag, 0, kPathCtlZeroed, stream), what)) return rc;
+    int launches = 0;
+    if (pc->npos < n) {
+        k_path_no_data<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, n, out, rem);
+        ++launches;
+    }
+    const PathCall<N> p{pc->order, pc->path_slot, pc->slot_first - pc->slot_base, a, as, b, bs, out, rem, static_cast<typename N::Slot*>(t->path_slots), flag};
     // test hooks: LUE_GB300_PATH_FREE_LONGEST (levels with longer paths use the look-back scan; 0: every
     // level) and LUE_GB300_PATH_POLLS (poll limit of a look-back wait; 0: every wait gives up at once,
     // and the walk engine redoes the call)
-    int free_longest = kPathFreeLongest, polls = kPathPolls;
+    int free_longest = -1, polls = kPathPolls;
     if (const char* e = getenv("LUE_GB300_PATH_FREE_LONGEST")) free_longest = std::max(0, atoi(e));
     if (const char* e = getenv("LUE_GB300_PATH_POLLS")) polls = std::max(0, atoi(e));
     PMap<K>* aggm = static_cast<PMap<K>*>(t->path_maps);
-    int launches = 1;
-    for (int l = 0; l < levels; ++l) {
-        const int64_t p0 = pc->level_offsets[l], p1 = pc->level_offsets[l + 1];
-        const int per = path_per(p0, p1);
-        const int64_t nt = path_level_tiles(p0, p1, per);
-        if (nt == 0) continue;
+    for (size_t l = 0; l < pc->levels.size(); ++l) {
+        const PathLevel& v = pc->levels[l];
         if (++t->path_epoch >= (1 << 29)) {  // status words of old launches could match again: clear them
             t->path_epoch = 1;
-            if (int rc = cuda_status(cudaMemsetAsync(t->path_status, 0, nt_max * sizeof(int), stream), what))
-                return rc;
+            if (int rc = cuda_status(cudaMemsetAsync(status, 0, nt_max * sizeof(int), stream), what)) return rc;
         }
-        const dim3 grid((unsigned)nt);
-        if (pc->level_longest[l] <= free_longest) {  // CTAs cut at path tops: no waits
-            const int64_t nf = (p1 - p0 + kPathThreads * per - 1) / (kPathThreads * per);
-            const dim3 gf((unsigned)nf);
-            switch (per * 2 + (l > 0)) {
-                case 16: k_path_free<R, K, 8, false><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                case 17: k_path_free<R, K, 8, true><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                case 8: k_path_free<R, K, 4, false><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                case 9: k_path_free<R, K, 4, true><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                case 4: k_path_free<R, K, 2, false><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                case 5: k_path_free<R, K, 2, true><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-                default: k_path_free<R, K, 1, true><<<gf, kPathThreads, 0, stream>>>(p, p0, p1); break;
-            }
-            ++launches;
-            continue;
-        }
-        PathScan<K> q{t->path_status, aggm, aggm + nt_max, tickets + l, t->path_epoch, polls};
-        switch (per * 2 + (l > 0)) {
-            case 16: k_path_level<R, K, 8, false><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            case 17: k_path_level<R, K, 8, true><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            case 8: k_path_level<R, K, 4, false><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            case 9: k_path_level<R, K, 4, true><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            case 4: k_path_level<R, K, 2, false><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            case 5: k_path_level<R, K, 2, true><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
-            default: k_path_level<R, K, 1, true><<<grid, kPathThreads, 0, stream>>>(p, p0, p1, q); break;
+        const int T = kPathThreads * v.per;
+        const bool free = v.longest <= (free_longest >= 0 ? free_longest : kPathFreeChunks * T);
+        const unsigned blocks =
+            free ? (unsigned)v.ncut : (unsigned)((v.p1 - (v.p0 & ~(v.per - 1)) + T - 1) / T);
+        if (blocks == 0) continue;
+        const PathScan<K> q{status, aggm, aggm + nt_max, tickets + l, t->path_epoch, polls};
+        switch (2 * (v.per > 1) + (l > 0)) {
+            case 0: launch_level<N, R, K, 1, false>(free, blocks, stream, p, v, q, pc->cut); break;
+            case 1: launch_level<N, R, K, 1, true>(free, blocks, stream, p, v, q, pc->cut); break;
+            case 2: launch_level<N, R, K, 4, false>(free, blocks, stream, p, v, q, pc->cut); break;
+            default: launch_level<N, R, K, 4, true>(free, blocks, stream, p, v, q, pc->cut); break;
         }
         ++launches;
     }
     // +-inf inputs, or a wait of the scan that gave up: the walk engine redoes the whole call (as behind
     // the tile engine of accu)
-    const unsigned long long* flag = t->path_flag;
     k_copy_words_if<<<grid_for(words_for(n), 256), 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(core->count),
                                                                      t->work_count, words_for(n), flag);
     WalkGrid g{core->fd, core->count, t->work_count, core->rows, core->cols, n};
-    RouteF32<R> v{core->upmask, a, as, b, bs, out, rem, t->lo, core->cols};
-    k_walk_if<<<grid_for(n, 256), 256, 0, stream>>>(g, v, flag);
+    k_walk_if<<<grid_for(n, 256), 256, 0, stream>>>(g, redo, flag);
     count_launches(launches + 2);
     return cuda_status(cudaGetLastError(), what);
+}
+
+template <Rule R, int K>
+static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const float* a, float as, const float* b, float bs,
+                        float* out, float* rem, cudaStream_t stream, const char* what)
+{
+    const RouteF32<R> redo{t->core->upmask, a, as, b, bs, out, rem, t->lo, t->core->cols};
+    return path_run<F32, R, K>(t, pc, a, as, b, bs, out, rem, redo, stream, what);
 }
 
 int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, const float* b, float bs, float* out,
@@ -1090,20 +1371,21 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
 {
     *done = false;
     if (path_engine_off()) return LUE_GPU_OK;
-    if (rule != (int)Rule::threshold && rule != (int)Rule::capacity && rule != (int)Rule::fraction &&
-        rule != (int)Rule::trigger)
-        return LUE_GPU_OK;
+    if (rule < (int)Rule::threshold || rule > (int)Rule::trigger) return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     if (int rc = path_core_get(t, stream, &pc)) return rc;
     if (!pc) return LUE_GPU_OK;
     *done = true;
     if (rule == (int)Rule::threshold)
-        return path_run<Rule::threshold, kMaxPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_threshold_f32 (paths)");
+        return path_run_f32<Rule::threshold, kMaxPlus>(t, pc, a, as, b, bs, out, rem, stream,
+                                                       "accu_threshold_f32 (paths)");
     if (rule == (int)Rule::fraction)
-        return path_run<Rule::fraction, kAffine>(t, pc, a, as, b, bs, out, rem, stream, "accu_fraction_f32 (paths)");
+        return path_run_f32<Rule::fraction, kAffine>(t, pc, a, as, b, bs, out, rem, stream,
+                                                     "accu_fraction_f32 (paths)");
     if (rule == (int)Rule::trigger)
-        return path_run<Rule::trigger, kTrigger>(t, pc, a, as, b, bs, out, rem, stream, "accu_trigger_f32 (paths)");
-    return path_run<Rule::capacity, kMinPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_capacity_f32 (paths)");
+        return path_run_f32<Rule::trigger, kTrigger>(t, pc, a, as, b, bs, out, rem, stream,
+                                                     "accu_trigger_f32 (paths)");
+    return path_run_f32<Rule::capacity, kMinPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_capacity_f32 (paths)");
 }
 
 }  // namespace lue_gb300

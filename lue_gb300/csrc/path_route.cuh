@@ -14,11 +14,12 @@
 // the largest upstream area (the heavy one); the other upstream neighbours (light) end paths of their
 // own.  A path's level is 0 when no cell of it has a light upstream neighbour, else one more than the
 // largest level of those light paths; every path crosses at most log2(cells) light edges, so there are
-// few levels.  Paths are laid out level by level, each from its top (a cell without inflow) to its
-// bottom (the cell whose downstream cell is on another path, off the array, a sink or no-data).  A call
-// runs the levels in order; within a level every path is one segment of a single scan (a path's top
-// map ignores its input, so segments need no flags), with the light inputs of a cell read from the
-// outflows of lower levels.
+// few levels.  Paths are laid out level by level, and within a level by the 64 x 64 tile of their bottom, each
+// from its top (a cell without inflow) to its bottom (the cell whose downstream cell is on another path, off the
+// array, a sink or no-data).  A call runs the levels in order; within a level every path is one segment of a
+// single scan (a path's top map ignores its input, so segments need no flags).  What leaves a path at its
+// bottom goes to a slot of the cell that it flows into; the slots of a cell are consecutive, and so are those
+// of neighbouring positions, so a level reads its light inflow densely and not by gathers over the raster.
 //
 // Built once per flow-direction raster (on the first call that needs it) and kept by the topology.
 #pragma once
@@ -31,14 +32,24 @@ namespace lue_gb300 {
 
 constexpr int kPathThreads = 256;  // CTA of the per-call kernels
 
+// One level: positions [p0, p1).
+struct PathLevel {
+    int32_t p0 = 0, p1 = 0;
+    int32_t cut0 = 0, ncut = 0;        // CTA ranges cut[cut0 + i] .. cut[cut0 + i + 1], i < ncut
+    int longest = 0;                   // cells of the longest path
+    int per = 1;                       // positions per thread
+};
+
 struct PathCore {
     int64_t npos = 0;                   // valid cells (positions)
     int32_t* order = nullptr;           // [npos] cell index, bit 31 set at the top cell of a path
-    uint8_t* light = nullptr;           // [npos] light upstream neighbours (bit k: neighbour k, walk order)
-    std::vector<int64_t> level_offsets; // [levels + 1] first position of each level
-    std::vector<int> level_longest;     // [levels] cells of the longest path of each level
+    int32_t* path_slot = nullptr;       // [npos] at the bottom of a path: the slot that takes its outflow, or -1
+    int32_t* slot_first = nullptr;      // [npos - slot_base + 1] first slot of a position
+    int32_t* cut = nullptr;             // path tops at which the CTAs of a level begin
+    int64_t slot_base = 0;              // first position of level 1 (level 0 has no light inflow)
+    int64_t nslots = 0;                 // light edges of the forest
+    std::vector<PathLevel> levels;
     int64_t tiles = 0;                  // most CTAs of one level's scan
-    int64_t longest_path = 0;           // cells of the longest path
     int64_t bytes = 0;
 };
 
