@@ -71,6 +71,8 @@ namespace lue_gb300 {
 // another engine.
 int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, const float* b, float bs, float* out,
                    float* rem, cudaStream_t stream, bool* done);
+// accu, float64: prefix sums along the paths in plain doubles (only additions of terms >= 0, so no cancellation).
+int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, cudaStream_t stream, bool* done);
 // Frees the handle's path-engine buffers.
 void path_buffers_free(lue_gpu_topology* t);
 // Builds the path layout of t now (lue_gpu_topology_prepare).

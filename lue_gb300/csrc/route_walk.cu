@@ -117,8 +117,8 @@ extern "C" int lue_gpu_accu_f32(lue_gpu_topology* t, const float* inflow, float 
     return cuda_status(cudaGetLastError(), "accu_f32");
 }
 
-// Float64 accu and the rules that are not plain sums run on the stage engine (stage_route.cuh) when the
-// topology has no flow cycles, else on the walk engine.  LUE_GB300_ENGINE=walk forces the walk engine.
+// The rules that are not plain sums, and float64 accu, run on the path engine (path_route.cuh) or the stage engine
+// (stage_route.cuh) when the topology has no flow cycles, else on the walk engine.  LUE_GB300_ENGINE=walk forces the walk engine.
 #define STAGE_OR_WALK(call)                          \
     do {                                             \
         bool done = false;                           \
@@ -131,6 +131,7 @@ extern "C" int lue_gpu_accu_f64(lue_gpu_topology* t, const double* inflow, doubl
 {
     if (int rc = check_topology(t, "accu_f64")) return rc;
     if (!outflow) return fail(LUE_GPU_EINVAL, "accu_f64: NULL output");
+    STAGE_OR_WALK(path_accu_f64(t, inflow, inflow_scalar, outflow, (cudaStream_t)stream, &done));
     STAGE_OR_WALK(stage_route_f64(t, (int)Rule::accu, inflow, inflow_scalar, nullptr, 0.0, outflow, nullptr,
                                   (cudaStream_t)stream, &done));
     return route_f64<Rule::accu>(t, inflow, inflow_scalar, nullptr, 0.0, outflow, nullptr, stream, "accu_f64");
