@@ -831,47 +831,64 @@ __device__ __forceinline__ int flow_wait(const int* p, int need, int* error, int
     return need;
 }
 
-// Shared memory of a stage of at most kStageMaxCap cells: the stage position of each in-tile cell, the
-// outflows by step parity and position, per position meta / history row / cell state / round starts, per
-// input (an upstream cell in another stage) its history row, value and cell, and per producer its
-// position, the earliest round that consumes it and the steps of it known to be in the history.
+// Shared memory of a stage of at most kStageMaxCap cells.  Values (outflows of the stage's cells, then its inputs:
+// upstream cells in other stages) lie by value index and step parity; a cell's upstream
+// outflows are listed by value index in neighbour order, the first one in its meta word and the others in
+// `src`, so that a cell step decodes no masks and neighbour offsets.  Per cell `meta`:
+//   x: in-tile cell (bits 0-9) | round (bits 10-19) | number of upstream cells (bits 20-23)
+//   y: the first upstream cell's value index (bits 0-15) | the other ones' first entry in src (bits 16-31)
+// and its history row and state; by round its first position and first input; per input its history row and its cell's round; per
+// producer its
+// position, the earliest round that consumes it and the steps of it known to be in the history.  While the
+// lists are built, the room of the values holds the stage position of each in-tile cell and each cell's first
+// entry.
 template <class R>
 struct FlowLayout {
-    uint8_t* local;
-    uint2* Qs;
     uint2* meta;
     int32_t* ex;
     typename R::Cell* cells;
     uint16_t* rstart;
-    uint2* in_vals;
+    uint16_t* rinput;
     int32_t* in_rows;
-    uint8_t* in_cell;
+    uint16_t* in_round;
     int2* prod;
     int* have;
+    uint16_t* src;
+    uint2* val;
+    uint8_t* local;   // [kStageCells], build
+    uint16_t* first;  // [count], build
     __device__ FlowLayout(unsigned char* base, int count, int nin, int np)
     {
-        local = base;
-        Qs = reinterpret_cast<uint2*>(local + kStageCells);
-        meta = Qs + 2 * count;
-        in_vals = meta + count;
-        ex = reinterpret_cast<int32_t*>(in_vals + nin);
-        in_rows = ex + count;
-        prod = reinterpret_cast<int2*>((reinterpret_cast<uintptr_t>(in_rows + nin) + 7) & ~uintptr_t(7));
-        have = reinterpret_cast<int*>(prod + np);
+        meta = reinterpret_cast<uint2*>(base);
+        prod = reinterpret_cast<int2*>(meta + count);
         // 16-byte aligned: a Cell may hold doubles
-        cells = reinterpret_cast<typename R::Cell*>((reinterpret_cast<uintptr_t>(have + np) + 15) & ~uintptr_t(15));
-        // round up to 4 bytes: a Cell may be a 1-byte empty struct
-        rstart = reinterpret_cast<uint16_t*>((reinterpret_cast<uintptr_t>(cells + count) + 3) & ~uintptr_t(3));
-        in_cell = reinterpret_cast<uint8_t*>(rstart + count + 2);
+        cells = reinterpret_cast<typename R::Cell*>((reinterpret_cast<uintptr_t>(prod + np) + 15) & ~uintptr_t(15));
+        // round up to 8 bytes: a Cell may be a 1-byte empty struct
+        val = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(cells + count) + 7) & ~uintptr_t(7));
+        local = reinterpret_cast<uint8_t*>(val);
+        first = reinterpret_cast<uint16_t*>(local + kStageCells);
+        ex = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(val) + value_bytes(count, nin));
+        in_rows = ex + count;
+        have = in_rows + nin;
+        rstart = reinterpret_cast<uint16_t*>(have + np);
+        rinput = rstart + count + 2;
+        src = rinput + count + 2;
+        in_round = src + count + nin;
+    }
+    static __host__ __device__ size_t value_bytes(size_t count, size_t nin)
+    {
+        const size_t v = 2 * (count + nin) * sizeof(uint2), b = (kStageCells + count * sizeof(uint16_t) + 7) & ~size_t(7);
+        return v > b ? v : b;
     }
 };
 
 template <class R>
 static size_t flow_smem(int64_t cells, int64_t inputs, int64_t producers)
 {
-    return kStageCells + cells * (3 * sizeof(uint2) + sizeof(int32_t) + sizeof(typename R::Cell)) +
-           (cells + 2) * sizeof(uint16_t) + inputs * (sizeof(uint2) + sizeof(int32_t) + 1) +
-           producers * (sizeof(int2) + sizeof(int)) + 32;  // + alignment
+    return cells * (sizeof(uint2) + sizeof(int32_t) + sizeof(typename R::Cell) + sizeof(uint16_t)) +
+           2 * (cells + 2) * sizeof(uint16_t) + FlowLayout<R>::value_bytes(cells, inputs) +
+           inputs * (sizeof(int32_t) + 2 * sizeof(uint16_t)) + producers * (sizeof(int2) + sizeof(int)) +
+           32;  // + alignment
 }
 
 // Waits until every producer has published the steps that round r consumes (round r consumes step
@@ -885,6 +902,15 @@ __device__ __forceinline__ void flow_wait_round(const StageFlowArgs& f, const in
         const int need = min(ns, r - pq.y + 1);
         if (need > have[i]) have[i] = flow_wait(f.progress + pq.x, need, f.error, f.polls);
     }
+}
+
+// The barrier of a stage's CTA; one warp needs no hardware barrier.  Either one orders the threads' memory
+// accesses.
+template <int NT>
+__device__ __forceinline__ void flow_sync()
+{
+    if (NT == 32) __syncwarp();
+    else __syncthreads();
 }
 
 constexpr int kFlowPrefetch = 2;  // inputs per thread loaded one round ahead into registers
@@ -902,7 +928,7 @@ __global__ void __launch_bounds__(NT) k_stage_flow(StageRunArgs a, StageFlowArgs
     __shared__ int s_ticket;
     __shared__ unsigned long long s_wait;  // tracing: time in waits
     if (threadIdx.x == 0) s_ticket = atomicAdd(f.ticket, 1);
-    __syncthreads();
+    flow_sync<NT>();
     const int64_t k = s_ticket;
     if (k >= f.nstages) return;
     if (f.trace && threadIdx.x == 0) {
@@ -933,78 +959,165 @@ __global__ void __launch_bounds__(NT) k_stage_flow(StageRunArgs a, StageFlowArgs
         const int p = (int)(m.x & 1023u);
         L.local[p] = (uint8_t)i;
         const int fi = (int)(m.y >> 16), ne = __popc((m.y >> 8) & 0xFFu);
-        for (int j = 0; j < ne; ++j) L.in_cell[fi + j] = (uint8_t)i;
+        for (int j = 0; j < ne; ++j) L.in_round[fi + j] = (uint16_t)((m.x >> 10) & 1023u);
         rule.load(L.cells[i], (row0 + (p >> 5)) * a.cols + col0 + (p & 31));
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < count; i += NT) {
-        const int rd = (int)((L.meta[i].x >> 10) & 1023u);
-        if (i == 0 || rd != (int)((L.meta[i - 1].x >> 10) & 1023u)) L.rstart[rd] = (uint16_t)i;
+    flow_sync<NT>();
+    if (threadIdx.x < 32) {  // first entries in src
+        int before = 0;
+        for (int i0 = 0; i0 < count; i0 += 32) {
+            const int i = i0 + (int)threadIdx.x;
+            const int n = i < count ? max(0, __popc(L.meta[i].y & 0xFFu) - 1) : 0;
+            int x = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if ((int)threadIdx.x >= o) x += y;
+            }
+            if (i < count) L.first[i] = (uint16_t)(before + x - n);
+            before += __shfl_sync(0xffffffffu, x, 31);
+        }
     }
-    if (threadIdx.x == 0) L.rstart[rounds] = (uint16_t)count;
+    flow_sync<NT>();
+    for (int i = threadIdx.x; i < count; i += NT) {
+        const uint2 m = L.meta[i];
+        const int rd = (int)((m.x >> 10) & 1023u);
+        if (i == 0 || rd != (int)((L.meta[i - 1].x >> 10) & 1023u)) {
+            L.rstart[rd] = (uint16_t)i;
+            L.rinput[rd] = (uint16_t)(m.y >> 16);
+        }
+        const int p = (int)(m.x & 1023u);
+        const unsigned em = (m.y >> 8) & 0xFFu;
+        const int f0 = L.first[i];
+        int n = 0, v0 = 0, in = count + (int)(m.y >> 16);
+        for (unsigned um = m.y & 0xFFu; um; um &= um - 1) {
+            const int q = __ffs(um) - 1;
+            const int v = ((em >> q) & 1u) ? in++ : L.local[p + nb_dr(q) * kStageSide + nb_dc(q)];
+            if (n == 0) v0 = v;
+            else L.src[f0 + n - 1] = (uint16_t)v;
+            ++n;
+        }
+        // the round bits stay as they are: the next position's thread reads them
+        L.meta[i] = make_uint2(m.x | ((unsigned)n << 20), (unsigned)v0 | ((unsigned)f0 << 16));
+    }
+    if (threadIdx.x == 0) {
+        L.rstart[rounds] = (uint16_t)count;
+        L.rinput[rounds] = (uint16_t)nin;
+    }
     const int max_exit = __ldg(f.max_exit_round + k);
     if (f.trace && threadIdx.x == 0) f.trace[4 * k + 1] = global_ns();
     // the inputs of round 0 (ONE: of every round)
     flow_wait_round<NT>(f, L.prod, L.have, np, ns, ONE ? ns + rounds : 0);
     if (k == f.stuck && threadIdx.x == 0) flow_wait(f.progress + k, ns + 1, f.error, f.polls);
-    __syncthreads();
+    flow_sync<NT>();
     if (f.trace && threadIdx.x == 0) s_wait += global_ns() - f.trace[4 * k + 1];
     {
-        const int s_hi = ONE ? nin : (rounds > 1 ? (int)(L.meta[L.rstart[1]].y >> 16) : nin);
-        for (int s = threadIdx.x; s < s_hi; s += NT) L.in_vals[s] = __ldcg(a.hist + (int64_t)L.in_rows[s] * ns);
+        const int s_hi = ONE ? nin : L.rinput[1];
+        for (int s = threadIdx.x; s < s_hi; s += NT)
+            L.val[2 * (count + s)] = __ldcg(a.hist + (int64_t)L.in_rows[s] * ns);  // step 0
     }
-    const int nrounds = rounds + ns - 1;
+    if (ONE && NT == 32) {
+        // One warp, one step: a round is a contiguous range of positions, and the next round's follows it.  The call
+        // lasts as long as its longest chain of rounds, so what a round needs besides its upstream values (range,
+        // meta, cell state, history row and the part of the rule before the upstream sum) is read and computed
+        // during the round before: 0.58 us a round on the critical chain (one kinematic-wave step at 2048^2), 0.90 us
+        // with the loop below.
+        flow_sync<NT>();  // the inputs
+        int hi = L.rstart[1];
+        int i = (int)threadIdx.x;
+        bool act = i < hi;
+        uint2 m = act ? L.meta[i] : make_uint2(0u, 0u);
+        int32_t e = act ? L.ex[i] : -1;
+        typename R::Cell cell{};
+        if (act) cell = L.cells[i];
+        for (int r = 0; r < rounds; ++r) {
+            const int hi2 = r + 2 <= rounds ? L.rstart[r + 2] : hi, i2 = hi + (int)threadIdx.x;
+            const bool act2 = i2 < hi2;
+            uint2 m2 = make_uint2(0u, 0u);
+            int32_t e2 = -1;
+            typename R::Cell cell2{};
+            if (act2) {
+                m2 = L.meta[i2];
+                e2 = L.ex[i2];
+                cell2 = L.cells[i2];
+            }
+            while (act) {
+                const int n = (int)((m.x >> 20) & 15u), p = (int)(m.x & 1023u);
+                const typename R::Pre pre = rule.pre(cell);
+                typename R::Acc acc = rule.begin();
+                if (n > 0) rule.first(acc, L.val[2 * (m.y & 0xFFFFu)]);
+                for (int j = (int)(m.y >> 16), j1 = j + n - 1; j < j1; ++j) rule.add(acc, L.val[2 * L.src[j]]);
+                const uint2 o = rule.step(cell, pre, acc, (row0 + (p >> 5)) * a.cols + col0 + (p & 31), 0);
+                L.val[2 * i] = o;
+                if (e >= 0) __stcg(a.hist + e, o);
+                if (R::kState) L.cells[i] = cell;
+                i += NT;
+                act = i < hi;
+                if (act) {  // a round of more than 32 cells
+                    m = L.meta[i];
+                    e = L.ex[i];
+                    cell = L.cells[i];
+                }
+            }
+            // orders every lane's history writes before lane 0's release, and the values before the next round
+            flow_sync<NT>();
+            if (threadIdx.x == 0 && r == max_exit) st_release(f.progress + k, 1);
+            hi = hi2;
+            i = i2;
+            act = act2;
+            m = m2;
+            e = e2;
+            cell = cell2;
+        }
+    }
+    const int nrounds = ONE && NT == 32 ? 0 : rounds + ns - 1;
     int published = 0;
     for (int r = 0; r < nrounds; ++r) {
         // the inputs of round r + 1: wait, then load into registers
         uint2 pv[kFlowPrefetch];
+        unsigned odd = 0;  // bit j: the parity of pv[j]'s step
         int s_lo = 0, s_hi = 0;
         if (!ONE && r + 1 < nrounds) {
             if (f.trace && threadIdx.x == 0) s_wait -= global_ns();
             flow_wait_round<NT>(f, L.prod, L.have, np, ns, r + 1);
-            __syncthreads();
+            flow_sync<NT>();
             if (f.trace && threadIdx.x == 0) s_wait += global_ns();
-            const int lo = L.rstart[max(0, r + 2 - ns)], hi = L.rstart[min(rounds, r + 2)];
-            s_lo = (int)(L.meta[lo].y >> 16);
-            s_hi = hi < count ? (int)(L.meta[hi].y >> 16) : nin;
+            s_lo = L.rinput[max(0, r + 2 - ns)];
+            s_hi = L.rinput[min(rounds, r + 2)];
 #pragma unroll
             for (int j = 0; j < kFlowPrefetch; ++j) {
                 const int s = s_lo + (int)threadIdx.x + j * NT;
                 if (s < s_hi) {
-                    const int t = r + 1 - (int)((L.meta[L.in_cell[s]].x >> 10) & 1023u);
+                    const int t = r + 1 - (int)L.in_round[s];
+                    odd |= (unsigned)(t & 1) << j;
                     pv[j] = __ldcg(a.hist + (int64_t)L.in_rows[s] * ns + t);
                 }
             }
         } else if (!ONE || r == 0) {
             // one step: the barrier that ends each round orders its outflows before the next round's
             // reads, so only round 0 (after the loads of the inputs) needs one here
-            __syncthreads();
+            flow_sync<NT>();
         }
         const int lo = L.rstart[max(0, r - ns + 1)], hi = L.rstart[min(rounds, r + 1)];
         for (int i = lo + (int)threadIdx.x; i < hi; i += NT) {
             const uint2 m = L.meta[i];
             const int t = r - (int)((m.x >> 10) & 1023u);
             const int p = (int)(m.x & 1023u);
-            const unsigned em = (m.y >> 8) & 0xFFu;
-            const int fi = (int)(m.y >> 16);
-            uint2* Qt = L.Qs + (t & 1) * count;
+            uint2* val = L.val + (t & 1);
+            const int n = (int)((m.x >> 20) & 15u);
+            typename R::Cell& cell = L.cells[i];
+            const typename R::Pre pre = rule.pre(cell);
             typename R::Acc acc = rule.begin();
-            unsigned um = m.y & 0xFFu;
-            while (um) {
-                const int q = __ffs(um) - 1;
-                um &= um - 1;
-                const uint2 v = ((em >> q) & 1u) ? L.in_vals[fi + __popc(em & ((1u << q) - 1u))]
-                                                  : Qt[L.local[p + nb_dr(q) * kStageSide + nb_dc(q)]];
-                rule.add(acc, v);
-            }
-            const uint2 o = rule.step(L.cells[i], acc, (row0 + (p >> 5)) * a.cols + col0 + (p & 31), t);
-            Qt[i] = o;
+            if (n > 0) rule.first(acc, val[2 * (m.y & 0xFFFFu)]);
+            for (int k = (int)(m.y >> 16), k1 = k + n - 1; k < k1; ++k) rule.add(acc, val[2 * L.src[k]]);
+            const uint2 o = rule.step(cell, pre, acc, (row0 + (p >> 5)) * a.cols + col0 + (p & 31), t);
+            val[2 * i] = o;
             const int32_t e = L.ex[i];
             if (e >= 0) __stcg(a.hist + (int64_t)e * ns + t, o);
         }
         // The barrier orders every thread's history writes before thread 0's release, which makes them
         // visible at GPU scope before the progress that announces them (the pattern of a grid barrier).
-        __syncthreads();
+        flow_sync<NT>();
         if (threadIdx.x == 0 && max_exit >= 0) {
             // every publish_every steps (a release fence each time), and the last step
             const int prog = min(ns, max(0, r + 1 - max_exit));
@@ -1017,11 +1130,11 @@ __global__ void __launch_bounds__(NT) k_stage_flow(StageRunArgs a, StageFlowArgs
 #pragma unroll
             for (int j = 0; j < kFlowPrefetch; ++j) {
                 const int s = s_lo + (int)threadIdx.x + j * NT;
-                if (s < s_hi) L.in_vals[s] = pv[j];
+                if (s < s_hi) L.val[2 * (count + s) + ((odd >> j) & 1u)] = pv[j];
             }
             for (int s = s_lo + (int)threadIdx.x + kFlowPrefetch * NT; s < s_hi; s += NT) {
-                const int t = r + 1 - (int)((L.meta[L.in_cell[s]].x >> 10) & 1023u);
-                L.in_vals[s] = __ldcg(a.hist + (int64_t)L.in_rows[s] * ns + t);
+                const int t = r + 1 - (int)L.in_round[s];
+                L.val[2 * (count + s) + (t & 1)] = __ldcg(a.hist + (int64_t)L.in_rows[s] * ns + t);
             }
         }
     }
@@ -1062,6 +1175,10 @@ struct StageF32 {
         cl.x = value_at(a, as, g);
         cl.b = RR == Rule::accu ? 0.0f : value_at(b, bs, g);
     }
+    struct Pre {};  // nothing before the upstream sum
+    static constexpr bool kState = false;
+    __device__ Pre pre(const Cell&) const { return Pre{}; }
+    __device__ void first(Acc& acc, uint2 v) const { add(acc, v); }
     __device__ Acc begin() const { return Acc{FF{0.0f, 0.0f}, false}; }
     __device__ void add(Acc& acc, uint2 v) const
     {
@@ -1069,7 +1186,7 @@ struct StageF32 {
         if (isnan(h)) acc.nan = true;
         else acc.t.add(h, __uint_as_float(v.y));
     }
-    __device__ uint2 step(Cell& cl, const Acc& acc, int64_t g, int) const
+    __device__ uint2 step(Cell& cl, const Pre&, const Acc& acc, int64_t g, int) const
     {
         float oh = 0.0f, ol = 0.0f, r = 0.0f;
         if (!rule_f32<RR>(acc.t, acc.nan, cl.x, cl.b, oh, ol, r)) {
@@ -1107,6 +1224,10 @@ struct StageF64 {
         cl.x = value_at(a, as, g);
         cl.b = RR == Rule::accu ? 0.0 : value_at(b, bs, g);
     }
+    struct Pre {};  // nothing before the upstream sum
+    static constexpr bool kState = false;
+    __device__ Pre pre(const Cell&) const { return Pre{}; }
+    __device__ void first(Acc& acc, uint2 v) const { add(acc, v); }
     __device__ Acc begin() const { return Acc{0.0, false}; }
     __device__ void add(Acc& acc, uint2 v) const
     {
@@ -1114,7 +1235,7 @@ struct StageF64 {
         if (isnan(h)) acc.nan = true;
         else acc.t += h;
     }
-    __device__ uint2 step(Cell& cl, const Acc& acc, int64_t g, int) const
+    __device__ uint2 step(Cell& cl, const Pre&, const Acc& acc, int64_t g, int) const
     {
         double o = 0.0, r = 0.0;
         if (!rule_f64<RR>(acc.t, acc.nan, cl.x, cl.b, o, r)) {
@@ -1150,6 +1271,10 @@ struct StageKW64 {
         cl.be = v.beta ? __ldg(v.beta + c) : v.beta_s;
         cl.len = v.dx ? __ldg(v.dx + c) : v.dx_s;
     }
+    struct Pre {};  // nothing before the upstream sum
+    static constexpr bool kState = false;
+    __device__ Pre pre(const Cell&) const { return Pre{}; }
+    __device__ void first(Acc& acc, uint2 v) const { add(acc, v); }
     __device__ Acc begin() const { return Acc{0.0, false}; }
     __device__ void add(Acc& acc, uint2 x) const
     {
@@ -1157,7 +1282,7 @@ struct StageKW64 {
         if (isnan(h)) acc.nan = true;
         else acc.up += h;
     }
-    __device__ uint2 step(Cell& cl, const Acc& acc, int64_t c, int) const
+    __device__ uint2 step(Cell& cl, const Pre&, const Acc& acc, int64_t c, int) const
     {
         const double o = rule_kw(acc.up, acc.nan, cl.qc, cl.q, cl.al, cl.be, v.dt, cl.len, v.br);
         v.out[c] = o;
@@ -1188,6 +1313,10 @@ struct StageKW32 {
         cl.be = v.beta ? __ldg(v.beta + c) : v.beta_s;
         cl.len = v.dx ? __ldg(v.dx + c) : v.dx_s;
     }
+    struct Pre {};  // nothing before the upstream sum
+    static constexpr bool kState = false;
+    __device__ Pre pre(const Cell&) const { return Pre{}; }
+    __device__ void first(Acc& acc, uint2 v) const { add(acc, v); }
     __device__ Acc begin() const { return Acc{0.0f, false}; }
     __device__ void add(Acc& acc, uint2 x) const
     {
@@ -1195,7 +1324,7 @@ struct StageKW32 {
         if (isnan(h)) acc.nan = true;
         else acc.up += h;
     }
-    __device__ uint2 step(Cell& cl, const Acc& acc, int64_t c, int) const
+    __device__ uint2 step(Cell& cl, const Pre&, const Acc& acc, int64_t c, int) const
     {
         const float o = rule_kw32(acc.up, acc.nan, cl.qc, cl.q, cl.al, cl.be, v.dt, cl.len);
         v.out[c] = o;
@@ -1204,7 +1333,10 @@ struct StageKW32 {
     __device__ void store(Cell&, int64_t) const {}
 };
 
-// kinematic wave, many steps, in float-float and the variable y = Q^(1/m) (kinematic_wave_ff.cuh).
+// kinematic wave, many steps, in float-float and the variable y = Q^(1/m) (kinematic_wave_ff.cuh).  Bound by
+// instruction issue and the latency of dependent instructions (53 % of the issue slots; more warps per SM make no
+// difference, since the stages that could fill them wait for producers).  With the nested solve for beta = 3/5 and
+// the listed upstream values, 100 steps at 8192^2 take 89 ms (before: 130 ms), one step at 2048^2 2.5 ms (5.2 ms).
 template <int P, int M>
 struct StageKWPoly {
     const double* qcur;
@@ -1222,25 +1354,39 @@ struct StageKWPoly {
         float lat, al;
     };
     struct Acc {
-        ffloat up;
-        bool nan;
+        ffloat up;  // hi NaN: no-data upstream
     };
     __device__ void load(Cell& cl, int64_t g) const
     {
         cl.lat = lateral ? __ldg(lateral + g) : lateral_s;
         cl.al = alpha ? __ldg(alpha + g) : alpha_s;
         cl.y = kw_poly_root<P, M>(ff_from_double(__ldg(qcur + g)), K);
+        // an input outside the domain: no-data, in this and every later step
+        if (K.bad || !(cl.lat >= 0.0f) || isnan(cl.al)) cl.y = ffloat{qnan<float>(), 0.0f};
     }
-    __device__ Acc begin() const { return Acc{ffloat{0.0f, 0.0f}, false}; }
+    static constexpr bool kState = true;  // a step changes the cell
+    static constexpr bool k35 = P == 3 && M == 5;
+    using Pre = KWBase35;
+    __device__ Pre pre(const Cell& cl) const
+    {
+        if constexpr (k35) return kw_base_35(cl.y, cl.lat, cl.al, K);
+        else return Pre{};
+    }
+    __device__ Acc begin() const { return Acc{ffloat{0.0f, 0.0f}}; }
+    __device__ void first(Acc& acc, uint2 x) const
+    {
+        acc.up = ffloat{__uint_as_float(x.x), __uint_as_float(x.y)};
+    }
     __device__ void add(Acc& acc, uint2 x) const
     {
-        const ffloat v{__uint_as_float(x.x), __uint_as_float(x.y)};
-        if (isnan(v.hi)) acc.nan = true;
-        else acc.up = ff_add_sloppy(acc.up, v);
+        const ffloat s = ff_two_sum(acc.up.hi, __uint_as_float(x.x));
+        acc.up = ffloat{s.hi, __fadd_rn(__fadd_rn(acc.up.lo, __uint_as_float(x.y)), s.lo)};
     }
-    __device__ uint2 step(Cell& cl, const Acc& acc, int64_t, int) const
+    __device__ uint2 step(Cell& cl, const Pre& pre, const Acc& acc, int64_t, int) const
     {
-        const ffloat q = kw_step_poly<P, M>(acc.up, acc.nan, cl.y, cl.lat, cl.al, K);
+        ffloat q;
+        if constexpr (k35) q = kw_step_35(pre, acc.up, cl.y, cl.lat, cl.al, K);
+        else q = kw_step_poly<P, M>(acc.up, isnan(acc.up.hi), cl.y, cl.lat, cl.al, K);
         return make_uint2(__float_as_uint(q.hi), __float_as_uint(q.lo));
     }
     __device__ void store(Cell& cl, int64_t g) const
@@ -1714,6 +1860,7 @@ static KWConstFF kw_constants(double beta, double dt, double dx, const BetaRatio
     K.k = ff_split(dt / dx);
     K.dt = ff_split(dt);
     K.kf = (float)(dt / dx);
+    K.lg2k = log2f(K.kf);
     K.beta_f = (float)beta;
     K.beta = beta;
     K.dt_d = dt;
