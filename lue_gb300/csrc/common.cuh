@@ -107,6 +107,13 @@ __device__ __forceinline__ T load_cg(const T* p)
 __device__ __forceinline__ int64_t grid_stride_begin() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int64_t grid_stride() { return (int64_t)gridDim.x * blockDim.x; }
 
+// Kernels of one call that follow each other on a stream (launch_after below): the next one starts while this one
+// still runs, once every CTA of this one has said so (or ended), and reads what no earlier kernel of the call
+// writes; it waits for the whole of this one before anything else.  Neither does anything in a kernel launched the
+// ordinary way.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Host side -----------------------------------------------------------------------------------------
 
 void set_error(const std::string& msg);
@@ -114,6 +121,25 @@ void set_error(const std::string& msg);
 void count_launches(int n);
 int fail(int status, const std::string& msg);
 int cuda_status(cudaError_t err, const char* what);
+
+// Launches a kernel that may start before the kernel before it on the stream has ended: it must call
+// wait_for_previous() before it reads what that one (or an earlier one of the call) writes and before its own first
+// write.  Errors are left to cudaGetLastError(), as with <<<>>>.
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
 
 // One thread per element, no grid-stride reuse (walk kernels: a thread that walks a long path must not
 // also own later cells, or the walks chain up behind each other).

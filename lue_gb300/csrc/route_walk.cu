@@ -66,6 +66,8 @@ static int route_f64(lue_gpu_topology* t, const double* a, double as, const doub
 
 __global__ void k_copy_words_if(const uint32_t* src, uint32_t* dst, int64_t nwords, const unsigned long long* flag)
 {
+    next_may_start();
+    wait_for_previous();
     if (flag[1] == 0) return;
     for (int64_t i = grid_stride_begin(); i < nwords; i += grid_stride()) dst[i] = src[i];
 }
@@ -104,16 +106,20 @@ extern "C" int lue_gpu_accu_f32(lue_gpu_topology* t, const float* inflow, float 
     if (!core->tiles || walk_engine_forced())
         return route_f32<Rule::accu>(t, inflow, inflow_scalar, nullptr, 0.0f, outflow, nullptr, stream_, "accu_f32");
     cudaStream_t stream = (cudaStream_t)stream_;
-    if (int rc = tile_accu_f32(core, &t->tile_scratch, inflow, inflow_scalar, outflow, stream)) return rc;
+    const unsigned long long* flag = nullptr;
+    bool reset = false;
+    if (int rc = tile_accu_f32(core, &t->tile_scratch, inflow, inflow_scalar, outflow, t->work_count, stream, &flag,
+                               &reset))
+        return rc;
     // +inf material or a total beyond the fixed-point range: the walk engine redoes the call
     const int64_t n = core->n;
-    const unsigned long long* flag = t->tile_scratch.total;
-    k_copy_words_if<<<grid_for(words_for(n), 256), 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(core->count),
-                                                                     t->work_count, words_for(n), flag);
+    if (!reset)
+        launch_after(k_copy_words_if, grid_for(words_for(n), 256), 256, 0, stream,
+                     reinterpret_cast<const uint32_t*>(core->count), t->work_count, words_for(n), flag);
     WalkGrid g{core->fd, core->count, t->work_count, core->rows, core->cols, n};
     RouteF32<Rule::accu> v{core->upmask, inflow, inflow_scalar, nullptr, 0.0f, outflow, nullptr, t->lo, core->cols};
-    k_walk_if<<<grid_for(n, 256), 256, 0, stream>>>(g, v, flag);
-    count_launches(2);
+    launch_after(k_walk_if<RouteF32<Rule::accu>>, grid_for(n, 256), 256, 0, stream, g, v, flag);
+    count_launches(reset ? 1 : 2);
     return cuda_status(cudaGetLastError(), "accu_f32");
 }
 

@@ -721,7 +721,7 @@ struct __align__(16) TileCallSmem {
     int seg_head[kTileThreads / 32];
     float carry_hi[kTileThreads], carry_lo[kTileThreads];        // pass 1: what each run's first segment carries in
     uint8_t run_first[kTileThreads];                             // pass 1: first segment head of each run (16: none)
-    int quit;                                                    // pass 3: the walk engine redoes the call
+    int quit;                                                    // the CTA leaves; the CTA is the last one
 };
 
 // The thread's run of a per-position table (cell_at or prev_at): eight coalesced 4-byte loads.
@@ -759,8 +759,9 @@ __device__ __forceinline__ bool tile_fallback(const unsigned long long* total)
     return *reinterpret_cast<const volatile unsigned long long*>(total + 1) != 0 || total[0] >= kTotalLimit;
 }
 
-constexpr int kScanItems = 8;
-constexpr int kScanBlock = kTileThreads * kScanItems;
+// Exits per thread of a scan block: 8 (63 registers, four CTAs per SM) where the scan fills the GPU, 2 on small
+// rasters, where fewer exits in a row per thread end the launch sooner.
+constexpr int kScanItems = 8, kScanItemsSmall = 2;
 constexpr int kScanPolls = 1 << 20;  // poll limit of one look-back wait (a second at most)
 
 __device__ __forceinline__ u128 block_exclusive_u128(u128 v, u128* warp_tot, u128& block_total)
@@ -799,7 +800,7 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// The exit forest's 128-bit inclusive scan, one chunk of consecutive scan blocks (kScanBlock exits each)
+// The exit forest's 128-bit inclusive scan, one chunk of consecutive scan blocks (256 x ITEMS exits each)
 // per CTA, with as many CTAs as fit on the GPU at once.  CTAs take chunks in ticket order; each sums its
 // chunk, publishes the sum (flag 1), then warp 0 adds up the sums of the chunks before it, 32 at a time,
 // until it meets a chunk that has published the sum up to and including itself (flag 2); the CTA
@@ -808,15 +809,19 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
 // sums before they wait for anything: no chain of waits forms.  Every wait is bounded: a wait that gives
 // up (or sees that one did) sets total[1] = 2, after which the walk engine redoes the call.
 // ctl = the ticket, then the chunk flags, zeroed before the call.
+template <int ITEMS>
 __global__ void __launch_bounds__(kTileThreads)
     k_scan_exits(const float2* __restrict__ P, int64_t n, int64_t chunk_blocks, unsigned long long* total,
                  unsigned* ctl, uint4* look_aggr, uint4* look_incl, uint4* __restrict__ S, int polls)
 {
+    constexpr int64_t kBlock = kTileThreads * ITEMS;
     __shared__ u128 warp_tot[kTileThreads / 32];
     __shared__ u128 prefix_sh;
     __shared__ unsigned ticket_sh;
     __shared__ int abort_sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    next_may_start();
+    wait_for_previous();
     // one thread decides, so that the whole CTA leaves or stays
     if (threadIdx.x == 0) ticket_sh = tile_fallback(total) ? ~0u : atomicAdd(ctl, 1u);
     __syncthreads();
@@ -824,15 +829,15 @@ __global__ void __launch_bounds__(kTileThreads)
     const int64_t g = ticket_sh;
     unsigned* flag = ctl + 1;
     const int F = fixed_point_bits(total[0]);
-    const int64_t first = g * chunk_blocks * kScanBlock;
-    const int64_t last = min(n, first + chunk_blocks * kScanBlock);
+    const int64_t first = g * chunk_blocks * kBlock;
+    const int64_t last = min(n, first + chunk_blocks * kBlock);
     // the chunk's sum
     u128 s = 0;
-    for (int64_t b0 = first; b0 < last; b0 += kScanBlock) {
-        const int64_t base = b0 + (int64_t)threadIdx.x * kScanItems;
+    for (int64_t b0 = first; b0 < last; b0 += kBlock) {
+        const int64_t base = b0 + (int64_t)threadIdx.x * ITEMS;
 #pragma unroll
-        for (int k = 0; k < kScanItems; ++k)
-            if (base + k < last) s += exit_value_fixed(__ldg(P + base + k), F);
+        for (int k = 0; k < ITEMS; ++k)
+            if (base + k < last) s += exit_value_fixed(__ldcg(P + base + k), F);
     }
     u128 bt;
     block_exclusive_u128(s, warp_tot, bt);
@@ -891,43 +896,50 @@ __global__ void __launch_bounds__(kTileThreads)
     __syncthreads();
     if (abort_sh) return;
     u128 carry = prefix_sh;
-    for (int64_t b0 = first; b0 < last; b0 += kScanBlock) {
-        const int64_t base = b0 + (int64_t)threadIdx.x * kScanItems;
-        u128 v[kScanItems];
+    for (int64_t b0 = first; b0 < last; b0 += kBlock) {
+        const int64_t base = b0 + (int64_t)threadIdx.x * ITEMS;
+        u128 v[ITEMS];
         u128 t = 0;
 #pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            v[k] = base + k < last ? exit_value_fixed(__ldg(P + base + k), F) : (u128)0;
+        for (int k = 0; k < ITEMS; ++k) {
+            v[k] = base + k < last ? exit_value_fixed(__ldcg(P + base + k), F) : (u128)0;
             t += v[k];
         }
         u128 blk;
         u128 run = carry + block_exclusive_u128(t, warp_tot, blk);
         carry += blk;
 #pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
+        for (int k = 0; k < ITEMS; ++k) {
             run += v[k];
             if (base + k < last) S[base + k] = from_u128(run);
         }
     }
 }
 
-// What enters each inflow slot (a border cell receiving flow from other tiles): the exact sum of the subtree
+// What enters an inflow slot (a border cell receiving flow from other tiles): the exact sum of the subtree
 // sums of the exits draining into it (each a difference of two inclusive prefix sums of the exit
 // forest), rounded to float once; NaN when one of them holds a no-data exit.
-__global__ void k_slot_inflow(int64_t nslot, const int32_t* __restrict__ slot_at,
-                              const int32_t* __restrict__ slot_first, const int2* __restrict__ slot_edge,
-                              const uint4* __restrict__ S, float* __restrict__ inflow,
-                              const unsigned long long* total)
+struct TileSlots {
+    const int32_t* base;   // [ntiles + 1] first slot of each tile
+    const int32_t* at;     // tile * kSlotStride + border index
+    const int32_t* first;  // first edge
+    const int2* edge;
+    const uint4* S;        // written by the kernel before: no read-only loads
+};
+__device__ __forceinline__ float slot_inflow(const TileSlots& q, int64_t i, int F)
+{
+    u128 src = 0;
+    for (int32_t k = __ldg(q.first + i), k1 = __ldg(q.first + i + 1); k < k1; ++k) {
+        const int2 e = __ldg(q.edge + k);
+        src += to_u128(__ldcg(q.S + e.x)) - (e.y >= 0 ? to_u128(__ldcg(q.S + e.y)) : (u128)0);
+    }
+    return (src >> 96) ? __int_as_float(0x7fc00000) : fixed128_to_float(src & kValueMask, F);
+}
+__global__ void k_slot_inflow(int64_t nslot, TileSlots q, float* __restrict__ inflow, const unsigned long long* total)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nslot || tile_fallback(total)) return;
-    const int F = fixed_point_bits(total[0]);
-    u128 src = 0;
-    for (int32_t k = __ldg(slot_first + i), k1 = __ldg(slot_first + i + 1); k < k1; ++k) {
-        const int2 e = __ldg(slot_edge + k);
-        src += to_u128(__ldcg(S + e.x)) - (e.y >= 0 ? to_u128(__ldcg(S + e.y)) : (u128)0);
-    }
-    inflow[__ldg(slot_at + i)] = (src >> 96) ? __int_as_float(0x7fc00000) : fixed128_to_float(src & kValueMask, F);
+    inflow[__ldg(q.at + i)] = slot_inflow(q, i, fixed_point_bits(total[0]));
 }
 
 // Build: per tile, its inflow slots and their upstream exits (one thread per tile, border order).
@@ -1093,28 +1105,15 @@ __device__ __forceinline__ SegSum seg_shfl_up(const SegSum& v, int d)
 // segmented prefix sum in float-float (relative error about 2^-35 of the segment's total in the worst
 // case, no cancellation), computed on the float pipes.  A NaN or negative term makes its segment NaN,
 // and with it the exit: no-data flows on from there through the exit forest.
-// vec: material rows can be read as float4 (16-byte aligned, columns a multiple of 4).
-__global__ void __launch_bounds__(kTileThreads, 4)
-    k_tile_exits(TileGeom g, const float* __restrict__ ext, float ext_s, bool vec, TileForest f,
-                 const int32_t* __restrict__ exit_base, const uint32_t* __restrict__ exit_span,
-                 const uint32_t* __restrict__ exit_pos, float2* __restrict__ P,
-                 unsigned long long* total, TileStat* __restrict__ stat)
+//
+// tile_exits: the tile's part of pass 1, from the material (xm) and the cell table (ca) in registers.  On return M
+// holds the material in cell order.  False: the walk engine must redo the call.  units: thread 0's share of
+// total[0] (kTotalLimit or more: out of range).
+__device__ __forceinline__ bool tile_exits(TileCallSmem& sm, const float4 (&xm)[4], const uint32_t (&ca)[kRunWords],
+                                           int ne, uint32_t span, uint32_t epos, float2* __restrict__ P,
+                                           TileStat& st, unsigned long long& units)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TileCallSmem& sm = *reinterpret_cast<TileCallSmem*>(smem_raw);
-    const int64_t tr = blockIdx.y, tc = blockIdx.x;  // grid = (tile columns, tile rows)
-    const int64_t tile = tr * g.tcols + tc;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    float4 xm[4];
-    load_material(xm, ext, ext_s, g, tr, tc, vec);
-    uint32_t ca[kRunWords];
-    load_run(f.cell_at + tile * kRunPositions, ca);
-    const int32_t e0 = __ldg(exit_base + tile), ne = __ldg(exit_base + tile + 1) - e0;
-    uint32_t span = 0, epos = 0;
-    if (t < ne) {  // a tile has at most 252 exits (its border cells)
-        span = __ldg(exit_span + e0 + t);
-        epos = __ldg(exit_pos + e0 + t);
-    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sm.M + quad_cell(j)) = xm[j];
     __syncthreads();
@@ -1201,10 +1200,8 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     const float bound = tile_bound(mx, 0u);
     const int F = tile_scale(bound);
     if (mx >= 0x7F800000u || !(bound < 1.0e38f) ||
-        (mn != 0xFFFFFFFFu && __uint_as_float(mn + 1u) * pow2f(F) < kMinQuantum)) {
-        if (t == 0) atomicOr(total + 1, 1ull);
-        return;  // uniform: every thread has the same reductions
-    }
+        (mn != 0xFFFFFFFFu && __uint_as_float(mn + 1u) * pow2f(F) < kMinQuantum))
+        return false;  // uniform: every thread has the same reductions
     __syncthreads();
     if (t < ne) {
         // the exit's position is the end of its segment; a segment that starts in an earlier run also
@@ -1219,14 +1216,109 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         P[epos] = isnan(h) ? make_float2(__int_as_float(0x7fc00000), 0.0f) : make_float2(h, __fsub_rn(lo, __fsub_rn(h, hi)));
     }
     if (t == 0) {
-        const double units = ldexp((double)sum * (1.0 + 1.0 / 1024.0) + ldexp(1.0, -100), 16) + 64.0;
-        if (units < (double)kTotalLimit) {
-            const unsigned long long u = (unsigned long long)units;
-            if (atomicAdd(total, u) + u < u) atomicOr(total + 1, 1ull);  // the sum wrapped
-        } else {
-            atomicOr(total + 1, 1ull);
+        const double u = ldexp((double)sum * (1.0 + 1.0 / 1024.0) + ldexp(1.0, -100), 16) + 64.0;
+        units = u < (double)kTotalLimit ? (unsigned long long)u : kTotalLimit;
+    }
+    st = TileStat{bound, mn, raw > 0x7F800000u ? 1u : 0u, 0u};
+    return true;
+}
+
+// Small rasters (kSmallTiles): a call is bound by its launches, so work that would be a launch of its own, after
+// all CTAs of a pass, is done by the CTA that finishes it last (an atomic counter; no CTA waits for another).
+struct TileTail {
+    int64_t ntiles, nexit;
+    unsigned* done;               // [2] finished CTAs of pass 1 and of pass 3
+    uint4* S;                     // pass 1: the exit forest's prefix sums, or null (k_scan_exits computes them)
+    unsigned long long* redo;     // pass 3: redo[1] = the walk engine must redo the call
+    const uint32_t* count;        // pass 3: inflow counts to reset the walk's counters with when it must
+    uint32_t* work;
+    int64_t nwords;
+    unsigned* ctl;                // pass 3: all of the call's control words, left at 0 for the next call
+    int64_t nctl;
+};
+
+// Whether the CTA is the last of the launch to get here; everything the others wrote before is then visible.  Ends
+// with a block barrier.
+__device__ __forceinline__ bool last_cta(int& flag, unsigned* done, int64_t n)
+{
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) flag = atomicAdd(done, 1u) == (unsigned)(n - 1);
+    __syncthreads();
+    const bool last = flag;
+    if (last) __threadfence();
+    __syncthreads();
+    return last;
+}
+
+// Most exits whose scan one CTA does within pass 1's launch: 16 per thread, about 3 us (a launch of its own takes 5
+// us and more).
+constexpr int64_t kTailExits = 4096;
+
+__device__ __forceinline__ void tail_scan(const float2* P, int64_t n, const unsigned long long* total, uint4* S)
+{
+    constexpr int64_t kBlock = kTileThreads * kScanItems;
+    __shared__ u128 warp_tot[kTileThreads / 32];
+    const int F = fixed_point_bits(*reinterpret_cast<const volatile unsigned long long*>(total));
+    u128 carry = 0;
+    for (int64_t b0 = 0; b0 < n; b0 += kBlock) {
+        const int64_t base = b0 + (int64_t)threadIdx.x * kScanItems;
+        u128 v[kScanItems], t = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = base + k < n ? exit_value_fixed(__ldcg(P + base + k), F) : (u128)0;
+            t += v[k];
         }
-        stat[tile] = TileStat{bound, mn, raw > 0x7F800000u ? 1u : 0u, 0u};
+        u128 blk;
+        u128 run = carry + block_exclusive_u128(t, warp_tot, blk);
+        carry += blk;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            run += v[k];
+            if (base + k < n) S[base + k] = from_u128(run);
+        }
+    }
+}
+
+// vec: material rows can be read as float4 (16-byte aligned, columns a multiple of 4).
+template <bool SMALL>
+__global__ void __launch_bounds__(kTileThreads, 4)
+    k_tile_exits(TileGeom g, const float* __restrict__ ext, float ext_s, bool vec, TileForest f,
+                 const int32_t* __restrict__ exit_base, const uint32_t* __restrict__ exit_span,
+                 const uint32_t* __restrict__ exit_pos, float2* P, unsigned long long* total,
+                 TileStat* __restrict__ stat, TileTail q)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TileCallSmem& sm = *reinterpret_cast<TileCallSmem*>(smem_raw);
+    const int64_t tr = blockIdx.y, tc = blockIdx.x;  // grid = (tile columns, tile rows)
+    const int64_t tile = tr * g.tcols + tc;
+    const int t = threadIdx.x;
+    if (SMALL) next_may_start();
+    float4 xm[4];
+    load_material(xm, ext, ext_s, g, tr, tc, vec);
+    uint32_t ca[kRunWords];
+    load_run(f.cell_at + tile * kRunPositions, ca);
+    const int32_t e0 = __ldg(exit_base + tile), ne = __ldg(exit_base + tile + 1) - e0;
+    uint32_t span = 0, epos = 0;
+    if (t < ne) {  // a tile has at most 252 exits (its border cells)
+        span = __ldg(exit_span + e0 + t);
+        epos = __ldg(exit_pos + e0 + t);
+    }
+    TileStat st{};
+    unsigned long long units = 0;
+    if (!tile_exits(sm, xm, ca, ne, span, epos, P, st, units)) {
+        if (t == 0) atomicOr(total + 1, 1ull);
+    } else if (t == 0) {
+        // the sum may wrap
+        if (units >= kTotalLimit || atomicAdd(total, units) + units < units) atomicOr(total + 1, 1ull);
+        stat[tile] = st;
+    }
+    if (SMALL && q.S && last_cta(sm.quit, q.done, q.ntiles)) {
+        if (t == 0)  // total[0] has changed during this launch
+            sm.quit = tile_fallback(total) ||
+                      *reinterpret_cast<const volatile unsigned long long*>(total) >= kTotalLimit;
+        __syncthreads();
+        if (!sm.quit) tail_scan(P, q.nexit, total, q.S);
     }
 }
 
@@ -1241,35 +1333,12 @@ __global__ void __launch_bounds__(kTileThreads, 4)
 // cells its prefix minus the prefix before its subtree; a cell without in-tile upstream cells keeps its
 // material (plus what enters) in M, which is its result.  Slow path: NaN / negative terms count as 0 and
 // are counted along the post-order; a cell whose subtree holds one is NaN.
-__global__ void __launch_bounds__(kTileThreads, 4)
-    k_tile_accu(TileGeom g, const float* __restrict__ ext, float ext_s, bool vec, float* __restrict__ out,
-                TileForest f, const TileStat* __restrict__ stat, unsigned long long* total)
+//
+// tile_enter: the warps' statistics of what enters (before a block barrier); tile_result: the rest, from M (the
+// material in cell order) and the tables in registers.  False: the walk engine must redo the call.
+__device__ __forceinline__ void tile_enter(TileCallSmem& sm, float entering)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TileCallSmem& sm = *reinterpret_cast<TileCallSmem*>(smem_raw);
-    const int64_t tr = blockIdx.y, tc = blockIdx.x;  // grid = (tile columns, tile rows)
-    const int64_t tile = tr * g.tcols + tc;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t == 0) {  // one thread decides (other CTAs may set the flag meanwhile), read after the barrier below
-        const bool fb = tile_fallback(total);
-        if (fb && *reinterpret_cast<volatile unsigned long long*>(total + 1) == 0) total[1] = 1ull;
-        sm.quit = fb;
-    }
-    float4 xm[4];
-    load_material(xm, ext, ext_s, g, tr, tc, vec);
-    uint32_t ca[kRunWords], pv[kRunWords];
-    load_run(f.cell_at + tile * kRunPositions, ca);
-    load_run(f.prev_at + tile * kRunPositions, pv);
-    const TileStat st = stat[tile];
-    // what enters through border cell t (0 where nothing does; NaN when no-data enters)
-    float entering = 0.0f;
-    int ecell = -1;
-    if (t < kBorderCells) {
-        entering = __ldg(f.inflow + tile * kSlotStride + t);
-        int rin, cin;
-        border_cell(t, rin, cin);
-        ecell = rin * kTile + cin;
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // over what enters: NaN anywhere, the float sum, and the smallest positive bits minus one
     const bool enan = isnan(entering);
     const float eclean = enan ? 0.0f : entering;
@@ -1283,10 +1352,28 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         sm.red[0][warp] = emn;
         sm.red[1][warp] = enan_any;
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sm.M + quad_cell(j)) = xm[j];
-    __syncthreads();
-    if (sm.quit) return;  // uniform
+}
+
+__device__ __forceinline__ TileStat tile_stat(const TileStat* stat, int64_t tile)
+{
+    const uint4 w = __ldcg(reinterpret_cast<const uint4*>(stat) + tile);  // written by the launch before
+    return TileStat{__uint_as_float(w.x), w.y, w.z, w.w};
+}
+
+// One thread decides whether the CTA leaves (other CTAs may set the flag meanwhile); read after a block barrier.
+__device__ __forceinline__ void tile_decide(TileCallSmem& sm, unsigned long long* total)
+{
+    const bool fb = tile_fallback(total);
+    if (fb && *reinterpret_cast<volatile unsigned long long*>(total + 1) == 0) total[1] = 1ull;
+    sm.quit = fb;
+}
+
+__device__ __forceinline__ bool tile_result(TileCallSmem& sm, const TileGeom& g, int64_t tr, int64_t tc, bool vec,
+                                            float* __restrict__ out, const uint32_t (&ca)[kRunWords],
+                                            const uint32_t (&pv)[kRunWords], const TileStat& st, float entering,
+                                            int ecell)
+{
+    const int t = threadIdx.x;
     if (ecell >= 0) {  // material out of the domain stays visible as NaN (the cell and all below are NaN)
         const float mat = sm.M[ecell];
         sm.M[ecell] = mat >= 0.0f ? mat + entering : __int_as_float(0x7fc00000);
@@ -1303,10 +1390,8 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     const unsigned nan_in = n0.x | n0.y | n0.z | n0.w | n1.x | n1.y | n1.z | n1.w;
     const float bound = (st.bound + in_total) * 1.0009765625f;
     const int F = tile_scale(bound);
-    if (!(bound < 1.0e38f) || (mn != 0xFFFFFFFFu && __uint_as_float(mn + 1u) * pow2f(F) < kMinQuantum)) {
-        if (t == 0) total[1] = 1ull;  // the walk engine redoes the call
-        return;                       // uniform
-    }
+    if (!(bound < 1.0e38f) || (mn != 0xFFFFFFFFu && __uint_as_float(mn + 1u) * pow2f(F) < kMinQuantum))
+        return false;  // uniform
     const bool exact = mn == 0xFFFFFFFFu || __uint_as_float(mn + 1u) * pow2f(F) >= 8388608.0f;
     const bool clean = !st.bad && !nan_in;  // uniform
     __syncthreads();  // M holds what enters
@@ -1381,6 +1466,72 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         const int cell = quad_cell(j);
         store_quad(out, g, tr * kTile + (cell >> 6), tc * kTile + (cell & 63), vec,
                    *reinterpret_cast<const float4*>(sm.M + cell));
+    }
+    return true;
+}
+
+// SMALL: what enters comes from the tile's slots, computed here, instead of from the array that k_slot_inflow fills (one
+// launch less; on a large raster that array is faster: accu at 16384^2 1.65 ms, 1.75 ms without it), and the kernel's
+// loads begin before the kernel before it has ended.  Three CTAs per SM, since the registers for that would spill.
+template <bool SMALL>
+__global__ void __launch_bounds__(kTileThreads, SMALL ? 3 : 4)
+    k_tile_accu(TileGeom g, const float* __restrict__ ext, float ext_s, bool vec, float* __restrict__ out,
+                TileForest f, const TileStat* __restrict__ stat, unsigned long long* total, TileSlots slots, TileTail q)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TileCallSmem& sm = *reinterpret_cast<TileCallSmem*>(smem_raw);
+    const int64_t tr = blockIdx.y, tc = blockIdx.x;  // grid = (tile columns, tile rows)
+    const int64_t tile = tr * g.tcols + tc;
+    const int t = threadIdx.x;
+    if (SMALL) next_may_start();
+    if (!SMALL && t == 0) tile_decide(sm, total);
+    float4 xm[4];
+    load_material(xm, ext, ext_s, g, tr, tc, vec);
+    uint32_t ca[kRunWords], pv[kRunWords];
+    load_run(f.cell_at + tile * kRunPositions, ca);
+    load_run(f.prev_at + tile * kRunPositions, pv);
+    if (SMALL) {
+        wait_for_previous();
+        if (t == 0) tile_decide(sm, total);
+    }
+    const TileStat st = SMALL ? tile_stat(stat, tile) : stat[tile];
+    // what enters through border cell t (0 where nothing does; NaN when no-data enters)
+    float entering = 0.0f;
+    int ecell = -1;
+    if (t < kBorderCells) {
+        int rin, cin;
+        border_cell(t, rin, cin);
+        ecell = rin * kTile + cin;
+    }
+    if (SMALL) {
+        float* enter = sm.carry_hi;  // pass 1's
+        enter[t] = 0.0f;
+        const int32_t s0 = __ldg(slots.base + tile), ns = __ldg(slots.base + tile + 1) - s0;
+        __syncthreads();
+        if (t < ns && !sm.quit)
+            enter[__ldg(slots.at + s0 + t) - (int)(tile * kSlotStride)] =
+                slot_inflow(slots, s0 + t, fixed_point_bits(total[0]));
+        __syncthreads();
+        if (t < kBorderCells) entering = enter[t];
+    } else if (t < kBorderCells) {
+        entering = __ldg(f.inflow + tile * kSlotStride + t);
+    }
+    tile_enter(sm, entering);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sm.M + quad_cell(j)) = xm[j];
+    __syncthreads();
+    if (!sm.quit) {  // uniform
+        if (!tile_result(sm, g, tr, tc, vec, out, ca, pv, st, entering, ecell) && t == 0) total[1] = 1ull;
+    }
+    if (SMALL && last_cta(sm.quit, q.done + 1, q.ntiles)) {
+        if (t == 0) {
+            sm.quit = tile_fallback(total);
+            q.redo[1] = sm.quit;
+        }
+        __syncthreads();
+        if (sm.quit)
+            for (int64_t i = t; i < q.nwords; i += kTileThreads) q.work[i] = q.count[i];
+        for (int64_t i = t; i < q.nctl; i += kTileThreads) q.ctl[i] = 0u;
     }
 }
 
@@ -1543,14 +1694,16 @@ int tile_core_build(TopologyCore* core, cudaStream_t stream)
         sbase[nt] = (int32_t)a;
         ebase[nt] = (int32_t)b;
         tc->nslot = a;
-        TRY(cudaMemcpyAsync(sc, sbase.data(), nt * sizeof(int32_t), cudaMemcpyHostToDevice, stream), "slot base");
         TRY(cudaMemcpyAsync(ec, ebase.data(), nt * sizeof(int32_t), cudaMemcpyHostToDevice, stream), "slot base");
+        TRY(cudaMalloc(&tc->slot_base, (nt + 1) * sizeof(int32_t)), "slot base");
+        TRY(cudaMemcpyAsync(tc->slot_base, sbase.data(), (nt + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, stream),
+            "slot base");
         TRY(cudaMalloc(&tc->slot_at, std::max<int64_t>(a, 1) * sizeof(int32_t)), "slots");
         TRY(cudaMalloc(&tc->slot_first, (a + 1) * sizeof(int32_t)), "slots");
         TRY(cudaMalloc(&tc->slot_edge, std::max<int64_t>(b, 1) * sizeof(int2)), "slots");
         TRY(cudaMemcpyAsync(tc->slot_first + a, &ebase[nt], sizeof(int32_t), cudaMemcpyHostToDevice, stream),
             "slot end");
-        k_slot_fill<<<blocks_for(nt, 256), 256, 0, stream>>>(nt, tc->border_in, tc->halo_exit, sc, ec,
+        k_slot_fill<<<blocks_for(nt, 256), 256, 0, stream>>>(nt, tc->border_in, tc->halo_exit, tc->slot_base, ec,
                                                              tc->exit_pos, tc->exit_start, tc->slot_at,
                                                              tc->slot_first, tc->slot_edge, flag);
         TRY(cudaGetLastError(), "slot fill");
@@ -1560,7 +1713,7 @@ int tile_core_build(TopologyCore* core, cudaStream_t stream)
             rc = fail(LUE_GPU_EINVAL, "tile topology: an inflow without an upstream exit");
             goto error;
         }
-        tc->bytes += a * 8 + 4 + b * 8;
+        tc->bytes += a * 8 + 4 + b * 8 + (nt + 1) * 4;
     }
     cudaFree(sc);
     cudaFree(ec);
@@ -1618,6 +1771,7 @@ void tile_core_free(TileCore* tc)
     cudaFree(tc->prev_at);
     cudaFree(tc->exit_span);
     cudaFree(tc->border_in);
+    cudaFree(tc->slot_base);
     cudaFree(tc->slot_at);
     cudaFree(tc->slot_first);
     cudaFree(tc->slot_edge);
@@ -1627,7 +1781,7 @@ void tile_core_free(TileCore* tc)
 int tile_scratch_alloc(const TileCore* tc, TileScratch* s)
 {
     const int64_t E = std::max<int64_t>(tc->nexit, 1);
-    const int64_t nb = (E + kScanBlock - 1) / kScanBlock;
+    const int64_t nb = (E + kTileThreads * kScanItemsSmall - 1) / (kTileThreads * kScanItemsSmall);
     int rc = 0;
     if ((rc = cuda_status(cudaMalloc(&s->P, E * sizeof(float2)), "tile scratch"))) return rc;
     if ((rc = cuda_status(cudaMalloc(&s->S, E * sizeof(uint4)), "tile scratch"))) return rc;
@@ -1638,10 +1792,11 @@ int tile_scratch_alloc(const TileCore* tc, TileScratch* s)
         return rc;
     if ((rc = cuda_status(cudaMalloc(&s->look_aggr, nb * sizeof(uint4)), "tile scratch"))) return rc;
     if ((rc = cuda_status(cudaMalloc(&s->look_incl, nb * sizeof(uint4)), "tile scratch"))) return rc;
-    // total[2], the scan's ticket, its block flags
-    s->ctl_bytes = 2 * sizeof(unsigned long long) + (1 + nb) * sizeof(unsigned);
+    // total[2], the finished CTAs of the passes, the scan's ticket, its block flags
+    s->ctl_bytes = 2 * sizeof(unsigned long long) + (3 + nb) * sizeof(unsigned);
     if ((rc = cuda_status(cudaMalloc(&s->total, s->ctl_bytes), "tile scratch"))) return rc;
     if ((rc = cuda_status(cudaMemset(s->total, 0, s->ctl_bytes), "tile scratch"))) return rc;
+    if ((rc = cuda_status(cudaMalloc(&s->redo, 2 * sizeof(unsigned long long)), "tile scratch"))) return rc;
     if ((rc = cuda_status(cudaMalloc(&s->stat, tc->ntiles * sizeof(TileStat)), "tile scratch"))) return rc;
     s->bytes = E * (8 + 16) + nb * 32 + s->ctl_bytes + tc->ntiles * (sizeof(TileStat) + kSlotStride * 4);
     return LUE_GPU_OK;
@@ -1655,6 +1810,7 @@ void tile_scratch_free(TileScratch* s)
     cudaFree(s->look_aggr);
     cudaFree(s->look_incl);
     cudaFree(s->total);
+    cudaFree(s->redo);
     cudaFree(s->stat);
     *s = TileScratch{};
 }
@@ -1667,7 +1823,7 @@ static int64_t scan_ctas()
         int dev = 0, sms = 0, per_sm = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_exits, kTileThreads, 0) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_exits<kScanItems>, kTileThreads, 0) != cudaSuccess ||
             sms <= 0 || per_sm <= 0) {
             cudaGetLastError();
             return (int64_t)152;
@@ -1677,11 +1833,26 @@ static int64_t scan_ctas()
     return n;
 }
 
-// accu (float32) on the tile engine.  Returns LUE_GPU_OK with `fallback` set on the device when the
-// material holds +inf or its total is beyond the fixed-point range; the caller then runs the walk
-// engine, guarded by that flag.
-int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, float ext_s, float* out,
-                  cudaStream_t stream)
+// Rasters of up to this many tiles (2048 x 2048 cells) are bound by their launches and the latency of each: three or
+// four launches that overlap take 22, 32 and 56 us a call at 256^2, 1024^2 and 2048^2, seven in turn 37, 46 and 63 us;
+// at 2800^2 they take 101 us against 92 us.
+constexpr int64_t kSmallTiles = 1024;
+
+template <bool SMALL>
+static bool tile_smem_ok()
+{
+    static const bool ok = cudaFuncSetAttribute(k_tile_exits<SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)sizeof(TileCallSmem)) == cudaSuccess &&
+                           cudaFuncSetAttribute(k_tile_accu<SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)sizeof(TileCallSmem)) == cudaSuccess;
+    return ok;
+}
+
+// accu (float32) on the tile engine.  Returns LUE_GPU_OK with (*redo)[1] set on the device when the material holds
+// +inf or its total is beyond the fixed-point range; the caller then runs the walk engine, guarded by that flag,
+// with its counters in `work` (reset here when *reset is true on return, else the caller resets them).
+int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, float ext_s, float* out, uint32_t* work,
+                  cudaStream_t stream, const unsigned long long** redo, bool* reset)
 {
     const TileCore* tc = core->tiles;
     TileGeom g{core->rows, core->cols, tc->trows, tc->tcols};
@@ -1690,38 +1861,59 @@ int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, fl
     const bool cols4 = (core->cols & 3) == 0;
     const bool vec_in = cols4 && (!ext || (reinterpret_cast<uintptr_t>(ext) & 15) == 0);
     const bool vec_out = cols4 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    static const bool smem_ok = cudaFuncSetAttribute(k_tile_exits, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)sizeof(TileCallSmem)) == cudaSuccess &&
-                                cudaFuncSetAttribute(k_tile_accu, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)sizeof(TileCallSmem)) == cudaSuccess;
-    if (!smem_ok) return fail(LUE_GPU_ECUDA, "accu_f32 (tiles): shared memory attribute");
+    const bool small = tc->ntiles <= kSmallTiles;
+    if (!(small ? tile_smem_ok<true>() : tile_smem_ok<false>()))
+        return fail(LUE_GPU_ECUDA, "accu_f32 (tiles): shared memory attribute");
     const dim3 tile_grid((unsigned)tc->tcols, (unsigned)tc->trows);
-    if (int rc = cuda_status(cudaMemsetAsync(s->total, 0, s->ctl_bytes, stream), "accu_f32 (tiles)")) return rc;
-    k_tile_exits<<<tile_grid, kTileThreads, sizeof(TileCallSmem), stream>>>(g, ext, ext_s, vec_in, f, tc->exit_base,
-                                                                            tc->exit_span, tc->exit_pos, s->P,
-                                                                            s->total, s->stat);
-    count_launches(1);
     const int64_t E = tc->nexit;
-    if (E > 0) {
-        const int64_t nb = (E + kScanBlock - 1) / kScanBlock;
+    unsigned* done = reinterpret_cast<unsigned*>(s->total + 2);
+    const bool tail = small && E <= kTailExits;
+    const TileTail q{tc->ntiles, E, done, tail && E > 0 ? s->S : nullptr, s->redo,
+                     reinterpret_cast<const uint32_t*>(core->count), work, words_for(core->n),
+                     reinterpret_cast<unsigned*>(s->total), s->ctl_bytes / 4};
+    const TileSlots slots{tc->slot_base, tc->slot_at, tc->slot_first, tc->slot_edge, s->S};
+    *redo = small ? s->redo : s->total;
+    *reset = small;
+    // a small call leaves its control words at 0
+    if (!small)
+        if (int rc = cuda_status(cudaMemsetAsync(s->total, 0, s->ctl_bytes, stream), "accu_f32 (tiles)")) return rc;
+    constexpr size_t smem = sizeof(TileCallSmem);
+    if (small)
+        k_tile_exits<true><<<tile_grid, kTileThreads, smem, stream>>>(g, ext, ext_s, vec_in, f, tc->exit_base,
+                                                                      tc->exit_span, tc->exit_pos, s->P, s->total,
+                                                                      s->stat, q);
+    else
+        k_tile_exits<false><<<tile_grid, kTileThreads, smem, stream>>>(g, ext, ext_s, vec_in, f, tc->exit_base,
+                                                                       tc->exit_span, tc->exit_pos, s->P, s->total,
+                                                                       s->stat, q);
+    count_launches(1);
+    if (E > 0 && !tail) {
+        const int64_t block = kTileThreads * (small ? kScanItemsSmall : kScanItems);
+        const int64_t nb = (E + block - 1) / block;
         const int64_t chunk_blocks = (nb + scan_ctas() - 1) / scan_ctas();
         const int64_t nchunk = (nb + chunk_blocks - 1) / chunk_blocks;
-        unsigned* ctl = reinterpret_cast<unsigned*>(s->total + 2);
         // test hook: LUE_GB300_TILE_POLLS (poll limit of a look-back wait; 0: every wait gives up at once,
         // and the walk engine redoes the call)
         int polls = kScanPolls;
         if (const char* e = getenv("LUE_GB300_TILE_POLLS")) polls = std::max(0, atoi(e));
-        k_scan_exits<<<(unsigned)nchunk, kTileThreads, 0, stream>>>(s->P, E, chunk_blocks, s->total, ctl,
-                                                                    s->look_aggr, s->look_incl, s->S, polls);
+        if (small)
+            launch_after(k_scan_exits<kScanItemsSmall>, (unsigned)nchunk, kTileThreads, 0, stream, s->P, E, chunk_blocks,
+                         s->total, done + 2, s->look_aggr, s->look_incl, s->S, polls);
+        else
+            k_scan_exits<kScanItems><<<(unsigned)nchunk, kTileThreads, 0, stream>>>(
+                s->P, E, chunk_blocks, s->total, done + 2, s->look_aggr, s->look_incl, s->S, polls);
         count_launches(1);
-        if (tc->nslot > 0) {
-            k_slot_inflow<<<blocks_for(tc->nslot, 256), 256, 0, stream>>>(tc->nslot, tc->slot_at, tc->slot_first,
-                                                                          tc->slot_edge, s->S, s->inflow, s->total);
+        if (!small && tc->nslot > 0) {
+            k_slot_inflow<<<blocks_for(tc->nslot, 256), 256, 0, stream>>>(tc->nslot, slots, s->inflow, s->total);
             count_launches(1);
         }
     }
-    k_tile_accu<<<tile_grid, kTileThreads, sizeof(TileCallSmem), stream>>>(g, ext, ext_s, vec_in && vec_out, out, f,
-                                                                           s->stat, s->total);
+    if (small)
+        launch_after(k_tile_accu<true>, tile_grid, kTileThreads, smem, stream, g, ext, ext_s, vec_in && vec_out, out, f,
+                     s->stat, s->total, slots, q);
+    else
+        k_tile_accu<false><<<tile_grid, kTileThreads, smem, stream>>>(g, ext, ext_s, vec_in && vec_out, out, f, s->stat,
+                                                                      s->total, slots, q);
     count_launches(1);
     return cuda_status(cudaGetLastError(), "accu_f32 (tiles)");
 }

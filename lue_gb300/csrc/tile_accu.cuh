@@ -18,6 +18,8 @@
 //      sums of the exits draining into it, rounded to float once.
 //   4. k_tile_accu: one CTA per tile adds to each border cell what enters it, takes the same prefix sum
 //      over the tile's post-order and writes every cell's result.
+// On small rasters, where launches and their latency bound a call, the last CTA of pass 1 computes the prefix sums (up to
+// 4096 exits; more: k_scan_exits), pass 3 computes what enters its tile itself, and the launches overlap.
 // Pass 1 reads the material and 2 bytes of post-order table per cell; pass 3 the material and 4 bytes of
 // tables, and writes the result.  The prefix sums stay in registers and shared memory.
 // Reference counterpart: the per-partition intra/inter split of ALG/definition/accumulating_router.hpp
@@ -84,6 +86,7 @@ struct TileCore {
     uint8_t* border_in = nullptr;              // [ntiles * kBorderCells] per border cell: outside neighbours draining in
     // Inflow slots (border cells that receive flow from other tiles), per tile in border order:
     int64_t nslot = 0;
+    int32_t* slot_base = nullptr;              // [ntiles + 1] first slot of each tile
     int32_t* slot_at = nullptr;                // [nslot] tile * kSlotStride + border index
     int32_t* slot_first = nullptr;             // [nslot + 1] first of the slot's upstream exits in slot_edge
     int2* slot_edge = nullptr;                 // [slot_first[nslot]] per exit draining into the slot: its
@@ -110,9 +113,11 @@ struct TileScratch {
     uint4* look_aggr = nullptr;                // [scan blocks] each block's sum (decoupled look-back)
     uint4* look_incl = nullptr;                // [scan blocks] the sum up to and including the block
     // Zeroed before each call, in one memset of ctl_bytes: total[0] = bound of the material total
-    // (2^-16 units, summed by pass 1), total[1] = fallback flag, then the scan's ticket and block flags.
+    // (2^-16 units, summed by pass 1), total[1] = fallback flag, then the finished CTAs of pass 1 and pass 3 (small
+    // rasters, whose calls leave all of it at 0 themselves), the scan's ticket and block flags.
     unsigned long long* total = nullptr;
     int64_t ctl_bytes = 0;
+    unsigned long long* redo = nullptr;        // [2] small rasters: redo[1] set when the walk engine must redo the call
     TileStat* stat = nullptr;                  // [ntiles]
     int64_t bytes = 0;
 };

@@ -76,8 +76,8 @@ inline PartitionGeom partition_geom(const TopologyCore* core)
 }
 
 // accu (float32) on the tile engine; see tile_accu.cuh.
-int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, float ext_s, float* out,
-                  cudaStream_t stream);
+int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, float ext_s, float* out, uint32_t* work,
+                  cudaStream_t stream, const unsigned long long** redo, bool* reset);
 
 // Launch of the walk engine: one thread per cell; cells without inflow start a downstream walk that
 // continues through a cell once all its upstream neighbours are done (definition/accumulating_router.hpp:

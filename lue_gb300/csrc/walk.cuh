@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(256) k_walk(WalkGrid g, Visitor v)
 template <class Visitor>
 __global__ void __launch_bounds__(256) k_walk_if(WalkGrid g, Visitor v, const unsigned long long* flag)
 {
+    wait_for_previous();
     if (flag[1] == 0) return;
     for (int64_t c = grid_stride_begin(); c < g.n; c += grid_stride()) {
         uint8_t code = __ldg(g.fd + c);
