@@ -1031,6 +1031,15 @@ struct Chunk {
     unsigned nan;            // bit j: no-data from the cell itself or its light inflow
     T e[PER], b[PER];
     typename N::V sum[PER];
+    // the positions' first slots, read with the inputs; with four positions their registers would spill
+    static constexpr bool kEarly = LIGHT && PER == 1;
+    int32_t f[kEarly ? PER + 1 : 1];
+
+    __device__ __forceinline__ int32_t first_slot(const PathCall<N>& p, int32_t first, int j) const
+    {
+        const bool used = ((on >> (j < PER ? j : PER - 1)) & 1u) || (j > 0 && ((on >> (j - 1)) & 1u));
+        return used ? __ldg(p.slot_first + first + j) : 0;
+    }
 
     // VEC: `first` is a multiple of PER and the order array is read with vector loads.
     template <bool VEC>
@@ -1047,8 +1056,12 @@ struct Chunk {
         }
     }
 
-    __device__ __forceinline__ void gather(const PathCall<N>& p)
+    __device__ __forceinline__ void gather(const PathCall<N>& p, int32_t first)
     {
+        if constexpr (kEarly) {
+#pragma unroll
+            for (int j = 0; j <= PER; ++j) f[j] = first_slot(p, first, j);
+        }
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             const int32_t c = w[j] & 0x7fffffff;
@@ -1066,18 +1079,18 @@ struct Chunk {
     {
         nan = 0;
         if (LIGHT) {
-            int32_t f[PER + 1];
+            int32_t at[PER + 1];
 #pragma unroll
-            for (int j = 0; j <= PER; ++j)
-                f[j] = ((on >> (j < PER ? j : PER - 1)) & 1u) || (j > 0 && ((on >> (j - 1)) & 1u))
-                           ? __ldg(p.slot_first + first + j)
-                           : 0;
+            for (int j = 0; j <= PER; ++j) {
+                if constexpr (kEarly) at[j] = f[j];
+                else at[j] = first_slot(p, first, j);
+            }
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
                 sum[j] = N::zero();
                 if (!((on >> j) & 1u)) continue;
                 bool bad = false;
-                for (int32_t k = f[j]; k < f[j + 1]; ++k) N::light(sum[j], bad, p.slots[k]);
+                for (int32_t k = at[j]; k < at[j + 1]; ++k) N::light(sum[j], bad, p.slots[k]);
                 nan |= bad ? 1u << j : 0u;
             }
         }
@@ -1141,13 +1154,15 @@ __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, P
     __shared__ PMap<K> s_warp[kPathThreads / 32];
     __shared__ PMap<K> s_prefix;
     __shared__ int s_tile;
+    next_may_start();
     if (threadIdx.x == 0) s_tile = atomicAdd(q.ticket, 1);
     __syncthreads();
     const int tile = s_tile;
     const int32_t first = (v.p0 & ~(PER - 1)) + tile * (kPathThreads * PER) + (int32_t)threadIdx.x * PER;
     Chunk<N, R, K, PER, LIGHT> ch;
     ch.template order<true>(p, first, v.p0, v.p1);
-    ch.gather(p);
+    ch.gather(p, first);
+    wait_for_previous();
     const PMap<K> acc = ch.maps(p, first);
     PMap<K> total;
     const PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
@@ -1197,12 +1212,14 @@ __global__ void __launch_bounds__(kPathThreads, 4)
     __shared__ PMap<K> s_warp[kPathThreads / 32];
     __shared__ PMap<K> s_carry;
     constexpr int32_t T = kPathThreads * PER;
+    next_may_start();
     const int32_t lo = __ldg(cut + v.cut0 + blockIdx.x), hi = __ldg(cut + v.cut0 + blockIdx.x + 1);
     if (threadIdx.x == 0) s_carry = pm_identity<K>();
     const int32_t at = (int32_t)threadIdx.x * PER;
     Chunk<N, R, K, PER, LIGHT> ch, nx;
     ch.template order<false>(p, lo + at, lo, hi);
-    ch.gather(p);
+    ch.gather(p, lo + at);
+    wait_for_previous();
     for (int32_t c0 = lo; c0 < hi; c0 += T) {  // uniform
         const int32_t first = c0 + at;
         const bool more = c0 + T < hi;
@@ -1214,7 +1231,7 @@ __global__ void __launch_bounds__(kPathThreads, 4)
         const PMap<K> E = compose<K>(s_carry, ex);
         __syncthreads();  // every thread has read s_carry
         if (threadIdx.x == 0) s_carry = compose<K>(s_carry, total);
-        if (more) nx.gather(p);
+        if (more) nx.gather(p, first + T);
         ch.store(p, first, hi, E);
         ch = nx;
     }
@@ -1296,12 +1313,19 @@ int path_prepare(lue_gpu_topology* t, cudaStream_t stream)
     return path_core_get(t, stream, &pc);
 }
 
+// A level reads its order, its inputs and its first slots while the level before still runs.  Level 0 follows whatever
+// wrote the inputs, so it starts after it.
 template <class N, Rule R, int K, int PER, bool LIGHT>
 static void launch_level(bool free, unsigned blocks, cudaStream_t stream, const PathCall<N>& p, const PathLevel& v,
                          const PathScan<K>& q, const int32_t* cut)
 {
-    if (free) k_path_free<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, cut);
-    else k_path_level<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, q);
+    if (!LIGHT) {
+        if (free) k_path_free<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, cut);
+        else k_path_level<N, R, K, PER, LIGHT><<<blocks, kPathThreads, 0, stream>>>(p, v, q);
+    } else {
+        if (free) launch_after(k_path_free<N, R, K, PER, LIGHT>, blocks, kPathThreads, 0, stream, p, v, cut);
+        else launch_after(k_path_level<N, R, K, PER, LIGHT>, blocks, kPathThreads, 0, stream, p, v, q);
+    }
 }
 
 template <class N, Rule R, int K, class Visitor>
@@ -1352,10 +1376,10 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
     }
     // +-inf inputs, or a wait of the scan that gave up: the walk engine redoes the whole call (as behind
     // the tile engine of accu)
-    k_copy_words_if<<<grid_for(words_for(n), 256), 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(core->count),
-                                                                     t->work_count, words_for(n), flag);
+    launch_after(k_copy_words_if, grid_for(words_for(n), 256), 256, 0, stream,
+                 reinterpret_cast<const uint32_t*>(core->count), t->work_count, words_for(n), (const unsigned long long*)flag);
     WalkGrid g{core->fd, core->count, t->work_count, core->rows, core->cols, n};
-    k_walk_if<<<grid_for(n, 256), 256, 0, stream>>>(g, redo, flag);
+    launch_after(k_walk_if<Visitor>, grid_for(n, 256), 256, 0, stream, g, redo, (const unsigned long long*)flag);
     count_launches(launches + 2);
     return cuda_status(cudaGetLastError(), what);
 }
