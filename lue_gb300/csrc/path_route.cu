@@ -421,12 +421,19 @@ static int64_t path_padded(int64_t npos) { return ((npos + 7) / 8 + 1) * 8; }
 // chains of dependent loads per thread).
 constexpr int64_t kPathSmallLevel = 1 << 20;
 
-// A level scans without look-back when its longest path is at most kPathFreeChunks chunks of a CTA; its CTA ranges
-// are then that many chunks, cut at path tops.  One chunk leaves most ranges a second one that is nearly empty
+// A level scans without look-back when its longest path is at most kPathFreeChunks chunks of a CTA; the CTA ranges of a
+// large level are then that many chunks, cut at path tops.  One chunk leaves most ranges a second one that is nearly empty
 // and more levels with look-back (accu_threshold at 16384^2: 11.3 ms), four lengthen the serial part of a CTA (6.8
 // ms; accu_fraction at 2311 x 1501: 189 us against 136 us); two: 6.6 ms.
 constexpr int kPathFreeChunks = 2;
-static int64_t path_cut_step(int per) { return (int64_t)kPathThreads * per * kPathFreeChunks; }
+// Small levels, which cannot fill the GPU, take half a chunk per CTA: most ranges are then one chunk, and the launch is
+// over sooner (accu_fraction at 2311 x 1501 119 -> 100 us, accu_trigger at 1500^2 161 -> 134 us; a quarter: 99 and 135).
+constexpr int64_t kPathTinyLevel = 1 << 18;
+static int64_t path_cut_step(int per, int64_t n)
+{
+    const int64_t T = (int64_t)kPathThreads * per;
+    return n < kPathTinyLevel ? T / 2 : T * kPathFreeChunks;
+}
 
 void path_core_free(PathCore* pc)
 {
@@ -516,7 +523,7 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
         v.longest = hstats[3 + l];
         v.per = v.p1 - v.p0 < kPathSmallLevel ? 1 : 4;
         v.cut0 = (int32_t)ncuts;
-        v.ncut = (int32_t)((v.p1 - v.p0 + path_cut_step(v.per) - 1) / path_cut_step(v.per));
+        v.ncut = (int32_t)((v.p1 - v.p0 + path_cut_step(v.per, v.p1 - v.p0) - 1) / path_cut_step(v.per, v.p1 - v.p0));
         ncuts += v.ncut + 1;
         pc->tiles = std::max<int64_t>(pc->tiles, (v.p1 - v.p0) / (kPathThreads * v.per) + 2);
     }
@@ -558,7 +565,7 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
         for (const PathLevel& v : pc->levels)
             if (v.ncut > 0)
                 k_path_cuts<<<(unsigned)(((v.ncut + 1) * 32 + 255) / 256), 256, 0, stream>>>(
-                    pc->order, v.p0, v.p1, path_cut_step(v.per), v.ncut, pc->cut + v.cut0);
+                    pc->order, v.p0, v.p1, path_cut_step(v.per, v.p1 - v.p0), v.ncut, pc->cut + v.cut0);
         launches += 8 + levels;
         long long hslots = 0;
         int bad = 0;
