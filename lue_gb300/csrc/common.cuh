@@ -141,6 +141,46 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
+// Several device arrays in one allocation: plan them with add(), then allocate().  Frees it unless released.
+class Arena {
+    size_t bytes_ = 0;
+    char* base_ = nullptr;
+    bool owned_ = false;
+
+public:
+    Arena() = default;
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+    ~Arena()
+    {
+        if (owned_) cudaFree(base_);
+    }
+    size_t add(int64_t n)
+    {
+        const size_t at = bytes_;
+        bytes_ += ((size_t)n + 255) & ~size_t(255);
+        return at;
+    }
+    size_t bytes() const { return bytes_; }
+    void reserve(size_t n) { bytes_ = bytes_ < n ? n : bytes_; }
+    cudaError_t allocate()
+    {
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&base_), bytes_ ? bytes_ : 256);
+        owned_ = e == cudaSuccess;
+        return e;
+    }
+    void* release()
+    {
+        owned_ = false;
+        return base_;
+    }
+    template <class T>
+    T* at(size_t offset) const
+    {
+        return reinterpret_cast<T*>(base_ + offset);
+    }
+};
+
 // One thread per element, no grid-stride reuse (walk kernels: a thread that walks a long path must not
 // also own later cells, or the walks chain up behind each other).
 inline unsigned grid_all(int64_t n, int threads)

@@ -1437,6 +1437,8 @@ static int stage_core_get(lue_gpu_topology* t, cudaStream_t stream, const StageC
         core->stages = sc;
         core->bytes += sc->bytes;
     }
+    if (core->stages)
+        if (int rc = stage_flag(t)) return rc;
     *out = core->stages;
     return LUE_GPU_OK;
 }

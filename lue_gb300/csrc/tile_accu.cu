@@ -1,6 +1,6 @@
 // tile_accu.cu — tiled accu engine (see tile_accu.cuh): topology build and per-call kernels.
 #include <algorithm>
-#include <vector>
+#include <cstring>
 
 #include "tile_accu.cuh"
 #include "topology.cuh"
@@ -97,42 +97,88 @@ __device__ __forceinline__ int64_t tile_of(const TileGeom& g, int64_t r, int64_t
     return (r / kTile) * g.tcols + c / kTile;
 }
 
-// Exit bitmap: one 64-bit word per tile row; bit c set when that cell's flow leaves the tile but not
-// the array.
-__global__ void k_exit_bitmap(const uint8_t* __restrict__ fd, TileGeom g, uint64_t* bitmap)
+// Whether the flow of in-tile cell (rin, cin) leaves the tile but not the array.
+__device__ __forceinline__ bool leaves_tile(const uint8_t* __restrict__ fd, const TileGeom& g, int64_t tr, int64_t tc,
+                                            int rin, int cin)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.trows * g.tcols * kTile) return;
-    int64_t tile = i / kTile;
-    int rin = (int)(i % kTile);
-    int64_t tr = tile / g.tcols, tc = tile % g.tcols;
-    int64_t r = tr * kTile + rin;
-    uint64_t m = 0;
-    if (r < g.rows) {
-        for (int cin = 0; cin < kTile; ++cin) {
-            int64_t c = tc * kTile + cin;
-            if (c >= g.cols) break;
-            int dr, dc;
-            uint8_t code = fd[r * g.cols + c];
-            if (code == kNoData || !d8_offset(code, dr, dc)) continue;
-            int64_t rd = r + dr, cd = c + dc;
-            if (rd < 0 || rd >= g.rows || cd < 0 || cd >= g.cols) continue;
-            if (rd / kTile != tr || cd / kTile != tc) m |= 1ull << cin;
-        }
-    }
-    bitmap[i] = m;
+    const int64_t r = tr * kTile + rin, c = tc * kTile + cin;
+    int dr, dc;
+    if (r >= g.rows || c >= g.cols) return false;
+    const uint8_t code = __ldg(fd + r * g.cols + c);
+    if (code == kNoData || !d8_offset(code, dr, dc)) return false;
+    const int64_t rd = r + dr, cd = c + dc;
+    if (rd < 0 || rd >= g.rows || cd < 0 || cd >= g.cols) return false;
+    return rin + dr < 0 || rin + dr >= kTile || cin + dc < 0 || cin + dc >= kTile;
 }
 
-__global__ void k_row_prefix(const uint64_t* bitmap, int64_t ntiles, uint16_t* rowpref, int32_t* count)
+// Exits of a tile, one warp each: a 64-bit word per tile row (bit c: that cell is an exit; only border cells can
+// be), the exits in the rows before each row, and their number.
+__global__ void __launch_bounds__(256) k_exit_bitmap(const uint8_t* __restrict__ fd, TileGeom g, uint64_t* bitmap,
+                                                     uint16_t* rowpref, int32_t* count)
 {
-    int64_t tile = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tile >= ntiles) return;
-    int acc = 0;
-    for (int r = 0; r < kTile; ++r) {
-        rowpref[tile * kTile + r] = (uint16_t)acc;
-        acc += __popcll(bitmap[tile * kTile + r]);
+    __shared__ uint64_t s_rows[8][kTile];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t tile = (int64_t)blockIdx.x * 8 + warp;
+    if (tile >= g.trows * g.tcols) return;
+    const int64_t tr = tile / g.tcols, tc = tile - tr * g.tcols;
+    uint64_t* rows = s_rows[warp];
+    for (int k = 0; k < 2; ++k) {  // the whole first and last row
+        const int rin = k * (kTile - 1);
+        const unsigned lo = __ballot_sync(0xffffffffu, leaves_tile(fd, g, tr, tc, rin, lane));
+        const unsigned hi = __ballot_sync(0xffffffffu, leaves_tile(fd, g, tr, tc, rin, lane + 32));
+        if (lane == 0) rows[rin] = ((uint64_t)hi << 32) | lo;
     }
-    count[tile] = acc;
+    for (int rin = 1 + lane; rin < kTile - 1; rin += 32)
+        rows[rin] = (leaves_tile(fd, g, tr, tc, rin, 0) ? 1ull : 0ull) |
+                    (leaves_tile(fd, g, tr, tc, rin, kTile - 1) ? 1ull << (kTile - 1) : 0ull);
+    __syncwarp();
+    int before = 0;
+    for (int k = 0; k < 2; ++k) {
+        const int rin = 32 * k + lane;
+        const uint64_t m = rows[rin];
+        const int n = __popcll(m);
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        bitmap[tile * kTile + rin] = m;
+        rowpref[tile * kTile + rin] = (uint16_t)(before + x - n);
+        before += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) count[tile] = before;
+}
+
+// Exclusive sums of up to two arrays of n counts (one CTA), with their totals at [n].
+__global__ void __launch_bounds__(1024) k_tile_scan(const int32_t* a, int32_t* a_base, const int32_t* b, int32_t* b_base,
+                                                    int64_t n)
+{
+    __shared__ int s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = 0; k < (b ? 2 : 1); ++k) {
+        const int32_t* x = k ? b : a;
+        int32_t* base = k ? b_base : a_base;
+        const int64_t per = (n + 1023) / 1024;
+        const int64_t i0 = min(n, (int64_t)threadIdx.x * per), i1 = min(n, i0 + per);
+        int sum = 0;
+        for (int64_t i = i0; i < i1; ++i) sum += x[i];
+        int v = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) s_warp[warp] = v;
+        __syncthreads();
+        int before = v - sum;
+        for (int w = 0; w < warp; ++w) before += s_warp[w];
+        for (int64_t i = i0; i < i1; ++i) {
+            base[i] = before;
+            before += x[i];
+        }
+        if (threadIdx.x == 1023) base[n] = before;
+        __syncthreads();
+    }
 }
 
 __device__ __forceinline__ int32_t exit_id_of(const TileGeom& g, const int32_t* exit_base, const uint64_t* bitmap,
@@ -144,8 +190,10 @@ __device__ __forceinline__ int32_t exit_id_of(const TileGeom& g, const int32_t* 
     return exit_base[tile] + rowpref[tile * kTile + rin] + __popcll(word & ((1ull << cin) - 1ull));
 }
 
+constexpr int kExitCounters = 5;  // children, children to come, positions handed out, depth, position seen
+
 __global__ void k_exit_list(TileGeom g, const uint64_t* bitmap, const uint16_t* rowpref, const int32_t* exit_base,
-                            uint16_t* exit_local, uint32_t* exit_cell)
+                            uint16_t* exit_local, uint32_t* exit_cell, uint32_t* size, int32_t* zero, int64_t stride)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.trows * g.tcols * kTile) return;
@@ -159,17 +207,20 @@ __global__ void k_exit_list(TileGeom g, const uint64_t* bitmap, const uint16_t* 
         m &= m - 1;
         exit_local[id] = (uint16_t)(rin * kTile + cin);
         exit_cell[id] = (uint32_t)((tr * kTile + rin) * g.cols + tc * kTile + cin);
+        size[id] = 1;
+        for (int k = 0; k < kExitCounters; ++k) zero[k * stride + id] = 0;
         ++id;
     }
 }
 
-// Parent of every exit: follow the flow from its downstream cell through that cell's tile.
-__global__ void k_exit_parent(const uint8_t* __restrict__ fd, TileGeom g, int64_t nexit, const uint32_t* exit_cell,
+// Parent of every exit: follow the flow from its downstream cell through that cell's tile.  plus: the cells from the
+// exit to its parent.
+__global__ void k_exit_parent(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* nexit, const uint32_t* exit_cell,
                               const int32_t* exit_base, const uint64_t* bitmap, const uint16_t* rowpref,
-                              int32_t* parent, int32_t* nchild, int* error)
+                              int32_t* parent, int32_t* nchild, int32_t* pending, int32_t* plus, int* cyclic)
 {
     int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= nexit) return;
+    if (y >= *nexit) return;
     int64_t cell = exit_cell[y];
     int64_t r = cell / g.cols, c = cell % g.cols;
     int dr, dc;
@@ -178,7 +229,8 @@ __global__ void k_exit_parent(const uint8_t* __restrict__ fd, TileGeom g, int64_
     c += dc;
     int64_t tile = tile_of(g, r, c);
     int32_t p = -1;
-    for (int step = 0; step <= kTileCells; ++step) {
+    int step = 0;
+    for (; step <= kTileCells; ++step) {
         uint8_t code = fd[r * g.cols + c];
         if (code == kNoData || !d8_offset(code, dr, dc)) break;  // sink (or flow into no-data): root
         int64_t r2 = r + dr, c2 = c + dc;
@@ -189,130 +241,102 @@ __global__ void k_exit_parent(const uint8_t* __restrict__ fd, TileGeom g, int64_
         }
         r = r2;
         c = c2;
-        if (step == kTileCells) atomicExch(error, 1);  // cycle inside a tile (excluded by the caller)
+        if (step == kTileCells) atomicExch(cyclic, 1);  // a cycle inside a tile
     }
     parent[y] = p;
-    if (p >= 0) atomicAdd(nchild + p, 1);
+    plus[y] = step + 1;
+    if (p >= 0) {
+        atomicAdd(nchild + p, 1);
+        atomicAdd(pending + p, 1);
+    }
 }
 
-// Subtree sizes and depths of the exit forest, with the counter walk of walk.cuh on the coarse forest.
-__global__ void k_exit_sizes(int64_t nexit, const int32_t* parent, const int32_t* nchild, int32_t* pending,
-                             uint32_t* size, int32_t* depth)
+// Subtree sizes, downstream levels and depth of the exit forest, with the counter walk of walk.cuh on the coarse
+// forest.  level: on entry each exit's level within its tile.  A subtree below a cycle never finishes.
+__global__ void k_exit_sizes(const int32_t* nexit, const int32_t* parent, const int32_t* nchild, const int32_t* plus,
+                             int32_t* pending, uint32_t* size, int32_t* level, int32_t* depth, int* max_depth)
 {
     int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= nexit || nchild[y] != 0) return;
+    if (y >= *nexit || nchild[y] != 0) return;
     uint32_t s = 1;
-    int32_t d = 1;
+    int32_t d = 1, lv = level[y];
     for (;;) {
         int32_t p = parent[y];
-        if (p < 0) return;
+        if (p < 0) {
+            if (d > *(volatile int*)max_depth) atomicMax(max_depth, d);
+            return;
+        }
         atomicAdd(size + p, s);
         atomicMax(depth + p, d + 1);
+        atomicMax(level + p, lv + plus[y]);
         __threadfence();
         if (atomicSub(pending + p, 1) != 1) return;
         __threadfence();
         s = atomicAdd(size + p, 0u);
         d = atomicAdd(depth + p, 0);
+        lv = atomicAdd(level + p, 0);
         y = p;
     }
 }
 
-__global__ void k_exit_offsets(int64_t nexit, const int32_t* parent, const uint32_t* size, uint32_t* acc,
-                               unsigned long long* root_acc, int64_t* D, int32_t* J)
+// The exit forest in post-order: link[y] = (offset of y's position from its parent's, the parent); the subtrees of a
+// parent's children follow one another in any order.
+__global__ void k_exit_offsets(const int32_t* nexit, const int32_t* parent, const int32_t* pending, const uint32_t* size,
+                               uint32_t* acc, unsigned* root_acc, int2* link, int* cyclic)
 {
-    int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= nexit) return;
-    int32_t p = parent[y];
-    if (p >= 0) {
-        uint32_t off = atomicAdd(acc + p, size[y]);
-        D[y] = (int64_t)off + size[y] - size[p];
-    } else {
-        unsigned long long off = atomicAdd(root_acc, (unsigned long long)size[y]);
-        D[y] = (int64_t)off + size[y] - 1;
+    const int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool in = y < *nexit;
+    const int32_t p = in ? parent[y] : 0;
+    const unsigned own = in ? size[y] : 0u;
+    if (in && pending[y] != 0) atomicExch(cyclic, 1);
+    // roots: one atomic per warp
+    unsigned x = in && p < 0 ? own : 0u;
+    const unsigned mine = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned z = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += z;
     }
-    J[y] = p;
+    unsigned base = 0;
+    if (lane == 31 && x) base = atomicAdd(root_acc, x);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (!in) return;
+    const unsigned off = p >= 0 ? atomicAdd(acc + p, own) - size[p] : base + x - mine - 1u;
+    link[y] = make_int2((int)(off + own), p);
 }
 
-// Pointer jumping: pos(y) = pos(parent) + D(y) summed to the root.
-__global__ void k_jump(int64_t nexit, const int64_t* D, const int32_t* J, int64_t* D2, int32_t* J2, int* more)
+// Pointer jumping, in place: position(y) = offset + position(parent) holds for every link at any time, and a link is
+// read and written as one 8-byte word.
+__global__ void k_jump(int64_t nexit, int2* link)
+{
+    const int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (y >= nexit) return;
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(link);
+    const unsigned long long w = __ldcg(words + y);
+    const int j = (int)(w >> 32);
+    if (j < 0) return;
+    const unsigned long long wj = __ldcg(words + j);
+    __stcg(words + y, (wj & 0xFFFFFFFF00000000ull) | (unsigned)((unsigned)w + (unsigned)wj));
+}
+
+// Positions from the links, checked: every post-order position must be a distinct index in [0, nexit) with start <= pos
+// (the per-call kernels scatter and gather with them, so the build refuses a forest that fails this check).
+__global__ void k_exit_positions(int64_t nexit, const int2* link, const uint32_t* size, uint32_t* pos, uint32_t* start,
+                                 int32_t* seen, int* error)
 {
     int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (y >= nexit) return;
-    int32_t j = J[y];
-    if (j >= 0) {
-        D2[y] = D[y] + D[j];
-        int32_t jj = J[j];
-        J2[y] = jj;
-        if (jj >= 0) *more = 1;
-    } else {
-        D2[y] = D[y];
-        J2[y] = -1;
-    }
-}
-
-__global__ void k_exit_positions(int64_t nexit, const int64_t* D, const uint32_t* size, uint32_t* pos, uint32_t* start)
-{
-    int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= nexit) return;
-    pos[y] = (uint32_t)D[y];
-    start[y] = (uint32_t)(D[y] - size[y] + 1);
-}
-
-// Every post-order position must be a distinct index in [0, nexit) with start <= pos: the per-call
-// kernels scatter and gather with them, so the build refuses a forest that fails this check.
-__global__ void k_check_positions(int64_t nexit, const uint32_t* pos, const uint32_t* start, int32_t* seen, int* error)
-{
-    int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= nexit) return;
-    uint32_t p = pos[y], s = start[y];
-    if (p >= (uint64_t)nexit || s > p) {
+    const int2 l = link[y];
+    const uint32_t p = (uint32_t)l.x, s = p - size[y] + 1u;
+    if (l.y >= 0 || p >= (uint64_t)nexit || s > p) {
+        pos[y] = start[y] = 0;
         atomicExch(error, 1);
         return;
     }
+    pos[y] = p;
+    start[y] = s;
     if (atomicAdd(seen + p, 1) != 0) atomicExch(error, 1);
-}
-
-__device__ __forceinline__ void halo_slot_coords(int s, int& hr, int& hc)
-{
-    if (s < kTile) { hr = -1; hc = s; }
-    else if (s < 2 * kTile) { hr = kTile; hc = s - kTile; }
-    else if (s < 3 * kTile) { hr = s - 2 * kTile; hc = -1; }
-    else if (s < 4 * kTile) { hr = s - 3 * kTile; hc = kTile; }
-    else if (s == 4 * kTile) { hr = -1; hc = -1; }
-    else if (s == 4 * kTile + 1) { hr = -1; hc = kTile; }
-    else if (s == 4 * kTile + 2) { hr = kTile; hc = -1; }
-    else { hr = kTile; hc = kTile; }
-}
-
-__device__ __forceinline__ int halo_slot_of(int hr, int hc)
-{
-    if (hr == -1) return hc == -1 ? 4 * kTile : (hc == kTile ? 4 * kTile + 1 : hc);
-    if (hr == kTile) return hc == -1 ? 4 * kTile + 2 : (hc == kTile ? 4 * kTile + 3 : kTile + hc);
-    return hc == -1 ? 2 * kTile + hr : 3 * kTile + hr;
-}
-
-__global__ void k_halo_exits(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* exit_base,
-                             const uint64_t* bitmap, const uint16_t* rowpref, int32_t* halo_exit)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t ntiles = g.trows * g.tcols;
-    if (i >= ntiles * kHaloSlots) return;
-    int64_t tile = i / kHaloSlots;
-    int s = (int)(i % kHaloSlots), hr, hc;
-    halo_slot_coords(s, hr, hc);
-    int64_t tr = tile / g.tcols, tc = tile % g.tcols;
-    int64_t r = tr * kTile + hr, c = tc * kTile + hc;
-    int32_t id = -1;
-    if (r >= 0 && r < g.rows && c >= 0 && c < g.cols) {
-        int dr, dc;
-        uint8_t code = fd[r * g.cols + c];
-        if (code != kNoData && d8_offset(code, dr, dc)) {
-            int64_t rd = r + dr, cd = c + dc;
-            if (rd >= 0 && rd < g.rows && cd >= 0 && cd < g.cols && tile_of(g, rd, cd) == tile)
-                id = exit_id_of(g, exit_base, bitmap, rowpref, r, c);
-        }
-    }
-    halo_exit[i] = id;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -321,60 +345,74 @@ __global__ void k_halo_exits(const uint8_t* __restrict__ fd, TileGeom g, const i
 
 constexpr uint16_t kNoCell = 0xFFFFu;
 
+// 49 KB: four CTAs of k_tile_forest on an SM.
 struct __align__(16) TileSmem {
-    float hi[kTileCells];
-    float lo[kTileCells];
-    uint32_t cnt[kTileCells / 4];  // in-tile inflow counters, 4 per word
+    uint32_t cell[kTileCells];     // high half: in-tile inflows to come, then the cell's round (its downstream level within
+                                   // the tile), then its subtree's first position; low half: the size of its subtree
     uint16_t dsl[kTileCells];      // downstream cell inside the tile, or kNoCell
     uint16_t queue[kTileCells];    // cells in the order they become ready (each cell once)
-    uint8_t up[kTileCells];        // in-tile upstream mask
+    uint16_t rstart[kTileCells + 1];  // round starts in the queue
+    __align__(16) uint8_t up[kTileCells];  // in-tile upstream mask
     uint8_t fd[kHalo][kHalo + 2];  // flow direction with a one-cell halo (255 outside the array)
-    uint8_t border[kBorderCells];  // per border cell: outside neighbours draining into it
+    int warp_tot[kTileThreads / 32];
+    int edges;                     // flow edges into the tile
+    int rounds;
     int round_count[3];            // cells queued for the next rounds (a ring of three counters)
 };
 
-// Load the flow direction with halo; fill in-tile upstream masks, counters and downstream indices, and
+// Downstream cell of in-tile cell (rin, cin) with flow direction `code`, if the flow goes to another cell of the tile;
+// q: the neighbour (nb_dr order) that the cell is to it.
+__device__ __forceinline__ bool tile_downstream(unsigned code, int rin, int cin, int& d, int& q)
+{
+    const unsigned pad = code - 1u;  // numeric pad: 0 .. 8 from the lower left, 4 in the middle
+    if (pad > 8u || pad == 4u) return false;
+    const int up = (int)(pad * 11u >> 5), right = (int)pad - 3 * up;  // 0, 1, 2
+    const int r = rin + 1 - up, c = cin + right - 1;
+    d = r * kTile + c;
+    const int seen = up * 3 + 2 - right;
+    q = seen - (seen > 4);
+    return (unsigned)r < (unsigned)kTile && (unsigned)c < (unsigned)kTile;
+}
+
+// Load the flow direction with halo; fill in-tile upstream masks, cell words and downstream indices, and
 // queue the cells without in-tile inflow (the first round).  Returns the number of queued cells.
 __device__ __forceinline__ int tile_prepare(TileSmem& sm, const uint8_t* __restrict__ fd, const TileGeom& g,
                                             int64_t tr, int64_t tc)
 {
-    const int t = threadIdx.x;
-    for (int i = t; i < kHalo * kHalo; i += kTileThreads) {
-        int hr = i / kHalo, hc = i % kHalo;
-        int64_t r = tr * kTile + hr - 1, c = tc * kTile + hc - 1;
-        sm.fd[hr][hc] = (r >= 0 && r < g.rows && c >= 0 && c < g.cols) ? __ldg(fd + r * g.cols + c) : kNoData;
+    const int t = threadIdx.x, lane = t & 31;
+    for (int hr = t >> 5; hr < kHalo; hr += kTileThreads / 32) {
+        const int64_t r = tr * kTile + hr - 1;
+        const bool row_in = r >= 0 && r < g.rows;
+        for (int hc = lane; hc < kHalo; hc += 32) {
+            const int64_t c = tc * kTile + hc - 1;
+            sm.fd[hr][hc] = row_in && c >= 0 && c < g.cols ? __ldg(fd + r * g.cols + c) : kNoData;
+        }
     }
+    uint32_t* up = reinterpret_cast<uint32_t*>(sm.up);
+    for (int i = t; i < kTileCells; i += kTileThreads) sm.cell[i] = 1u;
+    for (int i = t; i < kTileCells / 4; i += kTileThreads) up[i] = 0u;
     if (t < 3) sm.round_count[t] = 0;
+    if (t == 3) sm.edges = 0;
     __syncthreads();
-    uint8_t* cnt8 = reinterpret_cast<uint8_t*>(sm.cnt);
-    const int lane = t & 31;
 #pragma unroll 4
     for (int k = 0; k < kTileCells / kTileThreads; ++k) {
-        int i = t + k * kTileThreads;
-        int rin = i >> 6, cin = i & 63;
-        uint8_t code = sm.fd[rin + 1][cin + 1];
-        unsigned mask = 0;
-        uint16_t d = kNoCell;
-        if (code != kNoData) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                int rn = rin + nb_dr(q), cn = cin + nb_dc(q);
-                if (rn >= 0 && rn < kTile && cn >= 0 && cn < kTile && sm.fd[rn + 1][cn + 1] == nb_inflow_code(q))
-                    mask |= 1u << q;
-            }
-            int dr, dc;
-            if (d8_offset(code, dr, dc)) {
-                int r2 = rin + dr, c2 = cin + dc;
-                if (r2 >= 0 && r2 < kTile && c2 >= 0 && c2 < kTile && sm.fd[r2 + 1][c2 + 1] != kNoData)
-                    d = (uint16_t)(r2 * kTile + c2);
-            }
+        const int i = t + k * kTileThreads, rin = i >> 6, cin = i & 63;
+        int d = kNoCell, e, q;
+        if (tile_downstream(sm.fd[rin + 1][cin + 1], rin, cin, e, q) &&
+            sm.fd[(e >> 6) + 1][(e & 63) + 1] != kNoData) {
+            d = e;
+            atomicAdd(sm.cell + d, 0x10000u);
+            atomicOr(up + (d >> 2), 1u << (8 * (d & 3) + q));
         }
-        sm.up[i] = (uint8_t)mask;
-        sm.dsl[i] = d;
-        cnt8[i] = code == kNoData ? kNoData : (uint8_t)__popc(mask);
+        sm.dsl[i] = (uint16_t)d;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < kTileCells / kTileThreads; ++k) {
         // first round: valid cells without in-tile inflow (warp-aggregated queue appends)
-        bool start = code != kNoData && mask == 0;
-        unsigned ballot = __ballot_sync(0xffffffffu, start);
+        const int i = t + k * kTileThreads;
+        const bool start = sm.cell[i] == 1u && sm.fd[(i >> 6) + 1][(i & 63) + 1] != kNoData;
+        const unsigned ballot = __ballot_sync(0xffffffffu, start);
         int base = 0;
         if (lane == 0 && ballot) base = atomicAdd(&sm.round_count[0], __popc(ballot));
         base = __shfl_sync(0xffffffffu, base, 0);
@@ -435,24 +473,29 @@ __device__ __forceinline__ int block_exclusive_int(int v, int* warp_tot, int& to
 // (its subtree) get the positions start .. pos - 1 and the cell itself pos, so that the accu of any cell
 // is the difference of two prefix sums over the material laid out in post-order.  Cells with a no-data
 // flow direction (or outside the array) take the positions after the valid cells, flagged kNoValue.
-// Also: each exit's scan slots (its own, and the one before its subtree), and, per border cell, which
-// outside neighbours drain into it.
+// Also: each exit's scan slots (its own, and the one before its subtree), the cells' and exits' levels within the
+// tile, and, per border cell, which outside neighbours drain into it.
+// Bound by issue and by the chain of rounds (2048^2 fractal terrain: 126 us, 2.1 instructions per cycle; with separate
+// sweeps for counts and sizes, block barriers in every round and the tables stored cell by cell 264 us).
 __global__ void __launch_bounds__(kTileThreads)
     k_tile_forest(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* __restrict__ exit_base,
                   const uint16_t* __restrict__ exit_local, uint16_t* cell_at, uint16_t* prev_at,
-                  uint32_t* exit_span, uint8_t* border_in, int* error)
+                  uint32_t* exit_span, uint8_t* border_in, int32_t* nslot, int32_t* nedge, int32_t* exit_level,
+                  int32_t* __restrict__ level, int* error, int* cyclic)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileSmem& sm = *reinterpret_cast<TileSmem*>(smem_raw);
     const int64_t tr = blockIdx.y, tc = blockIdx.x;  // grid = (tile columns, tile rows)
     const int64_t tile = tr * g.tcols + tc;
     const int t = threadIdx.x, lane = t & 31;
-    uint16_t* rstart = reinterpret_cast<uint16_t*>(sm.hi);  // <= 4097 round starts
-    uint16_t* sz = reinterpret_cast<uint16_t*>(sm.lo);      // subtree size
-    uint16_t* st = sz + kTileCells;                         // first position of the subtree
+    uint16_t* rstart = sm.rstart;
+    const uint16_t* sz = reinterpret_cast<const uint16_t*>(sm.cell);  // [2 i] subtree size of cell i
+    uint16_t* st = reinterpret_cast<uint16_t*>(sm.cell) + 1;          // [2 i] its round, then its first position
     int head = 0, count = tile_prepare(sm, fd, g, tr, tc), r = 0;
-    // rounds: a round holds the cells whose in-tile upstream cells are all in earlier rounds
-    while (count > 0) {
+    // rounds: a round holds the cells whose in-tile upstream cells are all in earlier rounds; each hands its subtree's
+    // size down.  No round has more cells than the one before it: from the first with at most 32 on, one warp goes
+    // on without block barriers.
+    while (count > 32) {
         int* next = &sm.round_count[(r + 1) % 3];
         const int next_base = head + count;
         if (t == 0) {
@@ -460,13 +503,15 @@ __global__ void __launch_bounds__(kTileThreads)
             sm.round_count[(r + 2) % 3] = 0;  // read by everyone two rounds ago
         }
         for (int k0 = 0; k0 < count; k0 += kTileThreads) {
-            int k = k0 + t, d = kNoCell;
-            if (k < count) d = sm.dsl[sm.queue[head + k]];
+            const int k = k0 + t;
+            int d = kNoCell;
             bool ready = false;
-            if (d != kNoCell) {
-                unsigned shift = (unsigned)(d & 3) * 8u;
-                unsigned old = atomicSub(sm.cnt + (d >> 2), 1u << shift);
-                ready = ((old >> shift) & 0xFFu) == 1u;
+            if (k < count) {
+                const int i = sm.queue[head + k];
+                const unsigned size = sm.cell[i] & 0xFFFFu;
+                sm.cell[i] = ((unsigned)r << 16) | size;
+                d = sm.dsl[i];
+                if (d != kNoCell) ready = atomicAdd(sm.cell + d, size - 0x10000u) >> 16 == 1u;
             }
             unsigned ballot = __ballot_sync(0xffffffffu, ready);
             int base = 0;
@@ -479,13 +524,39 @@ __global__ void __launch_bounds__(kTileThreads)
         count = *next;
         ++r;
     }
-    const int rounds = r, nvalid = head;
-    if (t == 0) rstart[rounds] = (uint16_t)nvalid;
+    const int wide = r;  // rounds of more than 32 cells
+    if (t < 32) {
+        int i = t < count ? sm.queue[head + t] : kNoCell, d = i != kNoCell ? sm.dsl[i] : kNoCell;
+        unsigned size = i != kNoCell ? sm.cell[i] & 0xFFFFu : 0u;
+        while (count > 0) {
+            if (t == 0) rstart[r] = (uint16_t)head;
+            if (i != kNoCell) sm.cell[i] = ((unsigned)r << 16) | size;
+            bool ready = false;
+            int after = kNoCell;
+            if (d != kNoCell) {
+                after = sm.dsl[d];
+                const unsigned old = atomicAdd(sm.cell + d, size - 0x10000u);
+                ready = old >> 16 == 1u;
+                size = (old + size) & 0xFFFFu;
+            }
+            const unsigned ballot = __ballot_sync(0xffffffffu, ready);
+            head += count;
+            count = __popc(ballot);
+            if (ready) sm.queue[head + __popc(ballot & ((1u << lane) - 1u))] = (uint16_t)d;
+            i = ready ? d : kNoCell;
+            d = ready ? after : kNoCell;
+            ++r;
+        }
+        if (t == 0) {
+            rstart[r] = (uint16_t)head;
+            sm.rounds = r;
+        }
+    }
     // per border cell, the neighbours outside the tile that drain into it
-    for (int b = t; b < kBorderCells; b += kTileThreads) {
+    unsigned outside = 0;
+    if (t < kBorderCells) {
         int rin, cin;
-        border_cell(b, rin, cin);
-        unsigned outside = 0;
+        border_cell(t, rin, cin);
         if (sm.fd[rin + 1][cin + 1] != kNoData) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
@@ -494,65 +565,103 @@ __global__ void __launch_bounds__(kTileThreads)
                 if (sm.fd[hr + 1][hc + 1] == nb_inflow_code(q)) outside |= 1u << q;
             }
         }
-        border_in[tile * kBorderCells + b] = (uint8_t)outside;
+        border_in[tile * kBorderCells + t] = (uint8_t)outside;
     }
+    const int slots = __syncthreads_count(outside != 0);
+    int edges = __popc(outside);
+    edges = __reduce_add_sync(0xffffffffu, edges);
+    if (lane == 0) atomicAdd(&sm.edges, edges);
     __syncthreads();
-    // subtree sizes, upstream first
-    for (int q = 0; q < rounds; ++q) {
-        for (int k = rstart[q] + t; k < rstart[q + 1]; k += kTileThreads) {
-            const int i = sm.queue[k];
-            unsigned m = sm.up[i];
-            int size = 1;
-            while (m) {
-                size += sz[i + tile_nb_offset(__ffs(m) - 1)];
-                m &= m - 1;
-            }
-            sz[i] = (uint16_t)size;
-        }
-        __syncthreads();
+    if (t == 0) {
+        nslot[tile] = slots;
+        nedge[tile] = sm.edges;
     }
-    // roots (valid cells without an in-tile downstream cell) and invalid cells, in cell order: thread t
-    // owns cells 16 t .. 16 t + 15
-    int* wt = reinterpret_cast<int*>(sm.cnt);  // the counters are free after the rounds
+    const int rounds = sm.rounds, nvalid = rstart[rounds];
+    // roots (valid cells without an in-tile downstream cell) and invalid cells, in cell order: warp w owns the cells
+    // 512 w .. 512 w + 511
+    const int own = (t >> 5) * (kTileCells / (kTileThreads / 32)) + lane;
     int root_sum = 0, invalid = 0;
-    for (int j = 0; j < 16; ++j) {
-        const int i = 16 * t + j;
+    for (int i = own; i < own + 512; i += 32) {
         if (sm.fd[(i >> 6) + 1][(i & 63) + 1] == kNoData) ++invalid;
-        else if (sm.dsl[i] == kNoCell) root_sum += sz[i];
+        else if (sm.dsl[i] == kNoCell) root_sum += sz[2 * i];
     }
+    root_sum = __reduce_add_sync(0xffffffffu, root_sum);
+    invalid = __reduce_add_sync(0xffffffffu, invalid);
     int root_total, invalid_total;
-    int root_base = block_exclusive_int(root_sum, wt, root_total);
-    int invalid_base = root_total + block_exclusive_int(invalid, wt, invalid_total);
-    for (int j = 0; j < 16; ++j) {
-        const int i = 16 * t + j;
-        if (sm.fd[(i >> 6) + 1][(i & 63) + 1] == kNoData) {
-            st[i] = (uint16_t)invalid_base++;
-            sz[i] = 1;
-        } else if (sm.dsl[i] == kNoCell) {
-            st[i] = (uint16_t)root_base;
-            root_base += sz[i];
+    int root_base = block_exclusive_int(lane == 31 ? root_sum : 0, sm.warp_tot, root_total);
+    int invalid_base = root_total + block_exclusive_int(lane == 31 ? invalid : 0, sm.warp_tot, invalid_total);
+    root_base = __shfl_sync(0xffffffffu, root_base, 31);
+    invalid_base = __shfl_sync(0xffffffffu, invalid_base, 31);
+    if (nvalid + invalid_total != kTileCells) {  // uniform: cells on a cycle never become ready
+        if (t == 0) atomicExch(cyclic, 1);
+        return;
+    }
+    // levels within the tile
+    for (int i = t; i < kTileCells; i += kTileThreads) {
+        const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
+        if (row < g.rows && col < g.cols)
+            level[row * g.cols + col] = sm.fd[(i >> 6) + 1][(i & 63) + 1] == kNoData ? -1 : (int32_t)st[2 * i];
+    }
+    const int32_t e0 = exit_base[tile], ne = exit_base[tile + 1] - e0;
+    for (int e = t; e < ne; e += kTileThreads) exit_level[e0 + e] = st[2 * exit_local[e0 + e]];
+    __syncthreads();
+    // first positions of roots and invalid cells; the others' offset from their downstream cell's: after the siblings
+    // that come before them
+    for (int i = own; i < own + 512; i += 32) {
+        const bool bad = sm.fd[(i >> 6) + 1][(i & 63) + 1] == kNoData;
+        const int d = sm.dsl[i];
+        const int size = !bad && d == kNoCell ? sz[2 * i] : 0;
+        const unsigned bads = __ballot_sync(0xffffffffu, bad);
+        if (bad) st[2 * i] = (uint16_t)(invalid_base + __popc(bads & ((1u << lane) - 1u)));
+        invalid_base += __popc(bads);
+        if (__any_sync(0xffffffffu, size != 0)) {
+            int x = size;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (size) st[2 * i] = (uint16_t)(root_base + x - size);
+            root_base += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (d != kNoCell) {
+            int o = 0;
+            for (unsigned m = sm.up[d] & ((1u << nb_index_from(d, i)) - 1u); m; m &= m - 1)
+                o += sz[2 * (d + tile_nb_offset(__ffs(m) - 1))];
+            st[2 * i] = (uint16_t)o;
         }
     }
     __syncthreads();
-    // the other cells, downstream first: after the siblings that come before them
-    for (int q = rounds - 1; q >= 0; --q) {
+    // positions, downstream first; the narrow rounds read the next round's cells ahead
+    if (t < 32) {
+        int q = rounds - 1, k = q >= wide ? rstart[q] + t : 0;
+        int i = q >= wide && k < rstart[q + 1] ? sm.queue[k] : kNoCell, d = i != kNoCell ? sm.dsl[i] : kNoCell;
+        for (; q >= wide; --q) {
+            int i1 = kNoCell, d1 = kNoCell;
+            if (q > wide && rstart[q - 1] + t < rstart[q]) {
+                i1 = sm.queue[rstart[q - 1] + t];
+                d1 = sm.dsl[i1];
+            }
+            if (d != kNoCell) st[2 * i] += st[2 * d];
+            __syncwarp();
+            i = i1;
+            d = d1;
+        }
+    }
+    __syncthreads();
+    for (int q = wide - 1; q >= 0; --q) {
         for (int k = rstart[q] + t; k < rstart[q + 1]; k += kTileThreads) {
             const int i = sm.queue[k], d = sm.dsl[i];
-            if (d == kNoCell) continue;
-            unsigned m = sm.up[d] & ((1u << nb_index_from(d, i)) - 1u);
-            int o = st[d];
-            while (m) {
-                o += sz[d + tile_nb_offset(__ffs(m) - 1)];
-                m &= m - 1;
-            }
-            st[i] = (uint16_t)o;
+            if (d != kNoCell) st[2 * i] += st[2 * d];
         }
         __syncthreads();
     }
     // positions, checked distinct (every position 0 .. 4095 once), the first positions of the roots'
     // subtrees (segment heads), then the tables by position
     const int64_t T = tile * kRunPositions;
-    uint32_t* seen = reinterpret_cast<uint32_t*>(sm.queue);  // the queue is no longer read
+    // the tables are put together here: written cell by cell, each value would be a memory request of its own
+    uint16_t *s_cell = sm.queue, *s_prev = sm.rstart;
+    uint32_t* seen = reinterpret_cast<uint32_t*>(sm.up);
     uint32_t* heads = seen + kRunPositions / 32;
     for (int w = t; w < kRunPositions / 32; w += kTileThreads) {
         seen[w] = 0;
@@ -561,7 +670,7 @@ __global__ void __launch_bounds__(kTileThreads)
     __syncthreads();
     for (int i = t; i < kTileCells; i += kTileThreads) {
         const bool valid = sm.fd[(i >> 6) + 1][(i & 63) + 1] != kNoData;
-        const int s0 = st[i], p = s0 + sz[i] - 1;
+        const int s0 = st[2 * i], p = s0 + sz[2 * i] - 1;
         bool bad = p >= kRunPositions || s0 > p;
         if (!bad) bad = (atomicOr(&seen[p >> 5], 1u << (p & 31)) >> (p & 31)) & 1u;
         if (bad) {
@@ -573,19 +682,23 @@ __global__ void __launch_bounds__(kTileThreads)
     __syncthreads();
     for (int i = t; i < kTileCells; i += kTileThreads) {
         const bool valid = sm.fd[(i >> 6) + 1][(i & 63) + 1] != kNoData;
-        const int s0 = st[i], p = s0 + sz[i] - 1;
+        const int s0 = st[2 * i], p = s0 + sz[2 * i] - 1;
         if (p >= kRunPositions || s0 > p) continue;  // reported above
         const bool head = (heads[p >> 5] >> (p & 31)) & 1u;
-        cell_at[T + run_table_index(p)] =
+        s_cell[run_table_index(p)] =
             (uint16_t)(i | (valid ? 0u : kNoValue) | (head ? kSegHead : 0u) | (s0 == p ? kLoneCell : 0u));
-        prev_at[T + run_table_index(p)] = (uint16_t)(8 * (s0 > 0 ? scan_slot(s0 - 1) : kZeroSlot));
+        s_prev[run_table_index(p)] = (uint16_t)(8 * (s0 > 0 ? scan_slot(s0 - 1) : kZeroSlot));
     }
     __syncthreads();
+    static_assert(kRunPositions == kTileCells, "the tables are staged in arrays of one value per cell");
+    for (int i = t; i < kRunPositions / 8; i += kTileThreads) {
+        reinterpret_cast<uint4*>(cell_at + T)[i] = reinterpret_cast<const uint4*>(s_cell)[i];
+        reinterpret_cast<uint4*>(prev_at + T)[i] = reinterpret_cast<const uint4*>(s_prev)[i];
+    }
     if (t < kRunPositions / 32 && seen[t] != 0xFFFFFFFFu) *error = 1;
-    const int32_t e0 = exit_base[tile], ne = exit_base[tile + 1] - e0;
     for (int e = t; e < ne; e += kTileThreads) {
         const int loc = exit_local[e0 + e];
-        const int s0 = st[loc], p = s0 + sz[loc] - 1;
+        const int s0 = st[2 * loc], p = s0 + sz[2 * loc] - 1;
         exit_span[e0 + e] = (uint32_t)scan_slot(p) | ((uint32_t)(s0 > 0 ? scan_slot(s0 - 1) : kZeroSlot) << 16);
     }
 }
@@ -942,46 +1055,114 @@ __global__ void k_slot_inflow(int64_t nslot, TileSlots q, float* __restrict__ in
     inflow[__ldg(q.at + i)] = slot_inflow(q, i, fixed_point_bits(total[0]));
 }
 
-// Build: per tile, its inflow slots and their upstream exits (one thread per tile, border order).
-__global__ void k_slot_count(int64_t ntiles, const uint8_t* __restrict__ border_in, int32_t* nslot, int32_t* nexit)
+// Build, a CTA per tile: its inflow slots and their upstream exits, in border order (one thread per tile took 316 us
+// at 2048^2, this 6.5 us).
+__global__ void __launch_bounds__(kTileThreads)
+    k_slot_fill(TileGeom g, const uint8_t* __restrict__ border_in, const int32_t* __restrict__ exit_base,
+                const uint64_t* bitmap, const uint16_t* rowpref, const int32_t* __restrict__ slot_base,
+                const int32_t* __restrict__ edge_base, const uint32_t* __restrict__ exit_pos,
+                const uint32_t* __restrict__ exit_start, int32_t* slot_at, int32_t* slot_first, int2* slot_edge,
+                int64_t nexit, int* error)
 {
-    const int64_t tile = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tile >= ntiles) return;
-    int a = 0, b = 0;
-    for (int k = 0; k < kBorderCells; ++k) {
-        const unsigned m = border_in[tile * kBorderCells + k];
-        a += m != 0;
-        b += __popc(m);
+    __shared__ int warp_tot[kTileThreads / 32];
+    const int64_t tr = blockIdx.y, tc = blockIdx.x, tile = tr * g.tcols + tc;
+    const int t = threadIdx.x;
+    const unsigned m0 = t < kBorderCells ? border_in[tile * kBorderCells + t] : 0u;
+    int total;
+    const int32_t s = slot_base[tile] + block_exclusive_int(m0 != 0, warp_tot, total);
+    int32_t e = edge_base[tile] + block_exclusive_int(__popc(m0), warp_tot, total);
+    if (tile == g.trows * g.tcols - 1 && t == 0) slot_first[slot_base[tile + 1]] = edge_base[tile + 1];
+    if (!m0) return;
+    int rin, cin;
+    border_cell(t, rin, cin);
+    slot_at[s] = (int32_t)(tile * kSlotStride + t);
+    slot_first[s] = e;
+    for (unsigned m = m0; m; m &= m - 1) {
+        const int q = __ffs(m) - 1;
+        // a neighbour draining in is an exit of its tile
+        const int64_t y = exit_id_of(g, exit_base, bitmap, rowpref, tr * kTile + rin + nb_dr(q), tc * kTile + cin + nb_dc(q));
+        if (y >= nexit) {
+            atomicExch(error, 1);
+            return;
+        }
+        const uint32_t st = exit_start[y];
+        slot_edge[e++] = make_int2((int)exit_pos[y], st ? (int)(st - 1u) : -1);
     }
-    nslot[tile] = a;
-    nexit[tile] = b;
 }
 
-__global__ void k_slot_fill(int64_t ntiles, const uint8_t* __restrict__ border_in, const int32_t* __restrict__ halo_exit,
-                            const int32_t* __restrict__ slot_base, const int32_t* __restrict__ exit_base,
-                            const uint32_t* __restrict__ exit_pos, const uint32_t* __restrict__ exit_start,
-                            int32_t* slot_at, int32_t* slot_first, int2* slot_edge, int* error)
+// Build, a CTA per tile: the downstream level of every cell, from its level within the tile (k_tile_forest) and the
+// levels of the exits that drain into the tile (k_exit_sizes): each inflow raises the cells below it, up to the first
+// that is at least as high already.  And the raster's statistics [valid, ridge, outlet, sink, -, largest level].
+// A walk over the cells of the whole raster (k_walk) is bound by the longest flow path, a memory round trip per cell:
+// 0.99 ms at 2048^2, where k_exit_sizes, which takes those steps from tile to tile, and this kernel take 18 and 37 us.
+__global__ void __launch_bounds__(kTileThreads)
+    k_tile_levels(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* __restrict__ exit_base,
+                  const uint64_t* bitmap, const uint16_t* rowpref, const uint8_t* __restrict__ border_in,
+                  const int32_t* __restrict__ exit_level, int64_t nexit, int32_t* __restrict__ level,
+                  unsigned long long* stats)
 {
-    const int64_t tile = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tile >= ntiles) return;
-    int32_t s = slot_base[tile], e = exit_base[tile];
-    for (int b = 0; b < kBorderCells; ++b) {
-        const unsigned m0 = border_in[tile * kBorderCells + b];
-        if (!m0) continue;
-        int rin, cin;
-        border_cell(b, rin, cin);
-        slot_at[s] = (int32_t)(tile * kSlotStride + b);
-        slot_first[s] = e;
-        for (unsigned m = m0; m; m &= m - 1) {
-            const int q = __ffs(m) - 1;
-            const int32_t id = halo_exit[tile * kHaloSlots + halo_slot_of(rin + nb_dr(q), cin + nb_dc(q))];
-            if (id < 0) atomicExch(error, 1);  // a neighbour draining in must be an exit of its tile
-            const int32_t y = id < 0 ? 0 : id;
-            const uint32_t st = exit_start[y];
-            slot_edge[e++] = make_int2((int)exit_pos[y], st ? (int)(st - 1u) : -1);
-        }
-        ++s;
+    __shared__ int lv[kTileCells];
+    __shared__ uint8_t code[kTileCells];
+    __shared__ int tally[5];
+    const int64_t tr = blockIdx.y, tc = blockIdx.x, tile = tr * g.tcols + tc;
+    const int t = threadIdx.x, lane = t & 31;
+    if (t < 5) tally[t] = 0;
+    for (int i = t; i < kTileCells; i += kTileThreads) {
+        const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
+        const bool in = row < g.rows && col < g.cols;
+        code[i] = in ? fd[row * g.cols + col] : kNoData;
+        lv[i] = in ? level[row * g.cols + col] : -1;
     }
+    __syncthreads();
+    const unsigned from = t < kBorderCells ? border_in[tile * kBorderCells + t] : 0u;
+    if (from) {
+        int r, c, in = 0;
+        border_cell(t, r, c);
+        for (unsigned m = from; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            const int64_t y = exit_id_of(g, exit_base, bitmap, rowpref, tr * kTile + r + nb_dr(q), tc * kTile + c + nb_dc(q));
+            if (y < nexit) in = max(in, exit_level[y] + 1);
+        }
+        // the tile has no cycle (k_tile_forest): at most one step per cell
+        while (atomicMax(lv + r * kTile + c, in) < in) {
+            int dr, dc;
+            d8_offset(code[r * kTile + c], dr, dc);
+            r += dr;
+            c += dc;
+            if ((dr == 0 && dc == 0) || r < 0 || r >= kTile || c < 0 || c >= kTile || code[r * kTile + c] == kNoData) break;
+            ++in;
+        }
+    }
+    __syncthreads();
+    int valid = 0, ridge = 0, outlet = 0, sink = 0, most = 0;
+    for (int i = t; i < kTileCells; i += kTileThreads) {
+        if (code[i] == kNoData) continue;
+        const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
+        const int l = lv[i];
+        level[row * g.cols + col] = l;
+        ++valid;
+        ridge += l == 0;  // a cell has level 0 when nothing drains into it
+        int dr, dc;
+        if (!d8_offset(code[i], dr, dc)) ++sink;
+        else if (row + dr < 0 || row + dr >= g.rows || col + dc < 0 || col + dc >= g.cols) ++outlet;
+        most = max(most, l);
+    }
+    valid = __reduce_add_sync(0xffffffffu, valid);
+    ridge = __reduce_add_sync(0xffffffffu, ridge);
+    outlet = __reduce_add_sync(0xffffffffu, outlet);
+    sink = __reduce_add_sync(0xffffffffu, sink);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) {
+        atomicAdd(tally + 0, valid);
+        atomicAdd(tally + 1, ridge);
+        atomicAdd(tally + 2, outlet);
+        atomicAdd(tally + 3, sink);
+        atomicMax(tally + 4, most);
+    }
+    __syncthreads();
+    if (t < 4 && tally[t]) atomicAdd(stats + t, (unsigned long long)tally[t]);
+    if (t == 4 && (unsigned long long)tally[4] > *(volatile unsigned long long*)(stats + 5))
+        atomicMax(stats + 5, (unsigned long long)tally[4]);
 }
 
 // Inclusive prefix sums (modulo 2^64) of the thread runs a[0..15] over the whole tile, written to S by
@@ -1541,278 +1722,209 @@ __global__ void __launch_bounds__(kTileThreads, SMALL ? 3 : 4)
 
 static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-int tile_core_build(TopologyCore* core, cudaStream_t stream)
+// Most exits that a raster of this shape can have: a cell whose flow leaves its tile lies beside another tile.
+static int64_t most_exits(int64_t rows, int64_t cols)
 {
+    const int64_t trows = (rows + kTile - 1) / kTile, tcols = (cols + kTile - 1) / kTile;
+    return 2 * ((trows - 1) * cols + (tcols - 1) * rows);
+}
+
+namespace {
+
+// Arrays of the build only.
+struct TileTemp {
+    size_t ctl, bitmap, rowpref, count, nslot, nedge, edge_base, border_in, local, cell, size, counters, parent, plus, level,
+        link, start;
+};
+
+struct TileControl {
+    int cyclic, error, depth;
+    unsigned roots;
+    unsigned long long stats[6];
+};
+
+TileTemp plan_temp(int64_t nt, int64_t E, Arena& a)
+{
+    TileTemp p{};
+    p.ctl = a.add(sizeof(TileControl));
+    p.bitmap = a.add(nt * kTile * 8);
+    p.rowpref = a.add(nt * kTile * 2);
+    p.count = a.add(nt * 4);
+    p.nslot = a.add(nt * 4);
+    p.nedge = a.add(nt * 4);
+    p.edge_base = a.add((nt + 1) * 4);
+    p.border_in = a.add(nt * kBorderCells);
+    p.local = a.add(E * 2);
+    p.cell = a.add(E * 4);
+    p.size = a.add(E * 4);
+    p.counters = a.add(E * 4 * kExitCounters);
+    p.parent = a.add(E * 4);
+    p.plus = a.add(E * 4);
+    p.level = a.add(E * 4);
+    p.link = a.add(E * 8);
+    p.start = a.add(E * 4);
+    return p;
+}
+
+}  // namespace
+
+int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp)
+{
+    const int64_t nt = ((rows + kTile - 1) / kTile) * ((cols + kTile - 1) / kTile), E = most_exits(rows, cols);
+    if (E >= INT32_MAX) return fail(LUE_GPU_ERANGE, "tile topology: too many exits");
+    const size_t before = core.bytes();
+    p->exit_base = core.add((nt + 1) * 4);
+    p->slot_base = core.add((nt + 1) * 4);
+    p->cell_at = core.add(nt * kRunPositions * 2);
+    p->prev_at = core.add(nt * kRunPositions * 2);
+    // an inflow slot and its edges belong to exits of other tiles: at most E of each
+    p->exit_span = core.add(E * 4);
+    p->exit_pos = core.add(E * 4);
+    p->slot_at = core.add(E * 4);
+    p->slot_first = core.add((E + 1) * 4);
+    p->slot_edge = core.add(E * 8);
+    p->bytes = core.bytes() - before;
+    tile_scratch_plan(nt, E, scratch, sp);
+    Arena temp;
+    plan_temp(nt, E, temp);
+    scratch.reserve(temp.bytes());
+    return LUE_GPU_OK;
+}
+
+// Builds the tile structures, the downstream levels and the raster's statistics (hstats: valid, ridge, outlet, sink, 0,
+// largest level) in the planned arenas, and readies the scratch.  *acyclic is false, and core->tiles stays empty, when
+// the network has a flow cycle.  The build's own arrays lie in the handle's scratch.
+int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
+                    const TileScratchPlan& scratch_plan, cudaStream_t stream, bool* acyclic, unsigned long long* hstats)
+{
+    *acyclic = false;
     auto* tc = new (std::nothrow) TileCore();
     if (!tc) return fail(LUE_GPU_ENOMEM, "tile topology: host allocation");
     TileGeom g{core->rows, core->cols, (core->rows + kTile - 1) / kTile, (core->cols + kTile - 1) / kTile};
     tc->trows = g.trows;
     tc->tcols = g.tcols;
     tc->ntiles = g.trows * g.tcols;
-    const int64_t nt = tc->ntiles;
-    uint64_t* bitmap = nullptr;
-    uint16_t* rowpref = nullptr;
-    int32_t* count = nullptr;
-    uint32_t* exit_cell = nullptr;
-    int32_t *parent = nullptr, *nchild = nullptr, *pending = nullptr, *depth = nullptr, *J = nullptr, *J2 = nullptr;
-    uint32_t *size = nullptr, *acc = nullptr;
-    int64_t *D = nullptr, *D2 = nullptr;
-    unsigned long long* root_acc = nullptr;
-    int32_t *sc = nullptr, *ec = nullptr;
-    int* flag = nullptr;
-    std::vector<int32_t> hcount(nt), hbase(nt + 1);
-    int rc = 0, herr = 0;
-    int64_t E = 0;
+    const int64_t nt = tc->ntiles, most = most_exits(core->rows, core->cols);
+    const dim3 grid((unsigned)g.tcols, (unsigned)g.trows);
+    const unsigned exit_ctas = blocks_for(std::max<int64_t>(most, 1), 256);
+    tc->bytes = (int64_t)plan.bytes;
+    tc->exit_base = arena.at<int32_t>(plan.exit_base);
+    tc->slot_base = arena.at<int32_t>(plan.slot_base);
+    tc->cell_at = arena.at<uint16_t>(plan.cell_at);
+    tc->prev_at = arena.at<uint16_t>(plan.prev_at);
+    tc->exit_span = arena.at<uint32_t>(plan.exit_span);
+    tc->exit_pos = arena.at<uint32_t>(plan.exit_pos);
+    tc->slot_at = arena.at<int32_t>(plan.slot_at);
+    tc->slot_first = arena.at<int32_t>(plan.slot_first);
+    tc->slot_edge = arena.at<int2>(plan.slot_edge);
+    Arena sizes;
+    const TileTemp tmp = plan_temp(nt, most, sizes);
+    TileControl* ctl = scratch.at<TileControl>(tmp.ctl);
+    uint64_t* bitmap = scratch.at<uint64_t>(tmp.bitmap);
+    uint16_t* rowpref = scratch.at<uint16_t>(tmp.rowpref);
+    int32_t *count = scratch.at<int32_t>(tmp.count), *nslot = scratch.at<int32_t>(tmp.nslot),
+            *nedge = scratch.at<int32_t>(tmp.nedge), *edge_base = scratch.at<int32_t>(tmp.edge_base);
+    uint8_t* border_in = scratch.at<uint8_t>(tmp.border_in);
+    uint16_t* exit_local = scratch.at<uint16_t>(tmp.local);
+    uint32_t *exit_cell = scratch.at<uint32_t>(tmp.cell), *size = scratch.at<uint32_t>(tmp.size),
+             *exit_start = scratch.at<uint32_t>(tmp.start);
+    int32_t* nchild = scratch.at<int32_t>(tmp.counters);
+    int32_t *pending = nchild + most, *depth = nchild + 2 * most, *seen = nchild + 3 * most;
+    uint32_t* acc = reinterpret_cast<uint32_t*>(nchild + 4 * most);
+    int32_t *parent = scratch.at<int32_t>(tmp.parent), *plus = scratch.at<int32_t>(tmp.plus),
+            *exit_level = scratch.at<int32_t>(tmp.level);
+    int2* link = scratch.at<int2>(tmp.link);
+    int32_t *base = tc->exit_base, *nexit = base + nt, hexit = 0, hslot = 0;
+    TileControl h{};
+    int rc = 0;
 #define TRY(call, what) \
     if ((rc = cuda_status((call), what))) goto error
-    TRY(cudaMalloc(&bitmap, nt * kTile * sizeof(uint64_t)), "tile bitmap");
-    TRY(cudaMalloc(&rowpref, nt * kTile * sizeof(uint16_t)), "tile row prefix");
-    TRY(cudaMalloc(&count, nt * sizeof(int32_t)), "tile exit count");
-    TRY(cudaMalloc(&tc->exit_base, (nt + 1) * sizeof(int32_t)), "tile exit base");
-    TRY(cudaMalloc(&flag, 2 * sizeof(int)), "tile flag");
-    TRY(cudaMemsetAsync(flag, 0, 2 * sizeof(int), stream), "memset");
-    k_exit_bitmap<<<blocks_for(nt * kTile, 256), 256, 0, stream>>>(core->fd, g, bitmap);
-    k_row_prefix<<<blocks_for(nt, 256), 256, 0, stream>>>(bitmap, nt, rowpref, count);
-    TRY(cudaGetLastError(), "tile build");
-    TRY(cudaMemcpyAsync(hcount.data(), count, nt * sizeof(int32_t), cudaMemcpyDeviceToHost, stream), "tile counts");
-    TRY(cudaStreamSynchronize(stream), "tile counts");
-    hbase[0] = 0;
-    for (int64_t i = 0; i < nt; ++i) {
-        if ((int64_t)hbase[i] + hcount[i] > INT32_MAX) {
-            rc = fail(LUE_GPU_ERANGE, "tile topology: too many exits");
-            goto error;
-        }
-        hbase[i + 1] = hbase[i] + hcount[i];
-    }
-    E = hbase[nt];
-    tc->nexit = E;
-    TRY(cudaMemcpyAsync(tc->exit_base, hbase.data(), (nt + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, stream),
-        "tile exit base");
-    TRY(cudaMalloc(&tc->exit_local, std::max<int64_t>(E, 1) * sizeof(uint16_t)), "exit local");
-    TRY(cudaMalloc(&tc->exit_pos, std::max<int64_t>(E, 1) * sizeof(uint32_t)), "exit pos");
-    TRY(cudaMalloc(&tc->exit_start, std::max<int64_t>(E, 1) * sizeof(uint32_t)), "exit start");
-    TRY(cudaMalloc(&tc->halo_exit, nt * kHaloSlots * sizeof(int32_t)), "halo exits");
-    tc->bytes = (nt + 1) * 4 + E * 10 + nt * kHaloSlots * 4;
-    if (E > 0) {
-        TRY(cudaMalloc(&exit_cell, E * sizeof(uint32_t)), "exit cell");
-        TRY(cudaMalloc(&parent, E * sizeof(int32_t)), "exit parent");
-        TRY(cudaMalloc(&nchild, E * sizeof(int32_t)), "exit children");
-        TRY(cudaMalloc(&pending, E * sizeof(int32_t)), "exit pending");
-        TRY(cudaMalloc(&depth, E * sizeof(int32_t)), "exit depth");
-        TRY(cudaMalloc(&size, E * sizeof(uint32_t)), "exit size");
-        TRY(cudaMalloc(&acc, E * sizeof(uint32_t)), "exit acc");
-        TRY(cudaMalloc(&D, E * sizeof(int64_t)), "exit D");
-        TRY(cudaMalloc(&D2, E * sizeof(int64_t)), "exit D2");
-        TRY(cudaMalloc(&J, E * sizeof(int32_t)), "exit J");
-        TRY(cudaMalloc(&J2, E * sizeof(int32_t)), "exit J2");
-        TRY(cudaMalloc(&root_acc, sizeof(unsigned long long)), "root acc");
-        k_exit_list<<<blocks_for(nt * kTile, 256), 256, 0, stream>>>(g, bitmap, rowpref, tc->exit_base, tc->exit_local,
-                                                                     exit_cell);
-        TRY(cudaMemsetAsync(nchild, 0, E * sizeof(int32_t), stream), "memset");
-        k_exit_parent<<<blocks_for(E, 256), 256, 0, stream>>>(core->fd, g, E, exit_cell, tc->exit_base, bitmap, rowpref,
-                                                             parent, nchild, flag);
-        TRY(cudaMemcpyAsync(pending, nchild, E * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream), "copy");
-        {
-            std::vector<uint32_t> ones(E, 1u);
-            TRY(cudaMemcpyAsync(size, ones.data(), E * sizeof(uint32_t), cudaMemcpyHostToDevice, stream), "sizes");
-            TRY(cudaMemsetAsync(depth, 0, E * sizeof(int32_t), stream), "memset");
-            k_exit_sizes<<<blocks_for(E, 256), 256, 0, stream>>>(E, parent, nchild, pending, size, depth);
-            TRY(cudaMemsetAsync(acc, 0, E * sizeof(uint32_t), stream), "memset");
-            TRY(cudaMemsetAsync(root_acc, 0, sizeof(unsigned long long), stream), "memset");
-            k_exit_offsets<<<blocks_for(E, 256), 256, 0, stream>>>(E, parent, size, acc, root_acc, D, J);
-            TRY(cudaGetLastError(), "exit forest");
-            TRY(cudaStreamSynchronize(stream), "exit forest");  // `ones` must outlive the copy
-        }
-        for (int round = 0; round < 40; ++round) {
-            int more = 0;
-            TRY(cudaMemsetAsync(flag + 1, 0, sizeof(int), stream), "memset");
-            k_jump<<<blocks_for(E, 256), 256, 0, stream>>>(E, D, J, D2, J2, flag + 1);
-            std::swap(D, D2);
-            std::swap(J, J2);
-            TRY(cudaMemcpyAsync(&more, flag + 1, sizeof(int), cudaMemcpyDeviceToHost, stream), "jump flag");
-            TRY(cudaStreamSynchronize(stream), "jump");
-            if (!more) {
-                // one more round folds the last parents in (more == 0 means every J2 is now a root)
-                k_jump<<<blocks_for(E, 256), 256, 0, stream>>>(E, D, J, D2, J2, flag + 1);
-                std::swap(D, D2);
-                std::swap(J, J2);
-                break;
-            }
-        }
-        k_exit_positions<<<blocks_for(E, 256), 256, 0, stream>>>(E, D, size, tc->exit_pos, tc->exit_start);
-        TRY(cudaMemsetAsync(nchild, 0, E * sizeof(int32_t), stream), "memset");
-        k_check_positions<<<blocks_for(E, 256), 256, 0, stream>>>(E, tc->exit_pos, tc->exit_start, nchild, flag);
-        {
-            int32_t hmax = 0;
-            std::vector<int32_t> hd(E);
-            TRY(cudaMemcpyAsync(hd.data(), depth, E * sizeof(int32_t), cudaMemcpyDeviceToHost, stream), "depth");
-            TRY(cudaStreamSynchronize(stream), "depth");
-            for (int32_t v : hd) hmax = std::max(hmax, v);
-            tc->max_depth = std::max<int64_t>(hmax, 1);
-        }
-    }
-    k_halo_exits<<<blocks_for(nt * kHaloSlots, 256), 256, 0, stream>>>(core->fd, g, tc->exit_base, bitmap, rowpref,
-                                                                      tc->halo_exit);
-    // per-tile flow forests in post-order
-    TRY(cudaMalloc(&tc->cell_at, nt * kRunPositions * sizeof(uint16_t)), "tile forest");
-    TRY(cudaMalloc(&tc->prev_at, nt * kRunPositions * sizeof(uint16_t)), "tile forest");
-    TRY(cudaMalloc(&tc->exit_span, std::max<int64_t>(E, 1) * sizeof(uint32_t)), "exit span");
-    TRY(cudaMalloc(&tc->border_in, nt * kBorderCells), "tile border masks");
     TRY(cudaFuncSetAttribute(k_tile_forest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)),
-        "tile forest");
-    k_tile_forest<<<dim3((unsigned)g.tcols, (unsigned)g.trows), kTileThreads, sizeof(TileSmem), stream>>>(
-        core->fd, g, tc->exit_base, tc->exit_local, tc->cell_at, tc->prev_at, tc->exit_span, tc->border_in, flag);
-    tc->bytes += nt * kRunPositions * 4 + E * 4 + nt * kBorderCells;
+        "tile topology: shared memory");
+    TRY(cudaMemsetAsync(ctl, 0, sizeof(TileControl), stream), "tile topology");
+    k_exit_bitmap<<<blocks_for(nt, 8), 256, 0, stream>>>(core->fd, g, bitmap, rowpref, count);
+    k_tile_scan<<<1, 1024, 0, stream>>>(count, base, nullptr, nullptr, nt);
+    k_exit_list<<<blocks_for(nt * kTile, 256), 256, 0, stream>>>(g, bitmap, rowpref, base, exit_local, exit_cell, size,
+                                                                 nchild, most);
+    k_tile_forest<<<grid, kTileThreads, sizeof(TileSmem), stream>>>(core->fd, g, base, exit_local, tc->cell_at, tc->prev_at,
+                                                                    tc->exit_span, border_in, nslot, nedge, exit_level,
+                                                                    core->level, &ctl->error, &ctl->cyclic);
+    k_tile_scan<<<1, 1024, 0, stream>>>(nslot, tc->slot_base, nedge, edge_base, nt);
+    k_exit_parent<<<exit_ctas, 256, 0, stream>>>(core->fd, g, nexit, exit_cell, base, bitmap, rowpref, parent, nchild,
+                                                 pending, plus, &ctl->cyclic);
+    k_exit_sizes<<<exit_ctas, 256, 0, stream>>>(nexit, parent, nchild, plus, pending, size, exit_level, depth, &ctl->depth);
+    k_exit_offsets<<<exit_ctas, 256, 0, stream>>>(nexit, parent, pending, size, acc, &ctl->roots, link, &ctl->cyclic);
     TRY(cudaGetLastError(), "tile build");
-    TRY(cudaMemcpyAsync(&herr, flag, sizeof(int), cudaMemcpyDeviceToHost, stream), "tile flag");
+    TRY(cudaMemcpyAsync(&hexit, nexit, sizeof hexit, cudaMemcpyDeviceToHost, stream), "tile exits");
+    TRY(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, stream), "tile build");
     TRY(cudaStreamSynchronize(stream), "tile build");
-    if (herr) {
-        rc = fail(LUE_GPU_EINVAL, "tile topology: cycle inside a tile or inconsistent exit forest");
+    if (h.cyclic) goto error;  // rc == LUE_GPU_OK
+    tc->nexit = hexit;
+    tc->max_depth = std::max(h.depth, hexit > 0 ? 1 : 0);
+    if (hexit > 0) {
+        const unsigned ctas = blocks_for(hexit, 256);
+        for (int64_t reach = 1; reach < tc->max_depth; reach *= 2) k_jump<<<ctas, 256, 0, stream>>>(hexit, link);
+        k_exit_positions<<<ctas, 256, 0, stream>>>(hexit, link, size, tc->exit_pos, exit_start, seen, &ctl->error);
+    }
+    k_slot_fill<<<grid, kTileThreads, 0, stream>>>(g, border_in, base, bitmap, rowpref, tc->slot_base, edge_base, tc->exit_pos,
+                                                   exit_start, tc->slot_at, tc->slot_first, tc->slot_edge, hexit,
+                                                   &ctl->error);
+    k_tile_levels<<<grid, kTileThreads, 0, stream>>>(core->fd, g, base, bitmap, rowpref, border_in, exit_level, hexit,
+                                                     core->level, ctl->stats);
+    TRY(cudaGetLastError(), "tile build");
+    TRY(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, stream), "tile build");
+    TRY(cudaMemcpyAsync(&hslot, tc->slot_base + nt, sizeof hslot, cudaMemcpyDeviceToHost, stream), "tile build");
+    if ((rc = tile_scratch_clear(scratch, scratch_plan, stream))) goto error;
+    TRY(cudaStreamSynchronize(stream), "tile build");
+    if (h.error) {
+        rc = fail(LUE_GPU_EINVAL, "tile topology: inconsistent tile or exit forest");
         goto error;
     }
-    // inflow slots: per tile the border cells receiving flow from other tiles, and their upstream exits
-    {
-        std::vector<int32_t> hs(nt), he(nt), sbase(nt + 1), ebase(nt + 1);
-        TRY(cudaMalloc(&sc, nt * sizeof(int32_t)), "slot count");
-        TRY(cudaMalloc(&ec, nt * sizeof(int32_t)), "slot count");
-        k_slot_count<<<blocks_for(nt, 256), 256, 0, stream>>>(nt, tc->border_in, sc, ec);
-        TRY(cudaGetLastError(), "slot count");
-        TRY(cudaMemcpyAsync(hs.data(), sc, nt * sizeof(int32_t), cudaMemcpyDeviceToHost, stream), "slot count");
-        TRY(cudaMemcpyAsync(he.data(), ec, nt * sizeof(int32_t), cudaMemcpyDeviceToHost, stream), "slot count");
-        TRY(cudaStreamSynchronize(stream), "slot count");
-        int64_t a = 0, b = 0;
-        for (int64_t i = 0; i < nt; ++i) {
-            sbase[i] = (int32_t)a;
-            ebase[i] = (int32_t)b;
-            a += hs[i];
-            b += he[i];
-            if (a > INT32_MAX || b > INT32_MAX) {
-                rc = fail(LUE_GPU_ERANGE, "tile topology: too many inflow slots");
-                goto error;
-            }
-        }
-        sbase[nt] = (int32_t)a;
-        ebase[nt] = (int32_t)b;
-        tc->nslot = a;
-        TRY(cudaMemcpyAsync(ec, ebase.data(), nt * sizeof(int32_t), cudaMemcpyHostToDevice, stream), "slot base");
-        TRY(cudaMalloc(&tc->slot_base, (nt + 1) * sizeof(int32_t)), "slot base");
-        TRY(cudaMemcpyAsync(tc->slot_base, sbase.data(), (nt + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, stream),
-            "slot base");
-        TRY(cudaMalloc(&tc->slot_at, std::max<int64_t>(a, 1) * sizeof(int32_t)), "slots");
-        TRY(cudaMalloc(&tc->slot_first, (a + 1) * sizeof(int32_t)), "slots");
-        TRY(cudaMalloc(&tc->slot_edge, std::max<int64_t>(b, 1) * sizeof(int2)), "slots");
-        TRY(cudaMemcpyAsync(tc->slot_first + a, &ebase[nt], sizeof(int32_t), cudaMemcpyHostToDevice, stream),
-            "slot end");
-        k_slot_fill<<<blocks_for(nt, 256), 256, 0, stream>>>(nt, tc->border_in, tc->halo_exit, tc->slot_base, ec,
-                                                             tc->exit_pos, tc->exit_start, tc->slot_at,
-                                                             tc->slot_first, tc->slot_edge, flag);
-        TRY(cudaGetLastError(), "slot fill");
-        TRY(cudaMemcpyAsync(&herr, flag, sizeof(int), cudaMemcpyDeviceToHost, stream), "tile flag");
-        TRY(cudaStreamSynchronize(stream), "slot fill");  // the host vectors must outlive the copies
-        if (herr) {
-            rc = fail(LUE_GPU_EINVAL, "tile topology: an inflow without an upstream exit");
-            goto error;
-        }
-        tc->bytes += a * 8 + 4 + b * 8 + (nt + 1) * 4;
-    }
-    cudaFree(sc);
-    cudaFree(ec);
-    cudaFree(bitmap);
-    cudaFree(rowpref);
-    cudaFree(count);
-    cudaFree(exit_cell);
-    cudaFree(parent);
-    cudaFree(nchild);
-    cudaFree(pending);
-    cudaFree(depth);
-    cudaFree(size);
-    cudaFree(acc);
-    cudaFree(D);
-    cudaFree(D2);
-    cudaFree(J);
-    cudaFree(J2);
-    cudaFree(root_acc);
-    cudaFree(flag);
+    tc->nslot = hslot;
+    std::memcpy(hstats, h.stats, sizeof h.stats);
     core->tiles = tc;
+    *acyclic = true;
     return LUE_GPU_OK;
 error:
-    cudaFree(sc);
-    cudaFree(ec);
-    cudaFree(bitmap);
-    cudaFree(rowpref);
-    cudaFree(count);
-    cudaFree(exit_cell);
-    cudaFree(parent);
-    cudaFree(nchild);
-    cudaFree(pending);
-    cudaFree(depth);
-    cudaFree(size);
-    cudaFree(acc);
-    cudaFree(D);
-    cudaFree(D2);
-    cudaFree(J);
-    cudaFree(J2);
-    cudaFree(root_acc);
-    cudaFree(flag);
-    tile_core_free(tc);
+    delete tc;
     return rc;
 #undef TRY
 }
 
-void tile_core_free(TileCore* tc)
+// A handle's tile scratch, planned in its arena for up to nexit exits.
+void tile_scratch_plan(int64_t ntiles, int64_t nexit, Arena& a, TileScratchPlan* p)
 {
-    if (!tc) return;
-    cudaFree(tc->exit_base);
-    cudaFree(tc->exit_local);
-    cudaFree(tc->exit_pos);
-    cudaFree(tc->exit_start);
-    cudaFree(tc->halo_exit);
-    cudaFree(tc->cell_at);
-    cudaFree(tc->prev_at);
-    cudaFree(tc->exit_span);
-    cudaFree(tc->border_in);
-    cudaFree(tc->slot_base);
-    cudaFree(tc->slot_at);
-    cudaFree(tc->slot_first);
-    cudaFree(tc->slot_edge);
-    delete tc;
-}
-
-int tile_scratch_alloc(const TileCore* tc, TileScratch* s)
-{
-    const int64_t E = std::max<int64_t>(tc->nexit, 1);
+    const int64_t E = std::max<int64_t>(nexit, 1);
     const int64_t nb = (E + kTileThreads * kScanItemsSmall - 1) / (kTileThreads * kScanItemsSmall);
-    int rc = 0;
-    if ((rc = cuda_status(cudaMalloc(&s->P, E * sizeof(float2)), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->S, E * sizeof(uint4)), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->inflow, tc->ntiles * kSlotStride * sizeof(float)), "tile scratch")))
-        return rc;
-    // slots without inflow are never written: they stay 0
-    if ((rc = cuda_status(cudaMemset(s->inflow, 0, tc->ntiles * kSlotStride * sizeof(float)), "tile scratch")))
-        return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->look_aggr, nb * sizeof(uint4)), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->look_incl, nb * sizeof(uint4)), "tile scratch"))) return rc;
+    p->P = a.add(E * sizeof(float2));
+    p->S = a.add(E * sizeof(uint4));
+    p->look_aggr = a.add(nb * sizeof(uint4));
+    p->look_incl = a.add(nb * sizeof(uint4));
+    // zeroed once: slots without inflow are never written, and
     // total[2], the finished CTAs of the passes, the scan's ticket, its block flags
-    s->ctl_bytes = 2 * sizeof(unsigned long long) + (3 + nb) * sizeof(unsigned);
-    if ((rc = cuda_status(cudaMalloc(&s->total, s->ctl_bytes), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMemset(s->total, 0, s->ctl_bytes), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->redo, 2 * sizeof(unsigned long long)), "tile scratch"))) return rc;
-    if ((rc = cuda_status(cudaMalloc(&s->stat, tc->ntiles * sizeof(TileStat)), "tile scratch"))) return rc;
-    s->bytes = E * (8 + 16) + nb * 32 + s->ctl_bytes + tc->ntiles * (sizeof(TileStat) + kSlotStride * 4);
-    return LUE_GPU_OK;
+    p->inflow = a.add(ntiles * kSlotStride * sizeof(float));
+    p->ctl_bytes = 2 * sizeof(unsigned long long) + (3 + nb) * sizeof(unsigned);
+    p->total = a.add(p->ctl_bytes);
+    p->redo = a.add(2 * sizeof(unsigned long long));
+    p->stat = a.add(ntiles * sizeof(TileStat));
 }
 
-void tile_scratch_free(TileScratch* s)
+void tile_scratch_take(const Arena& a, const TileScratchPlan& p, TileScratch* s)
 {
-    cudaFree(s->P);
-    cudaFree(s->S);
-    cudaFree(s->inflow);
-    cudaFree(s->look_aggr);
-    cudaFree(s->look_incl);
-    cudaFree(s->total);
-    cudaFree(s->redo);
-    cudaFree(s->stat);
-    *s = TileScratch{};
+    s->P = a.at<float2>(p.P);
+    s->S = a.at<uint4>(p.S);
+    s->inflow = a.at<float>(p.inflow);
+    s->look_aggr = a.at<uint4>(p.look_aggr);
+    s->look_incl = a.at<uint4>(p.look_incl);
+    s->total = a.at<unsigned long long>(p.total);
+    s->ctl_bytes = (int64_t)p.ctl_bytes;
+    s->redo = a.at<unsigned long long>(p.redo);
+    s->stat = a.at<TileStat>(p.stat);
+}
+
+int tile_scratch_clear(const Arena& a, const TileScratchPlan& p, cudaStream_t stream)
+{
+    return cuda_status(cudaMemsetAsync(a.at<char>(p.inflow), 0, p.total + p.ctl_bytes - p.inflow, stream), "tile scratch");
 }
 
 // CTAs of k_scan_exits that fit on the device at once (chunks of the exit-forest scan).  The result does

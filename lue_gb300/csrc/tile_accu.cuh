@@ -34,7 +34,6 @@ namespace lue_gb300 {
 constexpr int kTile = 64;                 // tile side (cells)
 constexpr int kTileCells = kTile * kTile;
 constexpr int kHalo = kTile + 2;          // tile side with a one-cell halo
-constexpr int kHaloSlots = 4 * kTile + 4; // N row, S row, W column, E column, NW, NE, SW, SE corners
 constexpr int kTileThreads = 256;
 constexpr int kBorderCells = 4 * kTile - 4;  // cells on the tile's border ring
 
@@ -73,17 +72,12 @@ struct TileCore {
     int64_t nexit = 0;                         // exits (coarse nodes)
     int64_t max_depth = 0;                     // depth of the exit forest
     int32_t* exit_base = nullptr;              // [ntiles + 1] first exit id of each tile (tile-major ids)
-    uint16_t* exit_local = nullptr;            // [nexit] cell index inside its tile (row * 64 + col)
     uint32_t* exit_pos = nullptr;              // [nexit] post-order position
-    uint32_t* exit_start = nullptr;            // [nexit] post-order position of the first node of the subtree
-    int32_t* halo_exit = nullptr;              // [ntiles * kHaloSlots] exit id of the halo cell draining into
-                                               // the tile, or -1
     // Per-tile flow forests in post-order (built once from the flow direction), by post-order position:
     uint16_t* cell_at = nullptr;               // [ntiles * kRunPositions] cell at the position (| kNoValue)
     uint16_t* prev_at = nullptr;               // [ntiles * kRunPositions] 8 x the scan slot before the
                                                // subtree (kZeroSlot for a subtree at position 0)
     uint32_t* exit_span = nullptr;             // [nexit] scan slots of each exit cell: own | before << 16
-    uint8_t* border_in = nullptr;              // [ntiles * kBorderCells] per border cell: outside neighbours draining in
     // Inflow slots (border cells that receive flow from other tiles), per tile in border order:
     int64_t nslot = 0;
     int32_t* slot_base = nullptr;              // [ntiles + 1] first slot of each tile
@@ -119,14 +113,23 @@ struct TileScratch {
     int64_t ctl_bytes = 0;
     unsigned long long* redo = nullptr;        // [2] small rasters: redo[1] set when the walk engine must redo the call
     TileStat* stat = nullptr;                  // [ntiles]
-    int64_t bytes = 0;
+};
+
+// Offsets of a TileCore and of a TileScratch in their arenas.
+struct TileCorePlan {
+    size_t exit_base, slot_base, cell_at, prev_at, exit_span, exit_pos, slot_at, slot_first, slot_edge, bytes;
+};
+struct TileScratchPlan {
+    size_t P, S, look_aggr, look_incl, inflow, total, ctl_bytes, redo, stat;
 };
 
 struct TopologyCore;
 
-int tile_core_build(TopologyCore* core, cudaStream_t stream);
-void tile_core_free(TileCore* tc);
-int tile_scratch_alloc(const TileCore* tc, TileScratch* s);
-void tile_scratch_free(TileScratch* s);
+int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp);
+int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
+                    const TileScratchPlan& scratch_plan, cudaStream_t stream, bool* acyclic, unsigned long long* hstats);
+void tile_scratch_plan(int64_t ntiles, int64_t nexit, Arena& a, TileScratchPlan* p);
+void tile_scratch_take(const Arena& a, const TileScratchPlan& p, TileScratch* s);
+int tile_scratch_clear(const Arena& a, const TileScratchPlan& p, cudaStream_t stream);
 
 }  // namespace lue_gb300

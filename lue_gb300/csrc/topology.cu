@@ -127,39 +127,125 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The handle's stage_flow_error word (with core->stage_mutex held).  Pinned memory takes 110 us to allocate and 160 us
+// to release, more than a small raster's build: only handles that can come to run a stage engine launch have one.
+// A call that is being captured cannot allocate it, so it is there before: from the build of the stage structures on,
+// for the handle that builds them, and from a clone on for both handles (either may then use what the other built).
+int stage_flag(lue_gpu_topology* t)
+{
+    if (t->stage_flow_error) return LUE_GPU_OK;
+    int* flag = nullptr;
+    if (int rc = cuda_status(cudaHostAlloc(&flag, sizeof(int), cudaHostAllocDefault), "scratch flag")) return rc;
+    *flag = 0;
+    t->stage_flow_error = flag;
+    return LUE_GPU_OK;
+}
+
+namespace {
+
+struct ScratchPlan {
+    size_t count, lo;
+    TileScratchPlan tiles;
+};
+
+void plan_scratch(int64_t n, Arena& a, ScratchPlan* p)
+{
+    p->count = a.add(words_for(n) * 4);
+    p->lo = a.add(n * (int64_t)sizeof(float));
+}
+
+void take_scratch(lue_gpu_topology* t, Arena& a, const ScratchPlan& p)
+{
+    t->work_count = a.at<uint32_t>(p.count);
+    t->lo = a.at<float>(p.lo);
+    t->scratch_bytes = (int64_t)a.bytes();
+    if (t->core->tiles) tile_scratch_take(a, p.tiles, &t->tile_scratch);
+}
+
+}  // namespace
+
 int allocate_scratch(lue_gpu_topology* t)
 {
-    const int64_t n = t->core->n;
-    int rc = cuda_status(cudaMalloc(&t->work_count, words_for(n) * 4), "scratch counters");
-    if (rc) return rc;
-    rc = cuda_status(cudaMalloc(&t->lo, n * sizeof(float)), "scratch residuals");
-    if (rc) {
-        cudaFree(t->work_count);
-        t->work_count = nullptr;
+    Arena a;
+    ScratchPlan p{};
+    plan_scratch(t->core->n, a, &p);
+    if (t->core->tiles) tile_scratch_plan(t->core->tiles->ntiles, t->core->tiles->nexit, a, &p.tiles);
+    if (int rc = cuda_status(a.allocate(), "scratch")) return rc;
+    t->arena = a.release();
+    take_scratch(t, a, p);
+    if (!t->core->tiles) return LUE_GPU_OK;
+    if (int rc = tile_scratch_clear(a, p.tiles, nullptr)) return rc;
+    return cuda_status(cudaStreamSynchronize(nullptr), "tile scratch");  // the calls' streams may not wait for it
+}
+
+// The first build of a topology, in two allocations (its own and the handle's scratch, in which the build's arrays lie
+// too): cudaMalloc takes 35 us and cudaFree 30 to 60 us whatever the size, and with one of each for every array (45 and
+// 35) they took half of the build of a 2048^2 raster.  With `tiles`, *acyclic tells whether the network has no cycle; if it has one, or the raster has more
+// exits than the tile engine takes, nothing is kept.
+static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bool tiles, cudaStream_t stream, bool* acyclic,
+                          unsigned long long* hstats)
+{
+    TopologyCore* core = t->core;
+    const int64_t n = core->n, padded = words_for(n) * 4;
+    int rc = 0;
+    Arena a, s;
+    TileCorePlan tile_plan{};
+    ScratchPlan scratch{};
+    const size_t fd = a.add(padded), count = a.add(padded), upmask = a.add(padded),
+                 level = a.add(n * (int64_t)sizeof(int32_t));
+    core->bytes = (int64_t)a.bytes();
+    plan_scratch(n, s, &scratch);
+    *acyclic = false;
+    if (tiles && tile_core_plan(core->rows, core->cols, a, &tile_plan, s, &scratch.tiles)) return LUE_GPU_OK;
+    if ((rc = cuda_status(a.allocate(), "topology"))) return rc;
+    if ((rc = cuda_status(s.allocate(), "scratch"))) return rc;
+    core->fd = a.at<uint8_t>(fd);
+    core->count = a.at<uint8_t>(count);
+    core->upmask = a.at<uint8_t>(upmask);
+    core->level = a.at<int32_t>(level);
+    // the last word is padded with no-data
+    if ((rc = cuda_status(cudaMemsetAsync(core->fd + padded - 4, kNoData, 4, stream), "memset"))) return rc;
+    if ((rc = cuda_status(cudaMemcpyAsync(core->fd, flow_direction, n, cudaMemcpyDeviceToDevice, stream),
+                          "copy flow direction")))
         return rc;
+    if ((rc = cuda_status(cudaMemsetAsync(core->count + padded - 4, 0, 4, stream), "memset"))) return rc;
+    k_count_upmask<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, core->rows, core->cols, 1, core->count, core->upmask);
+    if (tiles) {
+        rc = tile_core_build(core, a, tile_plan, s, scratch.tiles, stream, acyclic, hstats);
+        if (!*acyclic) return rc == LUE_GPU_ECUDA || rc == LUE_GPU_ENOMEM ? rc : LUE_GPU_OK;
+        core->bytes += core->tiles->bytes;
+    } else {  // levels by a walk over the cells
+        uint32_t* work = s.at<uint32_t>(scratch.count);
+        unsigned long long* dstats = nullptr;
+        Arena d;
+        const size_t stats = d.add(6 * sizeof(unsigned long long));
+        if ((rc = cuda_status(d.allocate(), "topology stats"))) return rc;
+        dstats = d.at<unsigned long long>(stats);
+        k_fill_i32<<<grid_for(n, 256), 256, 0, stream>>>(core->level, n, -1);
+        if ((rc = cuda_status(cudaMemcpyAsync(work, core->count, padded, cudaMemcpyDeviceToDevice, stream), "reset counters")))
+            return rc;
+        WalkGrid g{core->fd, core->count, work, core->rows, core->cols, n};
+        LevelVisitor v{core->upmask, core->level, core->cols};
+        k_walk<<<grid_all(n, 256), 256, 0, stream>>>(g, v);
+        if ((rc = cuda_status(cudaMemsetAsync(dstats, 0, d.bytes(), stream), "memset"))) return rc;
+        k_stats<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, core->count, core->level, core->rows, core->cols, dstats);
+        if ((rc = cuda_status(cudaGetLastError(), "topology kernels"))) return rc;
+        if ((rc = cuda_status(cudaMemcpyAsync(hstats, dstats, 6 * sizeof *hstats, cudaMemcpyDeviceToHost, stream), "stats")))
+            return rc;
+        if ((rc = cuda_status(cudaStreamSynchronize(stream), "topology_create"))) return rc;
     }
-    t->scratch_bytes = words_for(n) * 4 + n * (int64_t)sizeof(float);
-    // the stage engine's timeout flag, read by the host on the next call (pinned, written by a copy)
-    rc = cuda_status(cudaHostAlloc(&t->stage_flow_error, sizeof(int), cudaHostAllocDefault), "scratch flag");
-    if (rc) return rc;
-    *t->stage_flow_error = 0;
-    if (t->core->tiles) {
-        rc = tile_scratch_alloc(t->core->tiles, &t->tile_scratch);
-        if (rc) return rc;
-        t->scratch_bytes += t->tile_scratch.bytes;
-    }
+    take_scratch(t, s, scratch);
+    core->arena = a.release();
+    t->arena = s.release();
     return LUE_GPU_OK;
 }
 
 static void free_core(TopologyCore* core)
 {
     if (!core) return;
-    cudaFree(core->fd);
-    cudaFree(core->count);
-    cudaFree(core->upmask);
-    cudaFree(core->level);
+    cudaFree(core->arena);
     cudaFree(core->order);
-    tile_core_free(core->tiles);
+    delete core->tiles;
     stage_core_free(core->stages);
     path_core_free(core->paths);
     delete core;
@@ -168,14 +254,12 @@ static void free_core(TopologyCore* core)
 static void free_handle(lue_gpu_topology* t)
 {
     if (!t) return;
-    cudaFree(t->work_count);
-    cudaFree(t->lo);
+    cudaFree(t->arena);
     cudaFree(t->history);
     cudaFree(t->planes);
     stage_buffers_free(t);
     path_buffers_free(t);
     cudaFreeHost(t->stage_flow_error);
-    tile_scratch_free(&t->tile_scratch);
     if (t->core && --t->core->refs == 0) free_core(t->core);
     delete t;
 }
@@ -218,41 +302,16 @@ extern "C" int lue_gpu_topology_create(const uint8_t* flow_direction, int64_t ro
     core->prow = partition_rows;
     core->pcol = partition_cols;
     core->n = rows * cols;
-    const int64_t n = core->n, padded = words_for(n) * 4;
-    int rc = 0;
-    unsigned long long* dstats = nullptr;
+    // the tile engine needs an acyclic network and 32-bit cell indices; its build gives the levels and statistics
+    bool acyclic = false;
     unsigned long long hstats[6] = {0, 0, 0, 0, 0, 0};
-    if ((rc = cuda_status(cudaMalloc(&core->fd, padded), "topology fd"))) goto error;
-    if ((rc = cuda_status(cudaMalloc(&core->count, padded), "topology count"))) goto error;
-    if ((rc = cuda_status(cudaMalloc(&core->upmask, padded), "topology upmask"))) goto error;
-    if ((rc = cuda_status(cudaMalloc(&core->level, n * sizeof(int32_t)), "topology level"))) goto error;
-    core->bytes = 3 * padded + n * (int64_t)sizeof(int32_t);
-    if ((rc = cuda_status(cudaMalloc(&t->work_count, padded), "scratch counters"))) goto error;
-    if ((rc = cuda_status(cudaMalloc(&dstats, sizeof hstats), "topology stats"))) goto error;
-    if ((rc = cuda_status(cudaMemsetAsync(core->fd, kNoData, padded, stream), "memset"))) goto error;
-    if ((rc = cuda_status(cudaMemcpyAsync(core->fd, flow_direction, n, cudaMemcpyDeviceToDevice, stream),
-                          "copy flow direction")))
-        goto error;
-    if ((rc = cuda_status(cudaMemsetAsync(core->count, 0, padded, stream), "memset"))) goto error;
-    k_count_upmask<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, rows, cols, 1, core->count, core->upmask);
-    k_fill_i32<<<grid_for(n, 256), 256, 0, stream>>>(core->level, n, -1);
-    if ((rc = cuda_status(cudaMemcpyAsync(t->work_count, core->count, padded, cudaMemcpyDeviceToDevice, stream),
-                          "reset counters")))
-        goto error;
-    {
-        WalkGrid g{core->fd, core->count, t->work_count, rows, cols, n};
-        LevelVisitor v{core->upmask, core->level, cols};
-        k_walk<<<grid_all(n, 256), 256, 0, stream>>>(g, v);
+    int rc = LUE_GPU_OK;
+    if (core->n < (int64_t(1) << 32)) rc = build_topology(t, flow_direction, true, stream, &acyclic, hstats);
+    if (!rc && !acyclic) rc = build_topology(t, flow_direction, false, stream, &acyclic, hstats);
+    if (rc) {
+        free_handle(t);
+        return rc;
     }
-    if ((rc = cuda_status(cudaMemsetAsync(dstats, 0, sizeof hstats, stream), "memset"))) goto error;
-    k_stats<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, core->count, core->level, rows, cols, dstats);
-    if ((rc = cuda_status(cudaGetLastError(), "topology kernels"))) goto error;
-    if ((rc = cuda_status(cudaMemcpyAsync(hstats, dstats, sizeof hstats, cudaMemcpyDeviceToHost, stream),
-                          "stats")))
-        goto error;
-    if ((rc = cuda_status(cudaStreamSynchronize(stream), "topology_create"))) goto error;
-    cudaFree(dstats);
-    dstats = nullptr;
     core->stats.rows = rows;
     core->stats.cols = cols;
     core->stats.partition_rows = partition_rows;
@@ -263,26 +322,12 @@ extern "C" int lue_gpu_topology_create(const uint8_t* flow_direction, int64_t ro
     core->stats.sink_cells = (int64_t)hstats[3];
     core->stats.cycle_cells = (int64_t)hstats[4];
     core->stats.max_level = (int64_t)hstats[5];
-    // the tile engine needs an acyclic network and 32-bit cell indices
-    if (core->stats.cycle_cells == 0 && n < (int64_t(1) << 32)) {
-        rc = tile_core_build(core, stream);
-        if (rc == LUE_GPU_ECUDA || rc == LUE_GPU_ENOMEM) goto error;
-        rc = LUE_GPU_OK;
-    }
     if (core->tiles) {
         core->stats.tile_exits = core->tiles->nexit;
         core->stats.exit_forest_depth = core->tiles->max_depth;
-        core->bytes += core->tiles->bytes;
     }
-    cudaFree(t->work_count);
-    t->work_count = nullptr;
-    if ((rc = allocate_scratch(t))) goto error;
     *out = t;
     return LUE_GPU_OK;
-error:
-    cudaFree(dstats);
-    free_handle(t);
-    return rc;
 }
 
 extern "C" int lue_gpu_topology_clone(const lue_gpu_topology* topology, lue_gpu_topology** clone)
@@ -294,6 +339,11 @@ extern "C" int lue_gpu_topology_clone(const lue_gpu_topology* topology, lue_gpu_
     t->core = topology->core;
     t->core->refs++;
     int rc = allocate_scratch(t);
+    if (!rc) {
+        std::lock_guard<std::mutex> lock(t->core->stage_mutex);
+        rc = stage_flag(t);
+        if (!rc) rc = stage_flag(const_cast<lue_gpu_topology*>(topology));
+    }
     if (rc) {
         free_handle(t);
         return rc;

@@ -14,6 +14,7 @@ namespace lue_gb300 {
 // Immutable part, shared by a topology and its clones.
 struct TopologyCore {
     int64_t rows = 0, cols = 0, prow = 0, pcol = 0, n = 0;
+    void* arena = nullptr;      // one allocation for fd, count, upmask and level
     uint8_t* fd = nullptr;      // device copy of the flow direction raster
     uint8_t* count = nullptr;   // inflow count, 255 where the flow direction is no-data
     uint8_t* upmask = nullptr;  // bit k set: neighbour k (NW, N, NE, W, E, SW, S, SE) drains here
@@ -37,6 +38,7 @@ struct TopologyCore {
 
 struct lue_gpu_topology {
     lue_gb300::TopologyCore* core = nullptr;
+    void* arena = nullptr;           // one allocation for work_count, lo and the tile scratch
     uint32_t* work_count = nullptr;  // per-call copy of the counts, 4 cells per word
     float* lo = nullptr;             // per-call float-float residuals of f32 routing
     lue_gb300::TileScratch tile_scratch;
@@ -61,6 +63,7 @@ struct lue_gpu_topology {
 namespace lue_gb300 {
 
 int allocate_scratch(lue_gpu_topology* t);
+int stage_flag(lue_gpu_topology* t);
 
 // The reference's partitions of a raster: the last partition of a row or column absorbs the remainder
 // (source/framework/core/include/lue/framework/core/domain_decomposition.hpp:90-175).
