@@ -213,38 +213,51 @@ __global__ void k_exit_list(TileGeom g, const uint64_t* bitmap, const uint16_t* 
     }
 }
 
-// Parent of every exit: follow the flow from its downstream cell through that cell's tile.  plus: the cells from the
-// exit to its parent.
+// Border cell b (0..251: N row, S row, W column, E column without corners) of a tile.
+__device__ __forceinline__ void border_cell(int b, int& rin, int& cin)
+{
+    if (b < kTile) { rin = 0; cin = b; }
+    else if (b < 2 * kTile) { rin = kTile - 1; cin = b - kTile; }
+    else if (b < 3 * kTile - 2) { rin = b - 2 * kTile + 1; cin = 0; }
+    else { rin = b - (3 * kTile - 2) + 1; cin = kTile - 1; }
+}
+
+// The border cell at (rin, cin).
+__device__ __forceinline__ int border_index(int rin, int cin)
+{
+    if (rin == 0) return cin;
+    if (rin == kTile - 1) return kTile + cin;
+    return (cin == 0 ? 2 * kTile : 3 * kTile - 2) + rin - 1;
+}
+
+// Parent of every exit: the root of its downstream cell in that cell's tile, if an exit.  plus: the cells from the exit
+// to its parent.
+// The roots come from k_tile_forest, which walks to them in shared memory: walking here, a round trip to memory per
+// cell, took 33 us at 2048^2 instead of 6.
 __global__ void k_exit_parent(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* nexit, const uint32_t* exit_cell,
                               const int32_t* exit_base, const uint64_t* bitmap, const uint16_t* rowpref,
-                              int32_t* parent, int32_t* nchild, int32_t* pending, int32_t* plus, int* cyclic)
+                              const uint32_t* __restrict__ border_root, int32_t* parent, int32_t* nchild, int32_t* pending,
+                              int32_t* plus)
 {
     int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (y >= *nexit) return;
-    int64_t cell = exit_cell[y];
+    const int64_t cell = exit_cell[y];
     int64_t r = cell / g.cols, c = cell % g.cols;
     int dr, dc;
     d8_offset(fd[cell], dr, dc);
     r += dr;
     c += dc;
-    int64_t tile = tile_of(g, r, c);
     int32_t p = -1;
-    int step = 0;
-    for (; step <= kTileCells; ++step) {
-        uint8_t code = fd[r * g.cols + c];
-        if (code == kNoData || !d8_offset(code, dr, dc)) break;  // sink (or flow into no-data): root
-        int64_t r2 = r + dr, c2 = c + dc;
-        if (r2 < 0 || r2 >= g.rows || c2 < 0 || c2 >= g.cols) break;  // leaves the array: root
-        if (tile_of(g, r2, c2) != tile) {
-            p = exit_id_of(g, exit_base, bitmap, rowpref, r, c);
-            break;
-        }
-        r = r2;
-        c = c2;
-        if (step == kTileCells) atomicExch(cyclic, 1);  // a cycle inside a tile
+    if (fd[r * g.cols + c] != kNoData) {
+        const int64_t tile = tile_of(g, r, c);
+        const uint32_t root = border_root[tile * kBorderCells + border_index((int)(r % kTile), (int)(c % kTile))];
+        const int rin = (int)((root & kIndexMask) >> 6), cin = (int)(root & 63u);
+        const uint64_t m = bitmap[tile * kTile + rin];
+        if ((m >> cin) & 1ull)
+            p = exit_base[tile] + rowpref[tile * kTile + rin] + __popcll(m & ((1ull << cin) - 1ull));
+        plus[y] = (int32_t)(root >> 12) + 1;
     }
     parent[y] = p;
-    plus[y] = step + 1;
     if (p >= 0) {
         atomicAdd(nchild + p, 1);
         atomicAdd(pending + p, 1);
@@ -437,15 +450,6 @@ __device__ __forceinline__ int nb_index_from(int d, int c)
     return idx < 4 ? idx : idx - 1;
 }
 
-// Border cell b (0..251: N row, S row, W column, E column without corners) of a tile.
-__device__ __forceinline__ void border_cell(int b, int& rin, int& cin)
-{
-    if (b < kTile) { rin = 0; cin = b; }
-    else if (b < 2 * kTile) { rin = kTile - 1; cin = b - kTile; }
-    else if (b < 3 * kTile - 2) { rin = b - 2 * kTile + 1; cin = 0; }
-    else { rin = b - (3 * kTile - 2) + 1; cin = kTile - 1; }
-}
-
 // Exclusive prefix of one int per thread over the block; `total` gets the block sum.
 __device__ __forceinline__ int block_exclusive_int(int v, int* warp_tot, int& total)
 {
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__(kTileThreads)
     k_tile_forest(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* __restrict__ exit_base,
                   const uint16_t* __restrict__ exit_local, uint16_t* cell_at, uint16_t* prev_at,
                   uint32_t* exit_span, uint8_t* border_in, int32_t* nslot, int32_t* nedge, int32_t* exit_level,
-                  int32_t* __restrict__ level, int* error, int* cyclic)
+                  int32_t* __restrict__ level, uint32_t* __restrict__ border_root, int* error, int* cyclic)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileSmem& sm = *reinterpret_cast<TileSmem*>(smem_raw);
@@ -566,6 +570,11 @@ __global__ void __launch_bounds__(kTileThreads)
             }
         }
         border_in[tile * kBorderCells + t] = (uint8_t)outside;
+        if (outside) {  // where that flow leaves the tile or ends
+            int i = rin * kTile + cin, steps = 0;
+            for (int d; (d = sm.dsl[i]) != kNoCell && steps < kTileCells; ++steps) i = d;
+            border_root[tile * kBorderCells + t] = (uint32_t)i | ((uint32_t)steps << 12);
+        }
     }
     const int slots = __syncthreads_count(outside != 0);
     int edges = __popc(outside);
@@ -1094,7 +1103,7 @@ __global__ void __launch_bounds__(kTileThreads)
 // levels of the exits that drain into the tile (k_exit_sizes): each inflow raises the cells below it, up to the first
 // that is at least as high already.  And the raster's statistics [valid, ridge, outlet, sink, -, largest level].
 // A walk over the cells of the whole raster (k_walk) is bound by the longest flow path, a memory round trip per cell:
-// 0.99 ms at 2048^2, where k_exit_sizes, which takes those steps from tile to tile, and this kernel take 18 and 37 us.
+// 0.99 ms at 2048^2, where k_exit_sizes, which takes those steps from tile to tile, and this kernel take 19 and 33 us.
 __global__ void __launch_bounds__(kTileThreads)
     k_tile_levels(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* __restrict__ exit_base,
                   const uint64_t* bitmap, const uint16_t* rowpref, const uint8_t* __restrict__ border_in,
@@ -1106,12 +1115,16 @@ __global__ void __launch_bounds__(kTileThreads)
     __shared__ int tally[5];
     const int64_t tr = blockIdx.y, tc = blockIdx.x, tile = tr * g.tcols + tc;
     const int t = threadIdx.x, lane = t & 31;
+    // thread t: column t & 63 of every fourth row
+    constexpr int kCells = kTileCells / kTileThreads, kStep = kTileThreads / kTile;
+    const int64_t row0 = tr * kTile + (t >> 6), col = tc * kTile + (t & 63), cell0 = row0 * g.cols + col, step = kStep * g.cols;
+    const int rows = col < g.cols ? (int)min((int64_t)kTile, max((int64_t)0, g.rows - row0)) : 0;  // this thread's, by kStep
     if (t < 5) tally[t] = 0;
-    for (int i = t; i < kTileCells; i += kTileThreads) {
-        const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
-        const bool in = row < g.rows && col < g.cols;
-        code[i] = in ? fd[row * g.cols + col] : kNoData;
-        lv[i] = in ? level[row * g.cols + col] : -1;
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) {
+        const bool in = k * kStep < rows;
+        code[t + k * kTileThreads] = in ? fd[cell0 + k * step] : kNoData;
+        lv[t + k * kTileThreads] = in ? level[cell0 + k * step] : -1;
     }
     __syncthreads();
     const unsigned from = t < kBorderCells ? border_in[tile * kBorderCells + t] : 0u;
@@ -1123,28 +1136,33 @@ __global__ void __launch_bounds__(kTileThreads)
             const int64_t y = exit_id_of(g, exit_base, bitmap, rowpref, tr * kTile + r + nb_dr(q), tc * kTile + c + nb_dc(q));
             if (y < nexit) in = max(in, exit_level[y] + 1);
         }
-        // the tile has no cycle (k_tile_forest): at most one step per cell
-        while (atomicMax(lv + r * kTile + c, in) < in) {
-            int dr, dc;
-            d8_offset(code[r * kTile + c], dr, dc);
-            r += dr;
-            c += dc;
-            if ((dr == 0 && dc == 0) || r < 0 || r >= kTile || c < 0 || c >= kTile || code[r * kTile + c] == kNoData) break;
-            ++in;
+        // the tile has no cycle (k_tile_forest): at most one step per cell.  The walk waits for its loads only, not for
+        // the maximum: whoever raised a cell first goes on below it.
+        for (int i = r * kTile + c; *(volatile int*)(lv + i) < in; ++in) {
+            atomicMax(lv + i, in);
+            int d, q;
+            if (!tile_downstream(code[i], i >> 6, i & 63, d, q) || code[d] == kNoData) break;
+            i = d;
         }
     }
     __syncthreads();
     int valid = 0, ridge = 0, outlet = 0, sink = 0, most = 0;
-    for (int i = t; i < kTileCells; i += kTileThreads) {
-        if (code[i] == kNoData) continue;
-        const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
-        const int l = lv[i];
-        level[row * g.cols + col] = l;
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) {
+        const unsigned c = code[t + k * kTileThreads];
+        if (c == kNoData) continue;
+        const int l = lv[t + k * kTileThreads];
+        level[cell0 + k * step] = l;
         ++valid;
         ridge += l == 0;  // a cell has level 0 when nothing drains into it
-        int dr, dc;
-        if (!d8_offset(code[i], dr, dc)) ++sink;
-        else if (row + dr < 0 || row + dr >= g.rows || col + dc < 0 || col + dc >= g.cols) ++outlet;
+        const unsigned pad = c - 1u;  // numeric pad: 0 .. 8 from the lower left, 4 in the middle
+        if (pad > 8u || pad == 4u) {
+            ++sink;
+        } else {
+            const int up = (int)(pad * 11u >> 5), right = (int)pad - 3 * up;
+            const int64_t row = row0 + k * kStep + 1 - up, to = col + right - 1;
+            outlet += row < 0 || row >= g.rows || to < 0 || to >= g.cols;
+        }
         most = max(most, l);
     }
     valid = __reduce_add_sync(0xffffffffu, valid);
@@ -1733,7 +1751,7 @@ namespace {
 
 // Arrays of the build only.
 struct TileTemp {
-    size_t ctl, bitmap, rowpref, count, nslot, nedge, edge_base, border_in, local, cell, size, counters, parent, plus, level,
+    size_t ctl, bitmap, rowpref, count, nslot, nedge, edge_base, border_in, border_root, local, cell, size, counters, parent, plus, level,
         link, start;
 };
 
@@ -1754,6 +1772,7 @@ TileTemp plan_temp(int64_t nt, int64_t E, Arena& a)
     p.nedge = a.add(nt * 4);
     p.edge_base = a.add((nt + 1) * 4);
     p.border_in = a.add(nt * kBorderCells);
+    p.border_root = a.add(nt * kBorderCells * 4);
     p.local = a.add(E * 2);
     p.cell = a.add(E * 4);
     p.size = a.add(E * 4);
@@ -1827,7 +1846,7 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
     uint8_t* border_in = scratch.at<uint8_t>(tmp.border_in);
     uint16_t* exit_local = scratch.at<uint16_t>(tmp.local);
     uint32_t *exit_cell = scratch.at<uint32_t>(tmp.cell), *size = scratch.at<uint32_t>(tmp.size),
-             *exit_start = scratch.at<uint32_t>(tmp.start);
+             *exit_start = scratch.at<uint32_t>(tmp.start), *border_root = scratch.at<uint32_t>(tmp.border_root);
     int32_t* nchild = scratch.at<int32_t>(tmp.counters);
     int32_t *pending = nchild + most, *depth = nchild + 2 * most, *seen = nchild + 3 * most;
     uint32_t* acc = reinterpret_cast<uint32_t*>(nchild + 4 * most);
@@ -1848,10 +1867,10 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
                                                                  nchild, most);
     k_tile_forest<<<grid, kTileThreads, sizeof(TileSmem), stream>>>(core->fd, g, base, exit_local, tc->cell_at, tc->prev_at,
                                                                     tc->exit_span, border_in, nslot, nedge, exit_level,
-                                                                    core->level, &ctl->error, &ctl->cyclic);
+                                                                    core->level, border_root, &ctl->error, &ctl->cyclic);
     k_tile_scan<<<1, 1024, 0, stream>>>(nslot, tc->slot_base, nedge, edge_base, nt);
-    k_exit_parent<<<exit_ctas, 256, 0, stream>>>(core->fd, g, nexit, exit_cell, base, bitmap, rowpref, parent, nchild,
-                                                 pending, plus, &ctl->cyclic);
+    k_exit_parent<<<exit_ctas, 256, 0, stream>>>(core->fd, g, nexit, exit_cell, base, bitmap, rowpref, border_root, parent,
+                                                 nchild, pending, plus);
     k_exit_sizes<<<exit_ctas, 256, 0, stream>>>(nexit, parent, nchild, plus, pending, size, exit_level, depth, &ctl->depth);
     k_exit_offsets<<<exit_ctas, 256, 0, stream>>>(nexit, parent, pending, size, acc, &ctl->roots, link, &ctl->cyclic);
     TRY(cudaGetLastError(), "tile build");
