@@ -417,22 +417,32 @@ __global__ void k_path_cuts(const int32_t* order, int64_t p0, int64_t p1, int64_
 // per-call kernels.
 static int64_t path_padded(int64_t npos) { return ((npos + 7) / 8 + 1) * 8; }
 
-// Positions per thread of a level's scan: 4 on large levels (2 and 8 were slower there), 1 on small ones (short
-// chains of dependent loads per thread).
-constexpr int64_t kPathSmallLevel = 1 << 20;
-
-// A level scans without look-back when its longest path is at most kPathFreeChunks chunks of a CTA; the CTA ranges of a
-// large level are then that many chunks, cut at path tops.  One chunk leaves most ranges a second one that is nearly empty
-// and more levels with look-back (accu_threshold at 16384^2: 11.3 ms), four lengthen the serial part of a CTA (6.8
-// ms; accu_fraction at 2311 x 1501: 189 us against 136 us); two: 6.6 ms.
-constexpr int kPathFreeChunks = 2;
-// Small levels, which cannot fill the GPU, take half a chunk per CTA: most ranges are then one chunk, and the launch is
-// over sooner (accu_fraction at 2311 x 1501 119 -> 100 us, accu_trigger at 1500^2 161 -> 134 us; a quarter: 99 and 135).
-constexpr int64_t kPathTinyLevel = 1 << 18;
-static int64_t path_cut_step(int per, int64_t n)
+// Positions per thread of a level's scan.  Level 0: 4 from 2^20 positions on (2 and 8 were slower there).  The levels
+// above wait for memory more than they compute (0.97 instructions per cycle with four positions a thread), and read
+// their first slots with their inputs when two positions leave the registers for it: 2 from 2^18 positions on
+// (accu_threshold at 8192^2 / 16384^2 in us: four positions 1963 / 6928, two 1803 / 6661, two and the shorter CTA
+// ranges below 1735 / 6445; one: 1908 at 8192^2).  Small levels: 1, short chains of dependent loads per thread.
+constexpr int64_t kPathSmallLevel = 1 << 20, kPathTinyLevel = 1 << 18;
+static int path_per(int level, int64_t n)
 {
-    const int64_t T = (int64_t)kPathThreads * per;
-    return n < kPathTinyLevel ? T / 2 : T * kPathFreeChunks;
+    if (level > 0) return n < kPathTinyLevel ? 1 : 2;
+    return n < kPathSmallLevel ? 1 : 4;
+}
+
+// A level scans without look-back when its longest path is at most this many positions.
+static int path_free_longest(int per) { return per == 1 ? 2 * kPathThreads : 8 * kPathThreads; }
+
+// Positions of a CTA's range in such a level, cut at path tops.  Level 0: two chunks less a sixteenth, as a range runs on
+// to the next top (accu_threshold at 8192^2: 1.2 % faster than two whole chunks; one chunk leaves most ranges a second
+// one that is nearly empty, 11.3 ms at 16384^2, and four lengthen the serial part of a CTA, 6.8 ms against 6.6).  Large
+// levels above: one chunk, more CTAs to wait on memory at once (two: 6661 us).  Small levels, which cannot fill
+// the GPU: half a chunk, so most ranges are one chunk and the launch is over sooner (accu_fraction at 2311 x 1501 119 ->
+// 100 us, accu_trigger at 1500^2 161 -> 134 us; a quarter: 99 and 135).
+static int64_t path_cut_step(int level, int64_t n)
+{
+    const int64_t T = (int64_t)kPathThreads * path_per(level, n);
+    if (n < kPathTinyLevel) return T / 2;
+    return level > 0 ? T : 2 * T - T / 16;
 }
 
 void path_core_free(PathCore* pc)
@@ -521,9 +531,9 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
         v.p0 = hstart[l];
         v.p1 = hstart[l + 1] = (int32_t)(hstart[l] + (int64_t)hcells[l]);
         v.longest = hstats[3 + l];
-        v.per = v.p1 - v.p0 < kPathSmallLevel ? 1 : 4;
+        v.per = path_per(l, v.p1 - v.p0);
         v.cut0 = (int32_t)ncuts;
-        v.ncut = (int32_t)((v.p1 - v.p0 + path_cut_step(v.per, v.p1 - v.p0) - 1) / path_cut_step(v.per, v.p1 - v.p0));
+        v.ncut = (int32_t)((v.p1 - v.p0 + path_cut_step(l, v.p1 - v.p0) - 1) / path_cut_step(l, v.p1 - v.p0));
         ncuts += v.ncut + 1;
         pc->tiles = std::max<int64_t>(pc->tiles, (v.p1 - v.p0) / (kPathThreads * v.per) + 2);
     }
@@ -562,10 +572,12 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
                                                           pc->slot_first, pc->slot_base, rows, cols, pc->path_slot,
                                                           stats + 2);
         // 6. CTA ranges of the scans
-        for (const PathLevel& v : pc->levels)
+        for (int l = 0; l < levels; ++l) {
+            const PathLevel& v = pc->levels[l];
             if (v.ncut > 0)
                 k_path_cuts<<<(unsigned)(((v.ncut + 1) * 32 + 255) / 256), 256, 0, stream>>>(
-                    pc->order, v.p0, v.p1, path_cut_step(v.per, v.p1 - v.p0), v.ncut, pc->cut + v.cut0);
+                    pc->order, v.p0, v.p1, path_cut_step(l, v.p1 - v.p0), v.ncut, pc->cut + v.cut0);
+        }
         launches += 8 + levels;
         long long hslots = 0;
         int bad = 0;
@@ -950,6 +962,9 @@ __device__ __forceinline__ void load_order(const P& p, int64_t first, int32_t (&
     if (PER == 4) {
         const int4 x = __ldg(reinterpret_cast<const int4*>(p.order + first));
         w[0] = x.x; w[1 % PER] = x.y; w[2 % PER] = x.z; w[3 % PER] = x.w;
+    } else if (PER == 2) {
+        const int2 x = __ldg(reinterpret_cast<const int2*>(p.order + first));
+        w[0] = x.x; w[1 % PER] = x.y;
     } else {
 #pragma unroll
         for (int j = 0; j < PER; ++j) w[j] = __ldg(p.order + first + j);
@@ -1038,9 +1053,7 @@ struct Chunk {
     unsigned nan;            // bit j: no-data from the cell itself or its light inflow
     T e[PER], b[PER];
     typename N::V sum[PER];
-    // the positions' first slots, read with the inputs; with four positions their registers would spill
-    static constexpr bool kEarly = LIGHT && PER == 1;
-    int32_t f[kEarly ? PER + 1 : 1];
+    int32_t f[LIGHT ? PER + 1 : 1];  // the positions' first slots
 
     __device__ __forceinline__ int32_t first_slot(const PathCall<N>& p, int32_t first, int j) const
     {
@@ -1065,7 +1078,7 @@ struct Chunk {
 
     __device__ __forceinline__ void gather(const PathCall<N>& p, int32_t first)
     {
-        if constexpr (kEarly) {
+        if constexpr (LIGHT) {
 #pragma unroll
             for (int j = 0; j <= PER; ++j) f[j] = first_slot(p, first, j);
         }
@@ -1086,18 +1099,12 @@ struct Chunk {
     {
         nan = 0;
         if (LIGHT) {
-            int32_t at[PER + 1];
-#pragma unroll
-            for (int j = 0; j <= PER; ++j) {
-                if constexpr (kEarly) at[j] = f[j];
-                else at[j] = first_slot(p, first, j);
-            }
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
                 sum[j] = N::zero();
                 if (!((on >> j) & 1u)) continue;
                 bool bad = false;
-                for (int32_t k = at[j]; k < at[j + 1]; ++k) N::light(sum[j], bad, p.slots[k]);
+                for (int32_t k = f[j]; k < f[j + 1]; ++k) N::light(sum[j], bad, p.slots[k]);
                 nan |= bad ? 1u << j : 0u;
             }
         }
@@ -1368,16 +1375,17 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
             if (int rc = cuda_status(cudaMemsetAsync(status, 0, nt_max * sizeof(int), stream), what)) return rc;
         }
         const int T = kPathThreads * v.per;
-        const bool free = v.longest <= (free_longest >= 0 ? free_longest : kPathFreeChunks * T);
+        const bool free = v.longest <= (free_longest >= 0 ? free_longest : path_free_longest(v.per));
         const unsigned blocks =
             free ? (unsigned)v.ncut : (unsigned)((v.p1 - (v.p0 & ~(v.per - 1)) + T - 1) / T);
         if (blocks == 0) continue;
         const PathScan<K> q{status, aggm, aggm + nt_max, tickets + l, t->path_epoch, polls};
-        switch (2 * (v.per > 1) + (l > 0)) {
-            case 0: launch_level<N, R, K, 1, false>(free, blocks, stream, p, v, q, pc->cut); break;
-            case 1: launch_level<N, R, K, 1, true>(free, blocks, stream, p, v, q, pc->cut); break;
-            case 2: launch_level<N, R, K, 4, false>(free, blocks, stream, p, v, q, pc->cut); break;
-            default: launch_level<N, R, K, 4, true>(free, blocks, stream, p, v, q, pc->cut); break;
+        if (l == 0) {
+            if (v.per == 1) launch_level<N, R, K, 1, false>(free, blocks, stream, p, v, q, pc->cut);
+            else launch_level<N, R, K, 4, false>(free, blocks, stream, p, v, q, pc->cut);
+        } else {
+            if (v.per == 1) launch_level<N, R, K, 1, true>(free, blocks, stream, p, v, q, pc->cut);
+            else launch_level<N, R, K, 2, true>(free, blocks, stream, p, v, q, pc->cut);
         }
         ++launches;
     }
