@@ -445,9 +445,27 @@ static int64_t path_cut_step(int level, int64_t n)
     return level > 0 ? T : 2 * T - T / 16;
 }
 
+// From this many cells on, the two results of a rule are collected by position and spread over the raster by a kernel of
+// its own (k_path_spread).  Below, the raster stays in L2, where partial writes cost little (accu_threshold 2048 x
+// 2500: 183 us straight, 194 spread; 2600 x 2700: 247 and 241; 2900^2: 288 and 271; 4000 x 4100: 528 and 460; 8192^2:
+// 1746 and 1415; 16384^2: 6461 and 4959).  accu has one result of 8 bytes, where it is slower at every size (8192^2: 1779
+// and 1912).  LUE_GB300_PATH_SPREAD: another limit (test hook).
+constexpr int64_t kPathSpreadCells = int64_t(1) << 23;
+static int64_t path_spread_cells()
+{
+    const char* e = getenv("LUE_GB300_PATH_SPREAD");
+    return e ? atoll(e) : kPathSpreadCells;
+}
+
+__global__ void k_path_at(const int32_t* order, int64_t npos, int32_t* at)
+{
+    for (int64_t i = grid_stride_begin(); i < npos; i += grid_stride()) at[order[i] & 0x7fffffff] = (int32_t)i;
+}
+
 void path_core_free(PathCore* pc)
 {
     if (!pc) return;
+    cudaFree(pc->at);
     cudaFree(pc->order);
     cudaFree(pc->path_slot);
     cudaFree(pc->slot_first);
@@ -589,6 +607,15 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
         if (bad) {
             rc = fail(LUE_GPU_ERANGE, "path topology: inconsistent layout (" + std::to_string(bad) + " misplaced)");
             goto done;
+        }
+        if (n >= path_spread_cells()) {  // in an array of the build that has served
+            TRY(cudaMemsetAsync(dtop, 0xFF, n * sizeof(int32_t), stream));
+            k_path_at<<<grid_for(npos, 256), 256, 0, stream>>>(pc->order, npos, dtop);
+            TRY(cudaStreamSynchronize(stream));
+            TRY(cudaGetLastError());
+            pc->at = dtop;
+            dtop = nullptr;
+            pc->bytes += n * 4;
         }
     }
     count_launches(launches);
@@ -941,6 +968,7 @@ struct PathCall {
     typename N::T* out;
     typename N::T* rem;
     typename N::Slot* slots;                 // what leaves each path; written by a level, read by higher ones
+    float2* dense;                           // both results by position, or nullptr: straight to out and rem
     unsigned long long* flag;
 };
 
@@ -1148,8 +1176,13 @@ struct Chunk {
             T rem = T(0);
             rule_total<R>(t, b[j], x, rem);
             odd |= !xnan && !(N::hi(t) < T(INFINITY));
-            p.out[c] = xnan ? qnan<T>() : N::hi(x);
-            if (R != Rule::accu) p.rem[c] = xnan ? qnan<T>() : rem;
+            const T o = xnan ? qnan<T>() : N::hi(x), left = xnan ? qnan<T>() : rem;
+            if (R != Rule::accu && p.dense) {
+                p.dense[first + j] = make_float2((float)o, (float)left);
+            } else {
+                p.out[c] = o;
+                if (R != Rule::accu) p.rem[c] = left;
+            }
             const int32_t next = j + 1 < PER && first + j + 1 < hi ? w[(j + 1) % PER] : after;
             if (next < 0) {  // a path bottom
                 const int32_t slot = __ldg(p.path_slot + first + j);
@@ -1251,6 +1284,41 @@ __global__ void __launch_bounds__(kPathThreads, 4)
     }
 }
 
+// The results from their positions to the raster, a CTA per 64 x 64 tile; no-data cells (without a position) get NaN.
+//
+// Stored cell by cell while a level runs, each result is a partial write of a sector of its own, most of them after
+// the rest of the sector has left L2: 2.4 of accu_threshold's 6.4 ms at 16384^2 (level 1: 1.21 ms, and 0.44 by position).
+// By position they are dense, and a tile's positions are close together, so this kernel's reads hit L1 and its
+// writes are whole rows: bound by memory, 0.88 ms at 16384^2 (20 bytes a cell, 6.1 TB/s).
+__global__ void __launch_bounds__(256)
+    k_path_spread(const int32_t* __restrict__ at, const float2* __restrict__ dense, int64_t rows, int64_t cols, int64_t tcols,
+                  float* __restrict__ out, float* __restrict__ rem)
+{
+    constexpr int kCells = 8, kStep = 256 / kPathTile;
+    const int64_t tr = blockIdx.x / tcols, tc = blockIdx.x - tr * tcols;
+    const int64_t row0 = tr * kPathTile + threadIdx.x / kPathTile, col = tc * kPathTile + threadIdx.x % kPathTile;
+    if (col >= cols) return;
+#pragma unroll
+    for (int h = 0; h < kPathTile / (kCells * kStep); ++h) {
+        int32_t i[kCells];
+        float2 v[kCells];
+#pragma unroll
+        for (int k = 0; k < kCells; ++k) {
+            const int64_t r = row0 + (h * kCells + k) * kStep;
+            i[k] = r < rows ? __ldcs(at + r * cols + col) : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < kCells; ++k) v[k] = i[k] >= 0 ? __ldg(dense + i[k]) : make_float2(qnan<float>(), qnan<float>());
+#pragma unroll
+        for (int k = 0; k < kCells; ++k) {
+            const int64_t r = row0 + (h * kCells + k) * kStep;
+            if (r >= rows) continue;
+            __stcs(out + r * cols + col, v[k].x);
+            __stcs(rem + r * cols + col, v[k].y);
+        }
+    }
+}
+
 template <class T>
 __global__ void k_path_no_data(const uint8_t* fd, int64_t n, T* out, T* rem)
 {
@@ -1293,6 +1361,8 @@ void path_buffers_free(lue_gpu_topology* t)
     cudaFree(t->path_maps);
     cudaFree(t->path_ctl);
     cudaFree(t->path_slots);
+    cudaFree(t->path_dense);
+    t->path_dense = nullptr;
     t->path_maps = nullptr;
     t->path_ctl = nullptr;
     t->path_slots = nullptr;
@@ -1315,6 +1385,14 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
         (rc = cuda_status(cudaMemsetAsync(t->path_ctl, 0, ctl, stream), what))) {
         path_buffers_free(t);
         return rc;
+    }
+    if (pc->at) {
+        if (cudaMalloc(&t->path_dense, pc->npos * 8) == cudaSuccess) {
+            t->scratch_bytes += pc->npos * 8;
+        } else {  // without it the levels write straight to the raster
+            t->path_dense = nullptr;
+            cudaGetLastError();
+        }
     }
     t->path_epoch = 0;
     t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (int64_t)ctl + ns * 8;
@@ -1356,11 +1434,13 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
     int* status = tickets + kPathMaxLevels + 2;
     if (int rc = cuda_status(cudaMemsetAsync(flag, 0, kPathCtlZeroed, stream), what)) return rc;
     int launches = 0;
-    if (pc->npos < n) {
+    float2* dense = R != Rule::accu ? static_cast<float2*>(t->path_dense) : nullptr;
+    if (pc->npos < n && !dense) {
         k_path_no_data<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, n, out, rem);
         ++launches;
     }
-    const PathCall<N> p{pc->order, pc->path_slot, pc->slot_first - pc->slot_base, a, as, b, bs, out, rem, static_cast<typename N::Slot*>(t->path_slots), flag};
+    const PathCall<N> p{pc->order, pc->path_slot, pc->slot_first - pc->slot_base, a, as, b, bs, out, rem, static_cast<typename N::Slot*>(t->path_slots),
+                        dense, flag};
     // test hooks: LUE_GB300_PATH_FREE_LONGEST (levels with longer paths use the look-back scan; 0: every
     // level) and LUE_GB300_PATH_POLLS (poll limit of a look-back wait; 0: every wait gives up at once,
     // and the walk engine redoes the call)
@@ -1388,6 +1468,13 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
             else launch_level<N, R, K, 2, true>(free, blocks, stream, p, v, q, pc->cut);
         }
         ++launches;
+    }
+    if constexpr (R != Rule::accu) {
+        if (dense) {
+            const int64_t tcols = (core->cols + kPathTile - 1) / kPathTile, trows = (core->rows + kPathTile - 1) / kPathTile;
+            k_path_spread<<<(unsigned)(trows * tcols), 256, 0, stream>>>(pc->at, dense, core->rows, core->cols, tcols, out, rem);
+            ++launches;
+        }
     }
     // +-inf inputs, or a wait of the scan that gave up: the walk engine redoes the whole call (as behind
     // the tile engine of accu)
