@@ -125,6 +125,8 @@ struct TileScratchPlan {
 
 struct TopologyCore;
 
+// Whether a grid holds the tile rows.
+inline bool tile_rows_fit(int64_t rows) { return (rows + kTile - 1) / kTile <= 65535; }
 int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp);
 int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
                     const TileScratchPlan& scratch_plan, cudaStream_t stream, bool* acyclic, unsigned long long* hstats);

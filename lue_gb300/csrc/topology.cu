@@ -345,9 +345,18 @@ extern "C" int lue_gpu_topology_create(const uint8_t* flow_direction, int64_t ro
     // the tile engine needs an acyclic network and 32-bit cell indices; its build gives the levels and statistics
     bool acyclic = false;
     unsigned long long hstats[6] = {0, 0, 0, 0, 0, 0};
-    int rc = LUE_GPU_OK;
-    if (core->n < (int64_t(1) << 32)) rc = build_topology(t, flow_direction, true, stream, &acyclic, hstats);
+    int rc = LUE_GPU_OK, tiles = LUE_GPU_OK;
+    if (core->n < (int64_t(1) << 32)) {
+        // without a grid or the memory for the tiles only rasters with cycles, which have none, are taken
+        if (tile_rows_fit(rows)) {
+            tiles = build_topology(t, flow_direction, true, stream, &acyclic, hstats);
+            if (tiles == LUE_GPU_ECUDA) rc = tiles;
+        } else {
+            tiles = LUE_GPU_ECUDA;
+        }
+    }
     if (!rc && !acyclic) rc = build_topology(t, flow_direction, false, stream, &acyclic, hstats);
+    if (!rc && tiles && hstats[4] == 0) rc = fail(tiles, "topology_create: no memory or grid for the tile structures");
     if (rc) {
         free_handle(t);
         return rc;

@@ -103,3 +103,12 @@ def test_build(lfr, name):
     if s["cycle_cells"] == 0:
         got = lfr.to_numpy(lfr.accu(a, lfr.from_numpy(np.ones(fd.shape, np.float32))))
         assert np.array_equal(got, accu.astype(np.float32), equal_nan=True)
+
+
+def test_more_tile_rows_than_a_grid_holds(lfr):
+    fd = np.full((64 * 65535 + 1, 1), 5, np.uint8)
+    with pytest.raises(RuntimeError):
+        lfr.from_numpy(fd).topology()
+    fd[0], fd[1] = 2, 8  # a cycle: no tiles are needed
+    s = lfr.from_numpy(fd).topology().stats()
+    assert s["cycle_cells"] == 2 and s["sink_cells"] == fd.size - 2
