@@ -109,15 +109,15 @@ int lue_gpu_topology_clone(const lue_gpu_topology* topology, lue_gpu_topology** 
 int lue_gpu_topology_destroy(lue_gpu_topology* topology);
 int lue_gpu_topology_get_stats(const lue_gpu_topology* topology, lue_gpu_topology_stats* stats);
 /* Builds now, on `stream`, what the first call of an operation would otherwise build: the path layout of
- * float32 accu_threshold / accu_capacity and the stage structures of accu_threshold / accu_fraction /
- * accu_capacity / accu_trigger / float64 accu / kinematic_wave (shared by the clones of the handle).
+ * float32 accu_threshold / accu_fraction / accu_capacity / accu_trigger and float64 accu, and the stage structures of
+ * the other float64 rules and kinematic_wave (shared by the clones of the handle).
  * Returns when they are built.  A serving loop
  * calls it when it loads a raster, so that no request pays for it.  (No reference counterpart: the
  * reference keeps no state between calls.) */
 int lue_gpu_topology_prepare(lue_gpu_topology* topology, void* stream);
 
-/* Schedule of the stage engine (accu_threshold, accu_fraction, accu_capacity, accu_trigger, float64 accu,
- * kinematic_wave).  No reference counterpart: the reference's schedule is HPX's task order over its
+/* Schedule of the stage engine (float64 accu_threshold, accu_fraction, accu_capacity and accu_trigger,
+ * kinematic_wave; with LUE_GB300_ENGINE=stage the float32 rules and float64 accu too).  No reference counterpart: the reference's schedule is HPX's task order over its
  * partitions.  Results do not depend on the schedule, only the time a call takes does.
  *   cap            most cells of one stage (1..256, default 128).  It belongs to the stage structures,
  *                  which the clones of a handle share: setting another cap frees them (they are rebuilt by

@@ -660,7 +660,7 @@ done:
 // (a1, b1 + b2, c1 + b2); with c1 < a2 what m1 holds back stays held back: (max(a1, a2 - b1), b1 + b2, c2).
 //
 // On the stage engine accu_trigger was bound by its chain of rounds (1500^2: 1595 us a call); as a scan it
-// takes 319 us.
+// takes 134 us.
 constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2, kTrigger = 3, kSum = 4;
 
 // a, b and c float-float.  flags bit 0: the map of a path's top cell, which ignores its input (its value is

@@ -1,12 +1,12 @@
-// path_route.cuh — the path engine: accu_threshold, accu_fraction, accu_capacity and accu_trigger (float32)
-// as prefix scans along the heavy paths of the flow forest.
+// path_route.cuh — the path engine: accu_threshold, accu_fraction, accu_capacity and accu_trigger (float32) and accu
+// (float64) as prefix scans along the heavy paths of the flow forest.
 //
 // Along one flow path the threshold rule maps the outflow x of the upstream cell to
 // max(x + s - threshold, 0), the fraction rule to fraction * (x + s), the capacity rule to
-// min(x + s, capacity) and the trigger rule to x + s where that reaches the trigger, else 0, where s is the material of the cell plus the outflow of its other upstream cells.
-// These maps compose into maps of the same form (path_route.cu, PMap), so the
-// outflows of a whole path follow from a prefix scan of the per-cell maps instead of a cell-by-cell walk
-// (ALG/definition/accumulating_router.hpp:525-599 walks them one cell after the other;
+// min(x + s, capacity) and the trigger rule to x + s where that reaches the trigger, else 0, where s is the material
+// of the cell plus the outflow of its other upstream cells.  These maps compose into maps of the same form
+// (path_route.cu, PMap), so the outflows of a whole path follow from a prefix scan of the per-cell maps instead of a
+// cell-by-cell walk (ALG/definition/accumulating_router.hpp:525-599 walks them one cell after the other;
 // ALG/definition/accu_threshold.hpp:124-169, ALG/definition/accu_fraction.hpp:124-162 and
 // ALG/definition/accu_capacity.hpp and accu_trigger.hpp enter_cell are the cell rules).
 //

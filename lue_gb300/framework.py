@@ -84,7 +84,7 @@ class Topology:
         return Topology._from_handle(h, self.shape, self.device)
 
     def prepare(self):
-        """Builds the structures that the first call of a stage-engine operation (accu_threshold,
+        """Builds the structures that the first call of a path- or stage-engine operation (accu_threshold,
         accu_fraction, accu_capacity, accu_trigger, float64 accu, kinematic_wave) would build."""
         import torch
         _lib.check(_lib.lib().lue_gpu_topology_prepare(self.handle,
