@@ -660,7 +660,7 @@ done:
 // (a1, b1 + b2, c1 + b2); with c1 < a2 what m1 holds back stays held back: (max(a1, a2 - b1), b1 + b2, c2).
 //
 // On the stage engine accu_trigger was bound by its chain of rounds (1500^2: 1595 us a call); as a scan it
-// takes 134 us.
+// takes 121 us.
 constexpr int kMaxPlus = 0, kMinPlus = 1, kAffine = 2, kTrigger = 3, kSum = 4;
 
 // a, b and c float-float.  flags bit 0: the map of a path's top cell, which ignores its input (its value is
@@ -1010,14 +1010,22 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v)
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Decoupled look-back of one level's launch: CTAs take tiles in ticket order; each publishes the
-// composition of its tile's maps (state 1), then the composition of everything before and including its
-// tile (state 2).  Status words carry the launch's epoch, so the arrays need no clearing between launches.
+// Look-back of one level's launch: CTAs take tiles in ticket order.  A tile publishes the composition of its own maps:
+// state 3 when that is a constant (a path's top is among its positions, so nothing before the tile matters), else
+// state 1, and then, if its number is a multiple of 32, also the composition of everything up to and including it
+// (state 2).  Status words carry the launch's epoch, so the arrays need no clearing between launches.
+//
+// A tile composes the tiles before it from the nearest constant one, or from the nearest published prefix (it is at most
+// 32 tiles away) if that comes first.  Which ones these are depends on the layout alone, not on which CTA is how far: the
+// same call gives the same bits every time, in plain doubles too.  The only chain of waits is that of the prefixes,
+// one every 32 tiles along a river.  Composing whatever tiles have published so far (every tile its prefix) takes longer as
+// well, since every tile publishes twice: accu (float64) over a basin of 3001 x 2777 264 us a call, this 246;
+// accu_trigger at 1500^2 138 and 121.
 template <int K>
 struct PathScan {
     int* status;  // [tiles] epoch << 2 | state
     PMap<K>* aggm;   // [tiles] the tile's own composition
-    PMap<K>* inclm;  // [tiles] the composition up to and including the tile
+    PMap<K>* inclm;  // [tiles] the composition up to and including the tile (multiples of 32)
     int* ticket;  // zeroed before the launch
     int epoch;
     int polls;    // poll limit of one wait
@@ -1025,48 +1033,42 @@ struct PathScan {
 
 constexpr int kPathPolls = 1 << 20;
 
-// Warp 0: the composition of all tiles before `tile` (in every lane).  Lane i looks at tile j - i, 32 at
-// a time, until a tile with a published prefix is among them.  Every wait is bounded: a wait that gives
-// up (or finds that another one did) sets flag[1], after which the walk engine redoes the call.
+// Warp 0: the composition of all tiles before `tile` (in every lane); lane i looks at tile `tile` - 1 - i.  The wait is
+// bounded: one that gives up (or finds that another one did) sets flag[1], after which the call is redone.
 template <int K>
-__device__ PMap<K> look_back(const PathScan<K>& q, int64_t tile, unsigned long long* flag)
+__device__ PMap<K> look_back(const PathScan<K>& q, int tile, unsigned long long* flag)
 {
-    const int lane = threadIdx.x & 31;
-    PMap<K> running = pm_identity<K>();
-    for (int64_t j = tile - 1;; j -= 32) {
-        const int64_t idx = j - lane;
-        int st = 2;
-        PMap<K> m = pm_identity<K>();
-        if (idx >= 0) {
-            int v = 0, k = 0;
-            for (; k < q.polls; ++k) {
-                v = ld_acquire_gpu(q.status + idx);
-                if ((v >> 2) == q.epoch && (v & 3) != 0) break;
-                if (*reinterpret_cast<volatile unsigned long long*>(flag + 1)) k = q.polls - 1;
-                __nanosleep(32);
-            }
-            if (k >= q.polls) {
-                st = -1;
-            } else {
-                st = v & 3;
-                m = pm_each(*(st == 2 ? q.inclm + idx : q.aggm + idx), [](const auto& v) { return __ldcg(&v); });
-            }
+    const int lane = threadIdx.x & 31, idx = tile - 1 - lane;
+    const bool fence = (idx & 31) == 0;
+    int state = 0, stop = -1;
+    for (int k = 0; k < q.polls; ++k) {
+        if (idx >= 0 && state < (fence ? 2 : 1)) {
+            const int v = ld_acquire_gpu(q.status + idx);
+            state = (v >> 2) == q.epoch ? v & 3 : 0;
         }
-        if (__ballot_sync(0xffffffffu, st < 0)) {
-            if (lane == 0) flag[1] = 1;
-            return pm_identity<K>();
+        const bool ready = state >= (fence ? 2 : 1);
+        const unsigned ends = __ballot_sync(0xffffffffu, ready && (fence || state == 3));
+        const unsigned missing = __ballot_sync(0xffffffffu, !ready);
+        // the nearest end counts, once every tile before it is there: farther ones may be there already
+        if (ends && !(missing & (ends ^ (ends - 1u)))) {
+            stop = __ffs(ends) - 1;
+            break;
         }
-        const unsigned incl = __ballot_sync(0xffffffffu, st == 2);
-        if (incl && lane > __ffs(incl) - 1) m = pm_identity<K>();
-        // lanes 31 .. 0 in this order (farther tiles come first)
-        for (int d = 1; d < 32; d <<= 1) {
-            const PMap<K> o = shfl_down(m, d);
-            if (lane + d < 32) m = compose<K>(o, m);
-        }
-        const PMap<K> window = pm_each(m, [](auto v) { return __shfl_sync(0xffffffffu, v, 0); });
-        running = compose<K>(window, running);
-        if (incl) return running;
+        if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned long long*>(flag + 1) != 0)) break;
+        __nanosleep(32);
     }
+    if (stop < 0) {
+        if (lane == 0) flag[1] = 1;
+        return pm_identity<K>();
+    }
+    PMap<K> m = pm_identity<K>();
+    if (lane <= stop) m = pm_each(*(state == 2 ? q.inclm + idx : q.aggm + idx), [](const auto& v) { return __ldcg(&v); });
+    // lanes 31 .. 0 in this order (farther tiles come first)
+    for (int d = 1; d < 32; d <<= 1) {
+        const PMap<K> o = shfl_down(m, d);
+        if (lane + d < 32) m = compose<K>(o, m);
+    }
+    return pm_each(m, [](auto v) { return __shfl_sync(0xffffffffu, v, 0); });
 }
 
 // The positions of one thread in one chunk of a scan: PER consecutive positions from `first`, those in
@@ -1194,7 +1196,7 @@ struct Chunk {
 };
 
 // The scan of one level with very long paths: tiles in ticket order, the composition of the tiles before each
-// one by decoupled look-back.
+// one by look-back.
 template <class N, Rule R, int K, int PER, bool LIGHT>
 __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, PathLevel v, PathScan<K> q)
 {
@@ -1214,26 +1216,20 @@ __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, P
     PMap<K> total;
     const PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
     if (threadIdx.x < 32) {
-        if (tile == 0) {
-            if (threadIdx.x == 0) {
-                q.inclm[0] = total;
-                __threadfence();
-                st_release_gpu(q.status, (q.epoch << 2) | 2);
-                s_prefix = pm_identity<K>();
-            }
-        } else {
-            if (threadIdx.x == 0) {
-                q.aggm[tile] = total;
-                __threadfence();
-                st_release_gpu(q.status + tile, (q.epoch << 2) | 1);
-            }
-            const PMap<K> before = look_back<K>(q, tile, p.flag);
-            if (threadIdx.x == 0) {
+        const bool constant = tile == 0 || (total.flags & 1);  // a level begins with a top
+        if (threadIdx.x == 0) {
+            q.aggm[tile] = total;
+            __threadfence();
+            st_release_gpu(q.status + tile, (q.epoch << 2) | (constant ? 3 : 1));
+        }
+        const PMap<K> before = tile ? look_back<K>(q, tile, p.flag) : pm_identity<K>();
+        if (threadIdx.x == 0) {
+            if (!constant && (tile & 31) == 0) {
                 q.inclm[tile] = compose<K>(before, total);
                 __threadfence();
                 st_release_gpu(q.status + tile, (q.epoch << 2) | 2);
-                s_prefix = before;
             }
+            s_prefix = before;
         }
     }
     __syncthreads();
