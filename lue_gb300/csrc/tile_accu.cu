@@ -2005,10 +2005,13 @@ int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, fl
     const TileSlots slots{tc->slot_base, tc->slot_at, tc->slot_first, tc->slot_edge, s->S};
     *redo = small ? s->redo : s->total;
     *reset = small;
-    // a small call leaves its control words at 0
-    if (!small)
+    // a small call leaves its control words at 0, unless one of its launches was refused
+    if (!small || s->dirty)
         if (int rc = cuda_status(cudaMemsetAsync(s->total, 0, s->ctl_bytes, stream), "accu_f32 (tiles)")) return rc;
+    s->dirty = small;
     constexpr size_t smem = sizeof(TileCallSmem);
+    // test hook: LUE_GB300_TILE_REFUSE asks for more shared memory than there is, so that pass 3's launch is refused
+    const size_t refused = getenv("LUE_GB300_TILE_REFUSE") ? size_t(1) << 20 : 0;
     if (small)
         k_tile_exits<true><<<tile_grid, kTileThreads, smem, stream>>>(g, ext, ext_s, vec_in, f, tc->exit_base,
                                                                       tc->exit_span, tc->exit_pos, s->P, s->total,
@@ -2040,13 +2043,15 @@ int tile_accu_f32(const TopologyCore* core, TileScratch* s, const float* ext, fl
         }
     }
     if (small)
-        launch_after(k_tile_accu<true>, tile_grid, kTileThreads, smem, stream, g, ext, ext_s, vec_in && vec_out, out, f,
+        launch_after(k_tile_accu<true>, tile_grid, kTileThreads, smem + refused, stream, g, ext, ext_s, vec_in && vec_out, out, f,
                      s->stat, s->total, slots, q);
     else
         k_tile_accu<false><<<tile_grid, kTileThreads, smem, stream>>>(g, ext, ext_s, vec_in && vec_out, out, f, s->stat,
                                                                       s->total, slots, q);
     count_launches(1);
-    return cuda_status(cudaGetLastError(), "accu_f32 (tiles)");
+    const int rc = cuda_status(cudaGetLastError(), "accu_f32 (tiles)");
+    if (!rc) s->dirty = false;
+    return rc;
 }
 
 }  // namespace lue_gb300

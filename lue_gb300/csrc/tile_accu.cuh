@@ -112,6 +112,8 @@ struct TileScratch {
     unsigned long long* total = nullptr;
     int64_t ctl_bytes = 0;
     unsigned long long* redo = nullptr;        // [2] small rasters: redo[1] set when the walk engine must redo the call
+    bool dirty = false;                        // a small raster's call whose launches were not all taken: its control
+                                               // words are not 0, and the next call clears them first
     TileStat* stat = nullptr;                  // [ntiles]
 };
 
