@@ -3,6 +3,7 @@
 // per path level.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 
 #include "route_walk_visitors.cuh"
@@ -1147,7 +1148,8 @@ struct Chunk {
             bad = bad || !in_domain<R>(e[j], b[j]);
             if constexpr (LIGHT) sum[j] = N::cell(sum[j], e[j]);
             else sum[j] = N::from(e[j]);
-            odd |= act && !bad && !(N::hi(sum[j]) < T(INFINITY) && b[j] < T(INFINITY));
+            // a trigger that nothing reaches is an ordinary map: its a is infinite, which compose() only compares
+            odd |= act && !bad && !(N::hi(sum[j]) < T(INFINITY) && (R == Rule::trigger || b[j] < T(INFINITY)));
             if (bad) {
                 sum[j] = N::zero();
                 b[j] = T(0);
@@ -1156,7 +1158,7 @@ struct Chunk {
             const PMap<K> m = cell_map<R, K>(w[j] < 0, sum[j], b[j], bad);
             if (act) acc = j == 0 ? m : compose<K>(acc, m);
         }
-        if (odd) p.flag[1] = 1;  // +inf: the walk engine redoes the call
+        if (odd) p.flag[1] = 1;  // +inf: the call is redone
         return acc;
     }
 
@@ -1315,6 +1317,261 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+__device__ __forceinline__ double from_lane(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ float2 from_lane(float2 v, int lane)
+{
+    return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+__device__ __forceinline__ FF from_lane(FF v, int lane)
+{
+    return FF{__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane)};
+}
+
+// What a step takes besides the flow along the path, from the lane that holds it.  bits: number of values added after that
+// flow (the first in `then`), kFlow when there is one, kAlone when nothing is added before it, kNone for no-data.
+constexpr unsigned kFlow = 16, kAlone = 32, kNone = 64;
+template <class Visitor>
+struct RedoStep {
+    decltype(Visitor::Total::t) t;
+    typename Visitor::Up then;
+    unsigned bits;
+    typename Visitor::T x, y;
+    template <class Total, class Up, class T>
+    static __device__ __forceinline__ RedoStep from(const Total& s, Up then, unsigned bits, T x, T y, int lane)
+    {
+        return RedoStep{from_lane(s.t, lane), from_lane(then, lane), __shfl_sync(0xffffffffu, bits, lane),
+                        __shfl_sync(0xffffffffu, x, lane), __shfl_sync(0xffffffffu, y, lane)};
+    }
+};
+
+// A slot without its value yet: a NaN that no rule gives.  A value is one word, so it needs no fence.
+constexpr unsigned long long kEmptySlot = ~0ull;
+template <class Up>
+__device__ __forceinline__ bool read_slot(const unsigned long long* p, Up& u)
+{
+    static_assert(sizeof(Up) == sizeof(unsigned long long), "a slot is one word");
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    memcpy(&u, &w, sizeof u);
+    return w != kEmptySlot;
+}
+template <class Up>
+__device__ __forceinline__ void write_slot(unsigned long long* p, Up u)
+{
+    unsigned long long w;
+    memcpy(&w, &u, sizeof w);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+
+// A call redone cell by cell (flag[1] of the engine: infinite values, or a look-back wait that gave up), with the cell rule of
+// the walk engine, so the results are that engine's bit for bit.  Persistent warps empty the slots, then take chunks
+// of positions in ticket order, each the paths whose tops lie in it.  A warp's lanes load what 32 positions need besides
+// the flow along their path, and the next 32 positions' inputs while the warp takes these steps one after the other,
+// every lane all of them.  It waits for the slots that its positions take: their paths are of lower levels, so lie at
+// lower positions, in chunks of earlier tickets, held by warps that run.  Waits are bounded, by far more than the paths before
+// can take; when one gives up, the last warp readies the counters of the walk over cells and sets walk[1].
+//
+// Bound by the chain of steps along the longest paths (55 to 120 ns a step), on large rasters also by issue (0.06 to 0.08
+// ns a cell).  With one infinite cell, 1500^2 / 4096^2 / 8192^2: accu (float64) 1.1 / 3.7 / 11.2 ms a call, accu_trigger 1.0 /
+// 3.1 / 9.3 ms; by the walk over cells (a dependent counter and its fences per step) 7.8 / 31 / 102 and 9.0 / 38 / 126 ms.
+constexpr int kRedoThreads = 256, kRedoChunk = 256, kRedoFill = 8192;
+struct PathRedo {
+    const int32_t* order;
+    const int32_t* path_slot;
+    const int32_t* slot_first;          // by position (the engine's array minus its base)
+    unsigned long long* slots;
+    int64_t npos, slot_base, nslots;
+    const unsigned long long* flag;
+    unsigned long long* walk;           // [2]
+    unsigned* ctl;                      // ticket, filled chunks of slots, finished warps, a wait gave up
+    long long polls;                    // poll limit of one wait
+    const uint32_t* count;              // what the walk's counters start from
+    uint32_t* work;
+    int64_t nwords;
+};
+
+// One position of a window: its order entry and inputs, loaded ahead.
+template <class Visitor>
+struct RedoCell {
+    typename Visitor::T x, y;
+    unsigned mask;       // upstream neighbours
+    int32_t slot;        // first of its slots
+    __device__ __forceinline__ void load(const PathRedo& q, const Visitor& v, int64_t i, int32_t w)
+    {
+        const int32_t c = w & 0x7fffffff;
+        const bool in = i < q.npos;
+        x = in ? v.first(c) : 0;
+        y = in ? v.second(c) : 0;
+        mask = in ? __ldg(v.upmask + c) : 0u;
+        slot = in && i >= q.slot_base ? __ldg(q.slot_first + i) : 0;
+    }
+};
+
+// The paths whose tops lie in [at, stop); false: a wait gave up.
+template <class Visitor>
+__device__ __forceinline__ bool redo_chunk(const PathRedo& q, Visitor& v, int64_t at, int64_t stop)
+{
+    using Up = typename Visitor::Up;
+    using T = typename Visitor::T;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t p1 = q.npos, first = next_top(q.order, at, stop);
+    if (first >= stop) return true;
+    // order entries of the window and of the next one
+    int32_t w = first + lane < p1 ? __ldg(q.order + first + lane) : -1;
+    int32_t w1 = first + 32 + lane < p1 ? __ldg(q.order + first + 32 + lane) : -1;
+    RedoCell<Visitor> cell;
+    cell.load(q, v, first + lane, w);
+    int32_t before_c = -1;  // the cell before the window's first
+    Up flow{};
+    for (int64_t i0 = first; i0 < p1; i0 += 32) {
+        const int32_t c = w & 0x7fffffff;
+        // the last window ends where the first path that another chunk takes begins
+        const int64_t i = i0 + lane;
+        const unsigned ends = __ballot_sync(kAll, i >= p1 || (i >= stop && w < 0));
+        const int steps = ends ? __ffs(ends) - 1 : 32;
+        const bool on = lane < steps;
+        // the flow along the path (none into its top) comes in the place of its neighbour: values before it and after
+        const int32_t up = __shfl_up_sync(kAll, c, 1), from = lane ? up : before_c;
+        int before = 0;
+        bool along = false;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (!((cell.mask >> k) & 1u) || along) continue;
+            if (c + nb_dr(k) * v.cols + nb_dc(k) == from) along = true;
+            else ++before;
+        }
+        const int n = on ? __popc(cell.mask) - (along ? 1 : 0) : 0;
+        Up u[8];
+        bool missing = n > 0;
+        for (long long k = 0; __any_sync(kAll, missing); ++k) {
+            if (k >= q.polls || __any_sync(kAll, *reinterpret_cast<volatile unsigned*>(q.ctl + 3) != 0)) return false;
+            if (missing) {
+                missing = false;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < n) missing |= !read_slot(q.slots + cell.slot + j, u[j]);
+            }
+            if (k) __nanosleep(128);
+        }
+        // the next window's inputs
+        RedoCell<Visitor> ahead;
+        ahead.load(q, v, i + 32, w1);
+        const int32_t w2 = i + 64 < p1 ? __ldg(q.order + i + 64) : -1;
+        typename Visitor::Total s;
+        Up then{};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j < n && j < before) Visitor::add(s, u[j]);
+            if (j < n && j == before) then = u[j];
+        }
+        const unsigned after = (unsigned)max(0, n - before);
+        const unsigned bits = after | (along ? kFlow : 0u) | (along && before == 0 ? kAlone : 0u) | (s.nan ? kNone : 0u);
+        Up mine{};
+        T rest = T(0);
+        const unsigned tops = __ballot_sync(kAll, w < 0);
+        if (__all_sync(kAll, n == 0)) {  // nothing but the flow along paths
+            T x = __shfl_sync(kAll, cell.x, 0), y = __shfl_sync(kAll, cell.y, 0);
+            for (int j = 0; j < steps; ++j) {
+                const T x1 = __shfl_sync(kAll, cell.x, (j + 1) & 31), y1 = __shfl_sync(kAll, cell.y, (j + 1) & 31);
+                // 0 + flow is the flow, bit for bit
+                const typename Visitor::Total t = (tops >> j) & 1u ? typename Visitor::Total{} : Visitor::total(flow);
+                T r;
+                flow = Visitor::apply(t, x, y, r);
+                mine = lane == j ? flow : mine;
+                rest = lane == j ? r : rest;
+                x = x1;
+                y = y1;
+            }
+        } else {
+            RedoStep<Visitor> now = RedoStep<Visitor>::from(s, then, bits, cell.x, cell.y, 0);
+            for (int j = 0; j < steps; ++j) {
+                const RedoStep<Visitor> next = RedoStep<Visitor>::from(s, then, bits, cell.x, cell.y, (j + 1) & 31);
+                typename Visitor::Total t{now.t, (now.bits & kNone) != 0};
+                if (now.bits & kAlone) t = Visitor::total(flow);
+                else if (now.bits & kFlow) Visitor::add(t, flow);
+                const unsigned more = now.bits & 15u;
+                if (more) Visitor::add(t, now.then);
+                if (more > 1u) {
+                    const int b = __shfl_sync(kAll, before, j);
+#pragma unroll
+                    for (int k = 1; k < 8; ++k) {
+                        const Up o = from_lane(u[k], j);
+                        if (k > b && k < b + (int)more) Visitor::add(t, o);
+                    }
+                }
+                T r;
+                flow = Visitor::apply(t, now.x, now.y, r);
+                mine = lane == j ? flow : mine;
+                rest = lane == j ? r : rest;
+                now = next;
+            }
+        }
+        // results, and at the bottoms of paths what flows on
+        int32_t below = __shfl_down_sync(kAll, w, 1);
+        const int32_t next_w = __shfl_sync(kAll, w1, 0);
+        if (lane == 31) below = next_w;
+        if (on) {
+            v.store(c, mine, rest);
+            if (below < 0) {
+                const int32_t slot = __ldg(q.path_slot + i);
+                if (slot >= 0) write_slot(q.slots + slot, mine);
+            }
+        }
+        if (steps < 32) break;
+        before_c = __shfl_sync(kAll, c, 31);
+        w = w1;
+        w1 = w2;
+        cell = ahead;
+    }
+    return true;
+}
+
+template <class Visitor>
+__global__ void __launch_bounds__(kRedoThreads) k_path_redo(PathRedo q, Visitor v)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    next_may_start();
+    wait_for_previous();
+    if (q.flag[1] == 0) return;
+    const int lane = threadIdx.x & 31;
+    unsigned *ticket = q.ctl, *filled = q.ctl + 1, *finished = q.ctl + 2, *gave_up = q.ctl + 3;
+    const int64_t fills = (q.nslots + kRedoFill - 1) / kRedoFill;
+    bool all_filled = false, ok = true;
+    while (ok) {
+        unsigned taken = 0;
+        if (lane == 0) taken = atomicAdd(ticket, 1u);
+        const int64_t k = __shfl_sync(kAll, taken, 0);
+        if (k < fills) {
+            for (int64_t i = k * kRedoFill + lane; i < min(q.nslots, (k + 1) * kRedoFill); i += 32) q.slots[i] = kEmptySlot;
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence();
+                atomicAdd(filled, 1u);
+            }
+            continue;
+        }
+        for (long long j = 0; !all_filled; ++j) {
+            all_filled = __all_sync(kAll, ld_acquire_gpu(reinterpret_cast<const int*>(filled)) >= fills);
+            if (j >= q.polls) break;
+        }
+        const int64_t at = (k - fills) * kRedoChunk;
+        if (at >= q.npos) break;
+        ok = all_filled && redo_chunk(q, v, at, min(at + kRedoChunk, q.npos));
+        if (!ok && lane == 0) atomicExch(gave_up, 1u);
+    }
+    unsigned ends = 0;
+    if (lane == 0) {
+        __threadfence();
+        ends = atomicAdd(finished, 1u);
+    }
+    ends = __shfl_sync(kAll, ends, 0);
+    if (ends + 1u == gridDim.x * (kRedoThreads / 32) && *reinterpret_cast<volatile unsigned*>(gave_up)) {
+        if (lane == 0) q.walk[1] = 1;
+        for (int64_t j = lane; j < q.nwords; j += 32) q.work[j] = q.count[j];
+    }
+}
+
 template <class T>
 __global__ void k_path_no_data(const uint8_t* fd, int64_t n, T* out, T* rem)
 {
@@ -1364,9 +1621,11 @@ void path_buffers_free(lue_gpu_topology* t)
     t->path_slots = nullptr;
 }
 
-// path_ctl: the redo flag (two words of 8 bytes) and one ticket per level, zeroed before each call, then the
-// status words of the scan tiles.
-constexpr size_t kPathCtlZeroed = 2 * sizeof(unsigned long long) + (kPathMaxLevels + 2) * sizeof(int);
+// path_ctl: the redo flag and the walk's (two words of 8 bytes each), one ticket per level and the control words of
+// k_path_redo, zeroed before each call, then the status words of the scan tiles.
+constexpr int kPathRedoCtl = 4;
+constexpr size_t kPathCtlZeroed =
+    4 * sizeof(unsigned long long) + (kPathMaxLevels + 2 + kPathRedoCtl) * sizeof(int);
 
 static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t stream)
 {
@@ -1426,8 +1685,9 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
     if (int rc = path_buffers(t, pc, stream)) return rc;
     const int64_t nt_max = std::max<int64_t>(pc->tiles, 1);
     unsigned long long* flag = static_cast<unsigned long long*>(t->path_ctl);
-    int* tickets = reinterpret_cast<int*>(flag + 2);
-    int* status = tickets + kPathMaxLevels + 2;
+    int* tickets = reinterpret_cast<int*>(flag + 4);
+    int* redo_ctl = tickets + kPathMaxLevels + 2;
+    int* status = redo_ctl + kPathRedoCtl;
     if (int rc = cuda_status(cudaMemsetAsync(flag, 0, kPathCtlZeroed, stream), what)) return rc;
     int launches = 0;
     float2* dense = R != Rule::accu ? static_cast<float2*>(t->path_dense) : nullptr;
@@ -1472,12 +1732,18 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
             ++launches;
         }
     }
-    // +-inf inputs, or a wait of the scan that gave up: the walk engine redoes the whole call (as behind
-    // the tile engine of accu)
-    launch_after(k_copy_words_if, grid_for(words_for(n), 256), 256, 0, stream,
-                 reinterpret_cast<const uint32_t*>(core->count), t->work_count, words_for(n), (const unsigned long long*)flag);
+    // the redo behind it; test hook: LUE_GB300_PATH_REDO_POLLS (poll limit of its waits; 0: each gives up at once, and
+    // the walk engine does the call).  A step along a path takes about a microsecond, and so does a poll.
+    int64_t chain = 0;
+    for (const PathLevel& v : pc->levels) chain += v.longest;
+    long long redo_polls = (1ll << 20) + 4 * chain + pc->npos / 64;
+    if (const char* e = getenv("LUE_GB300_PATH_REDO_POLLS")) redo_polls = std::max(0, atoi(e));
+    const PathRedo r{pc->order, pc->path_slot, p.slot_first, static_cast<unsigned long long*>(t->path_slots), pc->npos,
+                     pc->slot_base, pc->nslots, flag, flag + 2, reinterpret_cast<unsigned*>(redo_ctl), redo_polls,
+                     reinterpret_cast<const uint32_t*>(core->count), t->work_count, words_for(n)};
+    launch_after(k_path_redo<Visitor>, grid_for(pc->npos, kRedoChunk * (kRedoThreads / 32), 152 * 4), kRedoThreads, 0, stream, r, redo);
     WalkGrid g{core->fd, core->count, t->work_count, core->rows, core->cols, n};
-    launch_after(k_walk_if<Visitor>, grid_for(n, 256), 256, 0, stream, g, redo, (const unsigned long long*)flag);
+    launch_after(k_walk_if<Visitor>, grid_for(n, 256), 256, 0, stream, g, redo, (const unsigned long long*)(flag + 2));
     count_launches(launches + 2);
     return cuda_status(cudaGetLastError(), what);
 }

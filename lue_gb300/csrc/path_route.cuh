@@ -21,6 +21,9 @@
 // bottom goes to a slot of the cell that it flows into; the slots of a cell are consecutive, and so are those
 // of neighbouring positions, so a level reads its light inflow densely and not by gathers over the raster.
 //
+// Calls with infinite inputs or totals, which the float-float compositions cannot carry, are redone along the same paths
+// with the cell rules of the walk engine (k_path_redo).
+//
 // Built once per flow-direction raster (on the first call that needs it) and kept by the topology.
 #pragma once
 

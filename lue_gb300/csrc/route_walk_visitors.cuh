@@ -112,6 +112,20 @@ __device__ __forceinline__ bool rule_f32(FF t, bool nan, float x, float b, float
     return true;
 }
 
+// A cell on the walk: its upstream cells are done.
+template <class Visitor>
+__device__ __forceinline__ void enter_cell(Visitor& v, int64_t c)
+{
+    typename Visitor::Total s;
+    for (unsigned m = __ldg(v.upmask + c); m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        Visitor::add(s, v.upstream(c + nb_dr(k) * v.cols + nb_dc(k)));
+    }
+    typename Visitor::T r;
+    const typename Visitor::Up o = Visitor::apply(s, v.first(c), v.second(c), r);
+    v.store(c, o, r);
+}
+
 template <Rule R>
 struct RouteF32 {
     const uint8_t* upmask;
@@ -131,38 +145,62 @@ struct RouteF32 {
         if (R != Rule::accu) rem[c] = qnan<float>();
     }
 
-    __device__ void enter(int64_t c)
-    {
-        unsigned m = __ldg(upmask + c);
+    // A cell's step: what its upstream cells hand on, added in neighbour order, then the rule.
+    using T = float;
+    using Up = float2;  // outflow and its residual; NaN: no-data
+    struct Total {
         FF t{0.0f, 0.0f};
         bool nan = false;
-        while (m) {
-            int k = __ffs(m) - 1;
-            m &= m - 1;
-            int64_t u = c + nb_dr(k) * cols + nb_dc(k);
-            float h = load_cg(out + u);
-            if (isnan(h)) nan = true;
-            else t.add(h, load_cg(lo + u));
-        }
-        float oh = 0.0f, ol = 0.0f, r = 0.0f;
-        if (!rule_f32<R>(t, nan, value_at(a, as, c), R == Rule::accu ? 0.0f : value_at(b, bs, c), oh, ol, r)) {
-            no_data(c);
-            return;
-        }
-        out[c] = oh;
-        lo[c] = ol;
+    };
+    __device__ Up upstream(int64_t u) const { return make_float2(load_cg(out + u), load_cg(lo + u)); }
+    static __device__ void add(Total& s, Up u)  // once nan is set, t is not used: no branches
+    {
+        float h, e;
+        two_sum(s.t.hi, u.x, h, e);
+        s.nan |= isnan(u.x);
+        s.t.hi = h;
+        s.t.lo = fabsf(h) < INFINITY ? __fadd_rn(__fadd_rn(s.t.lo, e), u.y) : 0.0f;
+    }
+    static __device__ Total total(Up u) { return Total{FF{u.x, u.y}, isnan(u.x)}; }
+    __device__ float first(int64_t c) const { return value_at(a, as, c); }
+    __device__ float second(int64_t c) const { return R == Rule::accu ? 0.0f : value_at(b, bs, c); }
+    static __device__ Up apply(const Total& s, float x, float y, float& r)
+    {
+        Up o = make_float2(0.0f, 0.0f);
+        r = 0.0f;
+        if (rule_f32<R>(s.t, s.nan, x, y, o.x, o.y, r)) return o;
+        r = qnan<float>();
+        return make_float2(qnan<float>(), 0.0f);
+    }
+    __device__ void store(int64_t c, Up o, float r)
+    {
+        out[c] = o.x;
+        lo[c] = o.y;
         if (R != Rule::accu) rem[c] = r;
     }
+    __device__ void enter(int64_t c) { enter_cell(*this, c); }
 };
 
 // --- float64: plain double arithmetic, like the reference's double instantiation ---------------------
+
+// Comparisons on the integer pipes: the float64 pipe is slow on GB300.
+__device__ __forceinline__ bool is_nan_bits(double x)
+{
+    const unsigned lo = (unsigned)__double2loint(x);
+    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | ((lo | (0u - lo)) >> 31)) > 0x7ff00000u;
+}
+__device__ __forceinline__ bool is_non_negative(double x)  // x >= 0: false for NaN, true for -0
+{
+    const long long b = __double_as_longlong(x);
+    return (b >= 0 && b <= 0x7ff0000000000000ll) || b == (long long)0x8000000000000000ull;
+}
 
 // The float64 cell rule on the upstream sum t: outflow and state.  False: the cell is no-data.
 template <Rule R>
 __device__ __forceinline__ bool rule_f64(double t, bool nan, double x, double b, double& out, double& rem)
 {
     if (R == Rule::accu) {
-        if (nan || isnan(x) || !(x >= 0.0)) return false;
+        if (nan || !is_non_negative(x)) return false;
         out = t + x;
     } else if (R == Rule::threshold) {
         const double th = b;
@@ -223,24 +261,35 @@ struct RouteF64 {
         if (R != Rule::accu) rem[c] = qnan<double>();
     }
 
-    __device__ void enter(int64_t c)
-    {
-        unsigned m = __ldg(upmask + c);
+    using T = double;
+    using Up = double;
+    struct Total {
         double t = 0.0;
         bool nan = false;
-        while (m) {
-            int k = __ffs(m) - 1;
-            m &= m - 1;
-            double h = load_cg(out + c + nb_dr(k) * cols + nb_dc(k));
-            if (isnan(h)) nan = true;
-            else t += h;
-        }
-        double o = 0.0, r = 0.0;
-        if (!rule_f64<R>(t, nan, value_at(a, as, c), R == Rule::accu ? 0.0 : value_at(b, bs, c), o, r))
-            return no_data(c);
+    };
+    __device__ Up upstream(int64_t u) const { return load_cg(out + u); }
+    static __device__ void add(Total& s, Up u)
+    {
+        s.nan |= is_nan_bits(u);
+        s.t += u;
+    }
+    static __device__ Total total(Up u) { return Total{u, is_nan_bits(u)}; }
+    __device__ double first(int64_t c) const { return value_at(a, as, c); }
+    __device__ double second(int64_t c) const { return R == Rule::accu ? 0.0 : value_at(b, bs, c); }
+    static __device__ Up apply(const Total& s, double x, double y, double& r)
+    {
+        Up o = 0.0;
+        r = 0.0;
+        if (rule_f64<R>(s.t, s.nan, x, y, o, r)) return o;
+        r = qnan<double>();
+        return qnan<double>();
+    }
+    __device__ void store(int64_t c, Up o, double r)
+    {
         out[c] = o;
         if (R != Rule::accu) rem[c] = r;
     }
+    __device__ void enter(int64_t c) { enter_cell(*this, c); }
 };
 
 // --- kinematic wave (float64 discharge; lateral inflow and alpha as TIn) ------------------------------
