@@ -1756,12 +1756,22 @@ static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const float* a,
     return path_run<F32, R, K>(t, pc, a, as, b, bs, out, rem, redo, stream, what);
 }
 
+// A call in place: its inputs are overwritten before a redo would read them.
+static bool overlap(const lue_gpu_topology* t, const void* in, const void* out, size_t size)
+{
+    const char *a = static_cast<const char*>(in), *b = static_cast<const char*>(out);
+    const size_t bytes = (size_t)t->core->n * size;
+    return a && b && a < b + bytes && b < a + bytes;
+}
+
 int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, const float* b, float bs, float* out,
                    float* rem, cudaStream_t stream, bool* done)
 {
     *done = false;
     if (path_engine_off()) return LUE_GPU_OK;
     if (rule < (int)Rule::threshold || rule > (int)Rule::trigger) return LUE_GPU_OK;
+    if (rule == (int)Rule::trigger && (overlap(t, a, out, 4) || overlap(t, a, rem, 4) || overlap(t, b, out, 4) || overlap(t, b, rem, 4)))
+        return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     if (int rc = path_core_get(t, stream, &pc)) return rc;
     if (!pc) return LUE_GPU_OK;
@@ -1781,7 +1791,7 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
 int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, cudaStream_t stream, bool* done)
 {
     *done = false;
-    if (path_engine_off()) return LUE_GPU_OK;
+    if (path_engine_off() || overlap(t, a, out, 8)) return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     if (int rc = path_core_get(t, stream, &pc)) return rc;
     if (!pc) return LUE_GPU_OK;

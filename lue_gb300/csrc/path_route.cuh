@@ -71,11 +71,12 @@ struct lue_gpu_topology;
 namespace lue_gb300 {
 
 // accu_threshold (rule 1), accu_fraction (rule 2), accu_capacity (rule 3) and accu_trigger (rule 4), float32.
-// *done is false when the engine does not apply (flow cycles, a raster beyond its limits, LUE_GB300_ENGINE=walk or =stage): the caller then runs
-// another engine.
+// *done is false when the engine does not apply (flow cycles, a raster beyond its limits, accu_trigger in place,
+// LUE_GB300_ENGINE=walk or =stage): the caller then runs another engine.
 int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, const float* b, float bs, float* out,
                    float* rem, cudaStream_t stream, bool* done);
-// accu, float64: prefix sums along the paths in plain doubles (only additions of terms >= 0, so no cancellation).
+// accu, float64: prefix sums along the paths in plain doubles (only additions of terms >= 0, so no cancellation); not
+// in place.
 int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, cudaStream_t stream, bool* done);
 // Frees the handle's path-engine buffers.
 void path_buffers_free(lue_gpu_topology* t);
