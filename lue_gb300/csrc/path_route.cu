@@ -474,6 +474,31 @@ void path_core_free(PathCore* pc)
     delete pc;
 }
 
+// The positions of the cells, built on the first call that spreads its results.  Without the memory for them the
+// levels write straight to the raster.
+static int path_at_build(const TopologyCore* core, PathCore* pc, cudaStream_t stream)
+{
+    const int64_t n = core->n;
+    pc->at_decided = true;
+    if (n < path_spread_cells()) return LUE_GPU_OK;
+    int rc = cuda_status(cudaMalloc(&pc->at, n * sizeof(int32_t)), "path positions");
+    if (rc) {
+        pc->at = nullptr;
+        return rc == LUE_GPU_ENOMEM ? LUE_GPU_OK : rc;
+    }
+    if ((rc = cuda_status(cudaMemsetAsync(pc->at, 0xFF, n * sizeof(int32_t), stream), "path positions"))) return rc;
+    k_path_at<<<grid_for(pc->npos, 256), 256, 0, stream>>>(pc->order, pc->npos, pc->at);
+    count_launches(1);
+    if ((rc = cuda_status(cudaGetLastError(), "path positions"))) return rc;
+    return cuda_status(cudaStreamSynchronize(stream), "path positions");  // the calls' streams may not wait for it
+}
+
+static bool capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
 int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t stream, PathCore** out)
 {
     *out = nullptr;
@@ -608,15 +633,6 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
         if (bad) {
             rc = fail(LUE_GPU_ERANGE, "path topology: inconsistent layout (" + std::to_string(bad) + " misplaced)");
             goto done;
-        }
-        if (n >= path_spread_cells()) {  // in an array of the build that has served
-            TRY(cudaMemsetAsync(dtop, 0xFF, n * sizeof(int32_t), stream));
-            k_path_at<<<grid_for(npos, 256), 256, 0, stream>>>(pc->order, npos, dtop);
-            TRY(cudaStreamSynchronize(stream));
-            TRY(cudaGetLastError());
-            pc->at = dtop;
-            dtop = nullptr;
-            pc->bytes += n * 4;
         }
     }
     count_launches(launches);
@@ -1588,7 +1604,9 @@ static bool path_engine_off()
     return e && (e[0] == 'w' || e[0] == 's');
 }
 
-static int path_core_get(lue_gpu_topology* t, cudaStream_t stream, const PathCore** out)
+// The path layout of t, built on first use; nullptr when the engine does not apply.  at: for rules with two results, the
+// positions by cell, or nullptr where the levels write straight to the raster.
+static int path_core_get(lue_gpu_topology* t, cudaStream_t stream, const PathCore** out, const int32_t** at)
 {
     *out = nullptr;
     TopologyCore* core = t->core;
@@ -1604,6 +1622,14 @@ static int path_core_get(lue_gpu_topology* t, cudaStream_t stream, const PathCor
         if (rc) return rc;
         core->paths = pc;
         core->bytes += pc->bytes;
+    }
+    if (at && core->paths) {
+        // not while the call is captured: the allocation would be refused
+        if (!core->paths->at_decided && !capturing(stream)) {
+            if (int rc = path_at_build(core, core->paths, stream)) return rc;
+            if (core->paths->at) core->bytes += core->n * 4;
+        }
+        *at = core->paths->at;
     }
     *out = core->paths;
     return LUE_GPU_OK;
@@ -1641,23 +1667,32 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
         path_buffers_free(t);
         return rc;
     }
-    if (pc->at) {
-        if (cudaMalloc(&t->path_dense, pc->npos * 8) == cudaSuccess) {
-            t->scratch_bytes += pc->npos * 8;
-        } else {  // without it the levels write straight to the raster
-            t->path_dense = nullptr;
-            cudaGetLastError();
-        }
-    }
     t->path_epoch = 0;
     t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (int64_t)ctl + ns * 8;
     return LUE_GPU_OK;
 }
 
+// The two results of a call by position, for a handle's first call that spreads them; nullptr without the memory, or when
+// that call is captured: the levels write straight to the raster.
+static float2* path_dense(lue_gpu_topology* t, const PathCore* pc, cudaStream_t stream)
+{
+    if (!t->path_dense && !t->path_dense_tried && !capturing(stream)) {
+        t->path_dense_tried = true;
+        if (cudaMalloc(&t->path_dense, pc->npos * 8) == cudaSuccess) {
+            t->scratch_bytes += pc->npos * 8;
+        } else {
+            t->path_dense = nullptr;
+            cudaGetLastError();
+        }
+    }
+    return static_cast<float2*>(t->path_dense);
+}
+
 int path_prepare(lue_gpu_topology* t, cudaStream_t stream)
 {
     const PathCore* pc = nullptr;
-    return path_core_get(t, stream, &pc);
+    const int32_t* at = nullptr;
+    return path_core_get(t, stream, &pc, &at);
 }
 
 // A level reads its order, its inputs and its first slots while the level before still runs.  Level 0 follows whatever
@@ -1676,7 +1711,7 @@ static void launch_level(bool free, unsigned blocks, cudaStream_t stream, const 
 }
 
 template <class N, Rule R, int K, class Visitor>
-static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T* a, typename N::T as,
+static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, const typename N::T* a, typename N::T as,
                     const typename N::T* b, typename N::T bs, typename N::T* out, typename N::T* rem,
                     const Visitor& redo, cudaStream_t stream, const char* what)
 {
@@ -1690,7 +1725,7 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
     int* status = redo_ctl + kPathRedoCtl;
     if (int rc = cuda_status(cudaMemsetAsync(flag, 0, kPathCtlZeroed, stream), what)) return rc;
     int launches = 0;
-    float2* dense = R != Rule::accu ? static_cast<float2*>(t->path_dense) : nullptr;
+    float2* dense = at ? path_dense(t, pc, stream) : nullptr;
     if (pc->npos < n && !dense) {
         k_path_no_data<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, n, out, rem);
         ++launches;
@@ -1728,7 +1763,7 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
     if constexpr (R != Rule::accu) {
         if (dense) {
             const int64_t tcols = (core->cols + kPathTile - 1) / kPathTile, trows = (core->rows + kPathTile - 1) / kPathTile;
-            k_path_spread<<<(unsigned)(trows * tcols), 256, 0, stream>>>(pc->at, dense, core->rows, core->cols, tcols, out, rem);
+            k_path_spread<<<(unsigned)(trows * tcols), 256, 0, stream>>>(at, dense, core->rows, core->cols, tcols, out, rem);
             ++launches;
         }
     }
@@ -1749,11 +1784,11 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const typename N::T
 }
 
 template <Rule R, int K>
-static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const float* a, float as, const float* b, float bs,
+static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, const float* a, float as, const float* b, float bs,
                         float* out, float* rem, cudaStream_t stream, const char* what)
 {
     const RouteF32<R> redo{t->core->upmask, a, as, b, bs, out, rem, t->lo, t->core->cols};
-    return path_run<F32, R, K>(t, pc, a, as, b, bs, out, rem, redo, stream, what);
+    return path_run<F32, R, K>(t, pc, at, a, as, b, bs, out, rem, redo, stream, what);
 }
 
 // A call in place: its inputs are overwritten before a redo would read them.
@@ -1773,19 +1808,20 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
     if (rule == (int)Rule::trigger && (overlap(t, a, out, 4) || overlap(t, a, rem, 4) || overlap(t, b, out, 4) || overlap(t, b, rem, 4)))
         return LUE_GPU_OK;
     const PathCore* pc = nullptr;
-    if (int rc = path_core_get(t, stream, &pc)) return rc;
+    const int32_t* at = nullptr;
+    if (int rc = path_core_get(t, stream, &pc, &at)) return rc;
     if (!pc) return LUE_GPU_OK;
     *done = true;
     if (rule == (int)Rule::threshold)
-        return path_run_f32<Rule::threshold, kMaxPlus>(t, pc, a, as, b, bs, out, rem, stream,
+        return path_run_f32<Rule::threshold, kMaxPlus>(t, pc, at, a, as, b, bs, out, rem, stream,
                                                        "accu_threshold_f32 (paths)");
     if (rule == (int)Rule::fraction)
-        return path_run_f32<Rule::fraction, kAffine>(t, pc, a, as, b, bs, out, rem, stream,
+        return path_run_f32<Rule::fraction, kAffine>(t, pc, at, a, as, b, bs, out, rem, stream,
                                                      "accu_fraction_f32 (paths)");
     if (rule == (int)Rule::trigger)
-        return path_run_f32<Rule::trigger, kTrigger>(t, pc, a, as, b, bs, out, rem, stream,
+        return path_run_f32<Rule::trigger, kTrigger>(t, pc, at, a, as, b, bs, out, rem, stream,
                                                      "accu_trigger_f32 (paths)");
-    return path_run_f32<Rule::capacity, kMinPlus>(t, pc, a, as, b, bs, out, rem, stream, "accu_capacity_f32 (paths)");
+    return path_run_f32<Rule::capacity, kMinPlus>(t, pc, at, a, as, b, bs, out, rem, stream, "accu_capacity_f32 (paths)");
 }
 
 int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, cudaStream_t stream, bool* done)
@@ -1793,11 +1829,11 @@ int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, 
     *done = false;
     if (path_engine_off() || overlap(t, a, out, 8)) return LUE_GPU_OK;
     const PathCore* pc = nullptr;
-    if (int rc = path_core_get(t, stream, &pc)) return rc;
+    if (int rc = path_core_get(t, stream, &pc, nullptr)) return rc;
     if (!pc) return LUE_GPU_OK;
     *done = true;
     const RouteF64<Rule::accu> redo{t->core->upmask, a, as, nullptr, 0.0, out, nullptr, t->core->cols};
-    return path_run<F64, Rule::accu, kSum>(t, pc, a, as, nullptr, 0.0, out, nullptr, redo, stream,
+    return path_run<F64, Rule::accu, kSum>(t, pc, nullptr, a, as, nullptr, 0.0, out, nullptr, redo, stream,
                                            "accu_f64 (paths)");
 }
 

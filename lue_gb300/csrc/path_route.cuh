@@ -48,7 +48,9 @@ struct PathCore {
     int32_t* order = nullptr;           // [npos] cell index, bit 31 set at the top cell of a path
     int32_t* path_slot = nullptr;       // [npos] at the bottom of a path: the slot that takes its outflow, or -1
     int32_t* slot_first = nullptr;      // [npos - slot_base + 1] first slot of a position
-    int32_t* at = nullptr;              // large rasters: [cells] position of a cell, -1 for no-data
+    // Large rasters, from the first call with two results on: [cells] position of a cell, -1 for no-data.
+    int32_t* at = nullptr;
+    bool at_decided = false;
     int32_t* cut = nullptr;             // path tops at which the CTAs of a level begin
     int64_t slot_base = 0;              // first position of level 1 (level 0 has no light inflow)
     int64_t nslots = 0;                 // light edges of the forest

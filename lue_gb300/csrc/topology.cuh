@@ -56,7 +56,8 @@ struct lue_gpu_topology {
     void* path_maps = nullptr;       // path engine: per tile of a level's scan its own and its inclusive map
     void* path_ctl = nullptr;        // path engine: the redo flag, tickets and status words (path_route.cu)
     void* path_slots = nullptr;      // path engine: per light edge what flows over it, 8 bytes
-    void* path_dense = nullptr;      // path engine, large rasters: a call's two results by position, 8 bytes
+    void* path_dense = nullptr;      // path engine, large rasters, rules with two results: these by position, 8 bytes
+    bool path_dense_tried = false;
     int path_epoch = 0;              // path engine: tag of the last launch's status words
     int64_t scratch_bytes = 0;
 };
