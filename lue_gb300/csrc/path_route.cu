@@ -503,6 +503,9 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
 {
     *out = nullptr;
     const int64_t n = core->n, rows = core->rows, cols = core->cols;
+    // test hook: LUE_GB300_PATH_NO_MEMORY (layout or buffers: there is no memory for them)
+    if (const char* e = getenv("LUE_GB300_PATH_NO_MEMORY"))
+        if (e[0] == 'l') return fail(LUE_GPU_ENOMEM, "path topology: no memory (test hook)");
     // positions are 32-bit, and a CTA of the scan may look past the last one
     if (n >= (int64_t(1) << 31) - 65536) return fail(LUE_GPU_ERANGE, "path topology: about 2^31 cells or more");
     const int64_t npos = core->stats.valid_cells;
@@ -1657,6 +1660,8 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
 {
     if (t->path_maps) return LUE_GPU_OK;
     const char* what = "path engine buffers";
+    if (const char* e = getenv("LUE_GB300_PATH_NO_MEMORY"))
+        if (e[0] == 'b') return fail(LUE_GPU_ENOMEM, "path engine buffers: no memory (test hook)");
     const int64_t nt = std::max<int64_t>(pc->tiles, 1), ns = std::max<int64_t>(pc->nslots, 1);
     const size_t ctl = kPathCtlZeroed + nt * sizeof(int);
     int rc = LUE_GPU_OK;
@@ -1717,7 +1722,6 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, 
 {
     const TopologyCore* core = t->core;
     const int64_t n = core->n;
-    if (int rc = path_buffers(t, pc, stream)) return rc;
     const int64_t nt_max = std::max<int64_t>(pc->tiles, 1);
     unsigned long long* flag = static_cast<unsigned long long*>(t->path_ctl);
     int* tickets = reinterpret_cast<int*>(flag + 4);
@@ -1791,6 +1795,17 @@ static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const int32_t* 
     return path_run<F32, R, K>(t, pc, at, a, as, b, bs, out, rem, redo, stream, what);
 }
 
+// Layout and buffers for a call; *pc is nullptr when there are none, also for want of memory: the stage engine, which
+// then takes the call, builds other structures, which may fit (the layout takes 20 bytes a cell while it is built).
+static int path_ready(lue_gpu_topology* t, cudaStream_t stream, const PathCore** pc, const int32_t** at)
+{
+    int rc = path_core_get(t, stream, pc, at);
+    if (!rc && *pc) rc = path_buffers(t, *pc, stream);
+    if (rc != LUE_GPU_ENOMEM) return rc;
+    *pc = nullptr;
+    return LUE_GPU_OK;
+}
+
 // A call in place: its inputs are overwritten before a redo would read them.
 static bool overlap(const lue_gpu_topology* t, const void* in, const void* out, size_t size)
 {
@@ -1809,7 +1824,7 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
         return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     const int32_t* at = nullptr;
-    if (int rc = path_core_get(t, stream, &pc, &at)) return rc;
+    if (int rc = path_ready(t, stream, &pc, &at)) return rc;
     if (!pc) return LUE_GPU_OK;
     *done = true;
     if (rule == (int)Rule::threshold)
@@ -1829,7 +1844,7 @@ int path_accu_f64(lue_gpu_topology* t, const double* a, double as, double* out, 
     *done = false;
     if (path_engine_off() || overlap(t, a, out, 8)) return LUE_GPU_OK;
     const PathCore* pc = nullptr;
-    if (int rc = path_core_get(t, stream, &pc, nullptr)) return rc;
+    if (int rc = path_ready(t, stream, &pc, nullptr)) return rc;
     if (!pc) return LUE_GPU_OK;
     *done = true;
     const RouteF64<Rule::accu> redo{t->core->upmask, a, as, nullptr, 0.0, out, nullptr, t->core->cols};

@@ -49,3 +49,16 @@ def test_first_spread_call_captured(lfr, monkeypatch):
     g.replay()
     for x, y in zip(got, lfr.accu_threshold(a, m, b)):
         assert np.array_equal(lfr.to_numpy(x), lfr.to_numpy(y), equal_nan=True)
+
+
+@pytest.mark.parametrize("what", ["layout", "buffers"])
+@pytest.mark.parametrize("op", ["accu", "trigger"])
+def test_without_memory_another_engine_does_the_call(lfr, monkeypatch, op, what):
+    """Whole numbers: every engine gives the same bits."""
+    a, m, b, m64 = _inputs(lfr)
+    call = lambda: [lfr.accu(a, m64)] if op == "accu" else list(lfr.accu_trigger(a, m, b))  # noqa: E731
+    monkeypatch.setenv("LUE_GB300_PATH_NO_MEMORY", what)
+    got = [lfr.to_numpy(x) for x in call()]
+    monkeypatch.delenv("LUE_GB300_PATH_NO_MEMORY")
+    for x, y in zip(got, call()):
+        assert np.array_equal(x, lfr.to_numpy(y), equal_nan=True)
