@@ -110,7 +110,8 @@ int lue_gpu_topology_destroy(lue_gpu_topology* topology);
 int lue_gpu_topology_get_stats(const lue_gpu_topology* topology, lue_gpu_topology_stats* stats);
 /* Builds now, on `stream`, what the first call of an operation would otherwise build: the path layout of
  * float32 accu_threshold / accu_fraction / accu_capacity / accu_trigger and float64 accu, and the stage structures of
- * the other float64 rules and kinematic_wave (shared by the clones of the handle).
+ * the other float64 rules and kinematic_wave (shared by the clones of the handle), and this handle's buffers of the path
+ * engine, after which its calls there can be captured.
  * Returns when they are built.  A serving loop
  * calls it when it loads a raster, so that no request pays for it.  (No reference counterpart: the
  * reference keeps no state between calls.) */

@@ -1640,10 +1640,8 @@ static int path_core_get(lue_gpu_topology* t, cudaStream_t stream, const PathCor
 
 void path_buffers_free(lue_gpu_topology* t)
 {
-    cudaFree(t->path_maps);
-    cudaFree(t->path_ctl);
-    cudaFree(t->path_slots);
-    cudaFree(t->path_dense);
+    void* const buffers[2] = {t->path_maps, t->path_dense};
+    pool_release(buffers, 2);
     t->path_dense = nullptr;
     t->path_maps = nullptr;
     t->path_ctl = nullptr;
@@ -1662,18 +1660,26 @@ static int path_buffers(lue_gpu_topology* t, const PathCore* pc, cudaStream_t st
     const char* what = "path engine buffers";
     if (const char* e = getenv("LUE_GB300_PATH_NO_MEMORY"))
         if (e[0] == 'b') return fail(LUE_GPU_ENOMEM, "path engine buffers: no memory (test hook)");
+    if (capturing(stream))  // the buffers would belong to the graph
+        return fail(LUE_GPU_ECUDA, std::string(what) + ": the first call of a handle cannot be captured (call "
+                                                       "lue_gpu_topology_prepare on it first)");
     const int64_t nt = std::max<int64_t>(pc->tiles, 1), ns = std::max<int64_t>(pc->nslots, 1);
     const size_t ctl = kPathCtlZeroed + nt * sizeof(int);
-    int rc = LUE_GPU_OK;
-    if ((rc = cuda_status(cudaMalloc(&t->path_maps, 2 * nt * sizeof(PMap<kTrigger>)), what)) ||
-        (rc = cuda_status(cudaMalloc(&t->path_ctl, ctl), what)) ||
-        (rc = cuda_status(cudaMalloc(&t->path_slots, ns * sizeof(double)), what)) ||
-        (rc = cuda_status(cudaMemsetAsync(t->path_ctl, 0, ctl, stream), what))) {
+    Arena plan;  // the offsets of the three in one allocation
+    const size_t maps_at = plan.add(2 * nt * sizeof(PMap<kTrigger>)), ctl_at = plan.add(ctl),
+                 slots_at = plan.add(ns * sizeof(double));
+    void* base = nullptr;
+    if (int rc = pool_allocate(&base, plan.bytes(), stream, what)) return rc;
+    char* const b = static_cast<char*>(base);
+    t->path_maps = b + maps_at;
+    t->path_ctl = b + ctl_at;
+    t->path_slots = b + slots_at;
+    if (int rc = cuda_status(cudaMemsetAsync(t->path_ctl, 0, ctl, stream), what)) {
         path_buffers_free(t);
         return rc;
     }
     t->path_epoch = 0;
-    t->scratch_bytes += 2 * nt * (int64_t)sizeof(PMap<kTrigger>) + (int64_t)ctl + ns * 8;
+    t->scratch_bytes += (int64_t)plan.bytes();
     return LUE_GPU_OK;
 }
 
@@ -1683,12 +1689,8 @@ static float2* path_dense(lue_gpu_topology* t, const PathCore* pc, cudaStream_t 
 {
     if (!t->path_dense && !t->path_dense_tried && !capturing(stream)) {
         t->path_dense_tried = true;
-        if (cudaMalloc(&t->path_dense, pc->npos * 8) == cudaSuccess) {
+        if (pc->npos > 0 && !pool_allocate(&t->path_dense, pc->npos * 8, stream, "path results"))
             t->scratch_bytes += pc->npos * 8;
-        } else {
-            t->path_dense = nullptr;
-            cudaGetLastError();
-        }
     }
     return static_cast<float2*>(t->path_dense);
 }
@@ -1697,7 +1699,8 @@ int path_prepare(lue_gpu_topology* t, cudaStream_t stream)
 {
     const PathCore* pc = nullptr;
     const int32_t* at = nullptr;
-    return path_core_get(t, stream, &pc, &at);
+    if (int rc = path_core_get(t, stream, &pc, &at)) return rc;
+    return pc ? path_buffers(t, pc, stream) : LUE_GPU_OK;
 }
 
 // A level reads its order, its inputs and its first slots while the level before still runs.  Level 0 follows whatever

@@ -1543,15 +1543,37 @@ static cudaMemPool_t stage_pool()
 
 void stage_buffers_free(lue_gpu_topology* t)
 {
-    if (!t->stage_hist && !t->stage_flow) return;
-    cudaDeviceSynchronize();  // the handle's streams are unknown here: wait for all work
-    if (t->stage_hist) cudaFreeAsync(t->stage_hist, nullptr);
-    if (t->stage_flow) cudaFreeAsync(t->stage_flow, nullptr);
-    cudaStreamSynchronize(nullptr);
+    void* const buffers[2] = {t->stage_hist, t->stage_flow};
+    pool_release(buffers, 2);
     t->stage_hist = nullptr;
     t->stage_flow = nullptr;
     t->stage_hist_bytes = t->stage_flow_bytes = 0;
+}
+
+void pool_release(void* const* p, int n)
+{
+    if (std::all_of(p, p + n, [](void* x) { return !x; })) return;
+    cudaDeviceSynchronize();  // the handle's streams are unknown here: wait for all work
+    for (int i = 0; i < n; ++i)
+        if (p[i]) cudaFreeAsync(p[i], nullptr);
+    cudaStreamSynchronize(nullptr);
     if (cudaMemPool_t pool = stage_pool()) cudaMemPoolTrimTo(pool, 0);
+}
+
+int pool_allocate(void** p, size_t bytes, cudaStream_t stream, const char* what)
+{
+    *p = nullptr;
+    cudaMemPool_t pool = stage_pool();
+    if (!pool) return fail(LUE_GPU_ECUDA, std::string(what) + ": no memory pool");
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+    if (e == cudaSuccess) return LUE_GPU_OK;
+    *p = nullptr;
+    cudaGetLastError();  // not an error of the launches that follow
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    return fail(e == cudaErrorMemoryAllocation ? LUE_GPU_ENOMEM : LUE_GPU_ECUDA,
+                std::string(what) + ": " + cudaGetErrorString(e) + " (" + std::to_string(bytes >> 20) + " MiB asked, " +
+                    std::to_string(free_b >> 20) + " MiB free)");
 }
 
 template <class T>
@@ -1570,14 +1592,9 @@ static int grow(lue_gpu_topology* t, T*& p, size_t& have, size_t need, cudaStrea
     }
     p = nullptr;
     have = 0;
-    const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), need, pool, stream);
-    if (e != cudaSuccess) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        return fail(e == cudaErrorMemoryAllocation ? LUE_GPU_ENOMEM : LUE_GPU_ECUDA,
-                    std::string(what) + ": " + cudaGetErrorString(e) + " (" + std::to_string(need >> 20) +
-                        " MiB asked, " + std::to_string(free_b >> 20) + " MiB free)");
-    }
+    void* q = nullptr;
+    if (int rc = pool_allocate(&q, need, stream, what)) return rc;
+    p = static_cast<T*>(q);
     have = need;
     return LUE_GPU_OK;
 }

@@ -82,6 +82,10 @@ namespace lue_gb300 {
 // Frees the handle's stage buffers (history, flow counters) back to their pool, after the work queued so
 // far on the default stream.
 void stage_buffers_free(lue_gpu_topology* t);
+// Per-handle buffers come from a stream-ordered pool of the device: allocating one waits for nothing but its own stream.
+int pool_allocate(void** p, size_t bytes, cudaStream_t stream, const char* what);
+// Frees them, after all work on the device (the handle's streams are unknown by then).
+void pool_release(void* const* p, int n);
 // Builds the stage topology of t now (lue_gpu_topology_prepare).
 int stage_prepare(lue_gpu_topology* t, cudaStream_t stream);
 // Schedule of the stage engine for handle t: the cap of the shared stage structures and the handle's

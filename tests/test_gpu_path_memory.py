@@ -62,3 +62,29 @@ def test_without_memory_another_engine_does_the_call(lfr, monkeypatch, op, what)
     monkeypatch.delenv("LUE_GB300_PATH_NO_MEMORY")
     for x, y in zip(got, call()):
         assert np.array_equal(x, lfr.to_numpy(y), equal_nan=True)
+
+
+@pytest.mark.parametrize("op", ["accu", "trigger"])
+def test_first_call_captured_after_prepare(lfr, op):
+    """Whole numbers: a captured first call gives the bits of an ordinary one; so does an ordinary one after it."""
+    import torch
+    a, m, b, m64 = _inputs(lfr)
+    call = lambda: [lfr.accu(a, m64)] if op == "accu" else list(lfr.accu_trigger(a, m, b))  # noqa: E731
+    want = [lfr.to_numpy(x) for x in call()]
+    first, second = a.topology().clone(), None
+    a._topology, second = first, a._topology
+    try:
+        first.prepare()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            got = call()
+        for _ in range(2):
+            g.replay()
+        for results in (got, call()):
+            for x, w in zip(results, want):
+                assert np.array_equal(lfr.to_numpy(x), w, equal_nan=True)
+        del g
+    finally:
+        torch.cuda.synchronize()
+        a._topology = second
+        first.close()
