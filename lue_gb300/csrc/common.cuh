@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 #include "lue_gb300.h"
 
@@ -173,6 +174,12 @@ public:
     {
         owned_ = false;
         return base_;
+    }
+    void swap(Arena& o)
+    {
+        std::swap(bytes_, o.bytes_);
+        std::swap(base_, o.base_);
+        std::swap(owned_, o.owned_);
     }
     template <class T>
     T* at(size_t offset) const

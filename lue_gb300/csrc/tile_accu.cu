@@ -601,7 +601,19 @@ __global__ void __launch_bounds__(kTileThreads)
     int invalid_base = root_total + block_exclusive_int(lane == 31 ? invalid : 0, sm.warp_tot, invalid_total);
     root_base = __shfl_sync(0xffffffffu, root_base, 31);
     invalid_base = __shfl_sync(0xffffffffu, invalid_base, 31);
+    const int32_t e0 = exit_base[tile], ne = exit_base[tile + 1] - e0;
     if (nvalid + invalid_total != kTileCells) {  // uniform: cells on a cycle never become ready
+        // only the levels: -1 on the cycle (no cell drains out of one, so all others are in the queue)
+        uint32_t* ready = reinterpret_cast<uint32_t*>(sm.up);
+        for (int w = t; w < kTileCells / 32; w += kTileThreads) ready[w] = 0;
+        __syncthreads();
+        for (int k = t; k < nvalid; k += kTileThreads) atomicOr(ready + (sm.queue[k] >> 5), 1u << (sm.queue[k] & 31));
+        __syncthreads();
+        for (int i = t; i < kTileCells; i += kTileThreads) {
+            const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
+            if (row < g.rows && col < g.cols) level[row * g.cols + col] = (ready[i >> 5] >> (i & 31)) & 1u ? (int32_t)st[2 * i] : -1;
+        }
+        for (int e = t; e < ne; e += kTileThreads) exit_level[e0 + e] = st[2 * exit_local[e0 + e]];
         if (t == 0) atomicExch(cyclic, 1);
         return;
     }
@@ -611,7 +623,6 @@ __global__ void __launch_bounds__(kTileThreads)
         if (row < g.rows && col < g.cols)
             level[row * g.cols + col] = sm.fd[(i >> 6) + 1][(i & 63) + 1] == kNoData ? -1 : (int32_t)st[2 * i];
     }
-    const int32_t e0 = exit_base[tile], ne = exit_base[tile + 1] - e0;
     for (int e = t; e < ne; e += kTileThreads) exit_level[e0 + e] = st[2 * exit_local[e0 + e]];
     __syncthreads();
     // first positions of roots and invalid cells; the others' offset from their downstream cell's: after the siblings
@@ -1101,30 +1112,35 @@ __global__ void __launch_bounds__(kTileThreads)
 
 // Build, a CTA per tile: the downstream level of every cell, from its level within the tile (k_tile_forest) and the
 // levels of the exits that drain into the tile (k_exit_sizes): each inflow raises the cells below it, up to the first
-// that is at least as high already.  And the raster's statistics [valid, ridge, outlet, sink, -, largest level].
+// that is at least as high already.  Cells on a cycle keep -1: those that have it from k_tile_forest, and those below an
+// exit that k_exit_sizes did not finish (pending; nullptr without cycles).  And the raster's statistics [valid, ridge,
+// outlet, sink, cycle, largest level].
 // A walk over the cells of the whole raster (k_walk) is bound by the longest flow path, a memory round trip per cell:
 // 0.99 ms at 2048^2, where k_exit_sizes, which takes those steps from tile to tile, and this kernel take 19 and 33 us.
+constexpr int kOnCycle = 0x7fffffff;
 __global__ void __launch_bounds__(kTileThreads)
     k_tile_levels(const uint8_t* __restrict__ fd, TileGeom g, const int32_t* __restrict__ exit_base,
                   const uint64_t* bitmap, const uint16_t* rowpref, const uint8_t* __restrict__ border_in,
-                  const int32_t* __restrict__ exit_level, int64_t nexit, int32_t* __restrict__ level,
-                  unsigned long long* stats)
+                  const int32_t* __restrict__ exit_level, const int32_t* __restrict__ pending, int64_t nexit,
+                  int32_t* __restrict__ level, unsigned long long* stats)
 {
     __shared__ int lv[kTileCells];
     __shared__ uint8_t code[kTileCells];
-    __shared__ int tally[5];
+    __shared__ int tally[6];
     const int64_t tr = blockIdx.y, tc = blockIdx.x, tile = tr * g.tcols + tc;
     const int t = threadIdx.x, lane = t & 31;
     // thread t: column t & 63 of every fourth row
     constexpr int kCells = kTileCells / kTileThreads, kStep = kTileThreads / kTile;
     const int64_t row0 = tr * kTile + (t >> 6), col = tc * kTile + (t & 63), cell0 = row0 * g.cols + col, step = kStep * g.cols;
     const int rows = col < g.cols ? (int)min((int64_t)kTile, max((int64_t)0, g.rows - row0)) : 0;  // this thread's, by kStep
-    if (t < 5) tally[t] = 0;
+    if (t < 6) tally[t] = 0;
 #pragma unroll
     for (int k = 0; k < kCells; ++k) {
         const bool in = k * kStep < rows;
-        code[t + k * kTileThreads] = in ? fd[cell0 + k * step] : kNoData;
-        lv[t + k * kTileThreads] = in ? level[cell0 + k * step] : -1;
+        const unsigned c = in ? fd[cell0 + k * step] : kNoData;
+        const int l = in ? level[cell0 + k * step] : -1;
+        code[t + k * kTileThreads] = (uint8_t)c;
+        lv[t + k * kTileThreads] = c != kNoData && l < 0 ? kOnCycle : l;
     }
     __syncthreads();
     const unsigned from = t < kBorderCells ? border_in[tile * kBorderCells + t] : 0u;
@@ -1134,11 +1150,11 @@ __global__ void __launch_bounds__(kTileThreads)
         for (unsigned m = from; m; m &= m - 1) {
             const int q = __ffs(m) - 1;
             const int64_t y = exit_id_of(g, exit_base, bitmap, rowpref, tr * kTile + r + nb_dr(q), tc * kTile + c + nb_dc(q));
-            if (y < nexit) in = max(in, exit_level[y] + 1);
+            if (y < nexit) in = max(in, pending && pending[y] != 0 ? kOnCycle : exit_level[y] + 1);
         }
-        // the tile has no cycle (k_tile_forest): at most one step per cell.  The walk waits for its loads only, not for
-        // the maximum: whoever raised a cell first goes on below it.
-        for (int i = r * kTile + c; *(volatile int*)(lv + i) < in; ++in) {
+        // At most one step per cell: a cycle inside the tile stops the walk, as its cells have the highest value.  The walk
+        // waits for its loads only, not for the maximum: whoever raised a cell first goes on below it.
+        for (int i = r * kTile + c; *(volatile int*)(lv + i) < in; in += in != kOnCycle) {
             atomicMax(lv + i, in);
             int d, q;
             if (!tile_downstream(code[i], i >> 6, i & 63, d, q) || code[d] == kNoData) break;
@@ -1146,14 +1162,18 @@ __global__ void __launch_bounds__(kTileThreads)
         }
     }
     __syncthreads();
-    int valid = 0, ridge = 0, outlet = 0, sink = 0, most = 0;
+    int valid = 0, ridge = 0, outlet = 0, sink = 0, cycle = 0, most = 0;
 #pragma unroll
     for (int k = 0; k < kCells; ++k) {
         const unsigned c = code[t + k * kTileThreads];
         if (c == kNoData) continue;
-        const int l = lv[t + k * kTileThreads];
-        level[cell0 + k * step] = l;
         ++valid;
+        const int l = lv[t + k * kTileThreads];
+        level[cell0 + k * step] = l == kOnCycle ? -1 : l;
+        if (l == kOnCycle) {
+            ++cycle;
+            continue;
+        }
         ridge += l == 0;  // a cell has level 0 when nothing drains into it
         const unsigned pad = c - 1u;  // numeric pad: 0 .. 8 from the lower left, 4 in the middle
         if (pad > 8u || pad == 4u) {
@@ -1169,18 +1189,20 @@ __global__ void __launch_bounds__(kTileThreads)
     ridge = __reduce_add_sync(0xffffffffu, ridge);
     outlet = __reduce_add_sync(0xffffffffu, outlet);
     sink = __reduce_add_sync(0xffffffffu, sink);
+    cycle = __reduce_add_sync(0xffffffffu, cycle);
     most = __reduce_max_sync(0xffffffffu, most);
     if (lane == 0) {
         atomicAdd(tally + 0, valid);
         atomicAdd(tally + 1, ridge);
         atomicAdd(tally + 2, outlet);
         atomicAdd(tally + 3, sink);
-        atomicMax(tally + 4, most);
+        atomicAdd(tally + 4, cycle);
+        atomicMax(tally + 5, most);
     }
     __syncthreads();
-    if (t < 4 && tally[t]) atomicAdd(stats + t, (unsigned long long)tally[t]);
-    if (t == 4 && (unsigned long long)tally[4] > *(volatile unsigned long long*)(stats + 5))
-        atomicMax(stats + 5, (unsigned long long)tally[4]);
+    if (t < 5 && tally[t]) atomicAdd(stats + t, (unsigned long long)tally[t]);
+    if (t == 5 && (unsigned long long)tally[5] > *(volatile unsigned long long*)(stats + 5))
+        atomicMax(stats + 5, (unsigned long long)tally[5]);
 }
 
 // Inclusive prefix sums (modulo 2^64) of the thread runs a[0..15] over the whole tile, written to S by
@@ -1810,13 +1832,12 @@ int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Are
     return LUE_GPU_OK;
 }
 
-// Builds the tile structures, the downstream levels and the raster's statistics (hstats: valid, ridge, outlet, sink, 0,
-// largest level) in the planned arenas, and readies the scratch.  *acyclic is false, and core->tiles stays empty, when
-// the network has a flow cycle.  The build's own arrays lie in the handle's scratch.
+// Builds the tile structures, the downstream levels and the raster's statistics (hstats: valid, ridge, outlet, sink,
+// cycle, largest level) in the planned arenas, and readies the scratch.  core->tiles stays empty, and the levels and
+// statistics are all there is, when the network has a flow cycle.  The build's own arrays lie in the handle's scratch.
 int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
-                    const TileScratchPlan& scratch_plan, cudaStream_t stream, bool* acyclic, unsigned long long* hstats)
+                    const TileScratchPlan& scratch_plan, cudaStream_t stream, unsigned long long* hstats)
 {
-    *acyclic = false;
     auto* tc = new (std::nothrow) TileCore();
     if (!tc) return fail(LUE_GPU_ENOMEM, "tile topology: host allocation");
     TileGeom g{core->rows, core->cols, (core->rows + kTile - 1) / kTile, (core->cols + kTile - 1) / kTile};
@@ -1877,7 +1898,14 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
     TRY(cudaMemcpyAsync(&hexit, nexit, sizeof hexit, cudaMemcpyDeviceToHost, stream), "tile exits");
     TRY(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, stream), "tile build");
     TRY(cudaStreamSynchronize(stream), "tile build");
-    if (h.cyclic) goto error;  // rc == LUE_GPU_OK
+    if (h.cyclic) {
+        k_tile_levels<<<grid, kTileThreads, 0, stream>>>(core->fd, g, base, bitmap, rowpref, border_in, exit_level, pending,
+                                                         hexit, core->level, ctl->stats);
+        TRY(cudaGetLastError(), "tile build");
+        TRY(cudaMemcpyAsync(hstats, ctl->stats, sizeof h.stats, cudaMemcpyDeviceToHost, stream), "tile build");
+        TRY(cudaStreamSynchronize(stream), "tile build");
+        goto error;  // rc == LUE_GPU_OK
+    }
     tc->nexit = hexit;
     tc->max_depth = std::max(h.depth, hexit > 0 ? 1 : 0);
     if (hexit > 0) {
@@ -1888,8 +1916,8 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
     k_slot_fill<<<grid, kTileThreads, 0, stream>>>(g, border_in, base, bitmap, rowpref, tc->slot_base, edge_base, tc->exit_pos,
                                                    exit_start, tc->slot_at, tc->slot_first, tc->slot_edge, hexit,
                                                    &ctl->error);
-    k_tile_levels<<<grid, kTileThreads, 0, stream>>>(core->fd, g, base, bitmap, rowpref, border_in, exit_level, hexit,
-                                                     core->level, ctl->stats);
+    k_tile_levels<<<grid, kTileThreads, 0, stream>>>(core->fd, g, base, bitmap, rowpref, border_in, exit_level, nullptr,
+                                                     hexit, core->level, ctl->stats);
     TRY(cudaGetLastError(), "tile build");
     TRY(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, stream), "tile build");
     TRY(cudaMemcpyAsync(&hslot, tc->slot_base + nt, sizeof hslot, cudaMemcpyDeviceToHost, stream), "tile build");
@@ -1902,7 +1930,6 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
     tc->nslot = hslot;
     std::memcpy(hstats, h.stats, sizeof h.stats);
     core->tiles = tc;
-    *acyclic = true;
     return LUE_GPU_OK;
 error:
     delete tc;

@@ -131,7 +131,7 @@ struct TopologyCore;
 inline bool tile_rows_fit(int64_t rows) { return (rows + kTile - 1) / kTile <= 65535; }
 int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp);
 int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
-                    const TileScratchPlan& scratch_plan, cudaStream_t stream, bool* acyclic, unsigned long long* hstats);
+                    const TileScratchPlan& scratch_plan, cudaStream_t stream, unsigned long long* hstats);
 void tile_scratch_plan(int64_t ntiles, int64_t nexit, Arena& a, TileScratchPlan* p);
 void tile_scratch_take(const Arena& a, const TileScratchPlan& p, TileScratch* s);
 int tile_scratch_clear(const Arena& a, const TileScratchPlan& p, cudaStream_t stream);

@@ -220,9 +220,11 @@ int allocate_scratch(lue_gpu_topology* t)
 
 // The first build of a topology, in two allocations (its own and the handle's scratch, in which the build's arrays lie
 // too): cudaMalloc takes 35 us and cudaFree 30 to 60 us whatever the size, and with one of each for every array (45 and
-// 35) they took half of the build of a 2048^2 raster.  With `tiles`, *acyclic tells whether the network has no
-// cycle; if it has one, or the raster has more exits than the tile engine takes, nothing is kept.
-static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bool tiles, cudaStream_t stream, bool* acyclic,
+// 35) they took half of the build of a 2048^2 raster.  With `tiles`, *done stays false, and nothing is kept, when
+// the raster has more exits than the tile engine takes.  A raster with a flow cycle has its levels from the tiles too
+// (with one 2 x 2 cycle at 256^2 / 2048^2 / 8192^2: 0.42 / 0.93 / 5.4 ms; by a walk over its cells after the attempt with
+// tiles 1.5 / 9.6 / 54 ms), and keeps no tile structures.
+static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bool tiles, cudaStream_t stream, bool* done,
                           unsigned long long* hstats)
 {
     TopologyCore* core = t->core;
@@ -233,9 +235,10 @@ static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bo
     ScratchPlan scratch{};
     const size_t fd = a.add(padded), count = a.add(padded), upmask = a.add(padded),
                  level = a.add(n * (int64_t)sizeof(int32_t));
-    core->bytes = (int64_t)a.bytes();
+    const size_t base = a.bytes();
+    core->bytes = (int64_t)base;
     plan_scratch(n, s, &scratch);
-    *acyclic = false;
+    *done = false;
     if (tiles && tile_core_plan(core->rows, core->cols, a, &tile_plan, s, &scratch.tiles)) return LUE_GPU_OK;
     if ((rc = cuda_status(a.allocate(), "topology"))) return rc;
     if ((rc = cuda_status(s.allocate(), "scratch"))) return rc;
@@ -251,9 +254,27 @@ static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bo
     if ((rc = cuda_status(cudaMemsetAsync(core->count + padded - 4, 0, 4, stream), "memset"))) return rc;
     launch_count(core->fd, core->rows, core->cols, 1, core->count, core->upmask, stream);
     if (tiles) {
-        rc = tile_core_build(core, a, tile_plan, s, scratch.tiles, stream, acyclic, hstats);
-        if (!*acyclic) return rc == LUE_GPU_ECUDA || rc == LUE_GPU_ENOMEM ? rc : LUE_GPU_OK;
-        core->bytes += core->tiles->bytes;
+        rc = tile_core_build(core, a, tile_plan, s, scratch.tiles, stream, hstats);
+        if (rc) return rc == LUE_GPU_ECUDA || rc == LUE_GPU_ENOMEM ? rc : LUE_GPU_OK;
+        core->bytes += (int64_t)tile_plan.bytes;
+        Arena a0, s0;  // without the tiles: the same arrays come first in both
+        if (!core->tiles) {
+            ScratchPlan plain{};
+            a0.add((int64_t)base);
+            plan_scratch(n, s0, &plain);
+            if (!cuda_status(a0.allocate(), "topology") && !cuda_status(s0.allocate(), "scratch")) {
+                if ((rc = cuda_status(cudaMemcpyAsync(a0.at<char>(0), a.at<char>(0), base, cudaMemcpyDeviceToDevice, stream), "topology")) ||
+                    (rc = cuda_status(cudaStreamSynchronize(stream), "topology")))
+                    return rc;
+                core->bytes = (int64_t)base;
+                a.swap(a0);
+                s.swap(s0);
+                core->fd = a.at<uint8_t>(fd);
+                core->count = a.at<uint8_t>(count);
+                core->upmask = a.at<uint8_t>(upmask);
+                core->level = a.at<int32_t>(level);
+            }
+        }
     } else {  // levels by a walk over the cells
         uint32_t* work = s.at<uint32_t>(scratch.count);
         unsigned long long* dstats = nullptr;
@@ -277,6 +298,7 @@ static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bo
     take_scratch(t, s, scratch);
     core->arena = a.release();
     t->arena = s.release();
+    *done = true;
     return LUE_GPU_OK;
 }
 
@@ -342,20 +364,20 @@ extern "C" int lue_gpu_topology_create(const uint8_t* flow_direction, int64_t ro
     core->prow = partition_rows;
     core->pcol = partition_cols;
     core->n = rows * cols;
-    // the tile engine needs an acyclic network and 32-bit cell indices; its build gives the levels and statistics
-    bool acyclic = false;
+    // the tiles need 32-bit cell indices; their build gives the levels and statistics
+    bool done = false;
     unsigned long long hstats[6] = {0, 0, 0, 0, 0, 0};
     int rc = LUE_GPU_OK, tiles = LUE_GPU_OK;
     if (core->n < (int64_t(1) << 32)) {
         // without a grid or the memory for the tiles only rasters with cycles, which have none, are taken
         if (tile_rows_fit(rows)) {
-            tiles = build_topology(t, flow_direction, true, stream, &acyclic, hstats);
+            tiles = build_topology(t, flow_direction, true, stream, &done, hstats);
             if (tiles == LUE_GPU_ECUDA) rc = tiles;
         } else {
             tiles = LUE_GPU_ECUDA;
         }
     }
-    if (!rc && !acyclic) rc = build_topology(t, flow_direction, false, stream, &acyclic, hstats);
+    if (!rc && !done) rc = build_topology(t, flow_direction, false, stream, &done, hstats);
     if (!rc && tiles && hstats[4] == 0) rc = fail(tiles, "topology_create: no memory or grid for the tile structures");
     if (rc) {
         free_handle(t);
