@@ -150,6 +150,24 @@ __global__ void __launch_bounds__(256) k_exit_bitmap(const uint8_t* __restrict__
     if (lane == 0) count[tile] = before;
 }
 
+// The number of exits of the raster, one warp per tile.
+__global__ void __launch_bounds__(256) k_exit_count(const uint8_t* __restrict__ fd, TileGeom g, unsigned long long* total)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t tile = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (tile >= g.trows * g.tcols) return;
+    const int64_t tr = tile / g.tcols, tc = tile - tr * g.tcols;
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kTile; k += 32) {
+        const int i = k + lane;
+        n += leaves_tile(fd, g, tr, tc, 0, i) + leaves_tile(fd, g, tr, tc, kTile - 1, i);
+        if (i > 0 && i < kTile - 1) n += leaves_tile(fd, g, tr, tc, i, 0) + leaves_tile(fd, g, tr, tc, i, kTile - 1);
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0 && n) atomicAdd(total, (unsigned long long)n);
+}
+
 // Exclusive sums of up to two arrays of n counts (one CTA), with their totals at [n].
 __global__ void __launch_bounds__(1024) k_tile_scan(const int32_t* a, int32_t* a_base, const int32_t* b, int32_t* b_base,
                                                     int64_t n)
@@ -1809,9 +1827,34 @@ TileTemp plan_temp(int64_t nt, int64_t E, Arena& a)
 
 }  // namespace
 
-int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp)
+// From this many cells on, the exits are counted before the arrays are planned: a raster has about half of the most that
+// its shape can have (16384^2: 8.2 of 16.7 million, 0.4 GB less in the topology and its scratch).  Below, the
+// allocation, launch and synchronisation for it would cost more than the memory is worth (14 of 290 MB at 4000^2).
+constexpr int64_t kCountExitsCells = int64_t(1) << 24;
+
+int tile_exit_bound(const uint8_t* fd, int64_t rows, int64_t cols, cudaStream_t stream, int64_t* exits)
 {
-    const int64_t nt = ((rows + kTile - 1) / kTile) * ((cols + kTile - 1) / kTile), E = most_exits(rows, cols);
+    *exits = most_exits(rows, cols);
+    if (rows * cols < kCountExitsCells) return LUE_GPU_OK;
+    const TileGeom g{rows, cols, (rows + kTile - 1) / kTile, (cols + kTile - 1) / kTile};
+    Arena a;
+    const size_t at = a.add(sizeof(unsigned long long));
+    unsigned long long h = 0;
+    if (int rc = cuda_status(a.allocate(), "exit count")) return rc;
+    if (int rc = cuda_status(cudaMemsetAsync(a.at<char>(at), 0, sizeof h, stream), "exit count")) return rc;
+    k_exit_count<<<blocks_for(g.trows * g.tcols, 8), 256, 0, stream>>>(fd, g, a.at<unsigned long long>(at));
+    if (int rc = cuda_status(cudaGetLastError(), "exit count")) return rc;
+    if (int rc = cuda_status(cudaMemcpyAsync(&h, a.at<char>(at), sizeof h, cudaMemcpyDeviceToHost, stream), "exit count")) return rc;
+    if (int rc = cuda_status(cudaStreamSynchronize(stream), "exit count")) return rc;
+    *exits = (int64_t)h;
+    return LUE_GPU_OK;
+}
+
+int tile_core_plan(int64_t rows, int64_t cols, int64_t exits, Arena& core, TileCorePlan* p, Arena& scratch,
+                   TileScratchPlan* sp)
+{
+    const int64_t nt = ((rows + kTile - 1) / kTile) * ((cols + kTile - 1) / kTile), E = exits;
+    p->exits = E;
     if (E >= INT32_MAX) return fail(LUE_GPU_ERANGE, "tile topology: too many exits");
     const size_t before = core.bytes();
     p->exit_base = core.add((nt + 1) * 4);
@@ -1844,7 +1887,7 @@ int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& 
     tc->trows = g.trows;
     tc->tcols = g.tcols;
     tc->ntiles = g.trows * g.tcols;
-    const int64_t nt = tc->ntiles, most = most_exits(core->rows, core->cols);
+    const int64_t nt = tc->ntiles, most = plan.exits;
     const dim3 grid((unsigned)g.tcols, (unsigned)g.trows);
     const unsigned exit_ctas = blocks_for(std::max<int64_t>(most, 1), 256);
     tc->bytes = (int64_t)plan.bytes;

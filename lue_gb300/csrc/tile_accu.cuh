@@ -119,6 +119,7 @@ struct TileScratch {
 
 // Offsets of a TileCore and of a TileScratch in their arenas.
 struct TileCorePlan {
+    int64_t exits;  // the arrays have room for
     size_t exit_base, slot_base, cell_at, prev_at, exit_span, exit_pos, slot_at, slot_first, slot_edge, bytes;
 };
 struct TileScratchPlan {
@@ -129,7 +130,10 @@ struct TopologyCore;
 
 // Whether a grid holds the tile rows.
 inline bool tile_rows_fit(int64_t rows) { return (rows + kTile - 1) / kTile <= 65535; }
-int tile_core_plan(int64_t rows, int64_t cols, Arena& core, TileCorePlan* p, Arena& scratch, TileScratchPlan* sp);
+// The most exits that the raster has.
+int tile_exit_bound(const uint8_t* fd, int64_t rows, int64_t cols, cudaStream_t stream, int64_t* exits);
+int tile_core_plan(int64_t rows, int64_t cols, int64_t exits, Arena& core, TileCorePlan* p, Arena& scratch,
+                   TileScratchPlan* sp);
 int tile_core_build(TopologyCore* core, const Arena& arena, const TileCorePlan& plan, const Arena& scratch,
                     const TileScratchPlan& scratch_plan, cudaStream_t stream, unsigned long long* hstats);
 void tile_scratch_plan(int64_t ntiles, int64_t nexit, Arena& a, TileScratchPlan* p);

@@ -239,7 +239,11 @@ static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bo
     core->bytes = (int64_t)base;
     plan_scratch(n, s, &scratch);
     *done = false;
-    if (tiles && tile_core_plan(core->rows, core->cols, a, &tile_plan, s, &scratch.tiles)) return LUE_GPU_OK;
+    if (tiles) {
+        int64_t exits = 0;
+        if ((rc = tile_exit_bound(flow_direction, core->rows, core->cols, stream, &exits))) return rc;
+        if (tile_core_plan(core->rows, core->cols, exits, a, &tile_plan, s, &scratch.tiles)) return LUE_GPU_OK;
+    }
     if ((rc = cuda_status(a.allocate(), "topology"))) return rc;
     if ((rc = cuda_status(s.allocate(), "scratch"))) return rc;
     core->fd = a.at<uint8_t>(fd);
