@@ -25,6 +25,7 @@ __device__ __forceinline__ void upstream_window(const uint8_t* __restrict__ fd, 
                                                 const T* __restrict__ m, T* __restrict__ out)
 {
     const WindowAt<EDGE> w(rows, cols);
+    if (w.idle()) return;
     unsigned f[kWindowRows + 2];
     T v[kWindowRows + 2];
     w.load(f, fd, (unsigned)kNoData);
@@ -32,6 +33,7 @@ __device__ __forceinline__ void upstream_window(const uint8_t* __restrict__ fd, 
     T sum[kWindowRows + 2];
 #pragma unroll
     for (int j = 0; j < kWindowRows + 2; ++j) {
+        if (sizeof(T) == 8 && j >= 2 && w.below(j - 2)) break;
         const unsigned west = __shfl_up_sync(0xffffffffu, f[j], 1), east = __shfl_down_sync(0xffffffffu, f[j], 1);
         const T vw = __shfl_up_sync(0xffffffffu, v[j], 1), ve = __shfl_down_sync(0xffffffffu, v[j], 1);
         if (j + 1 <= kWindowRows) {
@@ -73,6 +75,7 @@ __device__ __forceinline__ void downstream_window(const uint8_t* __restrict__ fd
                                                   const T* __restrict__ m, T* __restrict__ out)
 {
     const WindowAt<EDGE> w(rows, cols);
+    if (w.idle()) return;
     unsigned f[kWindowRows + 2];
     T v[kWindowRows + 2];
     w.load(f, fd, (unsigned)kNoData);  // the first and the last row are not used: no loads of them
@@ -80,6 +83,7 @@ __device__ __forceinline__ void downstream_window(const uint8_t* __restrict__ fd
     const int west = (int)(threadIdx.x & 31) - 1;
 #pragma unroll
     for (int j = 1; j <= kWindowRows; ++j) {
+        if (w.below(j - 1)) break;
         unsigned k = f[j] - 1u;
         if (k > 8u) k = 4u;  // no-data, or a code that is not a direction: a sink
         const unsigned north = (k * 11u) >> 5;  // k / 3: 0 the row below, 1 the cell's, 2 the row above
@@ -124,11 +128,12 @@ static int one_hop(bool up, const uint8_t* fd, int64_t rows, int64_t cols, const
     if (!fd || !m || !out) return fail(LUE_GPU_EINVAL, std::string(what) + ": NULL argument");
     if (rows <= 0 || cols <= 0) return fail(LUE_GPU_EINVAL, std::string(what) + ": non-positive extent");
     dim3 grid;
-    if (!window_grid(rows, cols, grid)) return fail(LUE_GPU_ERANGE, std::string(what) + ": more than 524280 rows");
+    unsigned threads = 0;
+    if (!window_grid(rows, cols, grid, threads)) return fail(LUE_GPU_ERANGE, std::string(what) + ": more than 524280 rows");
     if (up)
-        k_upstream<T><<<grid, kWindowThreads, 0, (cudaStream_t)stream>>>(fd, rows, cols, m, out);
+        k_upstream<T><<<grid, threads, 0, (cudaStream_t)stream>>>(fd, rows, cols, m, out);
     else
-        k_downstream<T><<<grid, kWindowThreads, 0, (cudaStream_t)stream>>>(fd, rows, cols, m, out);
+        k_downstream<T><<<grid, threads, 0, (cudaStream_t)stream>>>(fd, rows, cols, m, out);
     count_launches(1);
     return cuda_status(cudaGetLastError(), what);
 }

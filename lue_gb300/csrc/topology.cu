@@ -48,6 +48,7 @@ __device__ __forceinline__ void count_window(const uint8_t* __restrict__ fd, int
                                              uint8_t* __restrict__ count, uint8_t* __restrict__ upmask)
 {
     const WindowAt<EDGE> w(rows, cols);
+    if (w.idle()) return;
     unsigned f[kWindowRows + 2], mask[kWindowRows + 2];
     w.load(f, fd, (unsigned)kNoData);
 #pragma unroll
@@ -114,8 +115,9 @@ static void launch_count(const uint8_t* fd, int64_t rows, int64_t cols, int valu
                          cudaStream_t stream)
 {
     dim3 grid;
-    if (window_grid(rows, cols, grid))
-        k_count_window<<<grid, kWindowThreads, 0, stream>>>(fd, rows, cols, value_policies, count, upmask);
+    unsigned threads = 0;
+    if (window_grid(rows, cols, grid, threads))
+        k_count_window<<<grid, threads, 0, stream>>>(fd, rows, cols, value_policies, count, upmask);
     else
         k_count_upmask<<<grid_for(rows * cols, 256), 256, 0, stream>>>(fd, rows, cols, value_policies, count, upmask);
 }
