@@ -105,6 +105,13 @@ __device__ __forceinline__ T load_cg(const T* p)
     return __ldcg(p);
 }
 
+// On the integer pipes: a warp's float64 operation, comparisons included, takes the float64 pipe of a GB300 SM 16 cycles.
+__device__ __forceinline__ bool is_nan_bits(double x)
+{
+    const unsigned lo = (unsigned)__double2loint(x);
+    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | ((lo | (0u - lo)) >> 31)) > 0x7ff00000u;
+}
+
 __device__ __forceinline__ int64_t grid_stride_begin() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int64_t grid_stride() { return (int64_t)gridDim.x * blockDim.x; }
 

@@ -183,12 +183,7 @@ struct RouteF32 {
 
 // --- float64: plain double arithmetic, like the reference's double instantiation ---------------------
 
-// Comparisons on the integer pipes: the float64 pipe is slow on GB300.
-__device__ __forceinline__ bool is_nan_bits(double x)
-{
-    const unsigned lo = (unsigned)__double2loint(x);
-    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | ((lo | (0u - lo)) >> 31)) > 0x7ff00000u;
-}
+// As is_nan_bits (common.cuh).
 __device__ __forceinline__ bool is_non_negative(double x)  // x >= 0: false for NaN, true for -0
 {
     const long long b = __double_as_longlong(x);
