@@ -1386,14 +1386,15 @@ __device__ __forceinline__ void write_slot(unsigned long long* p, Up u)
 // the walk engine, so the results are that engine's bit for bit.  Persistent warps empty the slots, then take chunks
 // of positions in ticket order, each the paths whose tops lie in it.  A warp's lanes load what 32 positions need besides
 // the flow along their path, and the next 32 positions' inputs while the warp takes these steps one after the other,
-// every lane all of them.  It waits for the slots that its positions take: their paths are of lower levels, so lie at
+// every lane all of them, or path by path where these are short.  It waits for the slots that its positions take: their paths are of lower levels, so lie at
 // lower positions, in chunks of earlier tickets, held by warps that run.  Waits are bounded, by far more than the paths before
 // can take; when one gives up, the last warp readies the counters of the walk over cells and sets walk[1].
 //
 // Bound by the chain of steps along the longest paths (55 to 120 ns a step), on large rasters also by issue (0.06 to 0.08
-// ns a cell).  With one infinite cell, 1500^2 / 4096^2 / 8192^2: accu (float64) 1.1 / 3.7 / 11.2 ms a call, accu_trigger 1.0 /
-// 3.1 / 9.3 ms; by the walk over cells (a dependent counter and its fences per step) 7.8 / 31 / 102 and 9.0 / 38 / 126 ms.
-constexpr int kRedoThreads = 256, kRedoChunk = 256, kRedoFill = 8192;
+// ns a cell).  With one infinite cell, 1500^2 / 3000^2 / 8192^2: accu (float64) 0.89 / 2.1 / 8.9 ms a call, accu_trigger 0.79 /
+// 1.9 / 7.7 ms; by the walk over cells (a dependent counter and its fences per step) 5.5 / 19 / 130 and 6.3 / 26 / 124 ms.
+// Path by path up to 12 cells: 1 x 2000000 of short paths 247 -> 111 us (accu float64), 500000 x 8 685 -> 520.
+constexpr int kRedoThreads = 256, kRedoChunk = 256, kRedoFill = 8192, kRedoShort = 12;
 struct PathRedo {
     const int32_t* order;
     const int32_t* path_slot;
@@ -1477,11 +1478,15 @@ __device__ __forceinline__ bool redo_chunk(const PathRedo& q, Visitor& v, int64_
         RedoCell<Visitor> ahead;
         ahead.load(q, v, i + 32, w1);
         const int32_t w2 = i + 64 < p1 ? __ldg(q.order + i + 64) : -1;
+        // (branches for the whole warp where a sum is rare: float64 additions that no lane needs take their time too)
         typename Visitor::Total s;
         Up then{};
+        const int most = __reduce_max_sync(kAll, n);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            if (j < n && j < before) Visitor::add(s, u[j]);
+            if (j >= most) break;
+            if (__any_sync(kAll, j < n && j < before))
+                if (j < n && j < before) Visitor::add(s, u[j]);
             if (j < n && j == before) then = u[j];
         }
         const unsigned after = (unsigned)max(0, n - before);
@@ -1489,7 +1494,31 @@ __device__ __forceinline__ bool redo_chunk(const PathRedo& q, Visitor& v, int64_
         Up mine{};
         T rest = T(0);
         const unsigned tops = __ballot_sync(kAll, w < 0);
-        if (__all_sync(kAll, n == 0)) {  // nothing but the flow along paths
+        // how far a lane is from the first one of its path in the window
+        const int offset = lane - (31 - __clz((tops | 1u) & (0xffffffffu >> (31 - lane))));
+        const int longest = __reduce_max_sync(kAll, on ? offset : 0) + 1;
+        if (longest <= kRedoShort) {  // short paths side by side
+            for (int j = 0; j < longest; ++j) {
+                Up in = from_lane(mine, lane ? lane - 1 : 0);
+                if (lane == 0) in = flow;
+                const bool turn = on && offset == j;
+                typename Visitor::Total t = s;
+                if (along && before == 0) t = Visitor::total(in);
+                if (__any_sync(kAll, turn && along && before > 0))
+                    if (along && before > 0) Visitor::add(t, in);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (k >= most) break;
+                    if (__any_sync(kAll, turn && k >= before && k < n))
+                        if (k >= before && k < n) Visitor::add(t, u[k]);
+                }
+                T r;
+                const Up o = Visitor::apply(t, cell.x, cell.y, r);
+                mine = turn ? o : mine;
+                rest = turn ? r : rest;
+            }
+            flow = from_lane(mine, max(steps - 1, 0));
+        } else if (__all_sync(kAll, n == 0)) {  // nothing but the flow along paths
             T x = __shfl_sync(kAll, cell.x, 0), y = __shfl_sync(kAll, cell.y, 0);
             for (int j = 0; j < steps; ++j) {
                 const T x1 = __shfl_sync(kAll, cell.x, (j + 1) & 31), y1 = __shfl_sync(kAll, cell.y, (j + 1) & 31);
