@@ -112,6 +112,23 @@ __device__ __forceinline__ bool is_nan_bits(double x)
     return (((unsigned)__double2hiint(x) & 0x7fffffffu) | ((lo | (0u - lo)) >> 31)) > 0x7ff00000u;
 }
 
+// Words by which CTAs wait for one another.
+__device__ __forceinline__ int ld_acquire(const int* p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
+{
+    return (unsigned)ld_acquire(reinterpret_cast<const int*>(p));
+}
+__device__ __forceinline__ void st_release(int* p, int v)
+{
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_release(unsigned* p, unsigned v) { st_release(reinterpret_cast<int*>(p), (int)v); }
+
 __device__ __forceinline__ int64_t grid_stride_begin() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int64_t grid_stride() { return (int64_t)gridDim.x * blockDim.x; }
 

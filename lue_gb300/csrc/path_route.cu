@@ -75,11 +75,6 @@ __device__ __forceinline__ int inflow_slot(uint8_t code)
     }
 }
 
-__global__ void k_fill(int32_t* p, int64_t n, int32_t v)
-{
-    for (int64_t i = grid_stride_begin(); i < n; i += grid_stride()) p[i] = v;
-}
-
 // next[c]: the cell below c on its path (c itself at the bottom), -1 for no-data.
 __global__ void k_path_next(const uint8_t* fd, const int32_t* heavy, int64_t rows, int64_t cols, int64_t n,
                             int32_t* next)
@@ -538,7 +533,7 @@ int path_core_build(const TopologyCore* core, uint32_t* work, cudaStream_t strea
     TRY(cudaMalloc(&cells, sizeof hcells));
     TRY(cudaMalloc(&pc->order, path_padded(npos) * sizeof(int32_t)));
     // 1. sizes, heavy neighbours, cells above on the path, path levels
-    k_fill<<<grid_for(n, 256), 256, 0, stream>>>(heavy, n, 8);
+    k_fill_i32<<<grid_for(n, 256), 256, 0, stream>>>(heavy, n, 8);
     TRY(cudaMemcpyAsync(work, core->count, words_for(n) * 4, cudaMemcpyDeviceToDevice, stream));
     {
         WalkGrid wg{core->fd, core->count, work, rows, cols, n};
@@ -711,8 +706,7 @@ template <int K>
 __device__ __forceinline__ PMap<K> pm_identity()
 {
     if constexpr (K == kSum) return PMap<K>{0.0, 0};
-    else
-    if constexpr (K == kAffine) return PMap<K>{1.0f, 0.0f, 0.0f, 0.0f, 0};
+    else if constexpr (K == kAffine) return PMap<K>{1.0f, 0.0f, 0.0f, 0.0f, 0};
     else if constexpr (K == kTrigger) return PMap<K>{-INFINITY, 0.0f, 0.0f, 0.0f, 0, 0.0f, 0.0f};
     else return PMap<K>{0.0f, 0.0f, K == kMinPlus ? INFINITY : -INFINITY, 0.0f, 0};
 }
@@ -920,20 +914,18 @@ __device__ __forceinline__ PMap<K> pm_each(const PMap<K>& m, F f)
     PMap<K> r;
     if constexpr (K == kSum) {
         r.b = f(m.b);
-        r.flags = f(m.flags);
-        return r;
     } else {
-    r.ah = f(m.ah);
-    r.al = f(m.al);
-    r.bh = f(m.bh);
-    r.bl = f(m.bl);
+        r.ah = f(m.ah);
+        r.al = f(m.al);
+        r.bh = f(m.bh);
+        r.bl = f(m.bl);
+    }
     r.flags = f(m.flags);
     if constexpr (K == kTrigger) {
         r.ch = f(m.ch);
         r.cl = f(m.cl);
     }
     return r;
-    }
 }
 template <int K>
 __device__ __forceinline__ PMap<K> shfl_up(const PMap<K>& m, int d)
@@ -1019,17 +1011,6 @@ __device__ __forceinline__ void load_order(const P& p, int64_t first, int32_t (&
     }
 }
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_gpu(int* p, int v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Look-back of one level's launch: CTAs take tiles in ticket order.  A tile publishes the composition of its own maps:
 // state 3 when that is a constant (a path's top is among its positions, so nothing before the tile matters), else
 // state 1, and then, if its number is a multiple of 32, also the composition of everything up to and including it
@@ -1063,7 +1044,7 @@ __device__ PMap<K> look_back(const PathScan<K>& q, int tile, unsigned long long*
     int state = 0, stop = -1;
     for (int k = 0; k < q.polls; ++k) {
         if (idx >= 0 && state < (fence ? 2 : 1)) {
-            const int v = ld_acquire_gpu(q.status + idx);
+            const int v = ld_acquire(q.status + idx);
             state = (v >> 2) == q.epoch ? v & 3 : 0;
         }
         const bool ready = state >= (fence ? 2 : 1);
@@ -1241,14 +1222,14 @@ __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, P
         if (threadIdx.x == 0) {
             q.aggm[tile] = total;
             __threadfence();
-            st_release_gpu(q.status + tile, (q.epoch << 2) | (constant ? 3 : 1));
+            st_release(q.status + tile, (q.epoch << 2) | (constant ? 3 : 1));
         }
         const PMap<K> before = tile ? look_back<K>(q, tile, p.flag) : pm_identity<K>();
         if (threadIdx.x == 0) {
             if (!constant && (tile & 31) == 0) {
                 q.inclm[tile] = compose<K>(before, total);
                 __threadfence();
-                st_release_gpu(q.status + tile, (q.epoch << 2) | 2);
+                st_release(q.status + tile, (q.epoch << 2) | 2);
             }
             s_prefix = before;
         }
@@ -1386,9 +1367,10 @@ __device__ __forceinline__ void write_slot(unsigned long long* p, Up u)
 // the walk engine, so the results are that engine's bit for bit.  Persistent warps empty the slots, then take chunks
 // of positions in ticket order, each the paths whose tops lie in it.  A warp's lanes load what 32 positions need besides
 // the flow along their path, and the next 32 positions' inputs while the warp takes these steps one after the other,
-// every lane all of them, or path by path where these are short.  It waits for the slots that its positions take: their paths are of lower levels, so lie at
-// lower positions, in chunks of earlier tickets, held by warps that run.  Waits are bounded, by far more than the paths before
-// can take; when one gives up, the last warp readies the counters of the walk over cells and sets walk[1].
+// every lane all of them, or path by path where these are short.  It waits for the slots that its positions take: their
+// paths are of lower levels, so lie at lower positions, in chunks of earlier tickets, held by warps that run.  Waits are
+// bounded, by far more than the paths before can take; when one gives up, the last warp readies the counters of the walk over
+// cells and sets walk[1].
 //
 // Bound by the chain of steps along the longest paths (55 to 120 ns a step), on large rasters also by issue (0.06 to 0.08
 // ns a cell).  With one infinite cell, 1500^2 / 3000^2 / 8192^2: accu (float64) 0.89 / 2.1 / 8.9 ms a call, accu_trigger 0.79 /
@@ -1600,7 +1582,7 @@ __global__ void __launch_bounds__(kRedoThreads) k_path_redo(PathRedo q, Visitor 
             continue;
         }
         for (long long j = 0; !all_filled; ++j) {
-            all_filled = __all_sync(kAll, ld_acquire_gpu(reinterpret_cast<const int*>(filled)) >= fills);
+            all_filled = __all_sync(kAll, ld_acquire(filled) >= fills);
             if (j >= q.polls) break;
         }
         const int64_t at = (k - fills) * kRedoChunk;
@@ -1766,8 +1748,8 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, 
         k_path_no_data<<<grid_for(n, 256), 256, 0, stream>>>(core->fd, n, out, rem);
         ++launches;
     }
-    const PathCall<N> p{pc->order, pc->path_slot, pc->slot_first - pc->slot_base, a, as, b, bs, out, rem, static_cast<typename N::Slot*>(t->path_slots),
-                        dense, flag};
+    const PathCall<N> p{pc->order, pc->path_slot, pc->slot_first - pc->slot_base, a, as, b, bs, out, rem,
+                        static_cast<typename N::Slot*>(t->path_slots), dense, flag};
     // test hooks: LUE_GB300_PATH_FREE_LONGEST (levels with longer paths use the look-back scan; 0: every
     // level) and LUE_GB300_PATH_POLLS (poll limit of a look-back wait; 0: every wait gives up at once,
     // and the walk engine redoes the call)
@@ -1812,7 +1794,8 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, 
     const PathRedo r{pc->order, pc->path_slot, p.slot_first, static_cast<unsigned long long*>(t->path_slots), pc->npos,
                      pc->slot_base, pc->nslots, flag, flag + 2, reinterpret_cast<unsigned*>(redo_ctl), redo_polls,
                      reinterpret_cast<const uint32_t*>(core->count), t->work_count, words_for(n)};
-    launch_after(k_path_redo<Visitor>, grid_for(pc->npos, kRedoChunk * (kRedoThreads / 32), 152 * 4), kRedoThreads, 0, stream, r, redo);
+    launch_after(k_path_redo<Visitor>, grid_for(pc->npos, kRedoChunk * (kRedoThreads / 32), 152 * 4), kRedoThreads, 0, stream,
+                 r, redo);
     WalkGrid g{core->fd, core->count, t->work_count, core->rows, core->cols, n};
     launch_after(k_walk_if<Visitor>, grid_for(n, 256), 256, 0, stream, g, redo, (const unsigned long long*)(flag + 2));
     count_launches(launches + 2);
@@ -1820,8 +1803,8 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, 
 }
 
 template <Rule R, int K>
-static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, const float* a, float as, const float* b, float bs,
-                        float* out, float* rem, cudaStream_t stream, const char* what)
+static int path_run_f32(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, const float* a, float as,
+                        const float* b, float bs, float* out, float* rem, cudaStream_t stream, const char* what)
 {
     const RouteF32<R> redo{t->core->upmask, a, as, b, bs, out, rem, t->lo, t->core->cols};
     return path_run<F32, R, K>(t, pc, at, a, as, b, bs, out, rem, redo, stream, what);
@@ -1852,7 +1835,8 @@ int path_route_f32(lue_gpu_topology* t, int rule, const float* a, float as, cons
     *done = false;
     if (path_engine_off()) return LUE_GPU_OK;
     if (rule < (int)Rule::threshold || rule > (int)Rule::trigger) return LUE_GPU_OK;
-    if (rule == (int)Rule::trigger && (overlap(t, a, out, 4) || overlap(t, a, rem, 4) || overlap(t, b, out, 4) || overlap(t, b, rem, 4)))
+    if (rule == (int)Rule::trigger &&
+        (overlap(t, a, out, 4) || overlap(t, a, rem, 4) || overlap(t, b, out, 4) || overlap(t, b, rem, 4)))
         return LUE_GPU_OK;
     const PathCore* pc = nullptr;
     const int32_t* at = nullptr;

@@ -124,7 +124,8 @@ extern "C" int lue_gpu_accu_f32(lue_gpu_topology* t, const float* inflow, float 
 }
 
 // The rules that are not plain sums, and float64 accu, run on the path engine (path_route.cuh) or the stage engine
-// (stage_route.cuh) when the topology has no flow cycles, else on the walk engine.  LUE_GB300_ENGINE=walk forces the walk engine.
+// (stage_route.cuh) when the topology has no flow cycles, else on the walk engine.  LUE_GB300_ENGINE=walk forces the walk
+// engine.
 #define STAGE_OR_WALK(call)                          \
     do {                                             \
         bool done = false;                           \

@@ -806,17 +806,6 @@ __device__ __forceinline__ unsigned long long global_ns()
     return v;
 }
 
-__device__ __forceinline__ int ld_acquire(const int* p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Waits until *p >= need and returns *p; gives up (returns `need`: the caller's results are then not
 // valid) after `polls` polls, setting *error, or once another wait has given up.
 __device__ __forceinline__ int flow_wait(const int* p, int need, int* error, int polls)

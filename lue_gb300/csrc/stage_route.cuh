@@ -2,7 +2,8 @@
 //
 // The float64 rules and kinematic_wave compute each cell from the sum of its upstream
 // outflows with a rule that does not distribute over sums, so they cannot use the prefix sums of the
-// tile engine (the float32 rules run as scans along flow paths: path_route.cuh).  The reference walks them cell by cell, partition by partition, with channel hand-off at
+// tile engine (the float32 rules run as scans along flow paths: path_route.cuh).  The reference walks them cell by cell,
+// partition by partition, with channel hand-off at
 // partition edges (ALG/definition/accumulating_router.hpp:525-599, 902-1209).  Here:
 //
 //   - The raster is cut into 32 x 32 tiles.  The crossing depth of a cell is the largest number of tile

@@ -629,7 +629,8 @@ __global__ void __launch_bounds__(kTileThreads)
         __syncthreads();
         for (int i = t; i < kTileCells; i += kTileThreads) {
             const int64_t row = tr * kTile + (i >> 6), col = tc * kTile + (i & 63);
-            if (row < g.rows && col < g.cols) level[row * g.cols + col] = (ready[i >> 5] >> (i & 31)) & 1u ? (int32_t)st[2 * i] : -1;
+            if (row < g.rows && col < g.cols)
+                level[row * g.cols + col] = (ready[i >> 5] >> (i & 31)) & 1u ? (int32_t)st[2 * i] : -1;
         }
         for (int e = t; e < ne; e += kTileThreads) exit_level[e0 + e] = st[2 * exit_local[e0 + e]];
         if (t == 0) atomicExch(cyclic, 1);
@@ -940,17 +941,6 @@ __device__ __forceinline__ u128 block_exclusive_u128(u128 v, u128* warp_tot, u12
     return before + x - v;
 }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // The exit forest's 128-bit inclusive scan, one chunk of consecutive scan blocks (256 x ITEMS exits each)
 // per CTA, with as many CTAs as fit on the GPU at once.  CTAs take chunks in ticket order; each sums its
 // chunk, publishes the sum (flag 1), then warp 0 adds up the sums of the chunks before it, 32 at a time,
@@ -996,14 +986,14 @@ __global__ void __launch_bounds__(kTileThreads)
         if (g == 0) {
             if (lane == 0) {
                 look_incl[0] = from_u128(bt);
-                st_release_u32(flag, 2u);
+                st_release(flag, 2u);
                 prefix_sh = 0;
                 abort_sh = 0;
             }
         } else {
             if (lane == 0) {
                 look_aggr[g] = from_u128(bt);
-                st_release_u32(flag + g, 1u);
+                st_release(flag + g, 1u);
             }
             u128 prefix = 0;
             bool failed = false;
@@ -1014,7 +1004,7 @@ __global__ void __launch_bounds__(kTileThreads)
                 if (j >= 0) {
                     int k = 0;
                     for (; k < polls; ++k) {
-                        f = ld_acquire_u32(flag + j);
+                        f = ld_acquire(flag + j);
                         if (f != 0u) break;
                         if (*reinterpret_cast<volatile unsigned long long*>(total + 1)) k = polls - 1;
                         __nanosleep(64);
@@ -1037,7 +1027,7 @@ __global__ void __launch_bounds__(kTileThreads)
                     total[1] = 2ull;
                 } else {
                     look_incl[g] = from_u128(prefix + bt);
-                    st_release_u32(flag + g, 2u);
+                    st_release(flag + g, 2u);
                 }
                 prefix_sh = prefix;
                 abort_sh = failed ? 1 : 0;
@@ -1844,7 +1834,8 @@ int tile_exit_bound(const uint8_t* fd, int64_t rows, int64_t cols, cudaStream_t 
     if (int rc = cuda_status(cudaMemsetAsync(a.at<char>(at), 0, sizeof h, stream), "exit count")) return rc;
     k_exit_count<<<blocks_for(g.trows * g.tcols, 8), 256, 0, stream>>>(fd, g, a.at<unsigned long long>(at));
     if (int rc = cuda_status(cudaGetLastError(), "exit count")) return rc;
-    if (int rc = cuda_status(cudaMemcpyAsync(&h, a.at<char>(at), sizeof h, cudaMemcpyDeviceToHost, stream), "exit count")) return rc;
+    if (int rc = cuda_status(cudaMemcpyAsync(&h, a.at<char>(at), sizeof h, cudaMemcpyDeviceToHost, stream), "exit count"))
+        return rc;
     if (int rc = cuda_status(cudaStreamSynchronize(stream), "exit count")) return rc;
     *exits = (int64_t)h;
     return LUE_GPU_OK;

@@ -269,7 +269,8 @@ static int build_topology(lue_gpu_topology* t, const uint8_t* flow_direction, bo
             a0.add((int64_t)base);
             plan_scratch(n, s0, &plain);
             if (!cuda_status(a0.allocate(), "topology") && !cuda_status(s0.allocate(), "scratch")) {
-                if ((rc = cuda_status(cudaMemcpyAsync(a0.at<char>(0), a.at<char>(0), base, cudaMemcpyDeviceToDevice, stream), "topology")) ||
+                if ((rc = cuda_status(cudaMemcpyAsync(a0.at<char>(0), a.at<char>(0), base, cudaMemcpyDeviceToDevice, stream),
+                                      "topology")) ||
                     (rc = cuda_status(cudaStreamSynchronize(stream), "topology")))
                     return rc;
                 core->bytes = (int64_t)base;

@@ -53,7 +53,8 @@ struct lue_gpu_topology {
     int* stage_flow_error = nullptr; // pinned: the error flag of the last dataflow launch, read by the next call
     int stage_threads = 0;           // stage engine: threads per stage CTA (0: LUE_GB300_STAGE_THREADS or by size)
     int publish_every = 0;           // stage engine: steps per progress publication (0: LUE_GB300_PUBLISH_EVERY or 4)
-    void* path_maps = nullptr;       // path engine (with path_ctl and path_slots one allocation): per tile of a level's scan its own and its inclusive map
+    // path engine, one allocation with path_ctl and path_slots: per tile of a level's scan its own and its inclusive map
+    void* path_maps = nullptr;
     void* path_ctl = nullptr;        // path engine: the redo flag, tickets and status words (path_route.cu)
     void* path_slots = nullptr;      // path engine: per light edge what flows over it, 8 bytes
     void* path_dense = nullptr;      // path engine, large rasters, rules with two results: these by position, 8 bytes

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(256) k_walk_if(WalkGrid g, Visitor v, const un
     }
 }
 
+__global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v);
 __global__ void k_copy_words_if(const uint32_t* src, uint32_t* dst, int64_t nwords, const unsigned long long* flag);
 
 }  // namespace lue_gb300
