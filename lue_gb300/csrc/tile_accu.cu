@@ -1142,13 +1142,18 @@ __global__ void __launch_bounds__(kTileThreads)
     const int64_t row0 = tr * kTile + (t >> 6), col = tc * kTile + (t & 63), cell0 = row0 * g.cols + col, step = kStep * g.cols;
     const int rows = col < g.cols ? (int)min((int64_t)kTile, max((int64_t)0, g.rows - row0)) : 0;  // this thread's, by kStep
     if (t < 6) tally[t] = 0;
+    unsigned c[kCells];
+    int l[kCells];
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) {  // all loads before the first use
+        const bool in = k * kStep < rows;
+        c[k] = in ? fd[cell0 + k * step] : kNoData;
+        l[k] = in ? level[cell0 + k * step] : -1;
+    }
 #pragma unroll
     for (int k = 0; k < kCells; ++k) {
-        const bool in = k * kStep < rows;
-        const unsigned c = in ? fd[cell0 + k * step] : kNoData;
-        const int l = in ? level[cell0 + k * step] : -1;
-        code[t + k * kTileThreads] = (uint8_t)c;
-        lv[t + k * kTileThreads] = c != kNoData && l < 0 ? kOnCycle : l;
+        code[t + k * kTileThreads] = (uint8_t)c[k];
+        lv[t + k * kTileThreads] = c[k] != kNoData && l[k] < 0 ? kOnCycle : l[k];
     }
     __syncthreads();
     const unsigned from = t < kBorderCells ? border_in[tile * kBorderCells + t] : 0u;
