@@ -1244,10 +1244,10 @@ __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, P
 // chunk's order is read before this chunk's scan, and its inputs before this chunk's rules, so that the two
 // dependent loads overlap the arithmetic.
 //
-// Bound by instruction issue (50 % of the slots) and by the requests of its scattered stores about equally: 270
-// thread instructions per position on level 0 at 8192^2, 0.71 ms; with branches in the compositions, a second
-// composition per cell in store() and 64-bit positions it was 486 and 1.0 ms.  accu_threshold at 16384^2: 8.4 -> 6.6
-// ms.  Tried and slower: one thread per short path (up to 16, 64 or 256 cells) with the cell rule itself, sorted by
+// Bound by instruction issue (54 % of the slots) and the waits for its loads: 230 thread instructions per position on level 0
+// at 8192^2, 0.56 ms with its results by position (0.71 ms straight to the raster, bound by the requests of the scattered
+// stores as well); with branches in the compositions, a second composition per cell in store() and 64-bit positions it was
+// 486 and 1.0 ms.  accu_threshold at 16384^2: 8.4 -> 6.6 ms with these steps, 4.9 with the ones since.  Tried and slower: one thread per short path (up to 16, 64 or 256 cells) with the cell rule itself, sorted by
 // length within a tile: 50 instructions per cell, but every lane of a store is a request of its own (8.3-10 ms at
 // 16384^2, with the results of a tile collected in shared memory as well); CTAs of 128 threads (6.9 ms).
 template <class N, Rule R, int K, int PER, bool LIGHT>

@@ -1323,9 +1323,10 @@ struct StageKW32 {
 };
 
 // kinematic wave, many steps, in float-float and the variable y = Q^(1/m) (kinematic_wave_ff.cuh).  Bound by
-// instruction issue and the latency of dependent instructions (53 % of the issue slots; more warps per SM make no
+// instruction issue and the latency of dependent instructions (59 % of the issue slots; more warps per SM make no
 // difference, since the stages that could fill them wait for producers).  With the nested solve for beta = 3/5 and
-// the listed upstream values, 100 steps at 8192^2 take 89 ms (before: 130 ms), one step at 2048^2 2.5 ms (5.2 ms).
+// the listed upstream values, 100 steps at 8192^2 take 91 ms (before: 130 ms), one step at 2048^2 1.8 to 2.1 ms (3.6 to
+// 5.1 ms).
 template <int P, int M>
 struct StageKWPoly {
     const double* qcur;
