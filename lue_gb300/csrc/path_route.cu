@@ -1011,22 +1011,24 @@ __device__ __forceinline__ void load_order(const P& p, int64_t first, int32_t (&
     }
 }
 
-// Look-back of one level's launch: CTAs take tiles in ticket order.  A tile publishes the composition of its own maps:
-// state 3 when that is a constant (a path's top is among its positions, so nothing before the tile matters), else
-// state 1, and then, if its number is a multiple of 32, also the composition of everything up to and including it
-// (state 2).  Status words carry the launch's epoch, so the arrays need no clearing between launches.
+// Look-back of one level's launch: CTAs take tiles in ticket order.  Each tile publishes the composition of its own maps: a
+// constant when a path's top is among its positions, so that nothing before the tile matters.  Tiles whose number is a
+// multiple of 32 (fences) also publish the composition of the 32 tiles up to and including themselves (their group), or,
+// at multiples of 1024, that of everything up to and including themselves (a prefix).  Status words carry the launch's
+// epoch, so the arrays need no clearing between launches.
 //
-// A tile composes the tiles before it from the nearest constant one, or from the nearest published prefix (it is at most
-// 32 tiles away) if that comes first.  Which ones these are depends on the layout alone, not on which CTA is how far: the
-// same call gives the same bits every time, in plain doubles too.  The only chain of waits is that of the prefixes,
-// one every 32 tiles along a river.  Composing whatever tiles have published so far (every tile its prefix) takes longer as
-// well, since every tile publishes twice: accu (float64) over a basin of 3001 x 2777 264 us a call, this 246;
-// accu_trigger at 1500^2 138 and 121.
+// A tile composes the tiles before it back to the nearest constant one, or to the fence before it, and from there the groups
+// back to the nearest constant one or to a prefix.  Which ones these are depends on the layout alone, not on which CTA is how
+// far: the same call gives the same bits every time, in plain doubles too.  The only chain of waits is that of the
+// prefixes, one every 1024 tiles along a river.  accu (float64) over a basin of 3001 x 2777 takes 203 us, accu_trigger at
+// 1500^2 124, accu over one path through 4000^2 cells 479; composing whatever tiles have published so far (every tile
+// its prefix, so twice as many publications) 216, 136 and 538; prefixes every 32 tiles without groups 1171 on the last.
+enum PathState { kOwn = 1, kGroup = 2, kConstant = 3, kConstantGroup = 4, kPrefix = 5 };
 template <int K>
 struct PathScan {
-    int* status;  // [tiles] epoch << 2 | state
+    int* status;  // [tiles] epoch << 3 | state
     PMap<K>* aggm;   // [tiles] the tile's own composition
-    PMap<K>* inclm;  // [tiles] the composition up to and including the tile (multiples of 32)
+    PMap<K>* inclm;  // [tiles] a fence's group or prefix
     int* ticket;  // zeroed before the launch
     int epoch;
     int polls;    // poll limit of one wait
@@ -1034,42 +1036,90 @@ struct PathScan {
 
 constexpr int kPathPolls = 1 << 20;
 
-// Warp 0: the composition of all tiles before `tile` (in every lane); lane i looks at tile `tile` - 1 - i.  The wait is
-// bounded: one that gives up (or finds that another one did) sets flag[1], after which the call is redone.
 template <int K>
-__device__ PMap<K> look_back(const PathScan<K>& q, int tile, unsigned long long* flag)
+__device__ __forceinline__ int path_state(const PathScan<K>& q, int tile)
 {
-    const int lane = threadIdx.x & 31, idx = tile - 1 - lane;
-    const bool fence = (idx & 31) == 0;
-    int state = 0, stop = -1;
-    for (int k = 0; k < q.polls; ++k) {
-        if (idx >= 0 && state < (fence ? 2 : 1)) {
-            const int v = ld_acquire(q.status + idx);
-            state = (v >> 2) == q.epoch ? v & 3 : 0;
-        }
-        const bool ready = state >= (fence ? 2 : 1);
-        const unsigned ends = __ballot_sync(0xffffffffu, ready && (fence || state == 3));
-        const unsigned missing = __ballot_sync(0xffffffffu, !ready);
-        // the nearest end counts, once every tile before it is there: farther ones may be there already
-        if (ends && !(missing & (ends ^ (ends - 1u)))) {
-            stop = __ffs(ends) - 1;
-            break;
-        }
-        if (__any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned long long*>(flag + 1) != 0)) break;
-        __nanosleep(32);
-    }
-    if (stop < 0) {
-        if (lane == 0) flag[1] = 1;
-        return pm_identity<K>();
-    }
-    PMap<K> m = pm_identity<K>();
-    if (lane <= stop) m = pm_each(*(state == 2 ? q.inclm + idx : q.aggm + idx), [](const auto& v) { return __ldcg(&v); });
-    // lanes 31 .. 0 in this order (farther tiles come first)
+    const int v = ld_acquire(q.status + tile);
+    return (v >> 3) == q.epoch ? v & 7 : 0;
+}
+template <int K>
+__device__ __forceinline__ void path_publish(const PathScan<K>& q, int tile, PMap<K>* to, const PMap<K>& m, int state)
+{
+    to[tile] = m;
+    __threadfence();
+    st_release(q.status + tile, (q.epoch << 3) | state);
+}
+
+// The lanes' maps composed, those of higher lanes (farther tiles) first, in every lane.
+template <int K>
+__device__ __forceinline__ PMap<K> compose_lanes(PMap<K> m)
+{
+    const int lane = threadIdx.x & 31;
     for (int d = 1; d < 32; d <<= 1) {
         const PMap<K> o = shfl_down(m, d);
         if (lane + d < 32) m = compose<K>(o, m);
     }
     return pm_each(m, [](auto v) { return __shfl_sync(0xffffffffu, v, 0); });
+}
+
+// Whether the lanes up to the first one of `ends` (all lanes without one) are ready; uniform.
+__device__ __forceinline__ bool lanes_ready(unsigned ends, unsigned missing) { return !(missing & (ends ^ (ends - 1u))); }
+
+// Warp 0: the composition of all tiles before `tile` (in every lane); publishes the group or prefix of a fence.  Waits are
+// bounded: one that gives up (or finds that another one did) sets flag[1], after which the call is redone.
+template <int K>
+__device__ PMap<K> look_back(const PathScan<K>& q, int tile, const PMap<K>& total, unsigned long long* flag)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, fence = (tile - 1) & ~31;
+    const int near = tile - 1 - lane, far = fence - 32 * lane;  // a lane's tile behind the fence, and its fence
+    const bool is_fence = (tile & 31) == 0 && !(total.flags & 1);
+    int own = near > fence ? 0 : -1, group = far >= 0 ? 0 : -1;
+    auto gave_up = [&] { return __any_sync(kAll, *reinterpret_cast<volatile unsigned long long*>(flag + 1) != 0) != 0; };
+    // the tiles after the fence
+    unsigned ends = 0;
+    bool ready = false;
+    for (int k = 0; k < q.polls && !ready; ++k) {
+        if (own == 0) own = path_state(q, near);
+        if (group >= 0 && group < kGroup) group = path_state(q, far);
+        ends = __ballot_sync(kAll, own == kConstant);
+        ready = lanes_ready(ends, __ballot_sync(kAll, own == 0));
+        if (!ready) {
+            if (gave_up()) break;
+            __nanosleep(32);
+        }
+    }
+    PMap<K> before = pm_identity<K>();
+    if (ready) {
+        const int stop = ends ? __ffs(ends) - 1 : 31;
+        PMap<K> m = pm_identity<K>();
+        if (own > 0 && lane <= stop) m = pm_each(q.aggm[near], [](const auto& v) { return __ldcg(&v); });
+        before = compose_lanes<K>(m);
+        if (is_fence && (ends || (tile & 1023)) && lane == 0)
+            path_publish(q, tile, q.inclm, compose<K>(before, total), ends ? kConstantGroup : kGroup);
+        if (ends) return before;
+        // the groups up to the fence
+        ready = false;
+        for (int k = 0; k < q.polls && !ready; ++k) {
+            if (group >= 0 && group < kGroup) group = path_state(q, far);
+            ends = __ballot_sync(kAll, group >= kConstant);
+            ready = ends && lanes_ready(ends, __ballot_sync(kAll, group >= 0 && group < kGroup));
+            if (!ready) {
+                if (gave_up()) break;
+                __nanosleep(32);
+            }
+        }
+    }
+    if (!ready) {
+        if (lane == 0) flag[1] = 1;
+        return pm_identity<K>();
+    }
+    PMap<K> m = pm_identity<K>();
+    if (lane <= __ffs(ends) - 1)
+        m = pm_each(*(group == kConstant ? q.aggm + far : q.inclm + far), [](const auto& v) { return __ldcg(&v); });
+    before = compose<K>(compose_lanes<K>(m), before);
+    if (is_fence && !(tile & 1023) && lane == 0) path_publish(q, tile, q.inclm, compose<K>(before, total), kPrefix);
+    return before;
 }
 
 // The positions of one thread in one chunk of a scan: PER consecutive positions from `first`, those in
@@ -1218,21 +1268,10 @@ __global__ void __launch_bounds__(kPathThreads, 4) k_path_level(PathCall<N> p, P
     PMap<K> total;
     const PMap<K> E = block_excl_scan<K, kPathThreads>(acc, s_warp, total);
     if (threadIdx.x < 32) {
-        const bool constant = tile == 0 || (total.flags & 1);  // a level begins with a top
-        if (threadIdx.x == 0) {
-            q.aggm[tile] = total;
-            __threadfence();
-            st_release(q.status + tile, (q.epoch << 2) | (constant ? 3 : 1));
-        }
-        const PMap<K> before = tile ? look_back<K>(q, tile, p.flag) : pm_identity<K>();
-        if (threadIdx.x == 0) {
-            if (!constant && (tile & 31) == 0) {
-                q.inclm[tile] = compose<K>(before, total);
-                __threadfence();
-                st_release(q.status + tile, (q.epoch << 2) | 2);
-            }
-            s_prefix = before;
-        }
+        // a level begins with a top
+        if (threadIdx.x == 0) path_publish(q, tile, q.aggm, total, tile == 0 || (total.flags & 1) ? kConstant : kOwn);
+        const PMap<K> before = tile ? look_back<K>(q, tile, total, p.flag) : pm_identity<K>();
+        if (threadIdx.x == 0) s_prefix = before;
     }
     __syncthreads();
     ch.store(p, first, v.p1, compose<K>(s_prefix, E));
@@ -1759,7 +1798,7 @@ static int path_run(lue_gpu_topology* t, const PathCore* pc, const int32_t* at, 
     PMap<K>* aggm = static_cast<PMap<K>*>(t->path_maps);
     for (size_t l = 0; l < pc->levels.size(); ++l) {
         const PathLevel& v = pc->levels[l];
-        if (++t->path_epoch >= (1 << 29)) {  // status words of old launches could match again: clear them
+        if (++t->path_epoch >= (1 << 28)) {  // status words of old launches could match again: clear them
             t->path_epoch = 1;
             if (int rc = cuda_status(cudaMemsetAsync(status, 0, nt_max * sizeof(int), stream), what)) return rc;
         }

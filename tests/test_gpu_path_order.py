@@ -58,3 +58,19 @@ def test_repeated_calls_give_the_same_bits(lfr, monkeypatch, op, longest):
     x = lfr.from_numpy(m.astype(np.float32))
     b = lfr.from_numpy(rng.random(fd.shape, dtype=np.float32) * np.float32(1.0 if op == "fraction" else 3.0))
     _repeat(lfr, lambda: getattr(lfr, f"accu_{op}")(a, x, b))
+
+
+def test_one_path_over_several_prefixes(lfr):
+    """4.2 million cells on one path: more than 4000 scan tiles, prefixes published at tiles 1024, 2048, ...; a position's sum
+    takes at most 4 + 5 + 8 + 2 x 6 + 1 + 5 additions one after the other."""
+    rows, cols = 2100, 2003
+    fd = np.full((rows, cols), 6, np.uint8)
+    fd[1::2] = 4
+    fd[0::2, -1] = 2
+    fd[1::2, 0] = 2
+    m = np.random.default_rng(3).lognormal(0.0, 1.0, fd.shape)
+    a, x = lfr.from_numpy(fd), lfr.from_numpy(m)
+    got = _repeat(lfr, lambda: [lfr.accu(a, x)])[0].cpu().numpy()
+    got[1::2], m[1::2] = got[1::2, ::-1].copy(), m[1::2, ::-1].copy()
+    want = np.cumsum(m.ravel().astype(np.longdouble)).reshape(m.shape)
+    assert np.all(np.abs(got - want) <= 64 * 2.0 ** -53 * want)
